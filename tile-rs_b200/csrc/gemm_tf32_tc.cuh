@@ -12,7 +12,7 @@
 //
 // The tensor core rounds its f32 accumulator toward zero at every instruction, so a long K accumulated in one go
 // drifts by about 2^-25.6 per instruction, all in one direction (3e-5 of the result at K = 4096).  The K loop is
-// therefore cut into chunks of kChunkKb k-blocks: each chunk is accumulated from zero in one of two tensor-memory
+// therefore cut into chunks of p.chunk_kb k-blocks: each chunk is accumulated from zero in one of two tensor-memory
 // accumulators and then added, round-to-nearest, to running sums that the eight epilogue warps keep in registers
 // (128 x 256 tile / 256 threads = 128 sums per thread) while the tensor core works on the next chunk.
 //
@@ -32,7 +32,6 @@ constexpr int kBN = 256;
 constexpr int kBK = 32;                  // 32 x f32 = one 128-byte swizzle row
 constexpr int kStages = 2;
 constexpr int kUmmaK = 8;                // 32 bytes of K per instruction
-constexpr int kChunkKb = 4;              // k-blocks per accumulation chunk: K = 128 per chunk
 constexpr int kThreads = 320;            // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
 constexpr int kAPlane = kBM * kBK * 4;   // 16 KiB
 constexpr int kBPlane = kBN * kBK * 4;   // 32 KiB
@@ -48,7 +47,11 @@ struct alignas(8) Barriers {
   uint32_t tmem_base;
   uint32_t abort_flag;
 };
-constexpr int kSmemBytes = kStages * kStageBytes + sizeof(Barriers) + 1024;
+// C is written in 32 x 32 blocks through shared memory, so that a warp's store covers whole 128-byte pieces of rows.
+constexpr int kStagingFloats = 32 * 32;                       // per epilogue warp
+constexpr int kStagingBytes = 8 * kStagingFloats * 4;
+constexpr int kSmemBytes = kStages * kStageBytes + kStagingBytes + sizeof(Barriers) + 1024;
+static_assert(kSmemBytes <= 227 * 1024, "shared memory budget of one CTA");
 
 struct Params {
   int32_t m, n, k, batch;
@@ -56,47 +59,68 @@ struct Params {
   int64_t c_batch_stride;  // elements
   int64_t ldc;             // row pitch of C in elements
   uint32_t* status;
+  int32_t vec_store;       // every row of C starts on a 16-byte boundary
+  int32_t chunk_kb;        // 32-deep k-blocks per accumulation chunk
+  // kRedo kernels: the operands as they came
+  int32_t b_transposed;
+  const float *a, *b;
+  int64_t lda, ldb, a_batch_stride, b_batch_stride;
 };
 
-// x rounded to the nearest TF32 number (10 explicit mantissa bits; ties away from zero)
+// x rounded to the nearest TF32 number (10 explicit mantissa bits; ties away from zero).  The conversion instruction, not
+// an add on the bits: that would carry a NaN of all ones into a zero.
 __device__ __forceinline__ float tf32_rn(float x) {
-  return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
+  uint32_t r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+  return __uint_as_float(r & 0xffffe000u);
 }
 
 // ---------------------------------------------------------------------------
 // the split pass
 // ---------------------------------------------------------------------------
-// src [rows][cols] with row pitch ld -> hi, lo [rows][cols] packed.  cols % 4 == 0; one thread per four values.
-// blockIdx.y = problem of the batch.
+// src [rows][cols] with row pitch ld -> hi, lo [rows][cols] with row pitch kp, a multiple of 4 >= cols, so that every
+// plane row starts on a 16-byte boundary whatever cols is (the columns from cols to kp are never read: the tensor maps
+// end at cols).  One thread per four values; kVec: rows of src start on 16-byte boundaries and cols % 4 == 0, else the
+// four values are loaded one by one.  blockIdx.y = problem of the batch.
+template <bool kVec>
 __global__ void __launch_bounds__(256)
 split_rows_kernel(const float* __restrict__ src, int64_t ld, int64_t src_batch_stride, float* __restrict__ hi,
-                  float* __restrict__ lo, int64_t rows, int32_t cols) {
-  const int64_t vec_per_row = cols >> 2;
+                  float* __restrict__ lo, int64_t rows, int32_t cols, int32_t kp) {
+  const int64_t vec_per_row = kp >> 2;
   const int64_t total = rows * vec_per_row;
   const float* s = src + blockIdx.y * src_batch_stride;
-  float* h = hi + blockIdx.y * rows * cols;
-  float* l = lo + blockIdx.y * rows * cols;
+  float* h = hi + blockIdx.y * rows * kp;
+  float* l = lo + blockIdx.y * rows * kp;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t r = i / vec_per_row, c4 = (i - r * vec_per_row) << 2;
-    const float4 x = *reinterpret_cast<const float4*>(s + r * ld + c4);
+    float4 x;
+    if (kVec) {
+      x = *reinterpret_cast<const float4*>(s + r * ld + c4);
+    } else {
+      const float* q = s + r * ld + c4;
+      x.x = q[0];  // c4 < cols, because kp - cols < 4
+      x.y = c4 + 1 < cols ? q[1] : 0.f;
+      x.z = c4 + 2 < cols ? q[2] : 0.f;
+      x.w = c4 + 3 < cols ? q[3] : 0.f;
+    }
     float4 a, b;
     a.x = tf32_rn(x.x), a.y = tf32_rn(x.y), a.z = tf32_rn(x.z), a.w = tf32_rn(x.w);
     b.x = tf32_rn(x.x - a.x), b.y = tf32_rn(x.y - a.y), b.z = tf32_rn(x.z - a.z), b.w = tf32_rn(x.w - a.w);
-    *reinterpret_cast<float4*>(h + r * cols + c4) = a;
-    *reinterpret_cast<float4*>(l + r * cols + c4) = b;
+    *reinterpret_cast<float4*>(h + r * kp + c4) = a;
+    *reinterpret_cast<float4*>(l + r * kp + c4) = b;
   }
 }
 
-// src [K][N] with row pitch ld -> hi, lo [N][K] packed (transposed), 32 x 32 tiles through shared memory.
+// src [K][N] with row pitch ld -> hi, lo [N][K] with row pitch kp (transposed), 32 x 32 tiles through shared memory.
 // grid (ceil(N/32), ceil(K/32), batch), 256 threads (32 x 8).
 __global__ void __launch_bounds__(256)
 split_transpose_kernel(const float* __restrict__ src, int64_t ld, int64_t src_batch_stride, float* __restrict__ hi,
-                       float* __restrict__ lo, int32_t k, int32_t n) {
+                       float* __restrict__ lo, int32_t k, int32_t n, int32_t kp) {
   __shared__ float tile[32][33];
   const float* s = src + blockIdx.z * src_batch_stride;
-  float* h = hi + static_cast<int64_t>(blockIdx.z) * n * k;
-  float* l = lo + static_cast<int64_t>(blockIdx.z) * n * k;
+  float* h = hi + static_cast<int64_t>(blockIdx.z) * n * kp;
+  float* l = lo + static_cast<int64_t>(blockIdx.z) * n * kp;
   const int n0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
 #pragma unroll
@@ -111,8 +135,8 @@ split_transpose_kernel(const float* __restrict__ src, int64_t ld, int64_t src_ba
     if (nn < n && kk < k) {
       const float x = tile[tx][ty + 8 * j];
       const float a = tf32_rn(x);
-      h[static_cast<int64_t>(nn) * k + kk] = a;
-      l[static_cast<int64_t>(nn) * k + kk] = tf32_rn(x - a);
+      h[static_cast<int64_t>(nn) * kp + kk] = a;
+      l[static_cast<int64_t>(nn) * kp + kk] = tf32_rn(x - a);
     }
   }
 }
@@ -120,6 +144,58 @@ split_transpose_kernel(const float* __restrict__ src, int64_t ld, int64_t src_ba
 // ---------------------------------------------------------------------------
 // the contraction
 // ---------------------------------------------------------------------------
+// One warp writes its 32 rows x 32 columns of C (lane = row of `sum`, first element C[row0][col0]), transposed through
+// `staging`: 16-byte unit u of row r lies at unit u ^ (r & 7), so neither side has bank conflicts.  vec_store: 16-byte
+// stores, four rows at a time, otherwise 4-byte stores of one row.  Writing rows from the lanes that hold them costs more
+// even where they are aligned: every store then touches 32 rows (2000 x 3000 x 1500 on 256 x 128 tiles: 127 us against 117).
+// kRedo (problems that the FP32 pipe could take as well): an output that comes out infinite or NaN is summed again in plain
+// f32, because infinity split into hi + lo is infinity + NaN.
+__device__ __noinline__ float dot_f32(const Params& p, int batch, int row, int col) {
+  const float* x = p.a + batch * p.a_batch_stride + row * p.lda;
+  const float* w = p.b + batch * p.b_batch_stride + (p.b_transposed ? col * p.ldb : static_cast<int64_t>(col));
+  const int64_t step = p.b_transposed ? 1 : p.ldb;
+  float s = 0.f;
+  for (int k = 0; k < p.k && s == s; ++k) s = fmaf(x[k], w[k * step], s);  // a NaN stays one
+  return s;
+}
+template <bool kRedo>
+__device__ __forceinline__ void store_block_32x32(float* __restrict__ c, const Params& p, int batch, int row0, int col0,
+                                                  const float (&sum)[32], float* staging, int lane) {
+  float* cb = c + batch * p.c_batch_stride;
+  uint32_t bad = 0;  // columns of this lane's row to sum again
+  if (kRedo) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) bad |= (fabsf(sum[i]) < INFINITY ? 0u : 1u) << i;
+    if (row0 + lane >= p.m) bad = 0;
+  }
+  float4* st4 = reinterpret_cast<float4*>(staging);
+  __syncwarp();  // the previous block has been read
+#pragma unroll
+  for (int i = 0; i < 8; ++i) st4[lane * 8 + (i ^ (lane & 7))] = make_float4(sum[4 * i], sum[4 * i + 1], sum[4 * i + 2], sum[4 * i + 3]);
+  __syncwarp();
+  const int rows = min(32, p.m - row0);
+  if (p.vec_store && col0 + 32 <= p.n) {
+    const int u = lane & 7;
+    float* dst = cb + static_cast<int64_t>(row0) * p.ldc + col0 + u * 4;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int r = i * 4 + (lane >> 3);
+      if (r < rows) *reinterpret_cast<float4*>(dst + r * p.ldc) = st4[r * 8 + (u ^ (r & 7))];
+    }
+  } else if (col0 + lane < p.n) {
+    float* dst = cb + static_cast<int64_t>(row0) * p.ldc + col0 + lane;
+    for (int r = 0; r < rows; ++r) dst[r * p.ldc] = staging[r * 32 + (((lane >> 2) ^ (r & 7)) << 2) + (lane & 3)];
+  }
+  if (kRedo && __any_sync(0xffffffffu, bad != 0)) {
+    __syncwarp();  // after the stores above: another lane may have written this lane's elements
+    __threadfence_block();
+    for (; bad != 0; bad &= bad - 1) {
+      const int col = col0 + __ffs(bad) - 1;
+      if (col < p.n) cb[static_cast<int64_t>(row0 + lane) * p.ldc + col] = dot_f32(p, batch, row0 + lane, col);
+    }
+  }
+}
+
 __device__ __forceinline__ void tile_coords(const Params& p, int tile, int& b, int& mb, int& nb) {
   const int per_batch = p.m_blocks * p.n_blocks;
   b = tile / per_batch;
@@ -151,19 +227,20 @@ __device__ __forceinline__ void tcgen05_mma_tf32_ss(uint32_t d_tmem, uint64_t a_
       : "memory");
 }
 
+template <bool kRedo>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tf32_tc_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_constant__ CUtensorMap tmap_a_lo,
                     const __grid_constant__ CUtensorMap tmap_b_hi, const __grid_constant__ CUtensorMap tmap_b_lo,
                     float* __restrict__ c, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  Barriers* bars = reinterpret_cast<Barriers*>(smem + kStages * kStageBytes);
+  Barriers* bars = reinterpret_cast<Barriers*>(smem + kStages * kStageBytes + kStagingBytes);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int num_tiles = p.batch * p.m_blocks * p.n_blocks;
   const int num_kb = (p.k + kBK - 1) / kBK;
-  const int num_chunks = (num_kb + kChunkKb - 1) / kChunkKb;
+  const int num_chunks = (num_kb + p.chunk_kb - 1) / p.chunk_kb;
   volatile uint32_t* abort_flag = &bars->abort_flag;
 
   if (threadIdx.x == 0) {
@@ -232,14 +309,14 @@ gemm_tf32_tc_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_
         for (int ch = 0; ch < num_chunks && ok; ++ch, ++chunk_count) {
           const uint32_t acc = chunk_count & 1u;
           const uint32_t acc_phase = (chunk_count >> 1) & 1u;
-          if (!ptx::mbar_wait(&bars->acc_empty[acc], acc_phase ^ 1u, abort_flag, p.status, 42)) {
+          if (!ptx::mbar_wait_relaxed(&bars->acc_empty[acc], acc_phase ^ 1u, abort_flag, p.status, 42)) {
             ok = false;
             break;
           }
           ptx::tcgen05_fence_after_thread_sync();
           const uint32_t d_tmem = tmem_base + acc * kBN;
-          const int kb_end = min(num_kb, (ch + 1) * kChunkKb);
-          for (int kb = ch * kChunkKb; kb < kb_end; ++kb) {
+          const int kb_end = min(num_kb, (ch + 1) * p.chunk_kb);
+          for (int kb = ch * p.chunk_kb; kb < kb_end; ++kb) {
             if (!ptx::mbar_wait_relaxed(&bars->full[stage], phase, abort_flag, p.status, 43)) {
               ok = false;
               break;
@@ -249,16 +326,18 @@ gemm_tf32_tc_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_
             const uint32_t a_lo = a_hi + kAPlane;
             const uint32_t b_hi = a_hi + 2 * kAPlane;
             const uint32_t b_lo = b_hi + kBPlane;
-            const bool first_kb = kb == ch * kChunkKb;
+            const bool first_kb = kb == ch * p.chunk_kb;
+            // the small products first, then the large ones
 #pragma unroll
             for (int kk = 0; kk < kBK / kUmmaK; ++kk) {
               const uint32_t off = kk * kstep;
-              // the two small products first, then the large one
               tcgen05_mma_tf32_ss(d_tmem, ptx::smem_desc(kmajor, a_lo + off), ptx::smem_desc(kmajor, b_hi + off), idesc,
                                   (first_kb && kk == 0) ? 0u : 1u);
               tcgen05_mma_tf32_ss(d_tmem, ptx::smem_desc(kmajor, a_hi + off), ptx::smem_desc(kmajor, b_lo + off), idesc, 1u);
-              tcgen05_mma_tf32_ss(d_tmem, ptx::smem_desc(kmajor, a_hi + off), ptx::smem_desc(kmajor, b_hi + off), idesc, 1u);
             }
+#pragma unroll
+            for (int kk = 0; kk < kBK / kUmmaK; ++kk)
+              tcgen05_mma_tf32_ss(d_tmem, ptx::smem_desc(kmajor, a_hi + kk * kstep), ptx::smem_desc(kmajor, b_hi + kk * kstep), idesc, 1u);
             ptx::tcgen05_commit(&bars->empty[stage]);  // stage reusable once these MMAs retire
             if (++stage == kStages) {
               stage = 0;
@@ -273,6 +352,7 @@ gemm_tf32_tc_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_
     // ------------------------------ chunk drain and output ----------------------
     const int quad = warp & 3;            // TMEM lanes [32*quad, 32*quad+32) belong to this warp
     const int half = (warp - 2) >> 2;     // which 128 columns of the 256-column accumulator
+    float* staging = reinterpret_cast<float*>(smem + kStages * kStageBytes) + (warp - 2) * kStagingFloats;
     const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + half * 128;
     uint32_t chunk_count = 0;
     bool alive = true;
@@ -307,23 +387,9 @@ gemm_tf32_tc_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_
         if (lane == 0) ptx::mbar_arrive(&bars->acc_empty[acc]);
       }
       if (!alive) break;
-      const int row = mb * kBM + quad * 32 + lane;
-      if (row < p.m) {
-        float* crow = c + static_cast<int64_t>(b) * p.c_batch_stride + static_cast<int64_t>(row) * p.ldc;
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-          const int col = nb * kBN + half * 128 + cc * 32;
-          if (col + 32 <= p.n) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-              reinterpret_cast<float4*>(crow + col)[i] = make_float4(sum[cc][4 * i], sum[cc][4 * i + 1], sum[cc][4 * i + 2], sum[cc][4 * i + 3]);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (col + i < p.n) crow[col + i] = sum[cc][i];
-          }
-        }
-      }
+      for (int cc = 0; cc < 4; ++cc)
+        store_block_32x32<kRedo>(c, p, b, mb * kBM + quad * 32, nb * kBN + half * 128 + cc * 32, sum[cc], staging, lane);
     }
   }
 
@@ -355,21 +421,33 @@ gemm_tf32_tc_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_
 namespace pair {
 constexpr int kPairM = 256;
 constexpr int kCtaM = 128;
-constexpr int kCtaN = 128;             // columns of B staged by each CTA
-constexpr int kStages = 3;
-constexpr int kPlane = kCtaM * kBK * 4;            // 16 KiB: every plane a CTA stages
-constexpr int kStageBytes = 4 * kPlane;            // A_hi, A_lo, B_hi, B_lo
 constexpr int kGroupM = 8;             // pair tiles per band
+constexpr int kMaxStages = 4;
+
+// BN: columns of a pair's tile, 256 or 128.  Half the width means twice the tiles, which fill the last wave better
+// (the host picks, see gemm_tf32_tc_launch), at 4/3 of the operand traffic per product.
+template <int BN>
+struct Shape {
+  static constexpr int kCtaN = BN / 2;                // columns of B staged by each CTA
+  static constexpr int kStages = BN == 256 ? 3 : 4;
+  static constexpr int kAPlane = kCtaM * kBK * 4;     // 16 KiB
+  static constexpr int kBPlane = kCtaN * kBK * 4;     // 16 or 8 KiB
+  static constexpr int kStageBytes = 2 * (kAPlane + kBPlane);  // A_hi, A_lo, B_hi, B_lo
+};
 
 struct alignas(8) Barriers {
-  uint64_t full[kStages];      // used in the leader: both CTAs' bytes of a stage have landed
-  uint64_t empty[kStages];     // in each CTA: the MMAs reading the stage have retired
+  uint64_t full[kMaxStages];   // used in the leader: both CTAs' bytes of a stage have landed
+  uint64_t empty[kMaxStages];  // in each CTA: the MMAs reading the stage have retired
   uint64_t acc_full[2];        // in each CTA: chunk accumulator complete
   uint64_t acc_empty[2];       // used in the leader: 16 epilogue warps of the pair have drained it
   uint32_t tmem_base;
   uint32_t abort_flag;
 };
-constexpr int kSmemBytes = kStages * kStageBytes + sizeof(Barriers) + 1024;
+template <int BN>
+constexpr int smem_bytes() {
+  return Shape<BN>::kStages * Shape<BN>::kStageBytes + kStagingBytes + sizeof(Barriers) + 1024;
+}
+static_assert(smem_bytes<256>() <= 227 * 1024 && smem_bytes<128>() <= 227 * 1024, "shared memory budget of one CTA");
 
 __device__ __forceinline__ void tile_coords(const Params& p, int tile, int& b, int& mb, int& nb) {
   const int per_batch = p.m_blocks * p.n_blocks;
@@ -396,14 +474,18 @@ __device__ __forceinline__ void tcgen05_mma_tf32_ss_pair(uint32_t d_tmem, uint64
       : "memory");
 }
 
-// m_blocks / n_blocks of Params count 256 x 256 pair tiles here.
+// m_blocks / n_blocks of Params count 256 x BN pair tiles here.
+template <int BN, bool kRedo>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_constant__ CUtensorMap tmap_a_lo,
                      const __grid_constant__ CUtensorMap tmap_b_hi, const __grid_constant__ CUtensorMap tmap_b_lo,
                      float* __restrict__ c, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  Barriers* bars = reinterpret_cast<Barriers*>(smem + kStages * kStageBytes);
+  using S = Shape<BN>;
+  constexpr int kStages = S::kStages, kStageBytes = S::kStageBytes, kCtaN = S::kCtaN;
+  constexpr int kAPlane = S::kAPlane, kBPlane = S::kBPlane;
+  Barriers* bars = reinterpret_cast<Barriers*>(smem + kStages * kStageBytes + kStagingBytes);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -412,7 +494,7 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
   const int num_pairs = gridDim.x >> 1;
   const int num_tiles = p.batch * p.m_blocks * p.n_blocks;
   const int num_kb = (p.k + kBK - 1) / kBK;
-  const int num_chunks = (num_kb + kChunkKb - 1) / kChunkKb;
+  const int num_chunks = (num_kb + p.chunk_kb - 1) / p.chunk_kb;
   volatile uint32_t* abort_flag = &bars->abort_flag;
 
   if (threadIdx.x == 0) {
@@ -450,7 +532,7 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
         int b, mb, nb;
         pair::tile_coords(p, tile, b, mb, nb);
         const int row0 = mb * kPairM + static_cast<int>(rank) * kCtaM;
-        const int col0 = nb * kBN + static_cast<int>(rank) * kCtaN;
+        const int col0 = nb * BN + static_cast<int>(rank) * kCtaN;
         for (int kb = 0; kb < num_kb; ++kb) {
           if (!ptx::mbar_wait(&bars->empty[stage], phase ^ 1u, abort_flag, p.status, 45)) {
             ok = false;
@@ -460,9 +542,9 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
           if (rank == 0) ptx::mbar_arrive_expect_tx(&bars->full[stage], 2 * kStageBytes);
           uint8_t* st = smem + stage * kStageBytes;
           ptx::tma_load_3d_pair(st, &tmap_a_hi, full_leader, kb * kBK, row0, b);
-          ptx::tma_load_3d_pair(st + kPlane, &tmap_a_lo, full_leader, kb * kBK, row0, b);
-          ptx::tma_load_3d_pair(st + 2 * kPlane, &tmap_b_hi, full_leader, kb * kBK, col0, b);
-          ptx::tma_load_3d_pair(st + 3 * kPlane, &tmap_b_lo, full_leader, kb * kBK, col0, b);
+          ptx::tma_load_3d_pair(st + kAPlane, &tmap_a_lo, full_leader, kb * kBK, row0, b);
+          ptx::tma_load_3d_pair(st + 2 * kAPlane, &tmap_b_hi, full_leader, kb * kBK, col0, b);
+          ptx::tma_load_3d_pair(st + 2 * kAPlane + kBPlane, &tmap_b_lo, full_leader, kb * kBK, col0, b);
           if (++stage == kStages) {
             stage = 0;
             phase ^= 1u;
@@ -473,7 +555,7 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
   } else if (warp == 1) {
     // ------------------------------ MMA issuer (leader CTA only) --------------
     if (lane == 0 && rank == 0) {
-      constexpr uint32_t idesc = make_idesc_tf32(kPairM, kBN);
+      constexpr uint32_t idesc = make_idesc_tf32(kPairM, BN);
       constexpr uint64_t kmajor = ptx::make_smem_desc_base(16, 1024);
       constexpr uint32_t kstep = kUmmaK * 4;
       int stage = 0;
@@ -484,30 +566,32 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
         for (int ch = 0; ch < num_chunks && ok; ++ch, ++chunk_count) {
           const uint32_t acc = chunk_count & 1u;
           const uint32_t acc_phase = (chunk_count >> 1) & 1u;
-          if (!ptx::mbar_wait(&bars->acc_empty[acc], acc_phase ^ 1u, abort_flag, p.status, 46)) {
+          if (!ptx::mbar_wait_relaxed(&bars->acc_empty[acc], acc_phase ^ 1u, abort_flag, p.status, 46)) {
             ok = false;
             break;
           }
           ptx::tcgen05_fence_after_thread_sync();
-          const uint32_t d_tmem = tmem_base + acc * kBN;
-          const int kb_end = min(num_kb, (ch + 1) * kChunkKb);
-          for (int kb = ch * kChunkKb; kb < kb_end; ++kb) {
+          const uint32_t d_tmem = tmem_base + acc * BN;
+          const int kb_end = min(num_kb, (ch + 1) * p.chunk_kb);
+          for (int kb = ch * p.chunk_kb; kb < kb_end; ++kb) {
             if (!ptx::mbar_wait_relaxed(&bars->full[stage], phase, abort_flag, p.status, 47)) {
               ok = false;
               break;
             }
             ptx::tcgen05_fence_after_thread_sync();
             const uint32_t a_hi = ptx::smem_u32(smem + stage * kStageBytes);
-            const uint32_t a_lo = a_hi + kPlane, b_hi = a_hi + 2 * kPlane, b_lo = a_hi + 3 * kPlane;
-            const bool first_kb = kb == ch * kChunkKb;
+            const uint32_t a_lo = a_hi + kAPlane, b_hi = a_lo + kAPlane, b_lo = b_hi + kBPlane;
+            const bool first_kb = kb == ch * p.chunk_kb;
 #pragma unroll
             for (int kk = 0; kk < kBK / kUmmaK; ++kk) {
               const uint32_t off = kk * kstep;
               tcgen05_mma_tf32_ss_pair(d_tmem, ptx::smem_desc(kmajor, a_lo + off), ptx::smem_desc(kmajor, b_hi + off), idesc,
                                        (first_kb && kk == 0) ? 0u : 1u);
               tcgen05_mma_tf32_ss_pair(d_tmem, ptx::smem_desc(kmajor, a_hi + off), ptx::smem_desc(kmajor, b_lo + off), idesc, 1u);
-              tcgen05_mma_tf32_ss_pair(d_tmem, ptx::smem_desc(kmajor, a_hi + off), ptx::smem_desc(kmajor, b_hi + off), idesc, 1u);
             }
+#pragma unroll
+            for (int kk = 0; kk < kBK / kUmmaK; ++kk)
+              tcgen05_mma_tf32_ss_pair(d_tmem, ptx::smem_desc(kmajor, a_hi + kk * kstep), ptx::smem_desc(kmajor, b_hi + kk * kstep), idesc, 1u);
             ptx::tcgen05_commit_pair(&bars->empty[stage], 3);  // frees the stage in both CTAs
             if (++stage == kStages) {
               stage = 0;
@@ -522,15 +606,17 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
     // ------------------------------ chunk drain and output (both CTAs) ----------
     const int quad = warp & 3;
     const int half = (warp - 2) >> 2;
-    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + half * 128;
+    constexpr int kChunks = BN / 64;      // 32-column blocks per warp
+    const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + half * (BN / 2);
+    float* staging = reinterpret_cast<float*>(smem + kStages * kStageBytes) + (warp - 2) * kStagingFloats;
     uint32_t chunk_count = 0;
     bool alive = true;
     for (int tile = pair_id; tile < num_tiles && alive; tile += num_pairs) {
       int b, mb, nb;
       pair::tile_coords(p, tile, b, mb, nb);
-      float sum[4][32];
+      float sum[kChunks][32];
 #pragma unroll
-      for (int cc = 0; cc < 4; ++cc)
+      for (int cc = 0; cc < kChunks; ++cc)
 #pragma unroll
         for (int i = 0; i < 32; ++i) sum[cc][i] = 0.f;
       for (int ch = 0; ch < num_chunks; ++ch, ++chunk_count) {
@@ -543,9 +629,9 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
         }
         ptx::tcgen05_fence_after_thread_sync();
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
+        for (int cc = 0; cc < kChunks; ++cc) {
           uint32_t v[32];
-          ptx::tmem_ld_32x32b_x32(lane_addr + acc * kBN + cc * 32, v);
+          ptx::tmem_ld_32x32b_x32(lane_addr + acc * BN + cc * 32, v);
           ptx::tmem_ld_wait();
 #pragma unroll
           for (int i = 0; i < 32; ++i) sum[cc][i] += __uint_as_float(v[i]);
@@ -555,23 +641,10 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
         if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa_shared(ptx::smem_u32(&bars->acc_empty[acc]), 0));
       }
       if (!alive) break;
-      const int row = mb * kPairM + static_cast<int>(rank) * kCtaM + quad * 32 + lane;
-      if (row < p.m) {
-        float* crow = c + static_cast<int64_t>(b) * p.c_batch_stride + static_cast<int64_t>(row) * p.ldc;
+      const int row0 = mb * kPairM + static_cast<int>(rank) * kCtaM + quad * 32;
 #pragma unroll
-        for (int cc = 0; cc < 4; ++cc) {
-          const int col = nb * kBN + half * 128 + cc * 32;
-          if (col + 32 <= p.n) {
-#pragma unroll
-            for (int i = 0; i < 8; ++i)
-              reinterpret_cast<float4*>(crow + col)[i] = make_float4(sum[cc][4 * i], sum[cc][4 * i + 1], sum[cc][4 * i + 2], sum[cc][4 * i + 3]);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (col + i < p.n) crow[col + i] = sum[cc][i];
-          }
-        }
-      }
+      for (int cc = 0; cc < kChunks; ++cc)
+        store_block_32x32<kRedo>(c, p, b, row0, nb * BN + half * (BN / 2) + cc * 32, sum[cc], staging, lane);
     }
   }
 

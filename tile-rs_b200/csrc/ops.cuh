@@ -599,10 +599,19 @@ inline cudaError_t keep_pool_memory_once() {
   return e;
 }
 
+// Columns of a pair's tile: the width whose waves of tiles over the SM pairs take the least time.  A 128-wide tile
+// costs two thirds of a 256-wide one, not half (its operand traffic per product is 4/3 and a chunk's drain overlaps
+// half the products): 4096^3 655 us in 4 wide waves, 757 in 7 narrow ones; 1536^3 79 us in one wide wave, 56 in one narrow.
+inline int gemm_tf32_pair_width(uint64_t m, uint64_t n, uint64_t batch, int sms) {
+  const uint64_t pairs = static_cast<uint64_t>(std::max(1, sms / 2)), rows = (m + 255) / 256 * batch;
+  const uint64_t wide = (rows * ((n + 255) / 256) + pairs - 1) / pairs, narrow = (rows * ((n + 127) / 128) + pairs - 1) / pairs;
+  return 67 * narrow < 100 * wide ? 128 : 256;
+}
+
 // f32 inputs on the tcgen05 tensor cores: split pass (hi / lo planes, B's planes K-major), then the
 // contraction with chunked accumulation (gemm_tf32_tc.cuh).  The planes live in stream-ordered scratch.
 inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
-                                   uint32_t* status, cudaStream_t s) {
+                                   uint32_t* status, bool rows_aligned, cudaStream_t s) {
   namespace g = gemm_tf32_tc;
   const uint64_t M = d->m, N = d->n, K = d->k, B = d->batch;
   const GemmPitch ld = gemm_pitch(d);
@@ -611,7 +620,8 @@ inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, 
   if (st != TSM100_OK) return st;
   cudaError_t e = keep_pool_memory_once();
   if (e != cudaSuccess) return cuda_ok(err, e, "cudaMemPoolSetAttribute");
-  const size_t a_plane = static_cast<size_t>(B) * M * K, b_plane = static_cast<size_t>(B) * N * K;  // elements
+  const uint64_t kp = (K + 3) / 4 * 4;  // row pitch of the planes: every row starts on a 16-byte boundary
+  const size_t a_plane = static_cast<size_t>(B) * M * kp, b_plane = static_cast<size_t>(B) * N * kp;  // elements
   float* ws = nullptr;
   e = cudaMallocAsync(reinterpret_cast<void**>(&ws), 2 * (a_plane + b_plane) * sizeof(float), s);
   if (e != cudaSuccess) {
@@ -621,74 +631,95 @@ inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, 
   float *a_hi = ws, *a_lo = ws + a_plane, *b_hi = ws + 2 * a_plane, *b_lo = b_hi + b_plane;
   const float* af = static_cast<const float*>(a);
   const float* bf = static_cast<const float*>(b);
-  auto grid1d = [&](uint64_t items) {
-    return static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((items + 255) / 256, static_cast<uint64_t>(sms) * 16)));
+  auto split_rows = [&](const float* src, int64_t pitch, uint64_t rows, float* hi, float* lo) {
+    const uint64_t items = rows * (kp / 4);
+    const dim3 grid(static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((items + 255) / 256, static_cast<uint64_t>(sms) * 16))),
+                    static_cast<unsigned>(B));
+    auto kern = kp == K && pitch % 4 == 0 && aligned16(src) ? g::split_rows_kernel<true> : g::split_rows_kernel<false>;
+    kern<<<grid, 256, 0, s>>>(src, pitch, static_cast<int64_t>(rows) * pitch, hi, lo, static_cast<int64_t>(rows),
+                              static_cast<int32_t>(K), static_cast<int32_t>(kp));
   };
-  g::split_rows_kernel<<<dim3(grid1d(M * K / 4), static_cast<unsigned>(B)), 256, 0, s>>>(
-      af, ld.lda, static_cast<int64_t>(M) * ld.lda, a_hi, a_lo, static_cast<int64_t>(M), static_cast<int32_t>(K));
+  split_rows(af, ld.lda, M, a_hi, a_lo);
   if (d->b_transposed) {
-    g::split_rows_kernel<<<dim3(grid1d(N * K / 4), static_cast<unsigned>(B)), 256, 0, s>>>(
-        bf, ld.ldb, static_cast<int64_t>(N) * ld.ldb, b_hi, b_lo, static_cast<int64_t>(N), static_cast<int32_t>(K));
+    split_rows(bf, ld.ldb, N, b_hi, b_lo);
   } else {
     g::split_transpose_kernel<<<dim3(static_cast<unsigned>((N + 31) / 32), static_cast<unsigned>((K + 31) / 32), static_cast<unsigned>(B)), 256, 0, s>>>(
-        bf, ld.ldb, static_cast<int64_t>(K) * ld.ldb, b_hi, b_lo, static_cast<int32_t>(K), static_cast<int32_t>(N));
+        bf, ld.ldb, static_cast<int64_t>(K) * ld.ldb, b_hi, b_lo, static_cast<int32_t>(K), static_cast<int32_t>(N), static_cast<int32_t>(kp));
   }
   st = cuda_ok(err, cudaGetLastError(), "gemm operand split launch");
   CUtensorMap ta_hi, ta_lo, tb_hi, tb_lo;
   const CUtensorMapDataType f32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  // Problems with more than one 128-row and 128-column block run on CTA pairs (256 x 256 tiles, each CTA staging
-  // 128 rows of A and 128 columns of B); the rest on single CTAs (128 x 256 tiles).
+  // Problems with more than one 128-row and 128-column block run on CTA pairs (256 x 256 or 256 x 128 tiles); the rest
+  // on single CTAs (128 x 256 tiles).
   const bool pairs = M > 128 && N > 128;
-  const uint32_t box_b = pairs ? g::pair::kCtaN : g::kBN;
-  if (st == TSM100_OK) st = make_tmap_3d(err, &ta_hi, a_hi, K, M, B, K, M * K, g::kBK, g::kBM, f32, 4);
-  if (st == TSM100_OK) st = make_tmap_3d(err, &ta_lo, a_lo, K, M, B, K, M * K, g::kBK, g::kBM, f32, 4);
-  if (st == TSM100_OK) st = make_tmap_3d(err, &tb_hi, b_hi, K, N, B, K, N * K, g::kBK, box_b, f32, 4);
-  if (st == TSM100_OK) st = make_tmap_3d(err, &tb_lo, b_lo, K, N, B, K, N * K, g::kBK, box_b, f32, 4);
+  const int bn = pairs ? gemm_tf32_pair_width(M, N, B, sms) : g::kBN;
+  const uint32_t box_b = pairs ? bn / 2 : g::kBN;
+  if (st == TSM100_OK) st = make_tmap_3d(err, &ta_hi, a_hi, K, M, B, kp, M * kp, g::kBK, g::kBM, f32, 4);
+  if (st == TSM100_OK) st = make_tmap_3d(err, &ta_lo, a_lo, K, M, B, kp, M * kp, g::kBK, g::kBM, f32, 4);
+  if (st == TSM100_OK) st = make_tmap_3d(err, &tb_hi, b_hi, K, N, B, kp, N * kp, g::kBK, box_b, f32, 4);
+  if (st == TSM100_OK) st = make_tmap_3d(err, &tb_lo, b_lo, K, N, B, kp, N * kp, g::kBK, box_b, f32, 4);
   if (st == TSM100_OK) {
     g::Params p;
     p.m = static_cast<int32_t>(M);
     p.n = static_cast<int32_t>(N);
     p.k = static_cast<int32_t>(K);
     p.batch = d->batch;
-    p.m_blocks = static_cast<int32_t>((M + (pairs ? g::pair::kPairM : g::kBM) - 1) / (pairs ? g::pair::kPairM : g::kBM));
-    p.n_blocks = static_cast<int32_t>((N + g::kBN - 1) / g::kBN);
+    const uint64_t bm = pairs ? g::pair::kPairM : g::kBM;
+    p.m_blocks = static_cast<int32_t>((M + bm - 1) / bm);
+    p.n_blocks = static_cast<int32_t>((N + bn - 1) / bn);
     p.c_batch_stride = static_cast<int64_t>(M) * ld.ldc;
     p.ldc = ld.ldc;
     p.status = status;
+    p.vec_store = aligned16(c) && ld.ldc % 4 == 0 ? 1 : 0;
+    // Accumulation chunk: 128 of K, or shorter for the problems that the FP32 pipe took before, whose error was smaller at
+    // short K (relative to the 64-bit result: FP32 pipe 2.9e-7 at K = 257, 6.9e-7 at 1501; here 9e-7 with chunks of 128,
+    // 3.8e-7 with 64, 1.4e-7 .. 1.8e-7 with 32)
+    p.chunk_kb = rows_aligned ? 4 : K >= 512 ? 2 : 1;
+    p.b_transposed = d->b_transposed;
+    p.a = af, p.b = bf;
+    p.lda = ld.lda, p.ldb = ld.ldb;
+    p.a_batch_stride = static_cast<int64_t>(M) * ld.lda;
+    p.b_batch_stride = static_cast<int64_t>(d->b_transposed ? N : K) * ld.ldb;
     const int64_t tiles = static_cast<int64_t>(p.m_blocks) * p.n_blocks * p.batch;
+    auto launch_pairs = [&](auto kern, int smem) -> cudaError_t {
+      cudaError_t pe = set_dyn_smem_once(kern, smem);
+      if (pe != cudaSuccess) return pe;
+      cudaLaunchConfig_t cfg = {};
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 2;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.blockDim = dim3(g::kThreads);
+      cfg.dynamicSmemBytes = static_cast<size_t>(smem);
+      cfg.stream = s;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      cfg.gridDim = dim3(static_cast<unsigned>(sms & ~1));
+      int max_clusters = sms / 2;
+      kernel_fact(reinterpret_cast<const void*>(kern), kFactClusters, &max_clusters, [&](int* out) {
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+          (void)cudaGetLastError();
+          return false;
+        }
+        *out = n;
+        return true;
+      });
+      const int64_t npairs = std::min<int64_t>(tiles, std::min<int64_t>(max_clusters, sms / 2));
+      cfg.gridDim = dim3(static_cast<unsigned>(2 * npairs));
+      return cudaLaunchKernelEx(&cfg, kern, ta_hi, ta_lo, tb_hi, tb_lo, static_cast<float*>(c), p);
+    };
     if (pairs) {
-      auto kern = g::pair::gemm_tf32_tc2_kernel;
-      e = set_dyn_smem_once(kern, g::pair::kSmemBytes);
-      if (e == cudaSuccess) {
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.blockDim = dim3(g::kThreads);
-        cfg.dynamicSmemBytes = g::pair::kSmemBytes;
-        cfg.stream = s;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        cfg.gridDim = dim3(static_cast<unsigned>(sms & ~1));
-        int max_clusters = sms / 2;
-        kernel_fact(reinterpret_cast<const void*>(kern), kFactClusters, &max_clusters, [&](int* out) {
-          int n = 0;
-          if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
-            (void)cudaGetLastError();
-            return false;
-          }
-          *out = n;
-          return true;
-        });
-        const int64_t npairs = std::min<int64_t>(tiles, std::min<int64_t>(max_clusters, sms / 2));
-        cfg.gridDim = dim3(static_cast<unsigned>(2 * npairs));
-        e = cudaLaunchKernelEx(&cfg, kern, ta_hi, ta_lo, tb_hi, tb_lo, static_cast<float*>(c), p);
-      }
+      if (rows_aligned)
+        e = bn == 256 ? launch_pairs(g::pair::gemm_tf32_tc2_kernel<256, false>, g::pair::smem_bytes<256>())
+                      : launch_pairs(g::pair::gemm_tf32_tc2_kernel<128, false>, g::pair::smem_bytes<128>());
+      else
+        e = bn == 256 ? launch_pairs(g::pair::gemm_tf32_tc2_kernel<256, true>, g::pair::smem_bytes<256>())
+                      : launch_pairs(g::pair::gemm_tf32_tc2_kernel<128, true>, g::pair::smem_bytes<128>());
       st = cuda_ok(err, e, "gemm_tf32_tc2_kernel launch");
     } else {
-      auto kern = g::gemm_tf32_tc_kernel;
+      auto kern = rows_aligned ? g::gemm_tf32_tc_kernel<false> : g::gemm_tf32_tc_kernel<true>;
       e = set_dyn_smem_once(kern, g::kSmemBytes);
       if (e == cudaSuccess) {
         const unsigned grid = static_cast<unsigned>(std::min<int64_t>(tiles, sms));
@@ -825,17 +856,15 @@ inline int32_t gemm(std::string* err, const tsm100_gemm_desc* d, const void* a, 
                                           static_cast<size_t>(d->batch) * d->m, s), "cudaMemset2DAsync");
   }
   if (d->dtype == TSM100_F32) {
-    // rows that start on 16-byte boundaries: tensor cores; anything else: the FP32 pipe
     const bool vec_ok = aligned16(a) && aligned16(b) && aligned16(c) && d->k % 4 == 0 && (d->b_transposed || d->n % 4 == 0) &&
                         d->n % 2 == 0 && ld.lda % 4 == 0 && ld.ldb % 4 == 0 && ld.ldc % 2 == 0;
-    if (vec_ok) {
-      // enough 128 x 256 tiles to occupy the GPU: the persistent tcgen05 kernels (operand planes from a split pass)
-      const int64_t tiles = ((d->m + 127) / 128) * ((d->n + 255) / 256) * d->batch;
-      if (status != nullptr && tiles >= 64 && tiles < 0x7fffffff && d->k >= 256) return gemm_tf32_tc_launch(err, d, a, b, c, status, s);
-      // fewer tiles (the 512^3 configuration has 8): the warp-level kernel, whose 64 x 64 tiles and cluster split-K
-      // spread a small problem over the SMs
-      return gemm_tf32x3_launch(err, d, a, b, c, s);
-    }
+    // enough work for the persistent tcgen05 kernels; their split pass takes rows of any alignment
+    const int64_t tiles = ((d->m + 127) / 128) * ((d->n + 255) / 256) * d->batch;
+    if (status != nullptr && tiles >= 64 && tiles < 0x7fffffff && d->k >= 256)
+      return gemm_tf32_tc_launch(err, d, a, b, c, status, vec_ok, s);
+    // fewer tiles (the 512^3 configuration has 8): the warp-level kernel, whose 64 x 64 tiles and cluster split-K
+    // spread a small problem over the SMs, if rows start on 16-byte boundaries, else the FP32 pipe
+    if (vec_ok) return gemm_tf32x3_launch(err, d, a, b, c, s);
     return gemm_simt_launch<float, float>(err, d, a, b, c, s);
   }
 
