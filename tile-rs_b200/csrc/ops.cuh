@@ -29,6 +29,7 @@
 #include "attention_tf32x3.cuh"
 #include "ewise.cuh"
 #include "gemm_simt.cuh"
+#include "gemm_skinny.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_tc2.cuh"
 #include "gemm_tf32_tc.cuh"
@@ -771,6 +772,71 @@ inline int32_t gemm_tc_launch(std::string* err, const tsm100_gemm_desc* d, const
   return cuda_ok(err, cudaGetLastError(), "gemm_tc_kernel launch");
 }
 
+// Few output tiles: 128 columns x NT rows of C per CTA, K split over clusters (gemm_skinny.cuh).
+template <typename OutT, bool kBT, bool kBf16, int NT>
+inline int32_t gemm_skinny_launch_nt(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
+                                     uint32_t* status, cudaStream_t s) {
+  namespace g = gemm_skinny;
+  CUtensorMap ta, tb;
+  const uint64_t M = d->m, N = d->n, K = d->k, B = d->batch;
+  const GemmPitch ld = gemm_pitch(d);
+  const uint64_t lda = ld.lda, ldb = ld.ldb;
+  int32_t st = make_tmap_16bit_3d(err, &ta, a, K, M, B, lda, M * lda, g::kBK, NT, kBf16);
+  if (st != TSM100_OK) return st;
+  if (kBT)
+    st = make_tmap_16bit_3d(err, &tb, b, K, N, B, ldb, N * ldb, g::kBK, g::kBN, kBf16);
+  else
+    st = make_tmap_16bit_3d(err, &tb, b, N, K, B, ldb, K * ldb, 64, g::kBK, kBf16);
+  if (st != TSM100_OK) return st;
+  int sms = 0;
+  st = sm_count(err, &sms);
+  if (st != TSM100_OK) return st;
+  g::Params p;
+  p.m = static_cast<int32_t>(M);
+  p.n = static_cast<int32_t>(N);
+  p.k = static_cast<int32_t>(K);
+  p.batch = d->batch;
+  p.m_blocks = static_cast<int32_t>((M + NT - 1) / NT);
+  p.n_blocks = static_cast<int32_t>((N + g::kBN - 1) / g::kBN);
+  p.c_batch_stride = static_cast<int64_t>(M) * ld.ldc;
+  p.ldc = ld.ldc;
+  p.status = status;
+  const int64_t tiles = static_cast<int64_t>(p.m_blocks) * p.n_blocks * p.batch;
+  if (tiles * g::kMaxSplit > 0x7fffffff) return op_fail(err, TSM100_ERR_INVALID, "gemm: too many tiles for one launch");
+  // K over a cluster while all CTAs still fit the GPU at once (two per SM) and each keeps at least four k-blocks
+  const int32_t kb = static_cast<int32_t>((K + g::kBK - 1) / g::kBK);
+  int splits = 1;
+  while (splits < g::kMaxSplit && tiles * splits * 2 <= 2ll * sms && kb / (2 * splits) >= 4) splits *= 2;
+  p.kb_per_cta = (kb + splits - 1) / splits;
+  splits = (kb + p.kb_per_cta - 1) / p.kb_per_cta;  // rounding up may leave a last CTA without work: drop it
+  auto kern = g::gemm_skinny_kernel<OutT, kBT, kBf16, NT>;
+  constexpr int smem = g::smem_bytes<NT>();
+  cudaError_t e = set_dyn_smem_once(kern, smem);
+  if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(gemm_skinny_kernel)");
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(splits);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cfg.blockDim = dim3(g::kThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
+  e = cudaLaunchKernelEx(&cfg, kern, ta, tb, static_cast<OutT*>(c), p);
+  return cuda_ok(err, e, "gemm_skinny_kernel launch");
+}
+template <typename OutT, bool kBT, bool kBf16>
+inline int32_t gemm_skinny_launch(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
+                                  uint32_t* status, cudaStream_t s) {
+  if (d->m <= 16) return gemm_skinny_launch_nt<OutT, kBT, kBf16, 16>(err, d, a, b, c, status, s);
+  if (d->m <= 32) return gemm_skinny_launch_nt<OutT, kBT, kBf16, 32>(err, d, a, b, c, status, s);
+  if (d->m <= 64) return gemm_skinny_launch_nt<OutT, kBT, kBf16, 64>(err, d, a, b, c, status, s);
+  return gemm_skinny_launch_nt<OutT, kBT, kBf16, 128>(err, d, a, b, c, status, s);
+}
+
 // CTA-pair kernel (256 x 256 tile per two SMs), launched as clusters of two.
 template <typename OutT, bool kBT, bool kBf16>
 inline int32_t gemm_tc2_launch(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
@@ -876,10 +942,20 @@ inline int32_t gemm(std::string* err, const tsm100_gemm_desc* d, const void* a, 
                       ld.lda % 8 == 0 && ld.ldb % 8 == 0 && (ld.ldc * dtype_size(d->out_dtype)) % 16 == 0 &&
                       (static_cast<int64_t>((d->m + 127) / 128) * ((d->n + 255) / 256) * d->batch < 0x7fffffff);
   if (tma_ok) {
-    const bool pair = d->m > 128 && d->n > 128;  // large enough for 256 x 256 tiles on CTA pairs
+    int sms = 0;
+    int32_t st = sm_count(err, &sms);
+    if (st != TSM100_OK) return st;
+    // CTA pairs where 256 x 256 tiles keep enough pairs busy.  Below, splitting K pays, unless K is short: 1024 x 2048 x 2048
+    // (32 pair tiles) 16.1 us on pairs, 16.8 split; 1024 x 1024 x 4096 24.8 / 16.0, 300 x 4096 x 16384 78.9 / 62.4.
+    const int64_t pair_tiles = ((d->m + 255) / 256) * ((d->n + 255) / 256) * d->batch;
+    const bool pair = d->m > 128 && d->n > 128 && (pair_tiles > sms / 4 || (pair_tiles > sms / 6 && d->k <= 2048));
+    // 65 .. 128 rows and 128 x 256 tiles for (nearly) all SMs: the persistent single-CTA kernel, whose accumulators alternate
+    // (128 x 16384 x 4096, batch 4: 95.4 us, 97.9 on the split kernel; batch 1, 64 tiles: 35.5 / 31.7)
+    const int64_t tiles = ((d->m + 127) / 128) * ((d->n + 255) / 256) * d->batch;
+    const bool single = d->m > 64 && d->n > 128 && d->m <= 128 && tiles * 8 >= sms * 6;
 #define TSM_GEMM_TC(OUT, BT, BF)                                                     \
-  return pair ? gemm_tc2_launch<OUT, BT, BF>(err, d, a, b, c, status, s) \
-              : gemm_tc_launch<OUT, BT, BF>(err, d, a, b, c, status, s)
+  return pair     ? gemm_tc2_launch<OUT, BT, BF>(err, d, a, b, c, status, s)         \
+         : single ? gemm_tc_launch<OUT, BT, BF>(err, d, a, b, c, status, s) : gemm_skinny_launch<OUT, BT, BF>(err, d, a, b, c, status, s)
     if (bf16) {
       if (out_f32) { if (d->b_transposed) TSM_GEMM_TC(float, true, true); else TSM_GEMM_TC(float, false, true); }
       else { if (d->b_transposed) TSM_GEMM_TC(__nv_bfloat16, true, true); else TSM_GEMM_TC(__nv_bfloat16, false, true); }
