@@ -28,6 +28,7 @@
 #include "attention_tc.cuh"
 #include "attention_tf32x3.cuh"
 #include "ewise.cuh"
+#include "gemm_pad.cuh"
 #include "gemm_simt.cuh"
 #include "gemm_skinny.cuh"
 #include "gemm_tc.cuh"
@@ -898,6 +899,62 @@ inline int32_t gemm_tc2_launch(std::string* err, const tsm100_gemm_desc* d, cons
   return cuda_ok(err, e, "gemm_tc2_kernel launch");
 }
 
+inline int32_t gemm(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
+                    uint32_t* status, void* stream);
+
+// A 16-bit problem whose rows start anywhere, on the tensor cores: operands that need it are copied into zero-padded
+// scratch (N and K rounded up to 8), the padded problem is computed and the result copied out.  The padding adds products
+// of zeros only, and columns that are not copied out.
+inline int32_t gemm_padded(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
+                           uint32_t* status, cudaStream_t s) {
+  namespace g = gemm_pad;
+  int sms = 0;
+  int32_t st = sm_count(err, &sms);
+  if (st != TSM100_OK) return st;
+  cudaError_t e = keep_pool_memory_once();
+  if (e != cudaSuccess) return cuda_ok(err, e, "cudaMemPoolSetAttribute");
+  const GemmPitch ld = gemm_pitch(d);
+  const int64_t np = (d->n + 7) / 8 * 8, kp = (d->k + 7) / 8 * 8, batch = d->batch;
+  const int64_t b_rows = d->b_transposed ? d->n : d->k, b_cols = d->b_transposed ? d->k : d->n;
+  const int64_t bp_rows = d->b_transposed ? np : kp, bp_cols = d->b_transposed ? kp : np;
+  const bool pad_a = kp != d->k || ld.lda % 8 != 0 || !aligned16(a);
+  const bool pad_b = bp_rows != b_rows || bp_cols != b_cols || ld.ldb % 8 != 0 || !aligned16(b);
+  const bool pad_c = np != d->n || ld.ldc % 8 != 0 || !aligned16(c);
+  const int64_t a_elems = pad_a ? batch * d->m * kp : 0, b_elems = pad_b ? batch * bp_rows * bp_cols : 0;  // multiples of 8
+  const int64_t c_elems = pad_c ? batch * d->m * np : 0;
+  uint16_t* ws = nullptr;
+  e = cudaMallocAsync(reinterpret_cast<void**>(&ws), static_cast<size_t>(a_elems + b_elems + c_elems) * 2, s);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    return op_fail(err, TSM100_ERR_MEMORY, std::string("gemm: scratch for padded operands: ") + cudaGetErrorString(e));
+  }
+  auto pad = [&](const void* src, int64_t pitch, int64_t rows, int64_t cols, uint16_t* dst, int64_t drows, int64_t dcols) {
+    const int64_t items = drows * (dcols / 8);
+    const dim3 grid(static_cast<unsigned>(std::min<int64_t>((items + g::kThreads - 1) / g::kThreads, 16ll * sms)), static_cast<unsigned>(batch));
+    g::pad_kernel<<<grid, g::kThreads, 0, s>>>(static_cast<const uint16_t*>(src), pitch, rows * pitch, static_cast<int32_t>(rows),
+                                              static_cast<int32_t>(cols), reinterpret_cast<uint4*>(dst), static_cast<int32_t>(drows),
+                                              static_cast<int32_t>(dcols));
+  };
+  tsm100_gemm_desc t = *d;
+  t.n = np, t.k = kp;
+  const void *ta = a, *tb = b;
+  void* tc = c;
+  if (pad_a) pad(a, ld.lda, d->m, d->k, ws, d->m, kp), ta = ws, t.lda = kp;
+  if (pad_b) pad(b, ld.ldb, b_rows, b_cols, ws + a_elems, bp_rows, bp_cols), tb = ws + a_elems, t.ldb = bp_cols;
+  if (pad_c) tc = ws + a_elems + b_elems, t.ldc = np;
+  st = cuda_ok(err, cudaGetLastError(), "gemm operand padding launch");
+  if (st == TSM100_OK) st = gemm(err, &t, ta, tb, tc, status, s);
+  if (st == TSM100_OK && pad_c) {
+    const dim3 grid(static_cast<unsigned>((d->n + g::kThreads - 1) / g::kThreads), static_cast<unsigned>(std::min<int64_t>(d->m, 4096)), static_cast<unsigned>(batch));
+    g::unpad_kernel<<<grid, g::kThreads, 0, s>>>(static_cast<const uint16_t*>(tc), static_cast<int32_t>(np), static_cast<uint16_t*>(c), ld.ldc,
+                                                d->m * ld.ldc, static_cast<int32_t>(d->m), static_cast<int32_t>(d->n));
+    st = cuda_ok(err, cudaGetLastError(), "gemm result copy launch");
+  }
+  e = cudaFreeAsync(ws, s);
+  if (st == TSM100_OK && e != cudaSuccess) st = cuda_ok(err, e, "cudaFreeAsync");
+  return st;
+}
+
 // `status` is a device word the tensor-core kernel writes if one of its bounded
 // waits runs out; it must be zero when the launch starts.
 inline int32_t gemm(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
@@ -965,6 +1022,12 @@ inline int32_t gemm(std::string* err, const tsm100_gemm_desc* d, const void* a, 
     }
 #undef TSM_GEMM_TC
   }
+  // Rows that start anywhere: worth the copies into padded scratch from about 2^26 products on.  Only for 16-bit results,
+  // whose last place hides the order of the f32 sums; an f32 result keeps the FP32 pipe's rounding to nearest.
+  const int64_t n8 = (d->n + 7) / 8 * 8, k8 = (d->k + 7) / 8 * 8;
+  if (status != nullptr && !out_f32 && d->m * d->n / 4096 * d->k * d->batch >= 1 << 14 && d->batch <= 65535 && n8 <= 0x7fffffff && k8 <= 0x7fffffff &&
+      ((d->m + 127) / 128) * ((n8 + 127) / 128) * d->batch * gemm_skinny::kMaxSplit <= 0x7fffffff)
+    return gemm_padded(err, d, a, b, c, status, s);
   if (bf16) {
     if (out_f32) return gemm_simt_launch<__nv_bfloat16, float>(err, d, a, b, c, s);
     return gemm_simt_launch<__nv_bfloat16, __nv_bfloat16>(err, d, a, b, c, s);
