@@ -1113,25 +1113,48 @@ inline int32_t attention_prefill_simt_launch(std::string* err, const tsm100_atte
   return cuda_ok(err, cudaGetLastError(), "attention_simt (prefill) launch");
 }
 
-// KV heads per band of the causal launch order: as many as keep K and V of the band (16-bit, head_dim 128) within
+// KV heads per band of the causal launch order: as many as keep K and V of the band (16-bit) within
 // 32 MiB, a quarter of the L2, so that the blocks in flight - a few weight levels of one band, at a band's end
 // together with the start of the next - read K and V from DRAM once.
-inline int32_t attention_kv_band(uint64_t kv_len, int64_t kv_heads) {
-  const uint64_t per_head = std::max<uint64_t>(1, kv_len * attn::kD * 2 * 2);
+inline int32_t attention_kv_band(uint64_t kv_len, int64_t kv_heads, uint64_t head_dim) {
+  const uint64_t per_head = std::max<uint64_t>(1, kv_len * head_dim * 2 * 2);
   const int64_t band = static_cast<int64_t>((32ull << 20) / per_head);
   return static_cast<int32_t>(std::max<int64_t>(1, std::min<int64_t>(band, std::max<int64_t>(kv_heads, 1))));
 }
 
-template <bool kBf16>
+// Launches the tcgen05 attention kernel over `blocks` query blocks.
+template <bool kBf16, bool kCache, int D>
+inline int32_t attention_fwd_launch(std::string* err, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, void* o,
+                                    attn::Params p, int64_t blocks, cudaStream_t s) {
+  namespace at = attn;
+  constexpr int smem = at::smem_bytes<D>();
+  p.blocks = static_cast<int32_t>(blocks);
+  auto kern = at::attention_fwd_kernel<kBf16, kCache, D>;
+  cudaError_t e = set_dyn_smem_once(kern, smem);
+  if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(attention_fwd_kernel)");
+  kern<<<static_cast<unsigned>(blocks), at::kThreads, smem, s>>>(tq, tk, tv, static_cast<uint16_t*>(o), p);
+  return cuda_ok(err, cudaGetLastError(), "attention_fwd_kernel launch");
+}
+
+// Which 16-bit problems run on the tcgen05 kernel: head_dim 128, and 32 and 64 on its 64-wide form.  96 stays on the TF32
+// kernel: the second P tile that keeps the probabilities' precision does not fit beside 128-wide tiles.  b4, 32 / 8 heads of
+// 64, 2000 tokens, causal: 724 us on the TF32 kernel, 171 here; both 1.6e-3 from the 64-bit result, the rounding of bf16.
+inline bool attention_tc_ok(int32_t dtype, int32_t head_dim, const uint32_t* status, const void* q, const void* k,
+                            const void* v, const void* o) {
+  return dtype != TSM100_F32 && (head_dim == attn::kD || head_dim == 32 || head_dim == 64) && status != nullptr &&
+         aligned16(q) && aligned16(k) && aligned16(v) && aligned16(o);
+}
+
+template <bool kBf16, int D>
 inline int32_t attention_prefill_tc_launch(std::string* err, const tsm100_attention_prefill_desc* d, const void* q, const void* k,
                                            const void* v, void* o, uint32_t* status, cudaStream_t s) {
   namespace at = attn;
   CUtensorMap tq, tk, tv;
-  const uint64_t D = at::kD, hq = d->heads_q, hkv = d->heads_kv, kv_len = static_cast<uint64_t>(d->start_pos) + d->seq_len;
+  const uint64_t d_row = d->head_dim, hq = d->heads_q, hkv = d->heads_kv, kv_len = static_cast<uint64_t>(d->start_pos) + d->seq_len;
   // token-major Q: row pitch heads_q * D, head pitch D; caches: row pitch D, head pitch max_seq * D, kv_len rows visible
-  int32_t st = make_tmap_16bit_3d(err, &tq, q, D, d->seq_len, hq, hq * D, D, 64, at::kBQ, kBf16);
-  if (st == TSM100_OK) st = make_tmap_16bit_3d(err, &tk, k, D, kv_len, hkv, D, static_cast<uint64_t>(d->max_seq) * D, 64, at::kBKV, kBf16);
-  if (st == TSM100_OK) st = make_tmap_16bit_3d(err, &tv, v, D, kv_len, hkv, D, static_cast<uint64_t>(d->max_seq) * D, 64, at::kBKV, kBf16);
+  int32_t st = make_tmap_16bit_3d(err, &tq, q, d_row, d->seq_len, hq, hq * d_row, d_row, 64, at::kBQ, kBf16);
+  if (st == TSM100_OK) st = make_tmap_16bit_3d(err, &tk, k, d_row, kv_len, hkv, d_row, static_cast<uint64_t>(d->max_seq) * d_row, 64, at::kBKV, kBf16);
+  if (st == TSM100_OK) st = make_tmap_16bit_3d(err, &tv, v, d_row, kv_len, hkv, d_row, static_cast<uint64_t>(d->max_seq) * d_row, 64, at::kBKV, kBf16);
   if (st != TSM100_OK) return st;
   at::Params p;
   p.seq = d->seq_len;
@@ -1140,20 +1163,17 @@ inline int32_t attention_prefill_tc_launch(std::string* err, const tsm100_attent
   p.batch = 1;
   p.causal = 1;
   p.q_blocks = (d->seq_len + 2 * at::kBQ - 1) / (2 * at::kBQ);
-  p.kv_band = attention_kv_band(kv_len, d->heads_kv);
-  p.scale_log2 = static_cast<float>((1.0 / std::sqrt(static_cast<double>(D))) * 1.4426950408889634);
+  p.kv_band = attention_kv_band(kv_len, d->heads_kv, d_row);
+  p.scale_log2 = static_cast<float>((1.0 / std::sqrt(static_cast<double>(d->head_dim))) * 1.4426950408889634);
   p.status = status;
   p.seq_kv = static_cast<int32_t>(kv_len);
   p.q_offset = d->start_pos;
-  p.o_row_stride = static_cast<int64_t>(hq * D);
-  p.o_head_stride = static_cast<int64_t>(D);
+  p.o_row_stride = static_cast<int64_t>(hq * d_row);
+  p.o_head_stride = static_cast<int64_t>(d_row);
+  p.head_dim = d->head_dim;
   const int64_t grid = static_cast<int64_t>(p.q_blocks) * d->heads_q;
   if (grid > 0x7fffffff) return op_fail(err, TSM100_ERR_INVALID, "attention_prefill: too many tiles for one launch");
-  auto kern = at::attention_fwd_kernel<kBf16, true>;
-  cudaError_t e = set_dyn_smem_once(kern, at::kSmemBytes);
-  if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(attention_fwd_kernel, cache)");
-  kern<<<static_cast<unsigned>(grid), at::kThreads, at::kSmemBytes, s>>>(tq, tk, tv, static_cast<uint16_t*>(o), p);
-  return cuda_ok(err, cudaGetLastError(), "attention_fwd_kernel (prefill) launch");
+  return attention_fwd_launch<kBf16, true, D>(err, tq, tk, tv, o, p, grid, s);
 }
 
 inline int32_t attention_prefill(std::string* err, const tsm100_attention_prefill_desc* d, const void* q, const void* k,
@@ -1168,11 +1188,13 @@ inline int32_t attention_prefill(std::string* err, const tsm100_attention_prefil
   if (d->head_dim > attn_simt::kMaxD) return op_fail(err, TSM100_ERR_INVALID, "attention_prefill: head_dim > 256 unsupported");
   if (d->seq_len == 0) return TSM100_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const bool tc_ok = d->dtype != TSM100_F32 && d->head_dim == attn::kD && status != nullptr && aligned16(q) && aligned16(k) &&
-                     aligned16(v) && aligned16(o);
-  if (tc_ok) {
-    if (d->dtype == TSM100_BF16) return attention_prefill_tc_launch<true>(err, d, q, k, v, o, status, s);
-    return attention_prefill_tc_launch<false>(err, d, q, k, v, o, status, s);
+  if (attention_tc_ok(d->dtype, d->head_dim, status, q, k, v, o)) {
+    const bool wide = d->head_dim == attn::kD;
+    if (d->dtype == TSM100_BF16)
+      return wide ? attention_prefill_tc_launch<true, 128>(err, d, q, k, v, o, status, s)
+                  : attention_prefill_tc_launch<true, 64>(err, d, q, k, v, o, status, s);
+    return wide ? attention_prefill_tc_launch<false, 128>(err, d, q, k, v, o, status, s)
+                : attention_prefill_tc_launch<false, 64>(err, d, q, k, v, o, status, s);
   }
   if (d->dtype == TSM100_F32) return attention_prefill_simt_launch<float>(err, d, q, k, v, o, s);
   if (d->dtype == TSM100_BF16) return attention_prefill_simt_launch<__nv_bfloat16>(err, d, q, k, v, o, s);
@@ -1377,16 +1399,16 @@ inline int32_t attention_decode(std::string* err, const tsm100_attention_decode_
   }
 }
 
-template <bool kBf16>
+template <bool kBf16, int D>
 inline int32_t attention_tc_launch(std::string* err, const tsm100_attention_desc* d, const void* q, const void* k,
                                    const void* v, void* o, uint32_t* status, cudaStream_t s) {
   namespace at = attn;
   CUtensorMap tq, tk, tv;
-  const uint64_t S = d->seq, D = at::kD;
+  const uint64_t S = d->seq, d_row = d->head_dim;
   const uint64_t nq = static_cast<uint64_t>(d->batch) * d->heads_q, nkv = static_cast<uint64_t>(d->batch) * d->heads_kv;
-  int32_t st = make_tmap_16bit_3d(err, &tq, q, D, S, nq, D, S * D, 64, at::kBQ, kBf16);
-  if (st == TSM100_OK) st = make_tmap_16bit_3d(err, &tk, k, D, S, nkv, D, S * D, 64, at::kBKV, kBf16);
-  if (st == TSM100_OK) st = make_tmap_16bit_3d(err, &tv, v, D, S, nkv, D, S * D, 64, at::kBKV, kBf16);
+  int32_t st = make_tmap_16bit_3d(err, &tq, q, d_row, S, nq, d_row, S * d_row, 64, at::kBQ, kBf16);
+  if (st == TSM100_OK) st = make_tmap_16bit_3d(err, &tk, k, d_row, S, nkv, d_row, S * d_row, 64, at::kBKV, kBf16);
+  if (st == TSM100_OK) st = make_tmap_16bit_3d(err, &tv, v, d_row, S, nkv, d_row, S * d_row, 64, at::kBKV, kBf16);
   if (st != TSM100_OK) return st;
   at::Params p;
   p.seq = d->seq;
@@ -1395,19 +1417,16 @@ inline int32_t attention_tc_launch(std::string* err, const tsm100_attention_desc
   p.batch = d->batch;
   p.causal = d->causal ? 1 : 0;
   p.q_blocks = (d->seq + 2 * at::kBQ - 1) / (2 * at::kBQ);
-  p.kv_band = attention_kv_band(S, static_cast<int64_t>(nkv));
-  p.scale_log2 = static_cast<float>((1.0 / std::sqrt(static_cast<double>(D))) * 1.4426950408889634);
+  p.kv_band = attention_kv_band(S, static_cast<int64_t>(nkv), d_row);
+  p.scale_log2 = static_cast<float>((1.0 / std::sqrt(static_cast<double>(d->head_dim))) * 1.4426950408889634);
   p.status = status;
   p.seq_kv = d->seq;
   p.q_offset = 0;
   p.o_row_stride = p.o_head_stride = 0;
+  p.head_dim = d->head_dim;
   const int64_t grid = static_cast<int64_t>(p.q_blocks) * nq;
   if (grid > 0x7fffffff) return op_fail(err, TSM100_ERR_INVALID, "attention: too many tiles for one launch");
-  auto kern = at::attention_fwd_kernel<kBf16>;
-  cudaError_t e = set_dyn_smem_once(kern, at::kSmemBytes);
-  if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(attention_fwd_kernel)");
-  kern<<<static_cast<unsigned>(grid), at::kThreads, at::kSmemBytes, s>>>(tq, tk, tv, static_cast<uint16_t*>(o), p);
-  return cuda_ok(err, cudaGetLastError(), "attention_fwd_kernel launch");
+  return attention_fwd_launch<kBf16, false, D>(err, tq, tk, tv, o, p, grid, s);
 }
 
 inline int32_t attention(std::string* err, const tsm100_attention_desc* d, const void* q, const void* k,
@@ -1421,11 +1440,11 @@ inline int32_t attention(std::string* err, const tsm100_attention_desc* d, const
     return op_fail(err, TSM100_ERR_INVALID, "attention: heads_q must be a positive multiple of heads_kv");
   if (d->head_dim > attn_simt::kMaxD) return op_fail(err, TSM100_ERR_INVALID, "attention: head_dim > 256 unsupported");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  const bool tc_ok = d->dtype != TSM100_F32 && d->head_dim == attn::kD && status != nullptr && aligned16(q) &&
-                     aligned16(k) && aligned16(v) && aligned16(o);
-  if (tc_ok) {
-    if (d->dtype == TSM100_BF16) return attention_tc_launch<true>(err, d, q, k, v, o, status, s);
-    return attention_tc_launch<false>(err, d, q, k, v, o, status, s);
+  if (attention_tc_ok(d->dtype, d->head_dim, status, q, k, v, o)) {
+    const bool wide = d->head_dim == attn::kD;
+    if (d->dtype == TSM100_BF16)
+      return wide ? attention_tc_launch<true, 128>(err, d, q, k, v, o, status, s) : attention_tc_launch<true, 64>(err, d, q, k, v, o, status, s);
+    return wide ? attention_tc_launch<false, 128>(err, d, q, k, v, o, status, s) : attention_tc_launch<false, 64>(err, d, q, k, v, o, status, s);
   }
   if (d->dtype == TSM100_F32) return attention_simt_launch<float>(err, d, q, k, v, o, s);
   if (d->dtype == TSM100_BF16) return attention_simt_launch<__nv_bfloat16>(err, d, q, k, v, o, s);
