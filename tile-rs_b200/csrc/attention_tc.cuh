@@ -34,6 +34,9 @@
 //               or the next step's product to do.  The running max is only raised
 //               when it grows by more than 2^8 (the accumulator in TMEM is then
 //               rescaled).
+// kSplit: too few query blocks to fill the GPU (a chunk of a prompt on a long cache, a few heads): the KV steps of a query
+// block are dealt to p.splits CTAs in contiguous ranges, which leave partial (max, sum, O) in memory for
+// attention_merge_kernel.
 // Launch order keeps CTAs that share K/V (the query blocks of a head, the heads of
 // a KV group) adjacent so that K/V tiles are served from L2.
 // Roofline: tensor pipe; 4*seq^2*d flop per head (half of it when causal).
@@ -107,6 +110,11 @@ struct Params {
   int64_t o_row_stride, o_head_stride;
   int32_t head_dim;        // D = 64 form: columns of Q, K, V and O that exist (a multiple of 8)
   int32_t blocks;          // query blocks of the launch: q_blocks * heads_q * batch
+  // kSplit: CTAs per query block, and their records.  part: [block][split][D / 4][256 rows] of four columns each, so that
+  // the lanes of a warp, which hold rows, write and read contiguous memory; part_ml: [block][split][256 rows] (max, sum)
+  int32_t splits;
+  float4* part;
+  float2* part_ml;
 };
 
 template <bool kIsBf16>
@@ -154,7 +162,7 @@ __device__ __forceinline__ void block_coords(const Params& p, int block, int& bh
 // kCache = false: plain attention, Q, O [batch*heads_q][seq][128], K, V [batch*heads_kv][seq][128] (the tensor
 // maps say so).  kCache = true: causal prefill against a KV cache - the tensor maps describe token-major Q and the
 // filled part of the caches, query rows are offset by q_offset, O is written with the strides of Params.
-template <bool kIsBf16, bool kCache = false, int D = 128>
+template <bool kIsBf16, bool kCache = false, int D = 128, bool kSplit = false>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                      const __grid_constant__ CUtensorMap tmap_v, uint16_t* __restrict__ o, const Params p) {
@@ -171,16 +179,25 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   volatile uint32_t* abort_flag = &bars->abort_flag;
+  if (kSplit) ptx::launch_dependents();  // the merge kernel may be set up meanwhile
 
+  const int splits = kSplit ? p.splits : 1;
+  const int rank = kSplit ? static_cast<int>(blockIdx.x) % splits : 0;
+  const int block = kSplit ? static_cast<int>(blockIdx.x) / splits : static_cast<int>(blockIdx.x);
   int bh, kvh, qb;
-  block_coords(p, static_cast<int>(blockIdx.x), bh, kvh, qb);
+  block_coords(p, block, bh, kvh, qb);
   const int q0 = qb * 2 * kBQ;
   const int seq_kv = kCache ? p.seq_kv : p.seq;
   const int q_off = kCache ? p.q_offset : 0;
   const int n_kv_all = (seq_kv + kBKV - 1) / kBKV;
   // number of KV steps each tile needs (causal: up to and including the step of its last row's own position)
-  const int n_a = p.causal ? min(n_kv_all, (q0 + kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
-  const int n_b = p.causal ? min(n_kv_all, (q0 + 2 * kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
+  const int n_a_all = p.causal ? min(n_kv_all, (q0 + kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
+  const int n_b_all = p.causal ? min(n_kv_all, (q0 + 2 * kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
+  // kSplit: this CTA's range [j0, j0 + n_b) of them, possibly empty
+  const int per_rank = kSplit ? (n_b_all + splits - 1) / splits : n_b_all;
+  const int j0 = kSplit ? min(rank * per_rank, n_b_all) : 0;
+  const int n_b = kSplit ? min(per_rank, n_b_all - j0) : n_b_all;
+  const int n_a = kSplit ? max(0, min(n_a_all - j0, n_b)) : n_a_all;
 
   if (threadIdx.x == 0) {
     ptx::mbar_init(&bars->q_full, 1);
@@ -237,7 +254,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         const bool is_v = idx == total - 1 || (idx >= 2 && (idx & 1) == 0);
         const int step = idx == 0 ? 0 : idx == total - 1 ? n_b - 1 : is_v ? (idx >> 1) - 1 : (idx + 1) >> 1;
         const CUtensorMap* tm = is_v ? &tmap_v : &tmap_k;
-        const int row0 = step * kBKV;
+        const int row0 = (j0 + step) * kBKV;
 #pragma unroll
         for (int c = 0; c < Sh::kHalves; ++c)
           ptx::tma_load_3d(smem_kv + slot * kTileBytes + c * kHalfBytes, tm, &bars->kv_full[slot], c * 64,
@@ -387,7 +404,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         break;
       }
       ptx::tcgen05_fence_after_thread_sync();
-      const int col0 = j * kBKV;
+      const int col0 = (j0 + j) * kBKV;
       const bool masked = col0 + kBKV - 1 > limit;
 
       // the whole score row of this step, read once
@@ -537,7 +554,26 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       ptx::mbar_arrive(&bars->p_ready[g]);
     }
 
-    if (alive && n_g > 0) {
+    if constexpr (kSplit) {
+      bool have = alive && n_g > 0;  // a range may be empty for this tile: weight 0, O zero
+      if (have) have = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done[g], (n_g - 1) & 1u, abort_flag, p.status, 20 + g));
+      ptx::tcgen05_fence_after_thread_sync();
+      const int64_t rec = static_cast<int64_t>(block) * splits + rank;
+      const int row = g * kBQ + r;
+      float4* part = p.part + rec * (D / 4) * (2 * kBQ) + row;
+#pragma unroll 1
+      for (int c = 0; c < D / 32; ++c) {
+        uint32_t ov[32];
+        ptx::tmem_ld_32x32b_x32(to + c * 32, ov);
+        ptx::tmem_ld_wait();
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          part[(c * 8 + i) * (2 * kBQ)] =
+              have ? make_float4(__uint_as_float(ov[4 * i]), __uint_as_float(ov[4 * i + 1]), __uint_as_float(ov[4 * i + 2]), __uint_as_float(ov[4 * i + 3]))
+                   : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      p.part_ml[rec * (2 * kBQ) + row] = have ? make_float2(m_used, l) : make_float2(-INFINITY, 0.f);
+    } else if (alive && n_g > 0) {
       bool ready = ptx::mbar_wait(&bars->pv_done[g], (n_g - 1) & 1u, abort_flag, p.status, 20 + g);
       if (__all_sync(0xffffffffu, ready)) {
         ptx::tcgen05_fence_after_thread_sync();
@@ -577,6 +613,48 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   if (warp == 9) {
     ptx::tcgen05_fence_after_thread_sync();
     ptx::tmem_dealloc(tmem_base, kTmemCols);
+  }
+}
+
+// The records of a query block's splits, in order, into O: one CTA per (block, 16 columns), one thread per row.  Launched as
+// a programmatic dependent of the kernel above, it waits for that kernel's results itself.
+template <bool kIsBf16, bool kCache, int D>
+__global__ void __launch_bounds__(2 * kBQ)
+attention_merge_kernel(uint16_t* __restrict__ o, const Params p) {
+  constexpr int kGroups = D / 16;
+  const int block = static_cast<int>(blockIdx.x) / kGroups, c0 = static_cast<int>(blockIdx.x) % kGroups * 16;
+  int bh, kvh, qb;
+  block_coords(p, block, bh, kvh, qb);
+  const int row = threadIdx.x, qrow = qb * 2 * kBQ + row;
+  const int cols = D == 64 ? p.head_dim : D;
+  ptx::wait_prior_grid();
+  if (qrow >= p.seq || c0 >= cols) return;
+  const int64_t rec0 = static_cast<int64_t>(block) * p.splits;
+  float gm = -INFINITY;
+  for (int q = 0; q < p.splits; ++q) gm = fmaxf(gm, p.part_ml[(rec0 + q) * (2 * kBQ) + row].x);
+  float acc[16], gl = 0.f;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+  for (int q = 0; q < p.splits; ++q) {
+    const float2 ml = p.part_ml[(rec0 + q) * (2 * kBQ) + row];
+    const float w = ml.x == -INFINITY ? 0.f : ptx::ex2_approx((ml.x - gm) * p.scale_log2);
+    gl = fmaf(w, ml.y, gl);
+    const float4* part = p.part + (rec0 + q) * (D / 4) * (2 * kBQ) + (c0 / 4) * (2 * kBQ) + row;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float4 x = part[i * (2 * kBQ)];
+      acc[4 * i] = fmaf(w, x.x, acc[4 * i]), acc[4 * i + 1] = fmaf(w, x.y, acc[4 * i + 1]);
+      acc[4 * i + 2] = fmaf(w, x.z, acc[4 * i + 2]), acc[4 * i + 3] = fmaf(w, x.w, acc[4 * i + 3]);
+    }
+  }
+  const float inv = 1.0f / gl;
+  uint16_t* orow = kCache ? o + bh * p.o_head_stride + qrow * p.o_row_stride : o + (static_cast<int64_t>(bh) * p.seq + qrow) * cols;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    uint4 out;
+    out.x = pack16x2<kIsBf16>(acc[8 * h] * inv, acc[8 * h + 1] * inv), out.y = pack16x2<kIsBf16>(acc[8 * h + 2] * inv, acc[8 * h + 3] * inv);
+    out.z = pack16x2<kIsBf16>(acc[8 * h + 4] * inv, acc[8 * h + 5] * inv), out.w = pack16x2<kIsBf16>(acc[8 * h + 6] * inv, acc[8 * h + 7] * inv);
+    *reinterpret_cast<uint4*>(orow + c0 + 8 * h) = out;  // head_dim is a multiple of 16
   }
 }
 

@@ -273,6 +273,10 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// Programmatic dependent launch: a kernel launched with that attribute starts while the kernel before it in the stream still
+// runs, and waits here before it touches memory; the other call lets the next such kernel be set up from now on.
+__device__ __forceinline__ void wait_prior_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // shared::cluster address of `smem_addr` (a shared::cta address) in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t mapa_shared(uint32_t smem_addr, uint32_t rank) {
   uint32_t r;
