@@ -24,6 +24,7 @@
 
 #include "../../include/tile_sm100.h"
 #include "attention_decode.cuh"
+#include "attention_f32_tc.cuh"
 #include "attention_simt.cuh"
 #include "attention_tc.cuh"
 #include "attention_tf32x3.cuh"
@@ -1077,14 +1078,87 @@ inline int32_t attention_tf32x3_launch(std::string* err, const attn_simt::Params
   }
 }
 
+// f32 on the tcgen05 kernel: two passes write the hi / lo planes of K and of V transposed into stream-ordered scratch.
+// kv_row 0 of every (batch, KV head) is kv_head_stride elements after the one before.
+template <int D>
+inline int32_t attention_f32_tc_launch_d(std::string* err, const attn_simt::Params& p, const float* q, const float* k,
+                                         const float* v, float* o, uint32_t* status, cudaStream_t s) {
+  namespace at = attn_f32_tc;
+  namespace g = gemm_tf32_tc;
+  int sms = 0;
+  int32_t st = sm_count(err, &sms);
+  if (st != TSM100_OK) return st;
+  cudaError_t e = keep_pool_memory_once();
+  if (e != cudaSuccess) return cuda_ok(err, e, "cudaMemPoolSetAttribute");
+  const uint64_t n_kv = static_cast<uint64_t>(p.batch) * p.heads_kv, len = p.seq_kv, len4 = (len + 3) / 4 * 4;
+  const size_t k_plane = n_kv * len * D, v_plane = n_kv * len4 * D;
+  float* ws = nullptr;
+  e = cudaMallocAsync(reinterpret_cast<void**>(&ws), 2 * (k_plane + v_plane) * sizeof(float), s);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    return op_fail(err, TSM100_ERR_MEMORY, std::string("attention: scratch for the K and V planes: ") + cudaGetErrorString(e));
+  }
+  float *k_hi = ws, *k_lo = ws + k_plane, *v_hi = ws + 2 * k_plane, *v_lo = v_hi + v_plane;
+  const uint64_t items = len * (D / 4);
+  g::split_rows_kernel<true><<<dim3(static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((items + 255) / 256, 16ull * sms))), static_cast<unsigned>(n_kv)), 256, 0, s>>>(
+      k, D, p.kv_head_stride, k_hi, k_lo, static_cast<int64_t>(len), D, D);
+  g::split_transpose_kernel<<<dim3(D / 32, static_cast<unsigned>((len + 31) / 32), static_cast<unsigned>(n_kv)), 256, 0, s>>>(
+      v, D, p.kv_head_stride, v_hi, v_lo, static_cast<int32_t>(len), D, static_cast<int32_t>(len4));
+  st = cuda_ok(err, cudaGetLastError(), "attention operand split launch");
+  CUtensorMap tk_hi, tk_lo, tv_hi, tv_lo;
+  const CUtensorMapDataType f32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  if (st == TSM100_OK) st = make_tmap_3d(err, &tk_hi, k_hi, D, len, n_kv, D, len * D, 32, at::kBKV, f32, 4);
+  if (st == TSM100_OK) st = make_tmap_3d(err, &tk_lo, k_lo, D, len, n_kv, D, len * D, 32, at::kBKV, f32, 4);
+  if (st == TSM100_OK) st = make_tmap_3d(err, &tv_hi, v_hi, len, D, n_kv, len4, len4 * D, at::kBKV, D, f32, 4);
+  if (st == TSM100_OK) st = make_tmap_3d(err, &tv_lo, v_lo, len, D, n_kv, len4, len4 * D, at::kBKV, D, f32, 4);
+  if (st == TSM100_OK) {
+    auto kern = at::attention_f32_tc_kernel<D>;
+    e = set_dyn_smem_once(kern, at::smem_bytes<D>());
+    if (e == cudaSuccess) {
+      at::Params pp;
+      pp.a = p;
+      pp.status = status;
+      const int64_t grid = static_cast<int64_t>((p.seq + at::kBQ - 1) / at::kBQ) * p.batch * p.heads_q;
+      kern<<<static_cast<unsigned>(grid), at::kThreads, at::smem_bytes<D>(), s>>>(tk_hi, tk_lo, tv_hi, tv_lo, q, o, pp);
+      e = cudaGetLastError();
+    }
+    st = cuda_ok(err, e, "attention_f32_tc_kernel launch");
+  }
+  e = cudaFreeAsync(ws, s);  // stream-ordered: after the kernel that reads the planes
+  if (st == TSM100_OK && e != cudaSuccess) st = cuda_ok(err, e, "cudaFreeAsync");
+  return st;
+}
+inline int32_t attention_f32_tc_launch(std::string* err, const attn_simt::Params& p, const void* q, const void* k, const void* v,
+                                       void* o, uint32_t* status, cudaStream_t s) {
+  const float *qf = static_cast<const float*>(q), *kf = static_cast<const float*>(k), *vf = static_cast<const float*>(v);
+  float* of = static_cast<float*>(o);
+  switch (p.head_dim) {
+    case 128: return attention_f32_tc_launch_d<128>(err, p, qf, kf, vf, of, status, s);
+    case 96: return attention_f32_tc_launch_d<96>(err, p, qf, kf, vf, of, status, s);
+    case 64: return attention_f32_tc_launch_d<64>(err, p, qf, kf, vf, of, status, s);
+    default: return attention_f32_tc_launch_d<32>(err, p, qf, kf, vf, of, status, s);
+  }
+}
+// The problems that attention_tf32x3_ok takes, with enough work to pay for the split passes and a kernel's start: 16 heads of
+// 4096 x 128, causal, 1450 us on the warp-level kernel, 504 here; 4 heads of 256 x 128 44 / 30; 2 heads of 512 x 64 43 / 27.
+// Error against the 64-bit result 8.6e-6 / 9e-7 at 4096 keys (the warp-level kernel accumulates all keys in one go).
+inline bool attention_f32_tc_ok(const attn_simt::Params& p, const uint32_t* status) {
+  const int64_t blocks = static_cast<int64_t>((p.seq + 127) / 128) * p.batch * p.heads_q;
+  const int64_t n_kv = static_cast<int64_t>(p.batch) * p.heads_kv;
+  return status != nullptr && p.seq >= 64 && p.seq_kv >= 256 && blocks <= 0x7fffffff && n_kv <= 65535 && p.seq_kv <= 1 << 20;
+}
+
 template <typename T>
 inline int32_t attention_simt_launch(std::string* err, const tsm100_attention_desc* d, const void* q, const void* k,
-                                     const void* v, void* o, cudaStream_t s) {
+                                     const void* v, void* o, uint32_t* status, cudaStream_t s) {
   const int64_t sd = static_cast<int64_t>(d->seq) * d->head_dim;
   attn_simt::Params p{d->seq, d->head_dim, d->heads_q, d->heads_kv, d->batch, d->causal,
                       static_cast<float>(1.0 / std::sqrt(static_cast<double>(d->head_dim))),
                       d->seq, 0, d->head_dim, sd, sd, d->head_dim, sd};
-  if (attention_tf32x3_ok<T>(p, q, k, v, o)) return attention_tf32x3_launch<T>(err, p, q, k, v, o, s);
+  if (attention_tf32x3_ok<T>(p, q, k, v, o)) {
+    if (sizeof(T) == 4 && attention_f32_tc_ok(p, status)) return attention_f32_tc_launch(err, p, q, k, v, o, status, s);
+    return attention_tf32x3_launch<T>(err, p, q, k, v, o, s);
+  }
   const int64_t rows = static_cast<int64_t>(d->batch) * d->heads_q * d->seq;
   const int64_t grid = (rows + attn_simt::kWarps - 1) / attn_simt::kWarps;
   if (grid > 0x7fffffff) return op_fail(err, TSM100_ERR_INVALID, "attention: too many query rows for one launch");
@@ -1098,13 +1172,16 @@ inline int32_t attention_simt_launch(std::string* err, const tsm100_attention_de
 // ---------------------------------------------------------------------------
 template <typename T>
 inline int32_t attention_prefill_simt_launch(std::string* err, const tsm100_attention_prefill_desc* d, const void* q,
-                                             const void* k, const void* v, void* o, cudaStream_t s) {
+                                             const void* k, const void* v, void* o, uint32_t* status, cudaStream_t s) {
   const int64_t hd = static_cast<int64_t>(d->heads_q) * d->head_dim;
   attn_simt::Params p{d->seq_len, d->head_dim, d->heads_q, d->heads_kv, 1, 1,
                       static_cast<float>(1.0 / std::sqrt(static_cast<double>(d->head_dim))),
                       d->start_pos + d->seq_len, d->start_pos, hd, d->head_dim,
                       static_cast<int64_t>(d->max_seq) * d->head_dim, hd, d->head_dim};
-  if (attention_tf32x3_ok<T>(p, q, k, v, o)) return attention_tf32x3_launch<T>(err, p, q, k, v, o, s);
+  if (attention_tf32x3_ok<T>(p, q, k, v, o)) {
+    if (sizeof(T) == 4 && attention_f32_tc_ok(p, status)) return attention_f32_tc_launch(err, p, q, k, v, o, status, s);
+    return attention_tf32x3_launch<T>(err, p, q, k, v, o, s);
+  }
   const int64_t rows = static_cast<int64_t>(d->heads_q) * d->seq_len;
   const int64_t grid = (rows + attn_simt::kWarps - 1) / attn_simt::kWarps;
   if (grid > 0x7fffffff) return op_fail(err, TSM100_ERR_INVALID, "attention_prefill: too many query rows for one launch");
@@ -1242,9 +1319,9 @@ inline int32_t attention_prefill(std::string* err, const tsm100_attention_prefil
     return wide ? attention_prefill_tc_launch<false, 128>(err, d, q, k, v, o, status, s)
                 : attention_prefill_tc_launch<false, 64>(err, d, q, k, v, o, status, s);
   }
-  if (d->dtype == TSM100_F32) return attention_prefill_simt_launch<float>(err, d, q, k, v, o, s);
-  if (d->dtype == TSM100_BF16) return attention_prefill_simt_launch<__nv_bfloat16>(err, d, q, k, v, o, s);
-  return attention_prefill_simt_launch<__half>(err, d, q, k, v, o, s);
+  if (d->dtype == TSM100_F32) return attention_prefill_simt_launch<float>(err, d, q, k, v, o, status, s);
+  if (d->dtype == TSM100_BF16) return attention_prefill_simt_launch<__nv_bfloat16>(err, d, q, k, v, o, status, s);
+  return attention_prefill_simt_launch<__half>(err, d, q, k, v, o, status, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -1492,9 +1569,9 @@ inline int32_t attention(std::string* err, const tsm100_attention_desc* d, const
       return wide ? attention_tc_launch<true, 128>(err, d, q, k, v, o, status, s) : attention_tc_launch<true, 64>(err, d, q, k, v, o, status, s);
     return wide ? attention_tc_launch<false, 128>(err, d, q, k, v, o, status, s) : attention_tc_launch<false, 64>(err, d, q, k, v, o, status, s);
   }
-  if (d->dtype == TSM100_F32) return attention_simt_launch<float>(err, d, q, k, v, o, s);
-  if (d->dtype == TSM100_BF16) return attention_simt_launch<__nv_bfloat16>(err, d, q, k, v, o, s);
-  return attention_simt_launch<__half>(err, d, q, k, v, o, s);
+  if (d->dtype == TSM100_F32) return attention_simt_launch<float>(err, d, q, k, v, o, status, s);
+  if (d->dtype == TSM100_BF16) return attention_simt_launch<__nv_bfloat16>(err, d, q, k, v, o, status, s);
+  return attention_simt_launch<__half>(err, d, q, k, v, o, status, s);
 }
 
 }  // namespace ops
