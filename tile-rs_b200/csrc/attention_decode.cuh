@@ -99,6 +99,10 @@ struct Params {
   int32_t head_base;    // first query head of the group handled by this launch (groups wider than G run in passes)
   int32_t heads_here;   // query heads of the group handled by this launch (<= G)
   float scale_log2;     // rsqrt(d) * log2(e)
+  // partial results in memory instead of a cluster (kGlobal kernels): CTAs per (batch, KV head), their records
+  // [unit][splits][16][D + 2] (weighted V, maximum, sum)
+  int32_t splits;
+  float* part;
 };
 
 template <typename T, int DPL>
@@ -324,7 +328,10 @@ __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
   return *reinterpret_cast<uint32_t*>(&h);
 }
 
-template <typename T, int D, int STAGES, int WARPS>
+// kGlobal: the ranges of a (batch, KV head) belong to p.splits independent CTAs, more than a cluster can have, which leave
+// their records in memory for attention_decode_merge_kernel.  For a handful of caches: eight KV heads fill 64 SMs as
+// clusters of 8 (of 16 the GPU holds only seven) and 144 this way.
+template <typename T, int D, int STAGES, int WARPS, bool kGlobal = false>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_decode_mma_kernel(const T* __restrict__ q, const T* __restrict__ kc, const T* __restrict__ vc, T* __restrict__ o,
                             const Params p) {
@@ -341,7 +348,9 @@ attention_decode_mma_kernel(const T* __restrict__ q, const T* __restrict__ kc, c
   float* part = reinterpret_cast<float*>(ring);                       // warp w's record at part + w * WARP_FLOATS
   float* mine = part + kRows * REC;                                   // the CTA's merged record [16][REC], behind warp 0's
 
-  const uint32_t rank = ptx::cluster_ctarank(), splits = ptx::cluster_nctarank();
+  if (kGlobal) ptx::launch_dependents();  // the merge kernel may be set up meanwhile
+  const uint32_t splits = kGlobal ? static_cast<uint32_t>(p.splits) : ptx::cluster_nctarank();
+  const uint32_t rank = kGlobal ? blockIdx.x % splits : ptx::cluster_ctarank();
   const int unit = blockIdx.x / splits;
   const int b = unit / p.heads_kv, g = unit % p.heads_kv;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -489,7 +498,9 @@ attention_decode_mma_kernel(const T* __restrict__ q, const T* __restrict__ kc, c
     }
   }
   __syncthreads();
-  for (int i = tid; i < kRows * D; i += kThreads) {
+  float* out = kGlobal ? p.part + (static_cast<int64_t>(unit) * splits + rank) * (kRows * REC) : mine;
+  const int rows = kGlobal ? p.heads_here : kRows;
+  for (int i = tid; i < rows * D; i += kThreads) {
     const int hh = i / D, dd = i % D;
     float mm = -INFINITY;
 #pragma unroll
@@ -502,15 +513,46 @@ attention_decode_mma_kernel(const T* __restrict__ q, const T* __restrict__ kc, c
       ll = fmaf(rec[D + 1], wgt, ll);
       oo = fmaf(rec[dd], wgt, oo);
     }
-    mine[hh * REC + dd] = oo;
+    out[hh * REC + dd] = oo;
     if (dd == 0) {
-      mine[hh * REC + D] = mm;
-      mine[hh * REC + D + 1] = ll;
+      out[hh * REC + D] = mm;
+      out[hh * REC + D + 1] = ll;
     }
   }
+  if (kGlobal) return;
   ptx::cluster_sync_all();
   cluster_merge<T, kRows, D, kThreads>(mine, part, rank, splits, p.heads_here, o + (static_cast<int64_t>(b) * p.heads_q + h0) * D);
   ptx::cluster_sync_all();  // nobody leaves while its shared memory may still be read
+}
+
+// One CTA of D threads per (unit, head): the splits' records, in order, into the output.  Launched as a programmatic
+// dependent of the kernel above, it waits for that kernel's results itself.  seq_len == 0: 0 / 0 = NaN, as above.
+constexpr int kMaxGlobalSplits = 128;
+template <typename T, int D>
+__global__ void __launch_bounds__(D)
+attention_decode_merge_kernel(T* __restrict__ o, const Params p) {
+  constexpr int REC = D + 2;
+  __shared__ float m[kMaxGlobalSplits], w[kMaxGlobalSplits], l[kMaxGlobalSplits];
+  const int unit = blockIdx.x / p.heads_here, hh = blockIdx.x % p.heads_here;
+  const int b = unit / p.heads_kv, g = unit % p.heads_kv;
+  const float* rec = p.part + (static_cast<int64_t>(unit) * p.splits * kRows + hh) * REC;
+  ptx::wait_prior_grid();
+  for (int i = threadIdx.x; i < p.splits; i += D) {
+    m[i] = rec[i * (kRows * REC) + D];
+    l[i] = rec[i * (kRows * REC) + D + 1];
+  }
+  __syncthreads();
+  float mm = -INFINITY;
+  for (int i = 0; i < p.splits; ++i) mm = fmaxf(mm, m[i]);
+  for (int i = threadIdx.x; i < p.splits; i += D) w[i] = m[i] == -INFINITY ? 0.f : ptx::ex2_approx(m[i] - mm);
+  __syncthreads();
+  float ll = 0.f, oo = 0.f;
+#pragma unroll 8
+  for (int i = 0; i < p.splits; ++i) {
+    ll = fmaf(l[i], w[i], ll);
+    oo = fmaf(rec[i * (kRows * REC) + threadIdx.x], w[i], oo);
+  }
+  softmax::Elem<T>::store1(o + (static_cast<int64_t>(b) * p.heads_q + g * p.group + p.head_base + hh) * D + threadIdx.x, oo / ll);
 }
 
 }  // namespace mma
@@ -542,7 +584,7 @@ __device__ __forceinline__ void split(float x, uint32_t& hi, uint32_t& lo) {
   lo = __float_as_uint(x - __uint_as_float(hi));  // exact; the tensor core reads its top 11 bits
 }
 __device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 template <int D, int STAGES, int WARPS>

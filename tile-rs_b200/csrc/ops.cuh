@@ -1412,6 +1412,57 @@ inline int32_t attention_decode_mma_launch(std::string* err, const tsm100_attent
   return cuda_ok(err, e, "attention_decode_mma_kernel launch");
 }
 
+// 16-bit caches, a few units: `splits` independent CTAs per unit and a merge kernel (programmatic dependent launch).
+template <typename T, int D>
+inline int32_t attention_decode_global_launch(std::string* err, const tsm100_attention_decode_desc* d, const T* q, const T* k,
+                                              const T* v, T* o, int splits, cudaStream_t s) {
+  namespace ad = attn_decode;
+  constexpr int WARPS = 8, STAGES = 3;
+  const int64_t units = static_cast<int64_t>(d->batch) * d->heads_kv;
+  cudaError_t e = keep_pool_memory_once();
+  if (e != cudaSuccess) return cuda_ok(err, e, "cudaMemPoolSetAttribute");
+  float* ws = nullptr;
+  e = cudaMallocAsync(reinterpret_cast<void**>(&ws), static_cast<size_t>(units) * splits * ad::mma::kRows * (D + 2) * sizeof(float), s);
+  if (e != cudaSuccess) {
+    (void)cudaGetLastError();
+    return op_fail(err, TSM100_ERR_MEMORY, std::string("attention_decode: scratch: ") + cudaGetErrorString(e));
+  }
+  ad::Params p;
+  p.batch = d->batch;
+  p.heads_q = d->heads_q;
+  p.heads_kv = d->heads_kv;
+  p.seq_len = d->seq_len;
+  p.max_seq = d->max_seq;
+  p.group = d->heads_q / d->heads_kv;
+  p.scale_log2 = static_cast<float>((1.0 / std::sqrt(static_cast<double>(D))) * 1.4426950408889634);
+  p.splits = splits;
+  p.part = ws;
+  auto kern = ad::mma::attention_decode_mma_kernel<T, D, STAGES, WARPS, true>;
+  constexpr int smem = ad::mma::smem_bytes<D, STAGES, WARPS>();
+  e = set_dyn_smem_once(kern, smem);
+  for (int base = 0; base < p.group && e == cudaSuccess; base += ad::mma::kRows) {
+    p.head_base = base;
+    p.heads_here = std::min(ad::mma::kRows, p.group - base);
+    kern<<<static_cast<unsigned>(units * splits), WARPS * 32, smem, s>>>(q, k, v, o, p);
+    e = cudaGetLastError();
+    if (e != cudaSuccess) break;
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.blockDim = dim3(D);
+    cfg.stream = s;
+    cfg.gridDim = dim3(static_cast<unsigned>(units * p.heads_here));
+    e = cudaLaunchKernelEx(&cfg, ad::mma::attention_decode_merge_kernel<T, D>, o, p);
+  }
+  int32_t st = cuda_ok(err, e, "attention_decode_mma_kernel (partial results) launch");
+  e = cudaFreeAsync(ws, s);
+  if (st == TSM100_OK && e != cudaSuccess) st = cuda_ok(err, e, "cudaFreeAsync");
+  return st;
+}
+
 // How many clusters of `size` CTAs of the eight-warp decode kernel the GPU holds at once (asked once per
 // kernel, size and device; 0 if such clusters cannot be placed at all).
 template <typename T, int D>
@@ -1476,6 +1527,14 @@ inline int32_t attention_decode_typed(std::string* err, const tsm100_attention_d
     if (splits == attn_decode::kMaxSplits && d->seq_len / (2 * attn_decode::kMaxSplitsWide) >= 256 &&
         units <= decode_lone_clusters<T, D>(attn_decode::kMaxSplitsWide))
       splits = attn_decode::kMaxSplitsWide;
+    // so few units that clusters leave a third of the SMs or more idle: one CTA per SM with 512 positions or more each,
+    // merged by a second kernel.  Eight KV heads: 35.2 us as clusters, 30.2 this way at 32768 positions, 15.3 / 11.0 at 8192;
+    // one KV head, 32768 positions 22.6 / 13.4.
+    if constexpr (sizeof(T) == 2) {
+      const int64_t wide = std::min<int64_t>({attn_decode::mma::kMaxGlobalSplits, sms / std::max<int64_t>(units, 1), d->seq_len / 512});
+      if (wide * 2 >= 3 * splits && wide > 1)
+        return attention_decode_global_launch<T, D>(err, d, qp, kp, vp, op, static_cast<int>(wide), s);
+    }
     // every CTA alone on its SM from start to end: eight warps and a deeper ring, so that it hides its own latencies
     const bool lone = units * splits <= sms && (splits < attn_decode::kMaxSplits || units <= decode_lone_clusters<T, D>(splits));
     for (int base = 0; base < group && st == TSM100_OK; base += 16)
