@@ -4,9 +4,9 @@
 // instantiate the same kernels with the same dispatch.
 //
 // Every function returns a TSM100_* status and, on failure, writes a message
-// to *err.  Nothing here synchronises; the one operator that needs device scratch (the
-// tcgen05 f32 GEMM: the hi / lo planes of its operands) takes it from, and returns it to,
-// the device's stream-ordered memory pool on the caller's stream.
+// to *err.  Nothing here synchronises; the operators that need device scratch (operand
+// planes of the tcgen05 f32 kernels, padded copies, partial results) take it from, and
+// return it to, the device's stream-ordered memory pool on the caller's stream.
 #pragma once
 
 #include <cuda.h>
@@ -248,6 +248,24 @@ inline cudaError_t launch_softmax_warp(const T* x, T* y, int64_t rows, int32_t c
   return cudaGetLastError();
 }
 
+// As many CTAs per row as its vectors need, one cluster per row.
+template <typename T, int VPT, int THREADS>
+inline int32_t softmax_cluster_launch(std::string* err, const T* x, T* y, int64_t rows, int64_t cols, int64_t ctas, cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(ctas);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cfg.blockDim = dim3(THREADS);
+  cfg.stream = s;
+  cfg.gridDim = dim3(static_cast<unsigned>(rows * ctas));
+  return cuda_ok(err, cudaLaunchKernelEx(&cfg, softmax::softmax_rows_cluster<T, VPT, THREADS>, x, y, rows, static_cast<int32_t>(cols)),
+                 "softmax_rows_cluster launch");
+}
+
 template <typename T>
 inline int32_t softmax_typed(std::string* err, const T* x, T* y, int64_t rows, int64_t cols, cudaStream_t s) {
   constexpr int PV = softmax::Elem<T>::kPerVec;
@@ -281,17 +299,46 @@ inline int32_t softmax_typed(std::string* err, const T* x, T* y, int64_t rows, i
   int sms = 0;
   int32_t st = sm_count(err, &sms);
   if (st != TSM100_OK) return st;
-  constexpr int64_t kMaxBlockCols = 56 * 1024;  // 224 KiB of f32 in shared memory
-  if (vec_ok && cols <= kMaxBlockCols) {
-    constexpr int THREADS = 512;
-    const size_t smem = static_cast<size_t>(cols) * sizeof(float);
-    auto kern = softmax::softmax_rows_block<T, THREADS>;
-    e = set_dyn_smem_once(kern, static_cast<int>(kMaxBlockCols * sizeof(float)));  // the most this path ever asks for
-    if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(softmax_rows_block)");
-    const int per_sm = static_cast<int>(std::max<size_t>(1, std::min<size_t>(4, (220 * 1024) / (smem + 1024))));
-    const unsigned grid = static_cast<unsigned>(std::min<int64_t>(rows, static_cast<int64_t>(sms) * per_sm));
-    kern<<<grid, THREADS, smem, s>>>(x, y, rows, static_cast<int32_t>(cols));
-    return cuda_ok(err, cudaGetLastError(), "softmax_rows_block launch");
+  // Rows that start anywhere, or too wide for one CTA's registers.  x and y must lie at the same offset from a 16-byte
+  // boundary, in every row alike (their row pitch is the same), a whole number of elements away from it.
+  const uintptr_t xa = reinterpret_cast<uintptr_t>(x), ya = reinterpret_cast<uintptr_t>(y);
+  const int64_t span = (cols + 2 * PV - 2) / PV;  // the most 16-byte vectors a row can touch
+  if (((xa ^ ya) & 15u) == 0 && xa % sizeof(T) == 0 && cols <= 1 << 30) {
+    const int32_t c = static_cast<int32_t>(cols);
+    if (span <= 32 * 8 && rows <= 4ll * 0x7fffffff) {
+      constexpr int WARPS = 4;
+      const unsigned grid = static_cast<unsigned>((rows + WARPS - 1) / WARPS);
+      if (span <= 32 * 2) softmax::softmax_rows_warp_any<T, 2, WARPS><<<grid, WARPS * 32, 0, s>>>(x, y, rows, c);
+      else if (span <= 32 * 4) softmax::softmax_rows_warp_any<T, 4, WARPS><<<grid, WARPS * 32, 0, s>>>(x, y, rows, c);
+      else softmax::softmax_rows_warp_any<T, 8, WARPS><<<grid, WARPS * 32, 0, s>>>(x, y, rows, c);
+      return cuda_ok(err, cudaGetLastError(), "softmax_rows_warp_any launch");
+    }
+    // up to 1024 vectors a row stays in registers: 8000 rows of 3501 bf16 78 us scalar, 66 read twice, 27 here; 3000 of 1111
+    // f32 17 / 23 / 8.5; 4000 of 8001 bf16 70 / 32 / 29
+    if (span <= 256 * 4) {
+      auto launch = [&](auto kern, int threads) {
+        kern<<<static_cast<unsigned>(std::min<int64_t>(rows, static_cast<int64_t>(sms) * blocks_per_sm(kern, threads))), threads, 0, s>>>(x, y, rows, c);
+      };
+      if (span <= 128 * 4) launch(softmax::softmax_rows_cta_any<T, 4, 128>, 128);
+      else launch(softmax::softmax_rows_cta_any<T, 4, 256>, 256);
+      return cuda_ok(err, cudaGetLastError(), "softmax_rows_cta_any launch");
+    }
+    // a row per SM or fewer (141 rows of 54588 f16: 21 us with a CTA per row, 11.5): a cluster per row, CTAs of 256 threads and 4 vectors each while eight of them hold a row
+    if (span <= 8 * 512 * 8 && rows <= sms) {
+      const int64_t ctas = (span + 1023) / 1024;
+      if (ctas <= 8) return softmax_cluster_launch<T, 4, 256>(err, x, y, rows, cols, ctas, s);
+      return softmax_cluster_launch<T, 8, 512>(err, x, y, rows, cols, (span + 4095) / 4096, s);
+    }
+    // one CTA per row, 1024 threads per SM in 4, 2 or 1 CTAs: as many as keep their rows within half of the L2 (126 MB).  1000
+    // rows of 50001 bf16: 97 us scalar, 49 here; 1212 of 97648 f32 286 / 214; 2000 of 16392 bf16 (in shared memory) 45 / 31
+    const int64_t fit = (64ll << 20) / (cols * static_cast<int64_t>(sizeof(T)) * sms);
+    auto launch = [&](auto kern, int threads) {
+      kern<<<static_cast<unsigned>(std::min<int64_t>(rows, sms * (1024ll / threads))), threads, 0, s>>>(x, y, rows, c);
+    };
+    if (fit >= 4) launch(softmax::softmax_rows_twice<T, 256>, 256);
+    else if (fit >= 2) launch(softmax::softmax_rows_twice<T, 512>, 512);
+    else launch(softmax::softmax_rows_twice<T, 1024>, 1024);
+    return cuda_ok(err, cudaGetLastError(), "softmax_rows_twice launch");
   }
   constexpr int THREADS = 512;
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>(rows, static_cast<int64_t>(sms) * 4));
