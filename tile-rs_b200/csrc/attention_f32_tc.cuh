@@ -9,20 +9,21 @@
 // see K-major operands only.  Then one CTA owns 128 query rows of one head and walks the keys in steps of 32:
 //   warp 8       TMA producer: K_0, K_1, V_0, K_2, V_1, ... (hi and lo together, 256 * D bytes a unit) through a 3-deep
 //                ring.  No multicast.
-//   warp 9       S = Q K^T: hi / lo tiles of Q stay in shared memory for the CTA's life (128 * D * 8 bytes).
+//   warp 9       S = Q K^T: the hi tile of Q stays in tensor memory for the CTA's life, the lo tile in shared memory.  A
+//                128 x 32 x 8 product reads 4 KiB of A against 1 KiB of B; from shared memory that takes 40 cycles, 16 of which
+//                the tensor core needs, so two of the three products take A from tensor memory.
 //   warp 10      O += P V: P_hi, P_lo are read from tensor memory.
 //   warps 0..3   softmax, one thread per query row; the running maximum is raised freely where a chunk of O begins and
 //                otherwise only when it grows by more than 2^8 (the chunk in tensor memory is then rescaled).
 //   warps 4..7   drain: the tensor core rounds its accumulator toward zero, so O is accumulated over kChunkSteps steps
 //                (128 keys) from zero and then added, round to nearest, to running sums in registers (D per thread).
-// S, P and the chunk of O are double-buffered (tensor memory: 2 * 128 + 2 * 32 + 4 * 32 of 512 columns at D = 128), so
-// that the products of one step run during the softmax of the next.
+// S and the chunk of O are double-buffered, so that the products of one step run during the softmax of the next; P is not
+// (tensor memory at D = 128: 2 * 128 of O, 2 * 32 of S, 32 + 32 of P, 128 of Q: all 512 columns).
 // Bound: tensor pipe at the TF32 rate / 3; shared-memory reads of Q by the 32-wide S products come close behind.  16 heads of
-// 4096 x 128: 137 TFLOP/s (half of a third of the TF32 rate), 48 on the warp-level kernel.
+// 4096 x 128: 170 TFLOP/s (0.63 of a third of the TF32 rate; 137 with both parts of Q in shared memory), 48 on the warp-level kernel.
 #pragma once
 
 #include "attention_simt.cuh"  // Params
-#include "attention_tc.cuh"    // kRegsOther
 #include "gemm_tf32_tc.cuh"    // split passes, tf32_rn, descriptors
 #include "ptx.cuh"
 
@@ -35,11 +36,11 @@ constexpr int kBQ = 128;           // query rows per CTA
 constexpr int kBKV = 32;           // keys per step: one 128-byte swizzle row of f32
 constexpr int kChunkSteps = 4;     // steps per accumulation chunk of O
 constexpr int kThreads = 384;
-constexpr int kRing = 3;
+constexpr int kRing = 5;
 constexpr int kRegsOther = 56, kRegsSoftmax = 168, kRegsDrain = 224;
 static_assert(128 * (kRegsOther + kRegsSoftmax + kRegsDrain) <= kThreads * 168, "setmaxnreg draws on the launch's registers");
 constexpr int kTmemCols = 512;
-constexpr int kTmemO = 0, kTmemS = 256, kTmemP = 320;  // two accumulators of 128, two of 32, two of (32 hi + 32 lo)
+constexpr int kTmemO = 0, kTmemS = 256, kTmemP = 320, kTmemQ = 384;  // two accumulators of 128, two of 32, 32 hi + 32 lo, 128
 constexpr float kRescaleThreshold = 8.0f;              // log2 units
 
 template <int D>
@@ -47,7 +48,7 @@ struct Shape {
   static constexpr int kQPlane = kBQ * D * 4;           // D / 32 groups of 128 rows x 128 bytes
   static constexpr int kUnitPlane = kBKV * D * 4;       // K: D / 32 groups of 32 rows x 128 bytes; V: D rows x 128 bytes
   static constexpr int kUnitBytes = 2 * kUnitPlane;     // hi, lo
-  static constexpr int kRingOff = 2 * kQPlane;
+  static constexpr int kRingOff = kQPlane;              // behind the lo tile of Q
   static constexpr int kRowsOff = kRingOff + kRing * kUnitBytes;  // float [3][128]: per chunk, the maximum it is scaled by
   static constexpr int kBarsOff = kRowsOff + 3 * kBQ * 4;
 };
@@ -55,7 +56,7 @@ struct alignas(8) Barriers {
   uint64_t q_ready;
   uint64_t kv_full[kRing], kv_empty[kRing];
   uint64_t s_full[2], s_free[2];
-  uint64_t p_ready[2], pv_done[2];
+  uint64_t p_ready, pv_done;
   uint64_t o_full[2], o_empty[2];
   uint64_t m_ready[3];   // the maximum of a chunk is in its row slot; the last one used after the last chunk: the row sums are
   uint64_t l_ready;
@@ -113,7 +114,9 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
   const int chunks = (n + kChunkSteps - 1) / kChunkSteps;
 
   if (threadIdx.x == 0) {
-    ptx::mbar_init(&bars->q_ready, 256);
+    ptx::mbar_init(&bars->q_ready, 128);
+    ptx::mbar_init(&bars->p_ready, 128);
+    ptx::mbar_init(&bars->pv_done, 1);
     for (int s = 0; s < kRing; ++s) {
       ptx::mbar_init(&bars->kv_full[s], 1);
       ptx::mbar_init(&bars->kv_empty[s], 1);
@@ -121,8 +124,6 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(&bars->s_full[i], 1);
       ptx::mbar_init(&bars->s_free[i], 128);
-      ptx::mbar_init(&bars->p_ready[i], 128);
-      ptx::mbar_init(&bars->pv_done[i], 1);
       ptx::mbar_init(&bars->o_full[i], 1);
       ptx::mbar_init(&bars->o_empty[i], 128);
     }
@@ -144,21 +145,29 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
   auto k_pos = [&](int j) { return j == 0 ? 0 : 2 * j - 1; };
   auto v_pos = [&](int j) { return j == n - 1 ? 2 * n - 1 : 2 * j + 2; };
 
-  // Q, split, into the swizzled K-major tiles (warps 0..7; 16-byte unit u of row r at position u ^ (r & 7) of its group)
-  if (warp < 8) {
-    constexpr int kUnits = D / 4;  // 16-byte units per row
-    const float* qh = q + bh * p.q_head_stride;
-    const uint32_t base = ptx::smem_u32(smem);
-    for (int i = threadIdx.x; i < kBQ * kUnits; i += 256) {
-      const int r = i / kUnits, u = i % kUnits;
-      float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (q0 + r < p.seq) x = *reinterpret_cast<const float4*>(qh + (q0 + r) * p.q_row_stride + u * 4);
-      const float4 h = make_float4(tf32_rn(x.x), tf32_rn(x.y), tf32_rn(x.z), tf32_rn(x.w));
-      const uint32_t at = base + (u >> 3) * (kBQ * 128) + r * 128 + (((u & 7) ^ (r & 7)) << 4);
-      ptx::st_shared_v4(at, __float_as_uint(h.x), __float_as_uint(h.y), __float_as_uint(h.z), __float_as_uint(h.w));
-      ptx::st_shared_v4(at + Sh::kQPlane, __float_as_uint(tf32_rn(x.x - h.x)), __float_as_uint(tf32_rn(x.y - h.y)),
-                        __float_as_uint(tf32_rn(x.z - h.z)), __float_as_uint(tf32_rn(x.w - h.w)));
+  // Q, split (warps 0..3, one row each): hi to tensor memory, lo to the swizzled K-major tile in shared memory (16-byte unit u
+  // of row r at position u ^ (r & 7) of its group of 32 columns)
+  if (warp < 4) {
+    const int r = warp * 32 + lane;
+    const bool valid = q0 + r < p.seq;
+    const float4* qr = reinterpret_cast<const float4*>(q + bh * p.q_head_stride + (q0 + r) * p.q_row_stride);
+    const uint32_t base = ptx::smem_u32(smem) + r * 128;
+#pragma unroll
+    for (int c = 0; c < D / 32; ++c) {
+      uint32_t hi[32];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const float4 x = valid ? qr[c * 8 + u] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 h = make_float4(tf32_rn(x.x), tf32_rn(x.y), tf32_rn(x.z), tf32_rn(x.w));
+        hi[4 * u] = __float_as_uint(h.x), hi[4 * u + 1] = __float_as_uint(h.y), hi[4 * u + 2] = __float_as_uint(h.z), hi[4 * u + 3] = __float_as_uint(h.w);
+        ptx::st_shared_v4(base + c * (kBQ * 128) + ((u ^ (r & 7)) << 4), __float_as_uint(tf32_rn(x.x - h.x)), __float_as_uint(tf32_rn(x.y - h.y)),
+                          __float_as_uint(tf32_rn(x.z - h.z)), __float_as_uint(tf32_rn(x.w - h.w)));
+      }
+      __syncwarp();
+      ptx::tmem_st_32x32b_x32(tmem + (static_cast<uint32_t>(warp * 32) << 16) + kTmemQ + c * 32, hi);
     }
+    ptx::tmem_st_wait();
+    ptx::tcgen05_fence_before_thread_sync();
     ptx::fence_proxy_async_smem();
     ptx::mbar_arrive(&bars->q_ready);
   }
@@ -203,6 +212,7 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
       constexpr uint32_t idesc = gemm_tf32_tc::make_idesc_tf32(kBQ, kBKV);
       const uint32_t q_lo32 = k_lo32 | (ptx::smem_u32(smem) >> 4);
       ok = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->q_ready, 0, abort_flag, status, 33));
+      ptx::tcgen05_fence_after_thread_sync();
       volatile uint32_t* pv_steps = &bars->pv_steps;
       for (int j = 0; j < n && ok; ++j) {
         // not before the P V of step j - 2 is queued: the tensor core would take this product first
@@ -218,13 +228,13 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
 #pragma unroll
           for (int kk = 0; kk < D / 8; ++kk) {
             const uint32_t a_off = (kk >> 2) * ((kBQ * 128) >> 4) + (kk & 3) * 2, b_off = (kk >> 2) * ((kBKV * 128) >> 4) + (kk & 3) * 2;
-            gemm_tf32_tc::tcgen05_mma_tf32_ss(d, desc(q_lo32 + (Sh::kQPlane >> 4) + a_off), desc(b_hi + b_off), idesc, kk != 0 ? 1u : 0u);
-            gemm_tf32_tc::tcgen05_mma_tf32_ss(d, desc(q_lo32 + a_off), desc(b_lo + b_off), idesc, 1u);
+            gemm_tf32_tc::tcgen05_mma_tf32_ss(d, desc(q_lo32 + a_off), desc(b_hi + b_off), idesc, kk != 0 ? 1u : 0u);
+            mma_tf32_ts(d, tmem + kTmemQ + kk * 8, desc(b_lo + b_off), idesc, 1u);
           }
 #pragma unroll
           for (int kk = 0; kk < D / 8; ++kk) {
-            const uint32_t a_off = (kk >> 2) * ((kBQ * 128) >> 4) + (kk & 3) * 2, b_off = (kk >> 2) * ((kBKV * 128) >> 4) + (kk & 3) * 2;
-            gemm_tf32_tc::tcgen05_mma_tf32_ss(d, desc(q_lo32 + a_off), desc(b_hi + b_off), idesc, 1u);
+            const uint32_t b_off = (kk >> 2) * ((kBKV * 128) >> 4) + (kk & 3) * 2;
+            mma_tf32_ts(d, tmem + kTmemQ + kk * 8, desc(b_hi + b_off), idesc, 1u);
           }
           ptx::tcgen05_commit(&bars->s_full[j & 1]);
           ptx::tcgen05_commit(&bars->kv_empty[k_pos(j) % kRing]);
@@ -238,10 +248,10 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
         const bool first = j % kChunkSteps == 0, last = j % kChunkSteps == kChunkSteps - 1 || j == n - 1;
         if (!(ok = wait_kv(v_pos(j)))) break;
         if (first && c >= 2 && !(ok = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&bars->o_empty[acc], ((c - 2) >> 1) & 1u, abort_flag, status, 36)))) break;
-        if (!(ok = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->p_ready[j & 1], (j >> 1) & 1u, abort_flag, status, 37)))) break;
+        if (!(ok = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->p_ready, j & 1u, abort_flag, status, 37)))) break;
         ptx::tcgen05_fence_after_thread_sync();
         const uint32_t d = tmem + kTmemO + acc * 128;
-        const uint32_t a_hi = tmem + kTmemP + (j & 1) * (2 * kBKV), a_lo = a_hi + kBKV;
+        const uint32_t a_hi = tmem + kTmemP, a_lo = a_hi + kBKV;
         const uint32_t b_hi = ring_lo + (v_pos(j) % kRing) * (Sh::kUnitBytes >> 4), b_lo = b_hi + (Sh::kUnitPlane >> 4);
         if (ptx::elect_one_sync()) {
 #pragma unroll
@@ -250,7 +260,7 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
             mma_tf32_ts(d, a_hi + kk * 8, desc(b_lo + kk * 2), idesc, 1u);
             mma_tf32_ts(d, a_hi + kk * 8, desc(b_hi + kk * 2), idesc, 1u);
           }
-          ptx::tcgen05_commit(&bars->pv_done[j & 1]);
+          ptx::tcgen05_commit(&bars->pv_done);
           ptx::tcgen05_commit(&bars->kv_empty[v_pos(j) % kRing]);
           if (last) ptx::tcgen05_commit(&bars->o_full[acc]);
           *const_cast<volatile uint32_t*>(&bars->pv_steps) = static_cast<uint32_t>(j + 1);
@@ -301,7 +311,7 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
           m_used = m_new;
         }
       } else if (__any_sync(0xffffffffu, (m_new - m_used) * sl2 > kRescaleThreshold)) {
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done[b ^ 1], ((j - 1) >> 1) & 1u, abort_flag, status, 39))) {
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done, (j - 1) & 1u, abort_flag, status, 39))) {
           alive = false;
           break;
         }
@@ -336,21 +346,21 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
         lo[i] = __float_as_uint(e - h);  // exact; the tensor core reads its top 11 bits
       }
       l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
-      // P of step j - 2 has been read
-      if (j >= 2 && !__all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done[b], ((j - 2) >> 1) & 1u, abort_flag, status, 40))) {
+      // P of step j - 1 has been read
+      if (j >= 1 && !__all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done, (j - 1) & 1u, abort_flag, status, 40))) {
         alive = false;
         break;
       }
       __syncwarp();
       ptx::tcgen05_fence_after_thread_sync();
-      const uint32_t tp = lane_base + kTmemP + b * (2 * kBKV);
+      const uint32_t tp = lane_base + kTmemP;
       ptx::tmem_st_32x32b_x32(tp, hi);
       ptx::tmem_st_32x32b_x32(tp + kBKV, lo);
       ptx::tmem_st_wait();
       ptx::tcgen05_fence_before_thread_sync();
-      ptx::mbar_arrive(&bars->p_ready[b]);
+      ptx::mbar_arrive(&bars->p_ready);
       if (j % kChunkSteps == kChunkSteps - 1 || j == n - 1) {
-        // slot c % 3: the wait above says that P V of step j - 2 was issued, which (accumulators alternate) says that
+        // slot c % 3: the wait above says that P V of step j - 1 was issued, which (accumulators alternate) says that
         // the drain warps are done with chunk c - 3
         const int c3 = (j / kChunkSteps) % 3;
         row_slot[c3 * kBQ + r] = m_used;
@@ -359,7 +369,7 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
     }
     // the row sum takes the slot after the last chunk's, once the last product has retired: by then the chunk that had it
     // (chunks - 3) is drained
-    if (alive && __all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done[(n - 1) & 1], ((n - 1) >> 1) & 1u, abort_flag, status, 41))) {
+    if (alive && __all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done, (n - 1) & 1u, abort_flag, status, 41))) {
       row_slot[(chunks % 3) * kBQ + r] = l;
       ptx::mbar_arrive(&bars->l_ready);
     }

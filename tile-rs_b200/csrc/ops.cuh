@@ -1187,7 +1187,7 @@ inline int32_t attention_f32_tc_launch(std::string* err, const attn_simt::Params
   }
 }
 // The problems that attention_tf32x3_ok takes, with enough work to pay for the split passes and a kernel's start: 16 heads of
-// 4096 x 128, causal, 1450 us on the warp-level kernel, 504 here; 4 heads of 256 x 128 44 / 30; 2 heads of 512 x 64 43 / 27.
+// 4096 x 128, causal, 1446 us on the warp-level kernel, 406 here; 4 heads of 256 x 128 44 / 30; 2 heads of 512 x 64 43 / 27.
 // Error against the 64-bit result 8.6e-6 / 9e-7 at 4096 keys (the warp-level kernel accumulates all keys in one go).
 inline bool attention_f32_tc_ok(const attn_simt::Params& p, const uint32_t* status) {
   const int64_t blocks = static_cast<int64_t>((p.seq + 127) / 128) * p.batch * p.heads_q;
