@@ -78,66 +78,85 @@ __device__ __forceinline__ float tf32_rn(float x) {
 // ---------------------------------------------------------------------------
 // the split pass
 // ---------------------------------------------------------------------------
-// src [rows][cols] with row pitch ld -> hi, lo [rows][cols] with row pitch kp, a multiple of 4 >= cols, so that every
+// One launch splits both operands (two launches cost a ramp and a tail more).
+// rows: src [rows][cols] with row pitch ld -> hi, lo [rows][cols] with row pitch kp, a multiple of 4 >= cols, so that every
 // plane row starts on a 16-byte boundary whatever cols is (the columns from cols to kp are never read: the tensor maps
 // end at cols).  One thread per four values; kVec: rows of src start on 16-byte boundaries and cols % 4 == 0, else the
-// four values are loaded one by one.  blockIdx.y = problem of the batch.
+// four values are loaded one by one.
+// transposed: src [cols][rows] with row pitch ld -> the same planes, 32 x 32 tiles through shared memory.
+struct SplitOperand {
+  const float* src;
+  float *hi, *lo;
+  int64_t ld, batch_stride;   // of src, in elements
+  int64_t rows;
+  int32_t cols, kp;
+  int32_t blocks;             // blocks of the launch that work on it
+};
+
 template <bool kVec>
-__global__ void __launch_bounds__(256)
-split_rows_kernel(const float* __restrict__ src, int64_t ld, int64_t src_batch_stride, float* __restrict__ hi,
-                  float* __restrict__ lo, int64_t rows, int32_t cols, int32_t kp) {
-  const int64_t vec_per_row = kp >> 2;
-  const int64_t total = rows * vec_per_row;
-  const float* s = src + blockIdx.y * src_batch_stride;
-  float* h = hi + blockIdx.y * rows * kp;
-  float* l = lo + blockIdx.y * rows * kp;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+__device__ __forceinline__ void split_rows(const SplitOperand& p, int block, int batch) {
+  const int64_t vec_per_row = p.kp >> 2;
+  const int64_t total = p.rows * vec_per_row;
+  const float* s = p.src + batch * p.batch_stride;
+  float* h = p.hi + batch * p.rows * p.kp;
+  float* l = p.lo + batch * p.rows * p.kp;
+  for (int64_t i = block * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total; i += static_cast<int64_t>(p.blocks) * blockDim.x) {
     const int64_t r = i / vec_per_row, c4 = (i - r * vec_per_row) << 2;
     float4 x;
     if (kVec) {
-      x = *reinterpret_cast<const float4*>(s + r * ld + c4);
+      x = *reinterpret_cast<const float4*>(s + r * p.ld + c4);
     } else {
-      const float* q = s + r * ld + c4;
+      const float* q = s + r * p.ld + c4;
       x.x = q[0];  // c4 < cols, because kp - cols < 4
-      x.y = c4 + 1 < cols ? q[1] : 0.f;
-      x.z = c4 + 2 < cols ? q[2] : 0.f;
-      x.w = c4 + 3 < cols ? q[3] : 0.f;
+      x.y = c4 + 1 < p.cols ? q[1] : 0.f;
+      x.z = c4 + 2 < p.cols ? q[2] : 0.f;
+      x.w = c4 + 3 < p.cols ? q[3] : 0.f;
     }
     float4 a, b;
     a.x = tf32_rn(x.x), a.y = tf32_rn(x.y), a.z = tf32_rn(x.z), a.w = tf32_rn(x.w);
     b.x = tf32_rn(x.x - a.x), b.y = tf32_rn(x.y - a.y), b.z = tf32_rn(x.z - a.z), b.w = tf32_rn(x.w - a.w);
-    *reinterpret_cast<float4*>(h + r * kp + c4) = a;
-    *reinterpret_cast<float4*>(l + r * kp + c4) = b;
+    *reinterpret_cast<float4*>(h + r * p.kp + c4) = a;
+    *reinterpret_cast<float4*>(l + r * p.kp + c4) = b;
   }
 }
 
-// src [K][N] with row pitch ld -> hi, lo [N][K] with row pitch kp (transposed), 32 x 32 tiles through shared memory.
-// grid (ceil(N/32), ceil(K/32), batch), 256 threads (32 x 8).
-__global__ void __launch_bounds__(256)
-split_transpose_kernel(const float* __restrict__ src, int64_t ld, int64_t src_batch_stride, float* __restrict__ hi,
-                       float* __restrict__ lo, int32_t k, int32_t n, int32_t kp) {
-  __shared__ float tile[32][33];
-  const float* s = src + blockIdx.z * src_batch_stride;
-  float* h = hi + static_cast<int64_t>(blockIdx.z) * n * kp;
-  float* l = lo + static_cast<int64_t>(blockIdx.z) * n * kp;
-  const int n0 = blockIdx.x * 32, k0 = blockIdx.y * 32;
+// One 32 x 32 tile per block, 256 threads (32 x 8).
+__device__ __forceinline__ void split_transposed(const SplitOperand& p, int block, int batch, float (&tile)[32][33]) {
+  const float* s = p.src + batch * p.batch_stride;
+  float* h = p.hi + batch * p.rows * p.kp;
+  float* l = p.lo + batch * p.rows * p.kp;
+  const int row_tiles = static_cast<int>((p.rows + 31) / 32);
+  const int n0 = block % row_tiles * 32, k0 = block / row_tiles * 32;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int kk = k0 + ty + 8 * j, nn = n0 + tx;
-    tile[ty + 8 * j][tx] = (kk < k && nn < n) ? s[static_cast<int64_t>(kk) * ld + nn] : 0.f;
+    tile[ty + 8 * j][tx] = (kk < p.cols && nn < p.rows) ? s[static_cast<int64_t>(kk) * p.ld + nn] : 0.f;
   }
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     const int nn = n0 + ty + 8 * j, kk = k0 + tx;
-    if (nn < n && kk < k) {
+    if (nn < p.rows && kk < p.cols) {
       const float x = tile[tx][ty + 8 * j];
       const float a = tf32_rn(x);
-      h[static_cast<int64_t>(nn) * kp + kk] = a;
-      l[static_cast<int64_t>(nn) * kp + kk] = tf32_rn(x - a);
+      h[static_cast<int64_t>(nn) * p.kp + kk] = a;
+      l[static_cast<int64_t>(nn) * p.kp + kk] = tf32_rn(x - a);
     }
+  }
+}
+
+// grid (a.blocks + b.blocks, batch); the blocks of the transposed operand come first.
+template <bool kVec, bool kTransposeB>
+__global__ void __launch_bounds__(256)
+split_operands_kernel(const SplitOperand a, const SplitOperand b) {
+  __shared__ float tile[kTransposeB ? 32 : 1][33];
+  const int block = static_cast<int>(blockIdx.x);
+  if (block < b.blocks) {
+    if constexpr (kTransposeB) split_transposed(b, block, blockIdx.y, tile);
+    else split_rows<kVec>(b, block, blockIdx.y);
+  } else {
+    split_rows<kVec>(a, block - b.blocks, blockIdx.y);
   }
 }
 

@@ -664,6 +664,30 @@ inline int gemm_tf32_pair_width(uint64_t m, uint64_t n, uint64_t batch, int sms)
   return 67 * narrow < 100 * wide ? 128 : 256;
 }
 
+// The hi / lo planes of two operands (gemm_tf32_tc.cuh), `batch` of them; `transpose_b`: b comes as [cols][rows].
+inline int32_t split_operands_launch(std::string* err, gemm_tf32_tc::SplitOperand a, gemm_tf32_tc::SplitOperand b, bool transpose_b,
+                                     int32_t batch, int sms, cudaStream_t s) {
+  namespace g = gemm_tf32_tc;
+  auto row_blocks = [&](const g::SplitOperand& p) {
+    const int64_t items = p.rows * (p.kp / 4);
+    return static_cast<int32_t>(std::max<int64_t>(1, std::min<int64_t>((items + 255) / 256, 16ll * sms)));
+  };
+  auto vec = [](const g::SplitOperand& p) { return p.kp == p.cols && p.ld % 4 == 0 && p.batch_stride % 4 == 0 && aligned16(p.src); };
+  const int64_t tiles = (b.rows + 31) / 32 * ((b.cols + 31) / 32);
+  a.blocks = row_blocks(a);
+  if (transpose_b && tiles > 0x7fffffff - a.blocks) return op_fail(err, TSM100_ERR_INVALID, "operand split: too many tiles for one launch");
+  b.blocks = transpose_b ? static_cast<int32_t>(tiles) : row_blocks(b);
+  const dim3 grid(static_cast<unsigned>(a.blocks) + static_cast<unsigned>(b.blocks), static_cast<unsigned>(batch));
+  if (transpose_b) {
+    if (vec(a)) g::split_operands_kernel<true, true><<<grid, 256, 0, s>>>(a, b);
+    else g::split_operands_kernel<false, true><<<grid, 256, 0, s>>>(a, b);
+  } else {
+    if (vec(a) && vec(b)) g::split_operands_kernel<true, false><<<grid, 256, 0, s>>>(a, b);
+    else g::split_operands_kernel<false, false><<<grid, 256, 0, s>>>(a, b);
+  }
+  return cuda_ok(err, cudaGetLastError(), "split_operands_kernel launch");
+}
+
 // f32 inputs on the tcgen05 tensor cores: split pass (hi / lo planes, B's planes K-major), then the
 // contraction with chunked accumulation (gemm_tf32_tc.cuh).  The planes live in stream-ordered scratch.
 inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
@@ -687,22 +711,9 @@ inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, 
   float *a_hi = ws, *a_lo = ws + a_plane, *b_hi = ws + 2 * a_plane, *b_lo = b_hi + b_plane;
   const float* af = static_cast<const float*>(a);
   const float* bf = static_cast<const float*>(b);
-  auto split_rows = [&](const float* src, int64_t pitch, uint64_t rows, float* hi, float* lo) {
-    const uint64_t items = rows * (kp / 4);
-    const dim3 grid(static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((items + 255) / 256, static_cast<uint64_t>(sms) * 16))),
-                    static_cast<unsigned>(B));
-    auto kern = kp == K && pitch % 4 == 0 && aligned16(src) ? g::split_rows_kernel<true> : g::split_rows_kernel<false>;
-    kern<<<grid, 256, 0, s>>>(src, pitch, static_cast<int64_t>(rows) * pitch, hi, lo, static_cast<int64_t>(rows),
-                              static_cast<int32_t>(K), static_cast<int32_t>(kp));
-  };
-  split_rows(af, ld.lda, M, a_hi, a_lo);
-  if (d->b_transposed) {
-    split_rows(bf, ld.ldb, N, b_hi, b_lo);
-  } else {
-    g::split_transpose_kernel<<<dim3(static_cast<unsigned>((N + 31) / 32), static_cast<unsigned>((K + 31) / 32), static_cast<unsigned>(B)), 256, 0, s>>>(
-        bf, ld.ldb, static_cast<int64_t>(K) * ld.ldb, b_hi, b_lo, static_cast<int32_t>(K), static_cast<int32_t>(N), static_cast<int32_t>(kp));
-  }
-  st = cuda_ok(err, cudaGetLastError(), "gemm operand split launch");
+  st = split_operands_launch(err, {af, a_hi, a_lo, ld.lda, static_cast<int64_t>(M) * ld.lda, static_cast<int64_t>(M), static_cast<int32_t>(K), static_cast<int32_t>(kp), 0},
+                             {bf, b_hi, b_lo, ld.ldb, static_cast<int64_t>(d->b_transposed ? N : K) * ld.ldb, static_cast<int64_t>(N), static_cast<int32_t>(K), static_cast<int32_t>(kp), 0},
+                             !d->b_transposed, d->batch, sms, s);
   CUtensorMap ta_hi, ta_lo, tb_hi, tb_lo;
   const CUtensorMapDataType f32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   // Problems with more than one 128-row and 128-column block run on CTA pairs (256 x 256 or 256 x 128 tiles); the rest
@@ -1152,12 +1163,9 @@ inline int32_t attention_f32_tc_launch_d(std::string* err, const attn_simt::Para
     return op_fail(err, TSM100_ERR_MEMORY, std::string("attention: scratch for the K and V planes: ") + cudaGetErrorString(e));
   }
   float *k_hi = ws, *k_lo = ws + k_plane, *v_hi = ws + 2 * k_plane, *v_lo = v_hi + v_plane;
-  const uint64_t items = len * (D / 4);
-  g::split_rows_kernel<true><<<dim3(static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((items + 255) / 256, 16ull * sms))), static_cast<unsigned>(n_kv)), 256, 0, s>>>(
-      k, D, p.kv_head_stride, k_hi, k_lo, static_cast<int64_t>(len), D, D);
-  g::split_transpose_kernel<<<dim3(D / 32, static_cast<unsigned>((len + 31) / 32), static_cast<unsigned>(n_kv)), 256, 0, s>>>(
-      v, D, p.kv_head_stride, v_hi, v_lo, static_cast<int32_t>(len), D, static_cast<int32_t>(len4));
-  st = cuda_ok(err, cudaGetLastError(), "attention operand split launch");
+  st = split_operands_launch(err, {k, k_hi, k_lo, D, p.kv_head_stride, static_cast<int64_t>(len), D, D, 0},
+                             {v, v_hi, v_lo, D, p.kv_head_stride, D, static_cast<int32_t>(len), static_cast<int32_t>(len4), 0}, true,
+                             static_cast<int32_t>(n_kv), sms, s);
   CUtensorMap tk_hi, tk_lo, tv_hi, tv_lo;
   const CUtensorMapDataType f32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   if (st == TSM100_OK) st = make_tmap_3d(err, &tk_hi, k_hi, D, len, n_kv, D, len * D, 32, at::kBKV, f32, 4);
