@@ -339,7 +339,8 @@ int32_t tsm100_attention_decode(tsm100_device_t dev, const tsm100_attention_deco
  * tsm100_gemm_host keeps B resident and streams A and C in row blocks, each a
  * launch of its own: a 16-bit result may differ from tsm100_gemm on the whole
  * problem by one rounding of the stored type in a few elements (the f32 sums
- * are taken in another order); f32 results do not differ. */
+ * are taken in another order); f32 results do not differ where a block is large
+ * enough for the kernel that the whole problem takes. */
 int32_t tsm100_softmax_host(tsm100_device_t dev, const tsm100_softmax_desc* desc, const void* x,
                             void* y);
 int32_t tsm100_gemm_host(tsm100_device_t dev, const tsm100_gemm_desc* desc, const void* a,

@@ -54,6 +54,18 @@ inline int32_t cuda_ok(std::string* err, cudaError_t e, const char* what) {
   return op_fail(err, code, std::string(what) + " failed: " + cudaGetErrorString(e));
 }
 
+// What an operator's launch function answers, without a message, when the pool cannot give it the scratch it would like
+// and a form without scratch exists: the dispatch then takes that one.
+constexpr int32_t kNoScratch = -1;
+inline int32_t take_scratch(std::string* err, void** ws, size_t bytes, cudaStream_t s) {
+  const cudaError_t e = cudaMallocAsync(ws, bytes, s);
+  if (e == cudaErrorMemoryAllocation) {
+    (void)cudaGetLastError();
+    return kNoScratch;
+  }
+  return cuda_ok(err, e, "cudaMallocAsync");
+}
+
 inline size_t dtype_size(int32_t dtype) { return dtype == TSM100_F32 ? 4 : 2; }
 inline bool dtype_valid(int32_t dtype) { return dtype == TSM100_F32 || dtype == TSM100_F16 || dtype == TSM100_BF16; }
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
@@ -703,10 +715,9 @@ inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, 
   const uint64_t kp = (K + 3) / 4 * 4;  // row pitch of the planes: every row starts on a 16-byte boundary
   const size_t a_plane = static_cast<size_t>(B) * M * kp, b_plane = static_cast<size_t>(B) * N * kp;  // elements
   float* ws = nullptr;
-  e = cudaMallocAsync(reinterpret_cast<void**>(&ws), 2 * (a_plane + b_plane) * sizeof(float), s);
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();
-    return op_fail(err, TSM100_ERR_MEMORY, std::string("gemm: scratch for the operand planes: ") + cudaGetErrorString(e));
+  {
+    const int32_t got = take_scratch(err, reinterpret_cast<void**>(&ws), 2 * (a_plane + b_plane) * sizeof(float), s);
+    if (got != TSM100_OK) return got;
   }
   float *a_hi = ws, *a_lo = ws + a_plane, *b_hi = ws + 2 * a_plane, *b_lo = b_hi + b_plane;
   const float* af = static_cast<const float*>(a);
@@ -988,10 +999,9 @@ inline int32_t gemm_padded(std::string* err, const tsm100_gemm_desc* d, const vo
   const int64_t a_elems = pad_a ? batch * d->m * kp : 0, b_elems = pad_b ? batch * bp_rows * bp_cols : 0;  // multiples of 8
   const int64_t c_elems = pad_c ? batch * d->m * np : 0;
   uint16_t* ws = nullptr;
-  e = cudaMallocAsync(reinterpret_cast<void**>(&ws), static_cast<size_t>(a_elems + b_elems + c_elems) * 2, s);
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();
-    return op_fail(err, TSM100_ERR_MEMORY, std::string("gemm: scratch for padded operands: ") + cudaGetErrorString(e));
+  {
+    const int32_t got = take_scratch(err, reinterpret_cast<void**>(&ws), static_cast<size_t>(a_elems + b_elems + c_elems) * 2, s);
+    if (got != TSM100_OK) return got;
   }
   auto pad = [&](const void* src, int64_t pitch, int64_t rows, int64_t cols, uint16_t* dst, int64_t drows, int64_t dcols) {
     const int64_t items = drows * (dcols / 8);
@@ -1048,8 +1058,10 @@ inline int32_t gemm(std::string* err, const tsm100_gemm_desc* d, const void* a, 
                         d->n % 2 == 0 && ld.lda % 4 == 0 && ld.ldb % 4 == 0 && ld.ldc % 2 == 0;
     // enough work for the persistent tcgen05 kernels; their split pass takes rows of any alignment
     const int64_t tiles = ((d->m + 127) / 128) * ((d->n + 255) / 256) * d->batch;
-    if (status != nullptr && tiles >= 64 && tiles < 0x7fffffff && d->k >= 256)
-      return gemm_tf32_tc_launch(err, d, a, b, c, status, vec_ok, s);
+    if (status != nullptr && tiles >= 64 && tiles < 0x7fffffff && d->k >= 256) {
+      const int32_t st = gemm_tf32_tc_launch(err, d, a, b, c, status, vec_ok, s);
+      if (st != kNoScratch) return st;
+    }
     // fewer tiles (the 512^3 configuration has 8): the warp-level kernel, whose 64 x 64 tiles and cluster split-K
     // spread a small problem over the SMs, if rows start on 16-byte boundaries, else the FP32 pipe
     if (vec_ok) return gemm_tf32x3_launch(err, d, a, b, c, s);
@@ -1091,8 +1103,10 @@ inline int32_t gemm(std::string* err, const tsm100_gemm_desc* d, const void* a, 
   // whose last place hides the order of the f32 sums; an f32 result keeps the FP32 pipe's rounding to nearest.
   const int64_t n8 = (d->n + 7) / 8 * 8, k8 = (d->k + 7) / 8 * 8;
   if (status != nullptr && !out_f32 && d->m * d->n / 4096 * d->k * d->batch >= 1 << 14 && d->batch <= 65535 && n8 <= 0x7fffffff && k8 <= 0x7fffffff &&
-      ((d->m + 127) / 128) * ((n8 + 127) / 128) * d->batch * gemm_skinny::kMaxSplit <= 0x7fffffff)
-    return gemm_padded(err, d, a, b, c, status, s);
+      ((d->m + 15) / 16) * ((n8 + 95) / 96) * d->batch * gemm_skinny::kMaxSplit <= 0x7fffffff) {
+    const int32_t st = gemm_padded(err, d, a, b, c, status, s);
+    if (st != kNoScratch) return st;
+  }
   if (bf16) {
     if (out_f32) return gemm_simt_launch<__nv_bfloat16, float>(err, d, a, b, c, s);
     return gemm_simt_launch<__nv_bfloat16, __nv_bfloat16>(err, d, a, b, c, s);
@@ -1157,10 +1171,9 @@ inline int32_t attention_f32_tc_launch_d(std::string* err, const attn_simt::Para
   const uint64_t n_kv = static_cast<uint64_t>(p.batch) * p.heads_kv, len = p.seq_kv, len4 = (len + 3) / 4 * 4;
   const size_t k_plane = n_kv * len * D, v_plane = n_kv * len4 * D;
   float* ws = nullptr;
-  e = cudaMallocAsync(reinterpret_cast<void**>(&ws), 2 * (k_plane + v_plane) * sizeof(float), s);
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();
-    return op_fail(err, TSM100_ERR_MEMORY, std::string("attention: scratch for the K and V planes: ") + cudaGetErrorString(e));
+  {
+    const int32_t got = take_scratch(err, reinterpret_cast<void**>(&ws), 2 * (k_plane + v_plane) * sizeof(float), s);
+    if (got != TSM100_OK) return got;
   }
   float *k_hi = ws, *k_lo = ws + k_plane, *v_hi = ws + 2 * k_plane, *v_lo = v_hi + v_plane;
   st = split_operands_launch(err, {k, k_hi, k_lo, D, p.kv_head_stride, static_cast<int64_t>(len), D, D, 0},
@@ -1217,7 +1230,10 @@ inline int32_t attention_simt_launch(std::string* err, const tsm100_attention_de
                       static_cast<float>(1.0 / std::sqrt(static_cast<double>(d->head_dim))),
                       d->seq, 0, d->head_dim, sd, sd, d->head_dim, sd};
   if (attention_tf32x3_ok<T>(p, q, k, v, o)) {
-    if (sizeof(T) == 4 && attention_f32_tc_ok(p, status)) return attention_f32_tc_launch(err, p, q, k, v, o, status, s);
+    if (sizeof(T) == 4 && attention_f32_tc_ok(p, status)) {
+      const int32_t st = attention_f32_tc_launch(err, p, q, k, v, o, status, s);
+      if (st != kNoScratch) return st;
+    }
     return attention_tf32x3_launch<T>(err, p, q, k, v, o, s);
   }
   const int64_t rows = static_cast<int64_t>(d->batch) * d->heads_q * d->seq;
@@ -1240,7 +1256,10 @@ inline int32_t attention_prefill_simt_launch(std::string* err, const tsm100_atte
                       d->start_pos + d->seq_len, d->start_pos, hd, d->head_dim,
                       static_cast<int64_t>(d->max_seq) * d->head_dim, hd, d->head_dim};
   if (attention_tf32x3_ok<T>(p, q, k, v, o)) {
-    if (sizeof(T) == 4 && attention_f32_tc_ok(p, status)) return attention_f32_tc_launch(err, p, q, k, v, o, status, s);
+    if (sizeof(T) == 4 && attention_f32_tc_ok(p, status)) {
+      const int32_t st = attention_f32_tc_launch(err, p, q, k, v, o, status, s);
+      if (st != kNoScratch) return st;
+    }
     return attention_tf32x3_launch<T>(err, p, q, k, v, o, s);
   }
   const int64_t rows = static_cast<int64_t>(d->heads_q) * d->seq_len;
@@ -1278,21 +1297,22 @@ inline int32_t attention_fwd_launch(std::string* err, const CUtensorMap& tq, con
   p.splits = static_cast<int32_t>(std::max<int64_t>(1, std::min<int64_t>(sms / blocks, kv_steps / kAttentionSplitSteps)));
   p.part = nullptr;
   p.part_ml = nullptr;
+  const size_t rows = static_cast<size_t>(blocks) * p.splits * (2 * at::kBQ);
+  float* ws = nullptr;
+  if (p.splits > 1) {
+    st = cuda_ok(err, keep_pool_memory_once(), "cudaMemPoolSetAttribute");
+    if (st != TSM100_OK) return st;
+    st = take_scratch(err, reinterpret_cast<void**>(&ws), rows * (D + 2) * sizeof(float), s);
+    if (st == kNoScratch) p.splits = 1;
+    else if (st != TSM100_OK) return st;
+  }
+  cudaError_t e = cudaSuccess;
   if (p.splits == 1) {
     auto kern = at::attention_fwd_kernel<kBf16, kCache, D>;
-    cudaError_t e = set_dyn_smem_once(kern, smem);
+    e = set_dyn_smem_once(kern, smem);
     if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(attention_fwd_kernel)");
     kern<<<static_cast<unsigned>(blocks), at::kThreads, smem, s>>>(tq, tk, tv, out, p);
     return cuda_ok(err, cudaGetLastError(), "attention_fwd_kernel launch");
-  }
-  cudaError_t e = keep_pool_memory_once();
-  if (e != cudaSuccess) return cuda_ok(err, e, "cudaMemPoolSetAttribute");
-  const size_t rows = static_cast<size_t>(blocks) * p.splits * (2 * at::kBQ);
-  float* ws = nullptr;
-  e = cudaMallocAsync(reinterpret_cast<void**>(&ws), rows * (D + 2) * sizeof(float), s);
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();
-    return op_fail(err, TSM100_ERR_MEMORY, std::string("attention: scratch for partial results: ") + cudaGetErrorString(e));
   }
   p.part = reinterpret_cast<float4*>(ws);
   p.part_ml = reinterpret_cast<float2*>(ws + rows * D);
@@ -1483,10 +1503,9 @@ inline int32_t attention_decode_global_launch(std::string* err, const tsm100_att
   cudaError_t e = keep_pool_memory_once();
   if (e != cudaSuccess) return cuda_ok(err, e, "cudaMemPoolSetAttribute");
   float* ws = nullptr;
-  e = cudaMallocAsync(reinterpret_cast<void**>(&ws), static_cast<size_t>(units) * splits * ad::mma::kRows * (D + 2) * sizeof(float), s);
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();
-    return op_fail(err, TSM100_ERR_MEMORY, std::string("attention_decode: scratch: ") + cudaGetErrorString(e));
+  {
+    const int32_t got = take_scratch(err, reinterpret_cast<void**>(&ws), static_cast<size_t>(units) * splits * ad::mma::kRows * (D + 2) * sizeof(float), s);
+    if (got != TSM100_OK) return got;
   }
   ad::Params p;
   p.batch = d->batch;
@@ -1593,8 +1612,11 @@ inline int32_t attention_decode_typed(std::string* err, const tsm100_attention_d
     // one KV head, 32768 positions 22.6 / 13.4.
     if constexpr (sizeof(T) == 2) {
       const int64_t wide = std::min<int64_t>({attn_decode::mma::kMaxGlobalSplits, sms / std::max<int64_t>(units, 1), d->seq_len / 512});
-      if (wide * 2 >= 3 * splits && wide > 1)
-        return attention_decode_global_launch<T, D>(err, d, qp, kp, vp, op, static_cast<int>(wide), s);
+      if (wide * 2 >= 3 * splits && wide > 1) {
+        st = attention_decode_global_launch<T, D>(err, d, qp, kp, vp, op, static_cast<int>(wide), s);
+        if (st != kNoScratch) return st;
+        st = TSM100_OK;
+      }
     }
     // every CTA alone on its SM from start to end: eight warps and a deeper ring, so that it hides its own latencies
     const bool lone = units * splits <= sms && (splits < attn_decode::kMaxSplits || units <= decode_lone_clusters<T, D>(splits));
