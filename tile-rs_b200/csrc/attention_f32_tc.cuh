@@ -5,7 +5,7 @@
 // crates/rustc_codegen_tile/src/mlir_to_gpu.rs:1657-1673); the scheme of three TF32 products per product on hi / lo
 // parts, and of accumulating in short chunks, is that of gemm_tf32_tc.cuh.
 //
-// Two streaming passes write the hi / lo planes of K ([keys][D]) and of V, transposed ([D][keys]), so that both products
+// One streaming launch writes the hi / lo planes of K ([keys][D]) and of V, transposed ([D][keys]), so that both products
 // see K-major operands only.  Then one CTA owns 128 query rows of one head and walks the keys in steps of 32:
 //   warp 8       TMA producer: K_0, K_1, V_0, K_2, V_1, ... (hi and lo together, 256 * D bytes a unit) through a 3-deep
 //                ring.  No multicast.

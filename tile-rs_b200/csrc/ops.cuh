@@ -1156,7 +1156,7 @@ inline int32_t attention_tf32x3_launch(std::string* err, const attn_simt::Params
   }
 }
 
-// f32 on the tcgen05 kernel: two passes write the hi / lo planes of K and of V transposed into stream-ordered scratch.
+// f32 on the tcgen05 kernel: one launch writes the hi / lo planes of K and of V transposed into stream-ordered scratch.
 // kv_row 0 of every (batch, KV head) is kv_head_stride elements after the one before.
 template <int D>
 inline int32_t attention_f32_tc_launch_d(std::string* err, const attn_simt::Params& p, const float* q, const float* k,
