@@ -34,3 +34,39 @@ def test_attention_steps_over_several_CTAs(dev, pkg, oracle, hq, s, d, causal):
     for row0, rows in ((0, 300), (s // 2, 64), (s - 200, 200)):
         ref, _ = oracle.attention_bf16(q, k, v, causal, row0, rows)
         util.assert_16bit_close(oracle, np.ascontiguousarray(o[:, :, row0:row0 + rows]), ref)
+
+
+# starts that are no multiple of the 128-key step, and ranges so short that the last one lies wholly behind the first rows of its
+# query tile: for them it holds no visible key
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("s,hq,hkv,d,start", [(256, 8, 2, 128, 32516), (100, 8, 8, 64, 36900), (256, 4, 1, 64, 32600), (100, 4, 1, 128, 78300),
+                                              (100, 1, 1, 128, 34721), (100, 1, 1, 64, 34721)])
+def test_prefill_rows_without_a_key_in_the_last_range(dev, pkg, oracle, s, hq, hkv, d, start, dtype):
+    capi = pkg.capi
+    qf = util.gen_normal(capi, (s, hq, d), 751)
+    kf, vf = (util.gen_normal(capi, (hkv, start + s, d), 752 + i) for i in range(2))
+    if dtype == "bf16":
+        q, k, v = (util.to_bf16(capi, t) for t in (qf, kf, vf))
+        wide = oracle.bf16_to_f32
+    else:
+        q, k, v = (util.f32_to_f16_bits(t) for t in (qf, kf, vf))
+        wide = lambda t: np.ascontiguousarray(t).view(np.float16).astype(np.float32)  # noqa: E731
+    o = wide(run_prefill(dev, capi, q, k, v, start, capi.BF16 if dtype == "bf16" else capi.F16).view(np.uint16))
+    util.assert_16bit_close(oracle, o, oracle.attention_prefill_f32(wide(q), wide(k), wide(v), start))
+
+
+# scores of -inf in a whole 128-key step, whose maximum then stays -inf: their keys weigh nothing, the others decide
+@pytest.mark.parametrize("d,first", [(128, True), (64, True), (64, False), (32, True)])
+def test_a_step_of_infinite_scores(dev, pkg, oracle, d, first):
+    capi = pkg.capi
+    q, k, v = bf16_qkv(capi, 1, 2, 1, 400, d, seed=761)
+    q[..., 0] = 0x3f80                      # 1.0
+    at = slice(0, 128) if first else slice(128, 256)
+    k[:, :, at, 0] = 0xff80                 # -inf
+    o = oracle.bf16_to_f32(run_attention(dev, capi, q, k, v, capi.BF16, False).view(np.uint16))
+    keep = np.r_[0:at.start, at.stop:400]
+    f = oracle.bf16_to_f32
+    qf, kf, vf = f(q)[0].astype(np.float64), f(k)[0, 0, keep].astype(np.float64), f(v)[0, 0, keep].astype(np.float64)
+    x = qf @ kf.T / np.sqrt(d)
+    p = np.exp(x - x.max(-1, keepdims=True))
+    util.assert_16bit_close(oracle, o[0], ((p / p.sum(-1, keepdims=True)) @ vf).astype(np.float32))

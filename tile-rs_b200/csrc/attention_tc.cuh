@@ -471,7 +471,9 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       // Of every 8 pairs, kPolyPairs go through the FMA-pipe polynomial and the rest through
       // MUFU ex2, so that neither pipe alone bounds the exponentials.  The row sum adds the
       // f32 probabilities before they are rounded (packed adds, two per instruction).
-      const float ms = m_used * sl2;
+      // A row whose scores so far are all -inf (a step, or in kSplit a whole range, may lie behind the row's last visible key):
+      // taking them against 0 gives them no weight, against their maximum of -inf NaN.
+      const float ms = m_used == -INFINITY ? 0.f : m_used * sl2;
       const ptx::f32x2_t sl2x2 = ptx::pack_f32x2(sl2, sl2);
       const ptx::f32x2_t nmsx2 = ptx::pack_f32x2(-ms, -ms);
       ptx::f32x2_t lsum[2] = {0ull, 0ull};  // (+0.0f, +0.0f)
@@ -577,7 +579,8 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       bool ready = ptx::mbar_wait(&bars->pv_done[g], (n_g - 1) & 1u, abort_flag, p.status, 20 + g);
       if (__all_sync(0xffffffffu, ready)) {
         ptx::tcgen05_fence_after_thread_sync();
-        const float inv = 1.0f / l;
+        // all scores -inf (or NaN): softmax is NaN there, l a stand-in (the wide form's cubic ends at 2^-125)
+        const float inv = m_used == -INFINITY ? NAN : 1.0f / l;
         const int cols = D == 64 ? p.head_dim : D;
         uint16_t* orow = kCache ? o + bh * p.o_head_stride + qrow * p.o_row_stride
                                 : o + (static_cast<int64_t>(bh) * p.seq + qrow) * cols;
@@ -637,6 +640,7 @@ attention_merge_kernel(uint16_t* __restrict__ o, const Params p) {
   for (int i = 0; i < 16; ++i) acc[i] = 0.f;
   for (int q = 0; q < p.splits; ++q) {
     const float2 ml = p.part_ml[(rec0 + q) * (2 * kBQ) + row];
+    // a range without a visible key weighs 0; it is added all the same, because a range of NaN scores has that maximum too
     const float w = ml.x == -INFINITY ? 0.f : ptx::ex2_approx((ml.x - gm) * p.scale_log2);
     gl = fmaf(w, ml.y, gl);
     const float4* part = p.part + (rec0 + q) * (D / 4) * (2 * kBQ) + (c0 / 4) * (2 * kBQ) + row;
