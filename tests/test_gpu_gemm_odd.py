@@ -55,3 +55,56 @@ def test_f32_infinities_and_nans_in_odd_rows(dev, pkg, oracle):
     rows = [r for r in (0, 4, 100, 2048)]
     assert np.abs(c[rows][finite[rows]] - want[rows][finite[rows]]).max() <= util.F32_REL * np.abs(want[rows][finite[rows]]).max()
     assert np.allclose(c[9][finite[9]], want[9][finite[9]], rtol=1e-5, atol=0)
+
+
+# every output infinite: all blocks are summed again, at about the FP32 pipe's rate, and nothing waits for it
+@pytest.mark.parametrize("bt", [False, True])
+def test_f32_odd_product_that_overflows_everywhere(dev, pkg, bt):
+    capi = pkg.capi
+    m, n, k = 2049, 2051, 301
+    rows, cols = np.where(np.arange(m) % 3 == 1, -1, 1), np.where(np.arange(n) % 5 == 2, -1, 1)
+    a = (np.abs(util.gen_uniform(capi, (m, k), 611)) + 1) * np.float32(1e20) * rows[:, None].astype(np.float32)
+    b = (np.abs(util.gen_uniform(capi, (k, n), 612)) + 1) * np.float32(1e20) * cols[None, :].astype(np.float32)
+    b = np.ascontiguousarray(b.T) if bt else b
+
+    def ms(a, b):
+        ad, bd = util.dev_tensor(torch, a), util.dev_tensor(torch, b)
+        cd = torch.full((m, n), 7, dtype=torch.float32, device="cuda:0")
+        t = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        for _ in range(2):
+            t[0].record()
+            dev.gemm(capi.F32, m, n, k, ad.data_ptr(), bd.data_ptr(), cd.data_ptr(), b_transposed=bt, stream=util.cur_stream(torch))
+            t[1].record()
+        torch.cuda.synchronize()
+        assert dev.status() == 0
+        return cd.cpu().numpy(), t[0].elapsed_time(t[1])
+
+    c, slow = ms(a, b)
+    assert np.array_equal(c, np.where(rows[:, None] * cols > 0, np.float32(np.inf), np.float32(-np.inf)))
+    _, fast = ms(a * np.float32(1e-20), b * np.float32(1e-20))
+    # one lane after the other took 20 ms more
+    assert slow <= 20 * fast + 1, (slow, fast)
+
+
+@pytest.mark.parametrize("m,n,k,bt", [(2305, 4099, 5001, False), (2305, 4099, 5001, True), (66, 16387, 2051, False)])
+def test_f32_an_infinite_row_of_a_long_product(dev, pkg, oracle, m, n, k, bt):
+    """Several tiles per CTA, among them some with infinities: those alone are replaced, by what the FP32 pipe gives."""
+    capi = pkg.capi
+    a, b = util.gen_uniform(capi, (m, k), 615), util.gen_uniform(capi, (n, k) if bt else (k, n), 616)
+    a[40, 3] = np.inf
+    col = n - 2
+    b[(col, 9) if bt else (9, col)] = -np.inf
+    c = run(dev, capi, capi.F32, a, b, m, n, k, bt)[0]
+    bk = lambda i: b[:, i] if bt else b[i]  # noqa: E731
+    want = np.sign(bk(3)) * np.float64(np.inf)
+    with np.errstate(invalid="ignore"):
+        want[col] += -np.sign(a[40, 9]) * np.inf
+    assert np.array_equal(c[40], want.astype(np.float32), equal_nan=True)
+    want = -np.sign(a[:, 9]) * np.inf
+    want[40] = c[40, col]
+    assert np.array_equal(c[:, col], want.astype(np.float32), equal_nan=True)
+    keep = np.delete(np.arange(n), col)
+    rows = np.array([0, 39, 41, 63, 64, m - 1])
+    truth = oracle.gemm_f32(np.ascontiguousarray(a[rows]), np.ascontiguousarray(b[keep] if bt else b[:, keep]), bt, f64_acc=True)
+    mt = oracle.compare(np.ascontiguousarray(c[rows][:, keep]), truth)
+    assert mt["rel_max"] <= util.F32_REL and mt["rel_fro"] <= util.F32_REL, mt

@@ -39,6 +39,11 @@ constexpr int kStageBytes = 2 * kAPlane + 2 * kBPlane;  // 96 KiB: A_hi, A_lo, B
 constexpr int kTmemCols = 512;           // two 256-column accumulators
 constexpr int kGroupM = 16;              // m-blocks per rasterisation band (L2 reuse)
 
+struct Redo {            // of a CTA's second pass (kRedo kernels)
+  uint32_t any;          // one of its blocks holds an infinity or a NaN
+  uint32_t pick, got;
+};
+
 struct alignas(8) Barriers {
   uint64_t full[kStages];
   uint64_t empty[kStages];
@@ -46,6 +51,7 @@ struct alignas(8) Barriers {
   uint64_t acc_empty[2];
   uint32_t tmem_base;
   uint32_t abort_flag;
+  Redo redo;
 };
 // C is written in 32 x 32 blocks through shared memory, so that a warp's store covers whole 128-byte pieces of rows.
 constexpr int kStagingFloats = 32 * 32;                       // per epilogue warp
@@ -61,7 +67,9 @@ struct Params {
   uint32_t* status;
   int32_t vec_store;       // every row of C starts on a 16-byte boundary
   int32_t chunk_kb;        // 32-deep k-blocks per accumulation chunk
-  // kRedo kernels: the operands as they came
+  // kRedo kernels: the operands as they came, and a word per 128 x 128 block of C, [batch][ceil(m / 128)][ceil(n / 128)], zero
+  // at the start (see second_pass)
+  uint32_t* flags;
   int32_t b_transposed;
   const float *a, *b;
   int64_t lda, ldb, a_batch_stride, b_batch_stride;
@@ -146,10 +154,13 @@ __device__ __forceinline__ void split_transposed(const SplitOperand& p, int bloc
   }
 }
 
-// grid (a.blocks + b.blocks, batch); the blocks of the transposed operand come first.
+// grid (a.blocks + b.blocks, batch); the blocks of the transposed operand come first.  zero[0 .. n_zero) is cleared on the way:
+// the flags of the contraction's second pass.
 template <bool kVec, bool kTransposeB>
 __global__ void __launch_bounds__(256)
-split_operands_kernel(const SplitOperand a, const SplitOperand b) {
+split_operands_kernel(const SplitOperand a, const SplitOperand b, uint32_t* zero, int64_t n_zero) {
+  if (blockIdx.y == 0)
+    for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n_zero; i += static_cast<int64_t>(gridDim.x) * blockDim.x) zero[i] = 0u;
   __shared__ float tile[kTransposeB ? 32 : 1][33];
   const int block = static_cast<int>(blockIdx.x);
   if (block < b.blocks) {
@@ -167,25 +178,23 @@ split_operands_kernel(const SplitOperand a, const SplitOperand b) {
 // `staging`: 16-byte unit u of row r lies at unit u ^ (r & 7), so neither side has bank conflicts.  vec_store: 16-byte
 // stores, four rows at a time, otherwise 4-byte stores of one row.  Writing rows from the lanes that hold them costs more
 // even where they are aligned: every store then touches 32 rows (2000 x 3000 x 1500 on 256 x 128 tiles: 127 us against 117).
-// kRedo (problems that the FP32 pipe could take as well): an output that comes out infinite or NaN is summed again in plain
-// f32, because infinity split into hi + lo is infinity + NaN.
-__device__ __noinline__ float dot_f32(const Params& p, int batch, int row, int col) {
-  const float* x = p.a + batch * p.a_batch_stride + row * p.lda;
-  const float* w = p.b + batch * p.b_batch_stride + (p.b_transposed ? col * p.ldb : static_cast<int64_t>(col));
-  const int64_t step = p.b_transposed ? 1 : p.ldb;
-  float s = 0.f;
-  for (int k = 0; k < p.k && s == s; ++k) s = fmaf(x[k], w[k * step], s);  // a NaN stays one
-  return s;
-}
+// Columns of an accumulator read at a time.  16 leave the kRedo kernels, whose second pass holds registers too, without spills:
+// 1999 x 3001 x 1501 130.2 us with 32, 124.7 with 16; no difference for the others.
+template <bool kRedo>
+constexpr int kDrain = kRedo ? 16 : 32;
+// kRedo (problems that the FP32 pipe could take as well): a block with an infinity or a NaN is marked for second_pass.
 template <bool kRedo>
 __device__ __forceinline__ void store_block_32x32(float* __restrict__ c, const Params& p, int batch, int row0, int col0,
-                                                  const float (&sum)[32], float* staging, int lane) {
+                                                  const float (&sum)[32], float* staging, int lane, Redo* redo) {
   float* cb = c + batch * p.c_batch_stride;
-  uint32_t bad = 0;  // columns of this lane's row to sum again
-  if (kRedo) {
+  if (kRedo && row0 < p.m && col0 < p.n) {
+    float z = 0.f;  // NaN where anything is infinite or NaN (rows and columns past C are so only beside such ones of C)
 #pragma unroll
-    for (int i = 0; i < 32; ++i) bad |= (fabsf(sum[i]) < INFINITY ? 0u : 1u) << i;
-    if (row0 + lane >= p.m) bad = 0;
+    for (int i = 0; i < 32; ++i) z = fmaf(sum[i], 0.f, z);
+    if (__any_sync(0xffffffffu, z != 0.f) && lane == 0) {
+      p.flags[(static_cast<int64_t>(batch) * ((p.m + 127) / 128) + row0 / 128) * ((p.n + 127) / 128) + col0 / 128] = 2u + blockIdx.x;
+      redo->any = 1u;
+    }
   }
   float4* st4 = reinterpret_cast<float4*>(staging);
   __syncwarp();  // the previous block has been read
@@ -205,12 +214,137 @@ __device__ __forceinline__ void store_block_32x32(float* __restrict__ c, const P
     float* dst = cb + static_cast<int64_t>(row0) * p.ldc + col0 + lane;
     for (int r = 0; r < rows; ++r) dst[r * p.ldc] = staging[r * 32 + (((lane >> 2) ^ (r & 7)) << 2) + (lane & 3)];
   }
-  if (kRedo && __any_sync(0xffffffffu, bad != 0)) {
-    __syncwarp();  // after the stores above: another lane may have written this lane's elements
-    __threadfence_block();
-    for (; bad != 0; bad &= bad - 1) {
-      const int col = col0 + __ffs(bad) - 1;
-      if (col < p.n) cb[static_cast<int64_t>(row0 + lane) * p.ldc + col] = dot_f32(p, batch, row0 + lane, col);
+}
+
+// ---------------------------------------------------------------------------
+// the second pass of kRedo kernels
+// ---------------------------------------------------------------------------
+// An infinity split into hi + lo is infinity + NaN, and a hi part can round up to infinity, so outputs that come out infinite or
+// NaN are summed again in plain f32 and replaced.  That runs when a CTA has written all of its tiles: no barrier of the
+// pipeline waits for it, however long it takes, and a CTA whose outputs are all finite does nothing.  A CTA that marked
+// blocks publishes them then, walks over the published blocks and sums those it can claim until it finds none, so that CTAs with few tiles
+// help those with many.  Nobody waits for a block to be published: its own CTA comes for it.
+// Every output infinite: 2049 x 2051 x 1501 590 us (610 on the FP32-pipe kernel), 1999 x 3001 x 1501 840 (770), 4097 x 4097 x
+// 2001 2900 (2650); 2049 x 2051 x 301 0.19 ms, 20 with one dependent sum per lane inside the epilogue.
+constexpr int kEpilogueThreads = 256;
+__device__ __forceinline__ void epilogue_sync() { asm volatile("barrier.cta.sync 1, 256;" ::: "memory"); }
+__device__ __forceinline__ bool epilogue_any(bool x) {
+  uint32_t r;
+  asm volatile(
+      "{\n"
+      ".reg .pred p, q;\n"
+      "setp.ne.u32 p, %1, 0;\n"
+      "barrier.cta.red.or.pred q, 1, 256, p;\n"
+      "selp.u32 %0, 1, 0, q;\n"
+      "}\n" : "=r"(r) : "r"(static_cast<uint32_t>(x)) : "memory");
+  return r != 0;
+}
+// One 128 x 128 block, 256 threads with 8 x 8 sums each, in the order of k; the next 16 of k are loaded meanwhile.
+// `panels`: kPanelFloats of shared memory.
+constexpr int kPanelK = 16, kPanelPitch = 132;
+constexpr int kPanelFloats = 2 * kPanelK * kPanelPitch;
+static_assert(kPanelFloats * 4 <= kStages * kStageBytes, "the panels take the place of the stages");
+__device__ __forceinline__ void sum_block_again(const Params& p, float* c, float* panels, int batch, int row0, int col0, int tid) {
+  float *sa = panels, *sb = panels + kPanelK * kPanelPitch;
+  const int tx = tid & 15, ty = tid >> 4;
+  // this thread's eight values of a panel of A: row (tid >> 4) + 16 i, k = tid & 15; of B the same, or, stored [K][N], column
+  // tid & 127, k = (tid >> 7) + 2 i
+  const bool bt = p.b_transposed != 0;
+  const int m = p.m, n = p.n, k = p.k;
+  const float* a = p.a + batch * p.a_batch_stride + (row0 + ty) * p.lda + tx;
+  const float* b = p.b + batch * p.b_batch_stride + (bt ? (col0 + ty) * p.ldb + tx : (tid >> 7) * p.ldb + col0 + (tid & 127));
+  const int64_t a_step = 16 * p.lda, b_step = (bt ? 16 : 2) * p.ldb, b_panel = bt ? kPanelK : kPanelK * p.ldb;
+  const int b_col = col0 + (bt ? ty : tid & 127), b_col_step = bt ? 16 : 0, b_k = bt ? tx : tid >> 7, b_k_step = bt ? 0 : 2;
+  float* const sa_at = sa + tx * kPanelPitch + ty;
+  float* const sb_at = bt ? sb + tx * kPanelPitch + ty : sb + (tid >> 7) * kPanelPitch + (tid & 127);
+  const int sb_step = bt ? 16 : 2 * kPanelPitch;
+  float acc[8][8], na[8], nb[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
+  auto fetch = [&](int k0) {
+    const float *pa = a, *pb = b;
+#pragma unroll
+    for (int i = 0; i < 8; ++i, pa += a_step, pb += b_step) {
+      na[i] = row0 + ty + 16 * i < m && k0 + tx < k ? *pa : 0.f;
+      nb[i] = b_col + i * b_col_step < n && k0 + b_k + i * b_k_step < k ? *pb : 0.f;
+    }
+    a += kPanelK;
+    b += b_panel;
+  };
+  fetch(0);
+  for (int k0 = 0; k0 < k; k0 += kPanelK) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      sa_at[i * 16] = na[i];
+      sb_at[i * sb_step] = nb[i];
+    }
+    epilogue_sync();
+    fetch(k0 + kPanelK);
+#pragma unroll 2
+    for (int kk = 0; kk < kPanelK; ++kk) {
+      alignas(16) float x[8], w[8];
+#pragma unroll
+      for (int i = 0; i < 8; i += 4) {
+        *reinterpret_cast<float4*>(x + i) = *reinterpret_cast<const float4*>(sa + kk * kPanelPitch + ty * 8 + i);
+        *reinterpret_cast<float4*>(w + i) = *reinterpret_cast<const float4*>(sb + kk * kPanelPitch + tx * 4 + i * 16);
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(x[i], w[j], acc[i][j]);
+    }
+    epilogue_sync();
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = row0 + ty * 8 + i;
+    if (r >= m) break;
+    float* out = c + batch * p.c_batch_stride + r * p.ldc + col0 + tx * 4;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int at = (j & 3) + (j >> 2) * 64;
+      if (col0 + tx * 4 + at < n && !(fabsf(__ldcg(out + at)) < INFINITY)) out[at] = acc[i][j];
+    }
+  }
+}
+// Called by all eight epilogue warps after their last tile, with `ok` false if a wait of theirs gave up.  The stages are free: the last
+// accumulator is complete, so every copy into them and every product from them has retired.
+__device__ __noinline__ void second_pass(const Params& p, float* c, float* panels, Redo* redo, bool ok) {
+  const int tid = static_cast<int>(threadIdx.x) - 64;
+  if (!epilogue_any(redo->any != 0u) || epilogue_any(!ok)) return;
+  const int rows = (p.m + 127) / 128, cols = (p.n + 127) / 128;
+  const int total = p.batch * rows * cols;
+  volatile uint32_t* flags = p.flags;
+  __threadfence();  // this thread's part of C before the flags that say it is there
+  epilogue_sync();
+  for (int i = tid; i < total; i += kEpilogueThreads)
+    if (flags[i] == 2u + blockIdx.x) atomicExch(&p.flags[i], 1u);
+  epilogue_sync();
+  const int start = static_cast<int>(static_cast<int64_t>(blockIdx.x) * total / gridDim.x);
+  bool found = true;
+  while (found) {
+    found = false;
+    for (int at = 0; at < total; at += kEpilogueThreads) {
+      const int i = (start + at + tid) % total;
+      for (;;) {
+        const bool ready = at + tid < total && flags[i] == 1u;
+        if (!epilogue_any(ready)) break;
+        if (tid == 0) redo->pick = kEpilogueThreads;
+        epilogue_sync();
+        if (ready) atomicMin(&redo->pick, static_cast<uint32_t>(tid));
+        epilogue_sync();
+        const int pick = static_cast<int>(redo->pick);
+        if (tid == pick) redo->got = atomicCAS(&p.flags[i], 1u, 0u) == 1u ? 1u : 0u;
+        epilogue_sync();
+        if (redo->got != 0u) {
+          __threadfence();
+          const int block = (start + at + pick) % total;
+          sum_block_again(p, c, panels, block / (rows * cols), block / cols % rows * 128, block % cols * 128, tid);
+          found = true;
+        }
+      }
     }
   }
 }
@@ -250,7 +384,7 @@ template <bool kRedo>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tf32_tc_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_constant__ CUtensorMap tmap_a_lo,
                     const __grid_constant__ CUtensorMap tmap_b_hi, const __grid_constant__ CUtensorMap tmap_b_lo,
-                    float* __restrict__ c, const Params p) {
+                    float* __restrict__ c, const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   Barriers* bars = reinterpret_cast<Barriers*>(smem + kStages * kStageBytes + kStagingBytes);
@@ -272,6 +406,7 @@ gemm_tf32_tc_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_
       ptx::mbar_init(&bars->acc_empty[a], 8);  // one arrival per epilogue warp
     }
     bars->abort_flag = 0;
+    bars->redo.any = 0;
     ptx::fence_mbar_init();
   }
   if (warp == 1) {
@@ -395,11 +530,15 @@ gemm_tf32_tc_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_
         ptx::tcgen05_fence_after_thread_sync();
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc) {
-          uint32_t v[32];
-          ptx::tmem_ld_32x32b_x32(lane_addr + acc * kBN + cc * 32, v);
-          ptx::tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) sum[cc][i] += __uint_as_float(v[i]);  // round-to-nearest add of the chunk
+          for (int h = 0; h < 32; h += kDrain<kRedo>) {
+            uint32_t v[kDrain<kRedo>];
+            if constexpr (kRedo) ptx::tmem_ld_32x32b_x16(lane_addr + acc * kBN + cc * 32 + h, v);
+            else ptx::tmem_ld_32x32b_x32(lane_addr + acc * kBN + cc * 32, v);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < kDrain<kRedo>; ++i) sum[cc][h + i] += __uint_as_float(v[i]);  // round-to-nearest add of the chunk
+          }
         }
         ptx::tcgen05_fence_before_thread_sync();
         __syncwarp();
@@ -408,8 +547,9 @@ gemm_tf32_tc_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_
       if (!alive) break;
 #pragma unroll
       for (int cc = 0; cc < 4; ++cc)
-        store_block_32x32<kRedo>(c, p, b, mb * kBM + quad * 32, nb * kBN + half * 128 + cc * 32, sum[cc], staging, lane);
+        store_block_32x32<kRedo>(c, p, b, mb * kBM + quad * 32, nb * kBN + half * 128 + cc * 32, sum[cc], staging, lane, &bars->redo);
     }
+    if (kRedo) second_pass(p, c, reinterpret_cast<float*>(smem), &bars->redo, alive);
   }
 
   // ------------------------------ teardown ------------------------------------
@@ -461,6 +601,7 @@ struct alignas(8) Barriers {
   uint64_t acc_empty[2];       // used in the leader: 16 epilogue warps of the pair have drained it
   uint32_t tmem_base;
   uint32_t abort_flag;
+  Redo redo;
 };
 template <int BN>
 constexpr int smem_bytes() {
@@ -498,7 +639,7 @@ template <int BN, bool kRedo>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_constant__ CUtensorMap tmap_a_lo,
                      const __grid_constant__ CUtensorMap tmap_b_hi, const __grid_constant__ CUtensorMap tmap_b_lo,
-                     float* __restrict__ c, const Params p) {
+                     float* __restrict__ c, const __grid_constant__ Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   using S = Shape<BN>;
@@ -526,6 +667,7 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
       ptx::mbar_init(&bars->acc_empty[a], 16);  // 8 epilogue warps in each CTA of the pair
     }
     bars->abort_flag = 0;
+    bars->redo.any = 0;
     ptx::fence_mbar_init();
   }
   if (warp == 1) {
@@ -649,11 +791,15 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
         ptx::tcgen05_fence_after_thread_sync();
 #pragma unroll
         for (int cc = 0; cc < kChunks; ++cc) {
-          uint32_t v[32];
-          ptx::tmem_ld_32x32b_x32(lane_addr + acc * BN + cc * 32, v);
-          ptx::tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) sum[cc][i] += __uint_as_float(v[i]);
+          for (int h = 0; h < 32; h += kDrain<kRedo>) {
+            uint32_t v[kDrain<kRedo>];
+            if constexpr (kRedo) ptx::tmem_ld_32x32b_x16(lane_addr + acc * BN + cc * 32 + h, v);
+            else ptx::tmem_ld_32x32b_x32(lane_addr + acc * BN + cc * 32, v);
+            ptx::tmem_ld_wait();
+#pragma unroll
+            for (int i = 0; i < kDrain<kRedo>; ++i) sum[cc][h + i] += __uint_as_float(v[i]);
+          }
         }
         ptx::tcgen05_fence_before_thread_sync();
         __syncwarp();
@@ -663,8 +809,9 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
       const int row0 = mb * kPairM + static_cast<int>(rank) * kCtaM + quad * 32;
 #pragma unroll
       for (int cc = 0; cc < kChunks; ++cc)
-        store_block_32x32<kRedo>(c, p, b, row0, nb * BN + half * (BN / 2) + cc * 32, sum[cc], staging, lane);
+        store_block_32x32<kRedo>(c, p, b, row0, nb * BN + half * (BN / 2) + cc * 32, sum[cc], staging, lane, &bars->redo);
     }
+    if (kRedo) second_pass(p, c, reinterpret_cast<float*>(smem), &bars->redo, alive);
   }
 
   // ------------------------------ teardown ------------------------------------

@@ -676,9 +676,10 @@ inline int gemm_tf32_pair_width(uint64_t m, uint64_t n, uint64_t batch, int sms)
   return 67 * narrow < 100 * wide ? 128 : 256;
 }
 
-// The hi / lo planes of two operands (gemm_tf32_tc.cuh), `batch` of them; `transpose_b`: b comes as [cols][rows].
+// The hi / lo planes of two operands (gemm_tf32_tc.cuh), `batch` of them; `transpose_b`: b comes as [cols][rows].  The same
+// launch clears zero[0 .. n_zero).
 inline int32_t split_operands_launch(std::string* err, gemm_tf32_tc::SplitOperand a, gemm_tf32_tc::SplitOperand b, bool transpose_b,
-                                     int32_t batch, int sms, cudaStream_t s) {
+                                     int32_t batch, int sms, cudaStream_t s, uint32_t* zero = nullptr, int64_t n_zero = 0) {
   namespace g = gemm_tf32_tc;
   auto row_blocks = [&](const g::SplitOperand& p) {
     const int64_t items = p.rows * (p.kp / 4);
@@ -691,11 +692,11 @@ inline int32_t split_operands_launch(std::string* err, gemm_tf32_tc::SplitOperan
   b.blocks = transpose_b ? static_cast<int32_t>(tiles) : row_blocks(b);
   const dim3 grid(static_cast<unsigned>(a.blocks) + static_cast<unsigned>(b.blocks), static_cast<unsigned>(batch));
   if (transpose_b) {
-    if (vec(a)) g::split_operands_kernel<true, true><<<grid, 256, 0, s>>>(a, b);
-    else g::split_operands_kernel<false, true><<<grid, 256, 0, s>>>(a, b);
+    if (vec(a)) g::split_operands_kernel<true, true><<<grid, 256, 0, s>>>(a, b, zero, n_zero);
+    else g::split_operands_kernel<false, true><<<grid, 256, 0, s>>>(a, b, zero, n_zero);
   } else {
-    if (vec(a) && vec(b)) g::split_operands_kernel<true, false><<<grid, 256, 0, s>>>(a, b);
-    else g::split_operands_kernel<false, false><<<grid, 256, 0, s>>>(a, b);
+    if (vec(a) && vec(b)) g::split_operands_kernel<true, false><<<grid, 256, 0, s>>>(a, b, zero, n_zero);
+    else g::split_operands_kernel<false, false><<<grid, 256, 0, s>>>(a, b, zero, n_zero);
   }
   return cuda_ok(err, cudaGetLastError(), "split_operands_kernel launch");
 }
@@ -714,17 +715,20 @@ inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, 
   if (e != cudaSuccess) return cuda_ok(err, e, "cudaMemPoolSetAttribute");
   const uint64_t kp = (K + 3) / 4 * 4;  // row pitch of the planes: every row starts on a 16-byte boundary
   const size_t a_plane = static_cast<size_t>(B) * M * kp, b_plane = static_cast<size_t>(B) * N * kp;  // elements
+  // rows that start anywhere: a flag per 128 x 128 block of C, behind the planes
+  const int64_t flags = rows_aligned ? 0 : static_cast<int64_t>(B * ((M + 127) / 128) * ((N + 127) / 128));
   float* ws = nullptr;
   {
-    const int32_t got = take_scratch(err, reinterpret_cast<void**>(&ws), 2 * (a_plane + b_plane) * sizeof(float), s);
+    const int32_t got = take_scratch(err, reinterpret_cast<void**>(&ws), (2 * (a_plane + b_plane) + flags) * sizeof(float), s);
     if (got != TSM100_OK) return got;
   }
   float *a_hi = ws, *a_lo = ws + a_plane, *b_hi = ws + 2 * a_plane, *b_lo = b_hi + b_plane;
+  uint32_t* flag_words = reinterpret_cast<uint32_t*>(b_lo + b_plane);
   const float* af = static_cast<const float*>(a);
   const float* bf = static_cast<const float*>(b);
   st = split_operands_launch(err, {af, a_hi, a_lo, ld.lda, static_cast<int64_t>(M) * ld.lda, static_cast<int64_t>(M), static_cast<int32_t>(K), static_cast<int32_t>(kp), 0},
                              {bf, b_hi, b_lo, ld.ldb, static_cast<int64_t>(d->b_transposed ? N : K) * ld.ldb, static_cast<int64_t>(N), static_cast<int32_t>(K), static_cast<int32_t>(kp), 0},
-                             !d->b_transposed, d->batch, sms, s);
+                             !d->b_transposed, d->batch, sms, s, flag_words, flags);
   CUtensorMap ta_hi, ta_lo, tb_hi, tb_lo;
   const CUtensorMapDataType f32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
   // Problems with more than one 128-row and 128-column block run on CTA pairs (256 x 256 or 256 x 128 tiles); the rest
@@ -753,6 +757,7 @@ inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, 
     // short K (relative to the 64-bit result: FP32 pipe 2.9e-7 at K = 257, 6.9e-7 at 1501; here 9e-7 with chunks of 128,
     // 3.8e-7 with 64, 1.4e-7 .. 1.8e-7 with 32)
     p.chunk_kb = rows_aligned ? 4 : K >= 512 ? 2 : 1;
+    p.flags = flag_words;
     p.b_transposed = d->b_transposed;
     p.a = af, p.b = bf;
     p.lda = ld.lda, p.ldb = ld.ldb;
