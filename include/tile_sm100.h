@@ -75,7 +75,7 @@ int32_t tsm100_mem_info(tsm100_device_t dev, size_t* free_bytes, size_t* total_b
 int32_t tsm100_device_sm_count(tsm100_device_t dev, int32_t* sms);
 /* Synchronises `stream`, then reads and clears the device's kernel status word:
  * 0, or 0x1000|site when a kernel gave up one of its bounded waits (mbarrier,
- * tensor-core completion).  The reference has no device-side error channel;
+ * tensor-core completion); a site number belongs to one kernel source file.  The reference has no device-side error channel;
  * check_cu (crates/tile_hal/src/cuda.rs:124-130) sees driver codes only. */
 int32_t tsm100_device_status(tsm100_device_t dev, void* stream, uint32_t* status);
 

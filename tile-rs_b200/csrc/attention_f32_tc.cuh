@@ -42,6 +42,7 @@ static_assert(128 * (kRegsOther + kRegsSoftmax + kRegsDrain) <= kThreads * 168, 
 constexpr int kTmemCols = 512;
 constexpr int kTmemO = 0, kTmemS = 256, kTmemP = 320, kTmemQ = 384;  // two accumulators of 128, two of 32, 32 hi + 32 lo, 128
 constexpr float kRescaleThreshold = 8.0f;              // log2 units
+// its bounded waits report sites 71 .. 84
 
 template <int D>
 struct Shape {
@@ -179,7 +180,7 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
       const int total = 2 * n;
       for (int idx = 0; idx < total; ++idx) {
         const int slot = idx % kRing;
-        if (!ptx::mbar_wait(&bars->kv_empty[slot], ((idx / kRing) & 1u) ^ 1u, abort_flag, status, 31)) break;
+        if (!ptx::mbar_wait(&bars->kv_empty[slot], ((idx / kRing) & 1u) ^ 1u, abort_flag, status, 71)) break;
         ptx::mbar_arrive_expect_tx(&bars->kv_full[slot], Sh::kUnitBytes);
         const bool is_v = idx == total - 1 || (idx >= 2 && (idx & 1) == 0);
         const int step = idx == 0 ? 0 : idx == total - 1 ? n - 1 : is_v ? (idx >> 1) - 1 : (idx + 1) >> 1;
@@ -204,21 +205,21 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
     auto desc = [](uint32_t lo) -> uint64_t { return (static_cast<uint64_t>(k_hi32) << 32) | lo; };
     const uint32_t ring_lo = k_lo32 | (ptx::smem_u32(ring) >> 4);
     auto wait_kv = [&](int idx) -> bool {
-      const bool r = ptx::mbar_wait_relaxed(&bars->kv_full[idx % kRing], (idx / kRing) & 1u, abort_flag, status, 32);
+      const bool r = ptx::mbar_wait_relaxed(&bars->kv_full[idx % kRing], (idx / kRing) & 1u, abort_flag, status, 72);
       return __all_sync(0xffffffffu, r);
     };
     bool ok = true;
     if (warp == 9) {
       constexpr uint32_t idesc = gemm_tf32_tc::make_idesc_tf32(kBQ, kBKV);
       const uint32_t q_lo32 = k_lo32 | (ptx::smem_u32(smem) >> 4);
-      ok = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->q_ready, 0, abort_flag, status, 33));
+      ok = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->q_ready, 0, abort_flag, status, 73));
       ptx::tcgen05_fence_after_thread_sync();
       volatile uint32_t* pv_steps = &bars->pv_steps;
       for (int j = 0; j < n && ok; ++j) {
         // not before the P V of step j - 2 is queued: the tensor core would take this product first
-        if (j >= 2 && !(ok = __all_sync(0xffffffffu, ptx::wait_counter_ge(pv_steps, static_cast<uint32_t>(j - 1), abort_flag, status, 34)))) break;
+        if (j >= 2 && !(ok = __all_sync(0xffffffffu, ptx::wait_counter_ge(pv_steps, static_cast<uint32_t>(j - 1), abort_flag, status, 74)))) break;
         if (!(ok = wait_kv(k_pos(j)))) break;
-        if (j >= 2 && !(ok = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&bars->s_free[j & 1], ((j - 2) >> 1) & 1u, abort_flag, status, 35)))) break;
+        if (j >= 2 && !(ok = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&bars->s_free[j & 1], ((j - 2) >> 1) & 1u, abort_flag, status, 75)))) break;
         ptx::tcgen05_fence_after_thread_sync();
         const uint32_t d = tmem + kTmemS + (j & 1) * kBKV;
         const uint32_t b_hi = ring_lo + (k_pos(j) % kRing) * (Sh::kUnitBytes >> 4), b_lo = b_hi + (Sh::kUnitPlane >> 4);
@@ -247,8 +248,8 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
         const int c = j / kChunkSteps, acc = c & 1;
         const bool first = j % kChunkSteps == 0, last = j % kChunkSteps == kChunkSteps - 1 || j == n - 1;
         if (!(ok = wait_kv(v_pos(j)))) break;
-        if (first && c >= 2 && !(ok = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&bars->o_empty[acc], ((c - 2) >> 1) & 1u, abort_flag, status, 36)))) break;
-        if (!(ok = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->p_ready, j & 1u, abort_flag, status, 37)))) break;
+        if (first && c >= 2 && !(ok = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&bars->o_empty[acc], ((c - 2) >> 1) & 1u, abort_flag, status, 76)))) break;
+        if (!(ok = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->p_ready, j & 1u, abort_flag, status, 77)))) break;
         ptx::tcgen05_fence_after_thread_sync();
         const uint32_t d = tmem + kTmemO + acc * 128;
         const uint32_t a_hi = tmem + kTmemP, a_lo = a_hi + kBKV;
@@ -282,7 +283,7 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
     bool alive = true;
     for (int j = 0; j < n; ++j) {
       const int b = j & 1;
-      if (!__all_sync(0xffffffffu, ptx::mbar_wait(&bars->s_full[b], (j >> 1) & 1u, abort_flag, status, 38))) {
+      if (!__all_sync(0xffffffffu, ptx::mbar_wait(&bars->s_full[b], (j >> 1) & 1u, abort_flag, status, 78))) {
         alive = false;
         break;
       }
@@ -311,7 +312,7 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
           m_used = m_new;
         }
       } else if (__any_sync(0xffffffffu, (m_new - m_used) * sl2 > kRescaleThreshold)) {
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done, (j - 1) & 1u, abort_flag, status, 39))) {
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done, (j - 1) & 1u, abort_flag, status, 79))) {
           alive = false;
           break;
         }
@@ -347,7 +348,7 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
       }
       l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
       // P of step j - 1 has been read
-      if (j >= 1 && !__all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done, (j - 1) & 1u, abort_flag, status, 40))) {
+      if (j >= 1 && !__all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done, (j - 1) & 1u, abort_flag, status, 80))) {
         alive = false;
         break;
       }
@@ -369,7 +370,7 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
     }
     // the row sum takes the slot after the last chunk's, once the last product has retired: by then the chunk that had it
     // (chunks - 3) is drained
-    if (alive && __all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done, (n - 1) & 1u, abort_flag, status, 41))) {
+    if (alive && __all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done, (n - 1) & 1u, abort_flag, status, 81))) {
       row_slot[(chunks % 3) * kBQ + r] = l;
       ptx::mbar_arrive(&bars->l_ready);
     }
@@ -387,8 +388,8 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
     bool alive = true;
     for (int c = 0; c < chunks; ++c) {
       const int acc = c & 1;
-      bool ready = ptx::mbar_wait(&bars->m_ready[c % 3], (c / 3) & 1u, abort_flag, status, 42);
-      ready = ready && ptx::mbar_wait(&bars->o_full[acc], (c >> 1) & 1u, abort_flag, status, 43);
+      bool ready = ptx::mbar_wait(&bars->m_ready[c % 3], (c / 3) & 1u, abort_flag, status, 82);
+      ready = ready && ptx::mbar_wait(&bars->o_full[acc], (c >> 1) & 1u, abort_flag, status, 83);
       if (!__all_sync(0xffffffffu, ready)) {
         alive = false;
         break;
@@ -408,7 +409,7 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
       ptx::tcgen05_fence_before_thread_sync();
       ptx::mbar_arrive(&bars->o_empty[acc]);
     }
-    if (alive && __all_sync(0xffffffffu, ptx::mbar_wait(&bars->l_ready, 0, abort_flag, status, 44))) {
+    if (alive && __all_sync(0xffffffffu, ptx::mbar_wait(&bars->l_ready, 0, abort_flag, status, 84))) {
       const float inv = 1.0f / row_slot[(chunks % 3) * kBQ + r];
       if (q0 + r < p.seq) {
         float4* orow = reinterpret_cast<float4*>(o + bh * p.o_head_stride + (q0 + r) * p.o_row_stride);
