@@ -246,7 +246,7 @@ int32_t tsm100_gemm_static_scratch(const tsm100_gemm_desc* desc, const void* a, 
  * __tile_attention_gqa_* as the NVIDIA emitter defines it
  * (mlir_to_gpu.rs:1624-1711): kv_head = h / (heads_q/heads_kv), always causal
  * there.  Replaces mlir_to_gpu.rs:1976-1979 (unhandled) and :1624-1711.
- * 16-bit Q/K/V use tensor cores with f32 softmax statistics (head_dim 32 / 64 / 128: tcgen05; 96: warp-level
+ * 16-bit Q/K/V use tensor cores with f32 softmax statistics (head_dim 32 / 64 / 128: tcgen05; 96, and short sequences of 32 and 64: warp-level
  * MMA); f32 Q/K/V with head_dim 32 / 64 / 96 / 128 use tensor cores with three TF32 products per product
  * (results agree with an f32 evaluation to 1e-5).  Other head sizes, or rows that do not start on 16-byte
  * boundaries: FP32 pipe. */

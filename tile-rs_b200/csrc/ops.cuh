@@ -36,6 +36,7 @@
 #include "gemm_tc2.cuh"
 #include "gemm_tf32_tc.cuh"
 #include "gemm_tf32x3.cuh"
+#include "route.hpp"
 #include "rowops.cuh"
 #include "softmax.cuh"
 
@@ -1347,11 +1348,17 @@ inline int32_t attention_fwd_launch(std::string* err, const CUtensorMap& tq, con
 
 // Which 16-bit problems run on the tcgen05 kernel: head_dim 128, and 32 and 64 on its 64-wide form.  96 stays on the TF32
 // kernel: the second P tile that keeps the probabilities' precision does not fit beside 128-wide tiles.  b4, 32 / 8 heads of
-// 64, 2000 tokens, causal: 724 us on the TF32 kernel, 171 here; both 1.6e-3 from the 64-bit result, the rounding of bf16.
-inline bool attention_tc_ok(int32_t dtype, int32_t head_dim, const uint32_t* status, const void* q, const void* k,
-                            const void* v, const void* o) {
-  return dtype != TSM100_F32 && (head_dim == attn::kD || head_dim == 32 || head_dim == 64) && status != nullptr &&
-         aligned16(q) && aligned16(k) && aligned16(v) && aligned16(o);
+// 64, 2000 tokens, causal: 724 us on the TF32 kernel, 171 here; both 1.6e-3 from the 64-bit result, the rounding of bf16.  Short
+// sequences of 32 and 64 stay there too (route.hpp).  rows: query rows per head, heads: of all problems.
+inline bool attention_tc_ok(int32_t dtype, int32_t head_dim, int64_t rows, int64_t heads, int64_t seq_kv, const uint32_t* status,
+                            const void* q, const void* k, const void* v, const void* o) {
+  if (dtype == TSM100_F32 || status == nullptr || !aligned16(q) || !aligned16(k) || !aligned16(v) || !aligned16(o)) return false;
+  if (head_dim == attn::kD) return true;
+  if (head_dim != 32 && head_dim != 64) return false;
+  int sms = 0;
+  std::string unused;
+  if (sm_count(&unused, &sms) != TSM100_OK) return false;
+  return route::attention_narrow_on_tcgen05(head_dim, seq_kv, route::div_up(rows, 2 * attn::kBQ) * heads, sms);
 }
 
 template <bool kBf16, int D>
@@ -1397,7 +1404,7 @@ inline int32_t attention_prefill(std::string* err, const tsm100_attention_prefil
   if (d->head_dim > attn_simt::kMaxD) return op_fail(err, TSM100_ERR_INVALID, "attention_prefill: head_dim > 256 unsupported");
   if (d->seq_len == 0) return TSM100_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (attention_tc_ok(d->dtype, d->head_dim, status, q, k, v, o)) {
+  if (attention_tc_ok(d->dtype, d->head_dim, d->seq_len, d->heads_q, static_cast<int64_t>(d->start_pos) + d->seq_len, status, q, k, v, o)) {
     const bool wide = d->head_dim == attn::kD;
     if (d->dtype == TSM100_BF16)
       return wide ? attention_prefill_tc_launch<true, 128>(err, d, q, k, v, o, status, s)
@@ -1710,7 +1717,7 @@ inline int32_t attention(std::string* err, const tsm100_attention_desc* d, const
     return op_fail(err, TSM100_ERR_INVALID, "attention: heads_q must be a positive multiple of heads_kv");
   if (d->head_dim > attn_simt::kMaxD) return op_fail(err, TSM100_ERR_INVALID, "attention: head_dim > 256 unsupported");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (attention_tc_ok(d->dtype, d->head_dim, status, q, k, v, o)) {
+  if (attention_tc_ok(d->dtype, d->head_dim, d->seq, static_cast<int64_t>(d->batch) * d->heads_q, d->seq, status, q, k, v, o)) {
     const bool wide = d->head_dim == attn::kD;
     if (d->dtype == TSM100_BF16)
       return wide ? attention_tc_launch<true, 128>(err, d, q, k, v, o, status, s) : attention_tc_launch<true, 64>(err, d, q, k, v, o, status, s);
