@@ -11,6 +11,10 @@ SOURCE = """
 #include "route.hpp"
 using namespace tsm100::route;
 extern "C" int attention_narrow(int d, long long kv, long long blocks, int sms) { return attention_narrow_on_tcgen05(d, kv, blocks, sms); }
+extern "C" void gemm16_plan(long long m, long long n, long long k, long long batch, int sms, long long* out) {
+  const Gemm16 r = gemm16(m, n, k, batch, sms);
+  out[0] = r.kind, out[1] = r.rows, out[2] = r.splits, out[3] = r.k_blocks_per_cta;
+}
 """
 
 
@@ -29,3 +33,45 @@ def lib(tmp_path_factory):
     (32, 64, 4096, False), (32, 128, 4096, False), (32, 129, 149, True), (32, 129, 148, False), (32, 448, 148, False), (32, 449, 1, True)])
 def test_short_sequences_of_narrow_heads_stay_on_the_warp_level_kernel(lib, d, kv, blocks, tcgen05):
     assert lib.attention_narrow(d, C.c_longlong(kv), C.c_longlong(blocks), SMS) == tcgen05
+
+
+PAIRS, SINGLES, FEW = 0, 1, 2
+
+
+def gemm16(lib, m, n, k, batch):
+    out = (C.c_longlong * 4)()
+    lib.gemm16_plan(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch), SMS, out)
+    return tuple(out)
+
+
+# the few-tiles kernel, and how far it splits K
+@pytest.mark.parametrize("m,n,k,batch,kind,splits", [
+    (16, 16384, 4096, 1, FEW, 2), (16, 4096, 16384, 1, FEW, 8), (300, 4096, 16384, 1, FEW, 2), (1024, 1024, 4096, 1, FEW, 4),
+    # two CTAs only for a long K; short ones unsplit or on the persistent kernels
+    (1024, 1024, 512, 1, FEW, 1), (192, 64, 512, 1, SINGLES, 1), (192, 64, 1024, 1, FEW, 4), (100, 16384, 2048, 1, SINGLES, 1),
+    # many small problems: persistent kernels
+    (1, 4096, 128, 1024, SINGLES, 1), (16, 4096, 64, 64, SINGLES, 1), (16, 512, 2048, 64, FEW, 1), (16, 512, 4096, 64, SINGLES, 1), (32, 512, 64, 1024, SINGLES, 1), (128, 64, 64, 1024, SINGLES, 1),
+    (128, 64, 512, 1, SINGLES, 1), (64, 4096, 128, 64, SINGLES, 1), (256, 256, 256, 128, PAIRS, 1),
+    # many rows of few columns
+    (65536, 64, 64, 1, SINGLES, 1), (65536, 64, 4096, 1, FEW, 1), (65536, 8, 1024, 1, FEW, 1),
+    # pairs from 38 pair tiles on
+    (256 * 37, 256, 1024, 1, FEW, 1), (256 * 38, 256, 1024, 1, PAIRS, 1), (8192, 8192, 8192, 1, PAIRS, 1)])
+def test_16_bit_products(lib, m, n, k, batch, kind, splits):
+    plan = gemm16(lib, m, n, k, batch)
+    assert plan[0] == kind and (kind != FEW or plan[2] == splits), plan
+
+
+def test_16_bit_plans_fit_a_launch(lib):
+    """Every CTA of a split has work, and no problem that the persistent kernels take is refused for its number of tiles."""
+    import random
+    rng = random.Random(5)
+    size = lambda top: int(2 ** rng.uniform(0, top))  # noqa: E731
+    for _ in range(20000):
+        m, n, k, batch = size(20), 8 * size(17), 8 * size(14), size(31 - 0.01)
+        kind, rows, splits, per = gemm16(lib, m, n, k, batch)
+        tiles, kb = -(-m // rows) * -(-n // 128) * batch, -(-k // 64)
+        if kind == FEW:
+            assert tiles * splits <= 0x7fffffff and (splits == 1 or tiles * splits <= 2 * SMS) and (-(-kb // per) - 1) * per < kb
+            assert rows == (16 if m <= 16 else 32 if m <= 32 else 64 if m <= 64 else 128)
+        assert (kind == PAIRS) <= (m > 128 and n > 128)
+    assert gemm16(lib, 1 << 20, 128, 8192, 1 << 20)[0] == SINGLES  # 2^33 tiles of 128 x 128

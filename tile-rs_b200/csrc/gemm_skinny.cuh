@@ -1,5 +1,5 @@
 // 16-bit GEMM for problems with few output tiles: a handful of rows of A against a large B (the projections of a decoding
-// step), and any shape whose 256 x 256 tiles leave most SM pairs of gemm_tc2.cuh without one.
+// step), and any shape whose 256 x 256 tiles leave most SM pairs of gemm_tc2.cuh without one (the rule is in route.hpp).
 //
 //   C[b][M,N] = A[b][M,K] * B[b], semantics and operand forms as in gemm_tc.cuh (crates/tile_std/src/tile.rs:1982-1986,
 //   :2017-2031; crates/rustc_codegen_tile/src/mlir_to_linalg.rs:1345-1393).

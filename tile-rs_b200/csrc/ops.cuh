@@ -856,9 +856,10 @@ inline int32_t gemm_tc_launch(std::string* err, const tsm100_gemm_desc* d, const
 }
 
 // Few output tiles: 128 columns x NT rows of C per CTA, K split over clusters (gemm_skinny.cuh).
+static_assert(gemm_skinny::kMaxSplit == route::kMaxGemmSplit && gemm_skinny::kBK == 64 && gemm_skinny::kBN == 128, "route.hpp plans in these units");
 template <typename OutT, bool kBT, bool kBf16, int NT>
 inline int32_t gemm_skinny_launch_nt(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
-                                     uint32_t* status, cudaStream_t s) {
+                                     const route::Gemm16& plan, uint32_t* status, cudaStream_t s) {
   namespace g = gemm_skinny;
   CUtensorMap ta, tb;
   const uint64_t M = d->m, N = d->n, K = d->k, B = d->batch;
@@ -871,9 +872,6 @@ inline int32_t gemm_skinny_launch_nt(std::string* err, const tsm100_gemm_desc* d
   else
     st = make_tmap_16bit_3d(err, &tb, b, N, K, B, ldb, K * ldb, 64, g::kBK, kBf16);
   if (st != TSM100_OK) return st;
-  int sms = 0;
-  st = sm_count(err, &sms);
-  if (st != TSM100_OK) return st;
   g::Params p;
   p.m = static_cast<int32_t>(M);
   p.n = static_cast<int32_t>(N);
@@ -885,13 +883,8 @@ inline int32_t gemm_skinny_launch_nt(std::string* err, const tsm100_gemm_desc* d
   p.ldc = ld.ldc;
   p.status = status;
   const int64_t tiles = static_cast<int64_t>(p.m_blocks) * p.n_blocks * p.batch;
-  if (tiles * g::kMaxSplit > 0x7fffffff) return op_fail(err, TSM100_ERR_INVALID, "gemm: too many tiles for one launch");
-  // K over a cluster while all CTAs still fit the GPU at once (two per SM) and each keeps at least four k-blocks
-  const int32_t kb = static_cast<int32_t>((K + g::kBK - 1) / g::kBK);
-  int splits = 1;
-  while (splits < g::kMaxSplit && tiles * splits * 2 <= 2ll * sms && kb / (2 * splits) >= 4) splits *= 2;
-  p.kb_per_cta = (kb + splits - 1) / splits;
-  splits = (kb + p.kb_per_cta - 1) / p.kb_per_cta;  // rounding up may leave a last CTA without work: drop it
+  p.kb_per_cta = static_cast<int32_t>(plan.k_blocks_per_cta);
+  const int64_t kb = (K + g::kBK - 1) / g::kBK, splits = (kb + p.kb_per_cta - 1) / p.kb_per_cta;  // a last CTA without work is dropped
   auto kern = g::gemm_skinny_kernel<OutT, kBT, kBf16, NT>;
   constexpr int smem = g::smem_bytes<NT>();
   cudaError_t e = set_dyn_smem_once(kern, smem);
@@ -913,11 +906,13 @@ inline int32_t gemm_skinny_launch_nt(std::string* err, const tsm100_gemm_desc* d
 }
 template <typename OutT, bool kBT, bool kBf16>
 inline int32_t gemm_skinny_launch(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
-                                  uint32_t* status, cudaStream_t s) {
-  if (d->m <= 16) return gemm_skinny_launch_nt<OutT, kBT, kBf16, 16>(err, d, a, b, c, status, s);
-  if (d->m <= 32) return gemm_skinny_launch_nt<OutT, kBT, kBf16, 32>(err, d, a, b, c, status, s);
-  if (d->m <= 64) return gemm_skinny_launch_nt<OutT, kBT, kBf16, 64>(err, d, a, b, c, status, s);
-  return gemm_skinny_launch_nt<OutT, kBT, kBf16, 128>(err, d, a, b, c, status, s);
+                                  const route::Gemm16& plan, uint32_t* status, cudaStream_t s) {
+  switch (plan.rows) {
+    case 16: return gemm_skinny_launch_nt<OutT, kBT, kBf16, 16>(err, d, a, b, c, plan, status, s);
+    case 32: return gemm_skinny_launch_nt<OutT, kBT, kBf16, 32>(err, d, a, b, c, plan, status, s);
+    case 64: return gemm_skinny_launch_nt<OutT, kBT, kBf16, 64>(err, d, a, b, c, plan, status, s);
+    default: return gemm_skinny_launch_nt<OutT, kBT, kBf16, 128>(err, d, a, b, c, plan, status, s);
+  }
 }
 
 // CTA-pair kernel (256 x 256 tile per two SMs), launched as clusters of two.
@@ -1085,17 +1080,11 @@ inline int32_t gemm(std::string* err, const tsm100_gemm_desc* d, const void* a, 
     int sms = 0;
     int32_t st = sm_count(err, &sms);
     if (st != TSM100_OK) return st;
-    // CTA pairs where 256 x 256 tiles keep enough pairs busy.  Below, splitting K pays, unless K is short: 1024 x 2048 x 2048
-    // (32 pair tiles) 16.1 us on pairs, 16.8 split; 1024 x 1024 x 4096 24.8 / 16.0, 300 x 4096 x 16384 78.9 / 62.4.
-    const int64_t pair_tiles = ((d->m + 255) / 256) * ((d->n + 255) / 256) * d->batch;
-    const bool pair = d->m > 128 && d->n > 128 && (pair_tiles > sms / 4 || (pair_tiles > sms / 6 && d->k <= 2048));
-    // 65 .. 128 rows and 128 x 256 tiles for (nearly) all SMs: the persistent single-CTA kernel, whose accumulators alternate
-    // (128 x 16384 x 4096, batch 4: 95.4 us, 97.9 on the split kernel; batch 1, 64 tiles: 35.5 / 31.7)
-    const int64_t tiles = ((d->m + 127) / 128) * ((d->n + 255) / 256) * d->batch;
-    const bool single = d->m > 64 && d->n > 128 && d->m <= 128 && tiles * 8 >= sms * 6;
-#define TSM_GEMM_TC(OUT, BT, BF)                                                     \
-  return pair     ? gemm_tc2_launch<OUT, BT, BF>(err, d, a, b, c, status, s)         \
-         : single ? gemm_tc_launch<OUT, BT, BF>(err, d, a, b, c, status, s) : gemm_skinny_launch<OUT, BT, BF>(err, d, a, b, c, status, s)
+    const route::Gemm16 plan = route::gemm16(d->m, d->n, d->k, d->batch, sms);
+#define TSM_GEMM_TC(OUT, BT, BF)                                                                                \
+  return plan.kind == route::Gemm16::kPairs     ? gemm_tc2_launch<OUT, BT, BF>(err, d, a, b, c, status, s) \
+         : plan.kind == route::Gemm16::kSingles ? gemm_tc_launch<OUT, BT, BF>(err, d, a, b, c, status, s)  \
+                                                : gemm_skinny_launch<OUT, BT, BF>(err, d, a, b, c, plan, status, s)
     if (bf16) {
       if (out_f32) { if (d->b_transposed) TSM_GEMM_TC(float, true, true); else TSM_GEMM_TC(float, false, true); }
       else { if (d->b_transposed) TSM_GEMM_TC(__nv_bfloat16, true, true); else TSM_GEMM_TC(__nv_bfloat16, false, true); }

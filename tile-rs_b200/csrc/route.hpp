@@ -22,5 +22,49 @@ inline bool attention_narrow_on_tcgen05(int32_t head_dim, int64_t seq_kv, int64_
   return seq_kv > (query_blocks > sms ? 128 : 448);
 }
 
+// 16-bit GEMM on the tensor cores: CTA pairs (256 x 256 tiles, gemm_tc2.cuh), single CTAs (128 x 256 tiles, gemm_tc.cuh; both
+// persistent) or the few-tiles kernel (128 columns x `rows` rows of C per CTA, K over `splits` CTAs of a cluster, gemm_skinny.cuh).
+struct Gemm16 {
+  enum Kind { kPairs, kSingles, kFewTiles } kind;
+  int rows;             // few tiles: rows of C per CTA
+  int splits;
+  int64_t k_blocks_per_cta;  // 64 of K each
+};
+constexpr int kMaxGemmSplit = 8;
+
+inline Gemm16 gemm16(int64_t m, int64_t n, int64_t k, int64_t batch, int sms) {
+  Gemm16 r{Gemm16::kFewTiles, m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128, 1, 0};
+  const bool wide = r.rows == 128;
+  const int64_t tiles = div_up(m, r.rows) * div_up(n, 128) * batch, kb = div_up(k, 64);
+  // K over a cluster while all CTAs fit the GPU at once, two per SM, and keep four k-blocks (128-row tiles: eight, once the
+  // second CTA of an SM is taken).  Two CTAs alone do not earn a cluster's launch while K is short: 192 x 64 x 512 7.5 unsplit,
+  // 9.3 in two; 300 x 4096 x 4096 24.0 / 21.6.
+  while (r.splits < kMaxGemmSplit && tiles * r.splits * 2 <= 2 * sms &&
+         kb / (2 * r.splits) >= (wide && tiles * r.splits * 2 > sms ? 8 : 4)) r.splits *= 2;
+  if (r.splits == 2 && kb < (wide ? 64 : 32)) r.splits = 1;
+  r.k_blocks_per_cta = div_up(kb, r.splits);
+  bool few;
+  if (m > 128 && n > 128) {
+    // pairs once 256 x 256 tiles are there for more than half of them: 24 .. 36 of them 0.83 .. 1.0 of the pairs' time at any K,
+    // 37 .. 48 0.99 .. 1.29
+    few = div_up(m, 256) * div_up(n, 256) * batch <= sms / 4;
+    if (!few) r.kind = Gemm16::kPairs;
+  } else {
+    // Unsplit, the few-tiles kernel starts a CTA per tile and hides nothing of its start and end but behind a second CTA; the
+    // persistent kernel loads the next tile meanwhile.  So it pays for tiles that are all there at once, and beyond that where a
+    // 256-wide tile would be half empty (n <= 128) and K long enough.  Persistent / few tiles: 16 x 4096 x
+    // 4096 23.3 / 8.4, 16 x 4096 x 128 of a batch of 256 48 / 93, 128 x 64 x 64 of 1024 11 / 21, 32 x 64 x 4096 of 1024 175 / 127.
+    if (r.splits > 1) few = true;
+    else if (m <= 16) few = tiles <= (kb < 64 ? 2 : 1) * sms || (n <= 128 && kb >= 8);
+    else if (m <= 32) few = tiles <= sms || (n <= 128 && (tiles <= 2 * sms || kb >= 16));
+    else if (m <= 64) few = n > 128 ? tiles <= sms : kb >= 16 || (kb >= 8 && tiles <= 2 * sms);
+    else few = n <= 128 && (kb >= 64 || (n <= 32 && tiles >= 2 * sms));
+    if (!few) r.kind = Gemm16::kSingles;
+  }
+  // one CTA per tile has to fit one launch
+  if (few && tiles * r.splits > 0x7fffffff) r.kind = m > 128 && n > 128 ? Gemm16::kPairs : Gemm16::kSingles;
+  return r;
+}
+
 }  // namespace route
 }  // namespace tsm100
