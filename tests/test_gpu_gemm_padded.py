@@ -11,7 +11,8 @@ pytestmark = pytest.mark.gpu
 # 16-bit rows that start anywhere: operands copied into padded scratch, in every combination of what needs it
 @pytest.mark.parametrize("m,n,k,bt,batch,offset,ldc", [
     (300, 301, 1203, False, 1, 0, 0), (300, 301, 1203, True, 1, 0, 0), (257, 512, 1001, True, 2, 0, 0), (511, 257, 1024, False, 3, 0, 0),
-    (400, 520, 512, False, 1, 1, 0), (400, 520, 512, True, 1, 0, 523), (28, 3134, 4883, False, 1, 0, 0)])
+    (400, 520, 512, False, 1, 1, 0), (400, 520, 512, True, 1, 0, 523), (28, 3134, 4883, False, 1, 0, 0),
+    (30, 101, 23003, False, 1, 0, 0), (1, 1001, 67103, True, 1, 0, 0), (30, 101, 1003, False, 23, 0, 0)])
 def test_bf16_rows_that_start_anywhere(dev, pkg, oracle, m, n, k, bt, batch, offset, ldc):
     capi = pkg.capi
     sigma = k ** -0.25

@@ -15,6 +15,7 @@ extern "C" void gemm16_plan(long long m, long long n, long long k, long long bat
   const Gemm16 r = gemm16(m, n, k, batch, sms);
   out[0] = r.kind, out[1] = r.rows, out[2] = r.splits, out[3] = r.k_blocks_per_cta;
 }
+extern "C" int padding_pays(long long m, long long n, long long k, long long batch) { return gemm16_padding_pays(m, n, k, batch); }
 """
 
 
@@ -75,3 +76,13 @@ def test_16_bit_plans_fit_a_launch(lib):
             assert rows == (16 if m <= 16 else 32 if m <= 32 else 64 if m <= 64 else 128)
         assert (kind == PAIRS) <= (m > 128 and n > 128)
     assert gemm16(lib, 1 << 20, 128, 8192, 1 << 20)[0] == SINGLES  # 2^33 tiles of 128 x 128
+
+
+@pytest.mark.parametrize("m,n,k,batch,pays", [
+    (2000, 3001, 2501, 1, True), (500, 1001, 999, 1, True), (28, 3134, 4883, 1, True),
+    (2000, 3001, 17, 1, False), (8001, 10001, 7, 1, False), (2000, 3001, 33, 1, False), (8001, 1001, 33, 1, True), (2000, 3001, 65, 1, True),
+    (100, 101, 103, 1, False), (64, 64, 65, 500, True), (64, 64, 65, 64, False),
+    # few outputs, long K: counted in products, not in 4096ths of outputs
+    (1, 3001, 50001, 1, True), (30, 101, 1003, 64, True), (1, 501, 4001, 1, False), ((1 << 31) - 1, (1 << 31) - 1, (1 << 31) - 1, 1, True)])
+def test_16_bit_products_of_odd_sizes(lib, m, n, k, batch, pays):
+    assert lib.padding_pays(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch)) == pays

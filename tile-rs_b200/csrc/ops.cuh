@@ -1094,11 +1094,11 @@ inline int32_t gemm(std::string* err, const tsm100_gemm_desc* d, const void* a, 
     }
 #undef TSM_GEMM_TC
   }
-  // Rows that start anywhere: worth the copies into padded scratch from about 2^26 products on.  Only for 16-bit results,
-  // whose last place hides the order of the f32 sums; an f32 result keeps the FP32 pipe's rounding to nearest.
+  // Rows that start anywhere: copied into padded scratch where that pays.  Only for 16-bit results, whose last place hides the
+  // order of the f32 sums; an f32 result keeps the FP32 pipe's rounding to nearest.
   const int64_t n8 = (d->n + 7) / 8 * 8, k8 = (d->k + 7) / 8 * 8;
-  if (status != nullptr && !out_f32 && d->m * d->n / 4096 * d->k * d->batch >= 1 << 14 && d->batch <= 65535 && n8 <= 0x7fffffff && k8 <= 0x7fffffff &&
-      ((d->m + 15) / 16) * ((n8 + 95) / 96) * d->batch * gemm_skinny::kMaxSplit <= 0x7fffffff) {
+  if (status != nullptr && !out_f32 && d->batch <= 65535 && n8 <= 0x7fffffff && k8 <= 0x7fffffff &&
+      route::gemm16_padding_pays(d->m, d->n, d->k, d->batch) && (d->m + 127) / 128 * ((n8 + 255) / 256) * d->batch < 0x7fffffff) {
     const int32_t st = gemm_padded(err, d, a, b, c, status, s);
     if (st != kNoScratch) return st;
   }

@@ -66,5 +66,13 @@ inline Gemm16 gemm16(int64_t m, int64_t n, int64_t k, int64_t batch, int sms) {
   return r;
 }
 
+// 16-bit products whose rows start anywhere: copies into padded scratch and the tensor cores (gemm_pad.cuh), or the FP32 pipe.  The
+// copies cost launches (hence the 2^26 products) and traffic per row, column and output, whatever K is: FP32 pipe / padded 2000 x 3001 x
+// 17 20.6 / 31.7, x 33 29 / 32, x 65 46 / 33; 8001 x 10001 x 7 130 / 280, x 17 226 / 282, x 33 328 / 282.
+inline bool gemm16_padding_pays(int64_t m, int64_t n, int64_t k, int64_t batch) {
+  const double outputs = static_cast<double>(m) * n * batch;
+  return outputs * k >= 67108864.0 && (k >= 64 || (k >= 32 && outputs >= 7340032.0));
+}
+
 }  // namespace route
 }  // namespace tsm100
