@@ -53,10 +53,17 @@ def test_any_start(dev, name, cols):
     check(dev, name, x, offset=1, offset_y=2)  # x and y at different offsets from a boundary
 
 
+# rows for all SMs, read twice by CTAs of 1024, 512 and 256 threads, whose steps end with the row or before it
 @pytest.mark.parametrize("name", ["f32", "bf16", "f16"])
-@pytest.mark.parametrize("cols", [33, 3001, 50001])
-def test_masks_and_specials(dev, name, cols):
-    x = rows_of(name, 8, cols, 9)
+@pytest.mark.parametrize("rows,cols", [(120, 8200), (148, 32771), (149, 16387), (149, 65536), (300, 16387), (300, 24576), (250, 520), (320, 1111)])
+def test_many_rows(dev, name, rows, cols):
+    check(dev, name, rows_of(name, rows, cols, cols))
+
+
+@pytest.mark.parametrize("name", ["f32", "bf16", "f16"])
+@pytest.mark.parametrize("rows,cols", [(8, 33), (8, 3001), (8, 50001), (149, 20001), (300, 1111), (300, 20001)])
+def test_masks_and_specials(dev, name, rows, cols):
+    x = rows_of(name, rows, cols, 9)
     low = torch.finfo(KIND[name][0]).min
     x[0, cols // 2:] = float("-inf")   # a half that is masked out: whole warps and CTAs see nothing but -inf
     x[1, :-1] = float("-inf")

@@ -16,6 +16,10 @@ extern "C" void gemm16_plan(long long m, long long n, long long k, long long bat
   out[0] = r.kind, out[1] = r.rows, out[2] = r.splits, out[3] = r.k_blocks_per_cta;
 }
 extern "C" int padding_pays(long long m, long long n, long long k, long long batch) { return gemm16_padding_pays(m, n, k, batch); }
+extern "C" int row_per_warp(long long span, long long rows, int sms) { return softmax_row_per_warp(span, rows, sms); }
+extern "C" int cluster(long long span, long long rows, int sms) { return softmax_cluster(span, rows, sms); }
+extern "C" int twice_skip(long long vectors, int threads) { return softmax_twice_skip(vectors, threads, 4); }
+extern "C" int twice_threads(long long bytes, long long rows, int sms) { return softmax_twice_threads(bytes, rows, sms); }
 """
 
 
@@ -86,3 +90,27 @@ def test_16_bit_plans_fit_a_launch(lib):
     (1, 3001, 50001, 1, True), (30, 101, 1003, 64, True), (1, 501, 4001, 1, False), ((1 << 31) - 1, (1 << 31) - 1, (1 << 31) - 1, 1, True)])
 def test_16_bit_products_of_odd_sizes(lib, m, n, k, batch, pays):
     assert lib.padding_pays(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch)) == pays
+
+
+@pytest.mark.parametrize("span,rows,warp", [(10, 1, True), (128, 1, True), (129, 1, False), (256, 296, False), (256, 297, True), (257, 5000, False)])
+def test_softmax_of_rows_that_start_anywhere(lib, span, rows, warp):
+    assert lib.row_per_warp(C.c_longlong(span), C.c_longlong(rows), SMS) == warp
+
+
+# vectors of a row, rows -> CTAs of a cluster, or 0: one CTA that reads the row twice
+@pytest.mark.parametrize("span,rows,ctas", [
+    (1026, 1, 2), (1026, 98, 2), (1026, 99, 0), (7501, 74, 8), (7501, 75, 0), (4098, 100, 5), (4098, 148, 0), (8192, 1, 8),
+    (8193, 32, 3), (8193, 74, 0), (16384, 32, 4), (16384, 148, 0), (32000, 32, 8), (32768, 1, 8), (32769, 1, 0), (2000, 149, 0)])
+def test_softmax_of_a_few_wide_rows(lib, span, rows, ctas):
+    assert lib.cluster(C.c_longlong(span), C.c_longlong(rows), SMS) == ctas
+
+
+@pytest.mark.parametrize("row_bytes,rows,threads", [
+    (100002, 1000, 256), (100002, 296, 512), (100002, 148, 1024), (200004, 1000, 512), (600000, 1000, 1024), (1 << 32, 1000, 1024)])
+def test_softmax_of_rows_read_twice(lib, row_bytes, rows, threads):
+    assert lib.twice_threads(C.c_longlong(row_bytes), C.c_longlong(rows), SMS) == threads
+
+
+@pytest.mark.parametrize("vectors,threads,skip", [(8192, 512, False), (8193, 512, True), (2250, 256, True), (3000, 256, False), (1026, 1024, True)])
+def test_softmax_steps_behind_the_row(lib, vectors, threads, skip):
+    assert lib.twice_skip(C.c_longlong(vectors), threads) == skip

@@ -318,7 +318,7 @@ inline int32_t softmax_typed(std::string* err, const T* x, T* y, int64_t rows, i
   const int64_t span = (cols + 2 * PV - 2) / PV;  // the most 16-byte vectors a row can touch
   if (((xa ^ ya) & 15u) == 0 && xa % sizeof(T) == 0 && cols <= 1 << 30) {
     const int32_t c = static_cast<int32_t>(cols);
-    if (span <= 32 * 8 && rows <= 4ll * 0x7fffffff) {
+    if (route::softmax_row_per_warp(span, rows, sms) && rows <= 4ll * 0x7fffffff) {
       constexpr int WARPS = 4;
       const unsigned grid = static_cast<unsigned>((rows + WARPS - 1) / WARPS);
       if (span <= 32 * 2) softmax::softmax_rows_warp_any<T, 2, WARPS><<<grid, WARPS * 32, 0, s>>>(x, y, rows, c);
@@ -336,21 +336,23 @@ inline int32_t softmax_typed(std::string* err, const T* x, T* y, int64_t rows, i
       else launch(softmax::softmax_rows_cta_any<T, 4, 256>, 256);
       return cuda_ok(err, cudaGetLastError(), "softmax_rows_cta_any launch");
     }
-    // a row per SM or fewer (141 rows of 54588 f16: 21 us with a CTA per row, 11.5): a cluster per row, CTAs of 256 threads and 4 vectors each while eight of them hold a row
-    if (span <= 8 * 512 * 8 && rows <= sms) {
-      const int64_t ctas = (span + 1023) / 1024;
-      if (ctas <= 8) return softmax_cluster_launch<T, 4, 256>(err, x, y, rows, cols, ctas, s);
-      return softmax_cluster_launch<T, 8, 512>(err, x, y, rows, cols, (span + 4095) / 4096, s);
+    if (const int ctas = route::softmax_cluster(span, rows, sms)) {
+      if (span <= 8 * 1024) return softmax_cluster_launch<T, 4, 256>(err, x, y, rows, cols, ctas, s);
+      return softmax_cluster_launch<T, 8, 512>(err, x, y, rows, cols, ctas, s);
     }
-    // one CTA per row, 1024 threads per SM in 4, 2 or 1 CTAs: as many as keep their rows within half of the L2 (126 MB).  1000
-    // rows of 50001 bf16: 97 us scalar, 49 here; 1212 of 97648 f32 286 / 214; 2000 of 16392 bf16 (in shared memory) 45 / 31
-    const int64_t fit = (64ll << 20) / (cols * static_cast<int64_t>(sizeof(T)) * sms);
-    auto launch = [&](auto kern, int threads) {
-      kern<<<static_cast<unsigned>(std::min<int64_t>(rows, sms * (1024ll / threads))), threads, 0, s>>>(x, y, rows, c);
-    };
-    if (fit >= 4) launch(softmax::softmax_rows_twice<T, 256>, 256);
-    else if (fit >= 2) launch(softmax::softmax_rows_twice<T, 512>, 512);
-    else launch(softmax::softmax_rows_twice<T, 1024>, 1024);
+    // one CTA per row.  1000 rows of 50001 bf16: 97 us scalar, 49 here; 1212 of 97648 f32 286 / 214; 2000 of 16392 bf16 (in shared
+    // memory) 45 / 31
+    const int threads = route::softmax_twice_threads(cols * static_cast<int64_t>(sizeof(T)), rows, sms);
+    auto launch = [&](auto kern) { kern<<<static_cast<unsigned>(std::min<int64_t>(rows, sms * (1024ll / threads))), threads, 0, s>>>(x, y, rows, c); };
+    if (route::softmax_twice_skip((cols + PV - 1) / PV, threads, softmax::kTwiceUnroll)) {
+      if (threads == 256) launch(softmax::softmax_rows_twice<T, 256, true>);
+      else if (threads == 512) launch(softmax::softmax_rows_twice<T, 512, true>);
+      else launch(softmax::softmax_rows_twice<T, 1024, true>);
+    } else {
+      if (threads == 256) launch(softmax::softmax_rows_twice<T, 256, false>);
+      else if (threads == 512) launch(softmax::softmax_rows_twice<T, 512, false>);
+      else launch(softmax::softmax_rows_twice<T, 1024, false>);
+    }
     return cuda_ok(err, cudaGetLastError(), "softmax_rows_twice launch");
   }
   constexpr int THREADS = 512;

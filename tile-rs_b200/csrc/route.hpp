@@ -74,5 +74,42 @@ inline bool gemm16_padding_pays(int64_t m, int64_t n, int64_t k, int64_t batch) 
   return outputs * k >= 67108864.0 && (k >= 64 || (k >= 32 && outputs >= 7340032.0));
 }
 
+// Row softmax whose rows start anywhere or are too wide for one CTA's registers (softmax.cuh); `span`: the most 16-byte vectors a row
+// can touch.
+// 129 .. 256 vectors: a warp per row while there are rows for all warps, else a CTA.  1111 bf16, 200 rows 3.7 a warp, 2.9 a CTA, 600
+// 3.7 / 3.6, 4000 8.1 / 14; 513 f32, 200 rows 2.5 / 2.4, 600 2.6 / 3.1.
+inline bool softmax_row_per_warp(int64_t span, int64_t rows, int sms) { return span <= 128 || (span <= 256 && rows > 2 * sms); }
+
+// More than 1024 vectors: how many CTAs of a cluster share a row, or 0 for one CTA per row that reads it twice.  CTAs of 256 threads
+// and 1024 vectors (four of which fit an SM) while eight of them hold a row, of 512 threads and 4096 vectors beyond.  A cluster
+// reads a row once, but has to fit the GPU with all others: a second wave costs more than the second read.  Cluster / twice: f32 74 rows of
+// 30001 6.1 / 7.6, 130 of 28000 9.4 / 8.0, 148 of 32776 19 / 8.6, 32 of 128000 16.5 / 23; bf16 74 of 50001 5.7 / 7.5, 148 of 65536 20 / 9.0.
+// Two or three CTAs for a hundred rows and more do not earn the exchange between them (f32 130 of 4099 4.0 / 3.5).
+inline int softmax_cluster(int64_t span, int64_t rows, int sms) {
+  if (rows > sms || span > 8 * 4096) return 0;
+  if (span <= 8 * 1024) {
+    const int64_t ctas = div_up(span, 1024);
+    const bool fits = 3 * rows <= 2 * sms ? rows * ctas <= 4 * sms : ctas >= 4 && rows * ctas < 4 * sms;
+    return fits ? static_cast<int>(ctas) : 0;
+  }
+  // a wave of such CTAs takes 5.3 us, reading rows twice 4.5 us and 1 us for 2048 vectors
+  const int64_t ctas = div_up(span, 4096), waves = div_up(rows * ctas, sms);
+  return 53 * waves < 45 + 10 * span / 2048 ? static_cast<int>(ctas) : 0;
+}
+
+// Threads of a CTA that reads its rows twice, 1024 of them per SM in all: as many CTAs as keep their rows within half of the L2 (126
+// MB), but not more than there are rows.  f32 149 rows of 16400 8.3 in CTAs of 256, 7.7 in CTAs of 512; bf16 149 of 50001 10.6 / 9.9.
+inline int softmax_twice_threads(int64_t row_bytes, int64_t rows, int sms) {
+  const int64_t fit = (64ll << 20) / (row_bytes * sms);
+  if (fit >= 4 && rows > 2 * sms) return 256;
+  return fit >= 2 && rows > sms ? 512 : 1024;
+}
+// Whether more than an eighth of the row's work would fall behind its end if every thread took whole steps of `unroll` vectors.  f32 1000
+// rows of 9000 18.7 with whole steps, 16.0 without; bf16 1000 of 65536 57 / 61.
+inline bool softmax_twice_skip(int64_t vectors, int threads, int unroll) {
+  const int64_t step = static_cast<int64_t>(threads) * unroll;
+  return (div_up(vectors, step) * step - vectors) * 8 > vectors;
+}
+
 }  // namespace route
 }  // namespace tsm100

@@ -18,7 +18,8 @@
 //     4096-wide configuration runs here with eight resident CTAs per SM).
 //   * softmax_rows_warp_any, softmax_rows_cta_any: a warp or a CTA per row that
 //     starts anywhere.
-//   * softmax_rows_twice: wider rows of any alignment, one CTA each, the second read from the L2.
+//   * softmax_rows_twice: wider rows of any alignment, one CTA each, read twice, the
+//     second time from the L2 up to 450 KB a row.
 //   * softmax_rows_cluster: a few such rows, a cluster of CTAs each.
 //   * softmax_rows_stream: any width, x and y at different offsets from a 16-byte
 //     boundary; online max/sum in a first pass, normalisation in a second (two
@@ -473,16 +474,19 @@ softmax_rows_cta_any(const T* __restrict__ x, T* __restrict__ y, int64_t rows, i
   }
 }
 
-// One CTA per row of any width and alignment, the row read twice, the second time from the L2 (the host keeps the rows in
-// flight small enough for that): online maximum and sum per thread, then the exponentials again.  No copy of the row in
-// shared memory or registers: several CTAs per SM are in different phases, and HBM reads, exponentials and writes overlap
-// (2000 rows of 16392 bf16: 44.8 us with the row in shared memory, 33.4 here).
-template <typename T, int THREADS>
+// One CTA per row of any width and alignment, the row read twice, the second time from the L2 as long as the rows in flight fit
+// half of it (one row per SM: 450 KB; wider rows come from HBM twice): online maximum and sum per thread, then the exponentials
+// again.  No copy of the row in shared memory or registers: several CTAs per SM are in different phases, and HBM reads,
+// exponentials and writes overlap (2000 rows of 16392 bf16: 44.8 us with the row in shared memory, 30.9 here).
+// kSkip: a thread's steps of four vectors end with the row (with 1024 threads a row of 1100 vectors would otherwise be four times
+// as much work); for rows that fill their steps the test costs 7 % and is left out.
+constexpr int kTwiceUnroll = 4;
+template <typename T, int THREADS, bool kSkip>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 softmax_rows_twice(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t cols) {
   constexpr int PV = Elem<T>::kPerVec;
   constexpr int NW = THREADS / 32;
-  constexpr int UNROLL = 4;
+  constexpr int UNROLL = kTwiceUnroll;
   __shared__ float2 slots[2][NW];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   int parity = 0;
@@ -493,9 +497,11 @@ softmax_rows_twice(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int
     for (int32_t i0 = tid; i0 < nvec; i0 += UNROLL * THREADS) {
       Vec16 raw[UNROLL];
 #pragma unroll
-      for (int u = 0; u < UNROLL; ++u) raw[u] = span.template load<true>(i0 + u * THREADS);
+      for (int u = 0; u < UNROLL; ++u)
+        if (!kSkip || i0 + u * THREADS < nvec) raw[u] = span.template load<true>(i0 + u * THREADS);
 #pragma unroll
       for (int u = 0; u < UNROLL; ++u) {
+        if (kSkip && i0 + u * THREADS >= nvec) break;
         float f[PV];
         Elem<T>::unpack(raw[u], f);
         float mv = f[0];
@@ -522,9 +528,11 @@ softmax_rows_twice(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int
     for (int32_t i0 = tid; i0 < nvec; i0 += UNROLL * THREADS) {
       Vec16 raw[UNROLL];
 #pragma unroll
-      for (int u = 0; u < UNROLL; ++u) raw[u] = span.load(i0 + u * THREADS);
+      for (int u = 0; u < UNROLL; ++u)
+        if (!kSkip || i0 + u * THREADS < nvec) raw[u] = span.load(i0 + u * THREADS);
 #pragma unroll
       for (int u = 0; u < UNROLL; ++u) {
+        if (kSkip && i0 + u * THREADS >= nvec) break;
         float f[PV];
         Elem<T>::unpack(raw[u], f);
 #pragma unroll
