@@ -18,6 +18,7 @@ extern "C" void gemm16_plan(long long m, long long n, long long k, long long bat
 extern "C" int padding_pays(long long m, long long n, long long k, long long batch) { return gemm16_padding_pays(m, n, k, batch); }
 extern "C" int row_per_warp(long long span, long long rows, int sms) { return softmax_row_per_warp(span, rows, sms); }
 extern "C" int cluster(long long span, long long rows, int sms) { return softmax_cluster(span, rows, sms); }
+extern "C" int rope_heads(long long blocks, int heads, int sms) { return rope_heads_per_thread(blocks, heads, sms); }
 extern "C" int twice_skip(long long vectors, int threads) { return softmax_twice_skip(vectors, threads, 4); }
 extern "C" int twice_threads(long long bytes, long long rows, int sms) { return softmax_twice_threads(bytes, rows, sms); }
 """
@@ -114,3 +115,9 @@ def test_softmax_of_rows_read_twice(lib, row_bytes, rows, threads):
 @pytest.mark.parametrize("vectors,threads,skip", [(8192, 512, False), (8193, 512, True), (2250, 256, True), (3000, 256, False), (1026, 1024, True)])
 def test_softmax_steps_behind_the_row(lib, vectors, threads, skip):
     assert lib.twice_skip(C.c_longlong(vectors), threads) == skip
+
+
+@pytest.mark.parametrize("blocks,heads,per", [
+    (1, 32, 4), (1, 3, 4), (1, 5, 8), (8, 32, 4), (74, 64, 16), (75, 12, 12), (75, 24, 8), (148, 64, 32), (149, 64, 64), (1184, 32, 32)])
+def test_rotary_head_groups(lib, blocks, heads, per):
+    assert lib.rope_heads(C.c_longlong(blocks), heads, SMS) == per

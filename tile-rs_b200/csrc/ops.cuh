@@ -519,9 +519,7 @@ inline int32_t rope(std::string* err, const tsm100_rope_desc* d, void* x, void* 
   auto launch = [&](auto* xt) {
     using T = std::remove_pointer_t<decltype(xt)>;
     if (vec) {
-      // groups of four heads or more, as many as make two blocks per SM
-      const int64_t want = (2ll * sms + grid - 1) / grid, groups = std::max<int64_t>(1, std::min<int64_t>(want, d->heads / 4));
-      const int32_t heads_per = static_cast<int32_t>(((d->heads + groups - 1) / groups + 3) / 4 * 4);
+      const int32_t heads_per = route::rope_heads_per_thread(grid, d->heads, sms);
       const dim3 grid2(grid, static_cast<unsigned>((d->heads + heads_per - 1) / heads_per));
       rowops::rope_vec_kernel<T><<<grid2, 256, 0, s>>>(xt, tokens, d->seq_len, d->heads, heads_per, d->head_dim, d->start_pos, d->theta);
     }
