@@ -270,7 +270,9 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+// The .aligned forms need the whole warp at the instruction: lanes that a loop or a branch before has parted meet here.
 __device__ __forceinline__ void cluster_sync_all() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 // Programmatic dependent launch: a kernel launched with that attribute starts while the kernel before it in the stream still

@@ -581,7 +581,6 @@ softmax_rows_cluster(const T* __restrict__ x, T* __restrict__ y, int64_t rows, i
     }
   s = warp_sum(s);
   if (lane == 0) slots[warp] = make_float2(m, s);
-  __syncwarp();
   ptx::cluster_sync_all();
   float gm = -INFINITY, gs = 0.f;
   float2 pair[(8 * NW + 31) / 32];
@@ -606,7 +605,6 @@ softmax_rows_cluster(const T* __restrict__ x, T* __restrict__ y, int64_t rows, i
     for (int e = 0; e < PV; ++e) v[k][e] *= factor;
     span.store(y_base, (k * ctas + rank) * THREADS + tid, v[k]);
   }
-  __syncwarp();
   ptx::cluster_sync_all();  // nobody leaves while its pairs may still be read
 }
 
