@@ -134,6 +134,19 @@ int32_t tsm100_launch(tsm100_module_t mod, const char* name, uint32_t blocks, vo
                       uint32_t nargs, void* stream);
 
 /* ---- operators on device memory ---------------------------------------- */
+/* Scratch.  Some operators take device memory for the length of a call:
+ *   tsm100_gemm, f32, 64 tiles of 128 x 256 and K >= 256 or more: 8 bytes per element of A and B (and 4 per 128 x 128 of C);
+ *   tsm100_gemm, 16 bit, sizes or rows that are no multiple of 16 bytes, 2^26 products or more: padded copies of A, B, C;
+ *   tsm100_attention and _prefill, f32, 64 query rows and 256 keys or more: twice the bytes of K and V;
+ *   the same in 16 bit, 4096 keys or more and query blocks for at most half of the SMs: up to 20 MB;
+ *   tsm100_attention_decode, 16 bit, few caches of 1024 positions or more: up to 2.5 MB.
+ * It is taken and returned on the caller's stream, from a pool of the library's own on each device (the device's default
+ * memory pool is neither used nor changed).  The pool keeps up to 1/16 of the device's memory for later calls and gives it
+ * back when the device's last handle is closed.  When the device has no memory left, such a call takes a form without
+ * scratch: slower, and with its sums in another order.
+ * While a stream is captured, taking and returning become allocation nodes of the graph.  The graph can be replayed any
+ * number of times; as CUDA has it for graphs with such nodes, it has one executable instance at a time and cannot be a
+ * child graph or be cloned. */
 /* Row softmax, y[r,:] = softmax(x[r,:]).  __tile_softmax_f32 / _f16
  * (crates/tile_std/src/tile.rs:189-190, :2162-2163; wrappers :2295-2305,
  * :2912-2920); semantics `linalg.softmax dimension(1)`

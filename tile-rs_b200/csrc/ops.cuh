@@ -6,7 +6,7 @@
 // Every function returns a TSM100_* status and, on failure, writes a message
 // to *err.  Nothing here synchronises; the operators that need device scratch (operand
 // planes of the tcgen05 f32 kernels, padded copies, partial results) take it from, and
-// return it to, the device's stream-ordered memory pool on the caller's stream.
+// return it to, the library's own memory pool on the caller's stream (scratch.hpp).
 #pragma once
 
 #include <cuda.h>
@@ -38,6 +38,7 @@
 #include "gemm_tf32x3.cuh"
 #include "route.hpp"
 #include "rowops.cuh"
+#include "scratch.hpp"
 #include "softmax.cuh"
 
 namespace tsm100 {
@@ -59,12 +60,12 @@ inline int32_t cuda_ok(std::string* err, cudaError_t e, const char* what) {
 // and a form without scratch exists: the dispatch then takes that one.
 constexpr int32_t kNoScratch = -1;
 inline int32_t take_scratch(std::string* err, void** ws, size_t bytes, cudaStream_t s) {
-  const cudaError_t e = cudaMallocAsync(ws, bytes, s);
-  if (e == cudaErrorMemoryAllocation) {
+  const cudaError_t e = scratch::take(ws, bytes, s);
+  if (e == cudaErrorMemoryAllocation || e == cudaErrorNotSupported) {
     (void)cudaGetLastError();
     return kNoScratch;
   }
-  return cuda_ok(err, e, "cudaMallocAsync");
+  return cuda_ok(err, e, "scratch from the library's memory pool");
 }
 
 inline size_t dtype_size(int32_t dtype) { return dtype == TSM100_F32 ? 4 : 2; }
@@ -650,24 +651,6 @@ inline int32_t gemm_tf32x3_launch(std::string* err, const tsm100_gemm_desc* d, c
   return cuda_ok(err, e, "gemm_tf32x3_kernel launch");
 }
 
-// The device's default memory pool keeps what is freed into it (no trimming at synchronisation points), so
-// that after the first call cudaMallocAsync / cudaFreeAsync are bookkeeping on the stream.  Once per device.
-inline cudaError_t keep_pool_memory_once() {
-  cudaError_t e = cudaSuccess;
-  int unused = 0;
-  kernel_fact(nullptr, 5, &unused, [&](int* out) {
-    int dev = 0;
-    cudaMemPool_t pool;
-    e = cudaGetDevice(&dev);
-    if (e == cudaSuccess) e = cudaDeviceGetDefaultMemPool(&pool, dev);
-    uint64_t keep = ~0ull;
-    if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-    *out = 1;
-    return e == cudaSuccess;
-  });
-  return e;
-}
-
 // Columns of a pair's tile: the width whose waves of tiles over the SM pairs take the least time.  A 128-wide tile
 // costs two thirds of a 256-wide one, not half (its operand traffic per product is 4/3 and a chunk's drain overlaps
 // half the products): 4096^3 655 us in 4 wide waves, 757 in 7 narrow ones; 1536^3 79 us in one wide wave, 56 in one narrow.
@@ -712,8 +695,7 @@ inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, 
   int sms = 0;
   int32_t st = sm_count(err, &sms);
   if (st != TSM100_OK) return st;
-  cudaError_t e = keep_pool_memory_once();
-  if (e != cudaSuccess) return cuda_ok(err, e, "cudaMemPoolSetAttribute");
+  cudaError_t e = cudaSuccess;
   const uint64_t kp = (K + 3) / 4 * 4;  // row pitch of the planes: every row starts on a 16-byte boundary
   const size_t a_plane = static_cast<size_t>(B) * M * kp, b_plane = static_cast<size_t>(B) * N * kp;  // elements
   // rows that start anywhere: a flag per 128 x 128 block of C, behind the planes
@@ -988,8 +970,7 @@ inline int32_t gemm_padded(std::string* err, const tsm100_gemm_desc* d, const vo
   int sms = 0;
   int32_t st = sm_count(err, &sms);
   if (st != TSM100_OK) return st;
-  cudaError_t e = keep_pool_memory_once();
-  if (e != cudaSuccess) return cuda_ok(err, e, "cudaMemPoolSetAttribute");
+  cudaError_t e = cudaSuccess;
   const GemmPitch ld = gemm_pitch(d);
   const int64_t np = (d->n + 7) / 8 * 8, kp = (d->k + 7) / 8 * 8, batch = d->batch;
   const int64_t b_rows = d->b_transposed ? d->n : d->k, b_cols = d->b_transposed ? d->k : d->n;
@@ -1161,8 +1142,7 @@ inline int32_t attention_f32_tc_launch_d(std::string* err, const attn_simt::Para
   int sms = 0;
   int32_t st = sm_count(err, &sms);
   if (st != TSM100_OK) return st;
-  cudaError_t e = keep_pool_memory_once();
-  if (e != cudaSuccess) return cuda_ok(err, e, "cudaMemPoolSetAttribute");
+  cudaError_t e = cudaSuccess;
   const uint64_t n_kv = static_cast<uint64_t>(p.batch) * p.heads_kv, len = p.seq_kv, len4 = (len + 3) / 4 * 4;
   const size_t k_plane = n_kv * len * D, v_plane = n_kv * len4 * D;
   float* ws = nullptr;
@@ -1295,8 +1275,6 @@ inline int32_t attention_fwd_launch(std::string* err, const CUtensorMap& tq, con
   const size_t rows = static_cast<size_t>(blocks) * p.splits * (2 * at::kBQ);
   float* ws = nullptr;
   if (p.splits > 1) {
-    st = cuda_ok(err, keep_pool_memory_once(), "cudaMemPoolSetAttribute");
-    if (st != TSM100_OK) return st;
     st = take_scratch(err, reinterpret_cast<void**>(&ws), rows * (D + 2) * sizeof(float), s);
     if (st == kNoScratch) p.splits = 1;
     else if (st != TSM100_OK) return st;
@@ -1501,8 +1479,7 @@ inline int32_t attention_decode_global_launch(std::string* err, const tsm100_att
   namespace ad = attn_decode;
   constexpr int WARPS = 8, STAGES = 3;
   const int64_t units = static_cast<int64_t>(d->batch) * d->heads_kv;
-  cudaError_t e = keep_pool_memory_once();
-  if (e != cudaSuccess) return cuda_ok(err, e, "cudaMemPoolSetAttribute");
+  cudaError_t e = cudaSuccess;
   float* ws = nullptr;
   {
     const int32_t got = take_scratch(err, reinterpret_cast<void**>(&ws), static_cast<size_t>(units) * splits * ad::mma::kRows * (D + 2) * sizeof(float), s);

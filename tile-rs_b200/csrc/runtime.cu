@@ -8,8 +8,11 @@
 #include <dlfcn.h>
 
 #include <cstring>
+#include <map>
+#include <mutex>
 
 #include "common.hpp"
+#include "scratch.hpp"
 
 namespace tsm100 {
 
@@ -50,6 +53,16 @@ int32_t read_status(tsm100_device_t dev, cudaStream_t stream, uint32_t* value) {
   *value = v;
   return TSM100_OK;
 }
+
+namespace {
+// Open handles of a device, after adding `change`.
+int open_handles(int ordinal, int change) {
+  static std::mutex mu;
+  static std::map<int, int> count;
+  std::lock_guard<std::mutex> lock(mu);
+  return count[ordinal] += change;
+}
+}  // namespace
 
 }  // namespace tsm100
 
@@ -105,6 +118,7 @@ int32_t tsm100_device_open(int32_t ordinal, tsm100_device_t* out) {
     delete d;
     return check_cuda(e, TSM100_ERR_MEMORY, "status word allocation");
   }
+  open_handles(ordinal, 1);
   *out = d;
   return TSM100_OK;
 }
@@ -121,6 +135,7 @@ int32_t tsm100_device_close(tsm100_device_t dev) {
   if (p.dev_buf) cudaFree(p.dev_buf);
   if (p.pin_buf) cudaFreeHost(p.pin_buf);
   if (dev->status) cudaFree(dev->status);
+  if (open_handles(dev->ordinal, -1) == 0) scratch::give_back(dev->ordinal);
   delete dev;
   return TSM100_OK;
 }
