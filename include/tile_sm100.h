@@ -139,7 +139,7 @@ int32_t tsm100_launch(tsm100_module_t mod, const char* name, uint32_t blocks, vo
  *   tsm100_gemm, 16 bit, sizes or rows that are no multiple of 16 bytes, 2^26 products or more: padded copies of A, B, C;
  *   tsm100_attention and _prefill, f32, 64 query rows and 256 keys or more: twice the bytes of K and V;
  *   the same in 16 bit, 4096 keys or more and query blocks for at most half of the SMs: up to 20 MB;
- *   tsm100_attention_decode, 16 bit, few caches of 1024 positions or more: up to 2.5 MB.
+ *   tsm100_attention_decode, 16 bit, few caches of 1024 positions or more: up to 1.3 MB.
  * It is taken and returned on the caller's stream, from a pool of the library's own on each device (the device's default
  * memory pool is neither used nor changed).  The pool keeps up to 1/16 of the device's memory for later calls and gives it
  * back when the device's last handle is closed.  When the device has no memory left, such a call takes a form without
@@ -313,7 +313,11 @@ int32_t tsm100_kv_cache_update(tsm100_device_t dev, const tsm100_kv_cache_update
  * __tile_attention_prefill_f32 (tile.rs:2134-2136; wrapper :3062-3074); arithmetic of
  * crates/rustc_codegen_tile/src/mlir_to_msl.rs:10928-11010 without that lowering's limit of 256 cache positions
  * (its `threadgroup float scores[256]`).  The same kernels as tsm100_attention serve it (tensor cores for
- * head_dim 128 in 16 bit and for head_dim 32 / 64 / 96 / 128 in f32 and 32 / 64 / 96 in 16 bit). */
+ * head_dim 32 / 64 / 96 / 128).  A prompt given in chunks yields the bits of the whole prompt in one call (and of causal
+ * tsm100_attention) while every call runs on the same kernel and its KV steps are not dealt to several CTAs: 16 bit,
+ * head_dim 128, fewer than 4096 positions; head_dim 64, the same with chunks that end behind position 64; head_dim 96 at any
+ * length; f32 with chunks of 64 tokens or more that end at 256 positions or more.  Otherwise the sums are taken in
+ * another order and agree to their rounding. */
 typedef struct {
   int32_t dtype;
   int32_t heads_q;

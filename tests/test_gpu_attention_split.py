@@ -70,3 +70,27 @@ def test_a_step_of_infinite_scores(dev, pkg, oracle, d, first):
     x = qf @ kf.T / np.sqrt(d)
     p = np.exp(x - x.max(-1, keepdims=True))
     util.assert_16bit_close(oracle, o[0], ((p / p.sum(-1, keepdims=True)) @ vf).astype(np.float32))
+
+
+# a prompt in two chunks against the whole prompt in one call: the same bits while neither is split (fewer than 4096 positions) and
+# both run on one kernel; beyond, the same to the rounding of sums in another order
+@pytest.mark.parametrize("dtype,d,total,first,same", [
+    ("bf16", 128, 4095, 3969, True), ("bf16", 128, 4095, 130, True), ("f16", 128, 4000, 3990, True), ("bf16", 64, 4095, 65, True),
+    ("bf16", 96, 5000, 4500, True), ("f32", 128, 700, 300, True), ("f32", 64, 5000, 4900, True),
+    ("bf16", 128, 4096, 3900, False), ("bf16", 64, 5000, 40, False), ("f32", 128, 700, 680, False)])
+def test_prompt_in_chunks(dev, pkg, dtype, d, total, first, same):
+    capi = pkg.capi
+    code = {"bf16": capi.BF16, "f16": capi.F16, "f32": capi.F32}[dtype]
+    narrow = {"bf16": lambda t: util.to_bf16(capi, t), "f16": util.f32_to_f16_bits, "f32": lambda t: t}[dtype]
+    q = narrow(util.gen_normal(capi, (total, 2, d), 771))
+    k, v = (narrow(util.gen_normal(capi, (1, total, d), 772 + i)) for i in range(2))
+    whole = run_prefill(dev, capi, q, k, v, 0, code)
+    parts = np.concatenate([run_prefill(dev, capi, np.ascontiguousarray(q[:first]), k, v, 0, code),
+                            run_prefill(dev, capi, np.ascontiguousarray(q[first:]), k, v, first, code)])
+    if same:
+        assert np.array_equal(whole.view(np.uint8), parts.view(np.uint8))
+        return
+    wide = {"bf16": lambda t: (t.view(np.uint16).astype(np.uint32) << 16).view(np.float32), "f16": lambda t: t.view(np.float16), "f32": lambda t: t}[dtype]
+    a, b = wide(whole).astype(np.float64), wide(parts).astype(np.float64)
+    # f32: the bound of the operator; bf16: each side rounds the probabilities and the result once, 2^-9 each
+    assert np.linalg.norm(a - b) <= (1e-5 if dtype == "f32" else 2.0 ** -7) * np.linalg.norm(a)

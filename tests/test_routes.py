@@ -18,6 +18,7 @@ extern "C" void gemm16_plan(long long m, long long n, long long k, long long bat
 extern "C" int padding_pays(long long m, long long n, long long k, long long batch) { return gemm16_padding_pays(m, n, k, batch); }
 extern "C" int row_per_warp(long long span, long long rows, int sms) { return softmax_row_per_warp(span, rows, sms); }
 extern "C" int cluster(long long span, long long rows, int sms) { return softmax_cluster(span, rows, sms); }
+extern "C" int splits(long long blocks, long long keys, int sms) { return attention_splits(blocks, keys, sms); }
 extern "C" int rope_heads(long long blocks, int heads, int sms) { return rope_heads_per_thread(blocks, heads, sms); }
 extern "C" int twice_skip(long long vectors, int threads) { return softmax_twice_skip(vectors, threads, 4); }
 extern "C" int twice_threads(long long bytes, long long rows, int sms) { return softmax_twice_threads(bytes, rows, sms); }
@@ -121,3 +122,9 @@ def test_softmax_steps_behind_the_row(lib, vectors, threads, skip):
     (1, 32, 4), (1, 3, 4), (1, 5, 8), (8, 32, 4), (74, 64, 16), (75, 12, 12), (75, 24, 8), (148, 64, 32), (149, 64, 64), (1184, 32, 32)])
 def test_rotary_head_groups(lib, blocks, heads, per):
     assert lib.rope_heads(C.c_longlong(blocks), heads, SMS) == per
+
+
+@pytest.mark.parametrize("blocks,keys,ctas", [
+    (1, 1, 1), (1, 3969, 1), (1, 4095, 1), (1, 4096, 2), (64, 16384, 2), (74, 1 << 20, 2), (75, 1 << 20, 1), (9, 34000, 16), (1, 1 << 20, 148), (1 << 20, 8192, 1)])
+def test_attention_steps_over_several_ctas(lib, blocks, keys, ctas):
+    assert lib.splits(C.c_longlong(blocks), C.c_longlong(keys), SMS) == ctas

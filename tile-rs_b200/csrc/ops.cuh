@@ -1254,14 +1254,11 @@ inline int32_t attention_kv_band(uint64_t kv_len, int64_t kv_heads, uint64_t hea
   return static_cast<int32_t>(std::max<int64_t>(1, std::min<int64_t>(band, std::max<int64_t>(kv_heads, 1))));
 }
 
-// Launches the tcgen05 attention kernel over `blocks` query blocks of at most kv_steps 128-key steps.  With blocks for at
-// most half of the SMs (one CTA fills an SM) the steps of a block are dealt to as many CTAs as the SMs allow, 16 steps (2048
-// keys) or more each, and merged by a second kernel.  512 tokens on 15872, 32 heads (64 blocks): 212 us unsplit, 122 split.
-// Up to 4095 keys a call is never split, so a prompt in chunks gives the bits of the whole one.
-constexpr int64_t kAttentionSplitSteps = 16;
+// Launches the tcgen05 attention kernel over `blocks` query blocks that see at most `keys` keys, the KV steps of a block dealt to
+// several CTAs and merged by a second kernel where route.hpp says so.
 template <bool kBf16, bool kCache, int D>
 inline int32_t attention_fwd_launch(std::string* err, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, void* o,
-                                    attn::Params p, int64_t blocks, int64_t kv_steps, cudaStream_t s) {
+                                    attn::Params p, int64_t blocks, int64_t keys, cudaStream_t s) {
   namespace at = attn;
   constexpr int smem = at::smem_bytes<D>();
   int sms = 0;
@@ -1269,7 +1266,7 @@ inline int32_t attention_fwd_launch(std::string* err, const CUtensorMap& tq, con
   if (st != TSM100_OK) return st;
   uint16_t* out = static_cast<uint16_t*>(o);
   p.blocks = static_cast<int32_t>(blocks);
-  p.splits = static_cast<int32_t>(std::max<int64_t>(1, std::min<int64_t>(sms / blocks, kv_steps / kAttentionSplitSteps)));
+  p.splits = route::attention_splits(blocks, keys, sms);
   p.part = nullptr;
   p.part_ml = nullptr;
   const size_t rows = static_cast<size_t>(blocks) * p.splits * (2 * at::kBQ);
@@ -1356,7 +1353,7 @@ inline int32_t attention_prefill_tc_launch(std::string* err, const tsm100_attent
   p.head_dim = d->head_dim;
   const int64_t grid = static_cast<int64_t>(p.q_blocks) * d->heads_q;
   if (grid > 0x7fffffff) return op_fail(err, TSM100_ERR_INVALID, "attention_prefill: too many tiles for one launch");
-  return attention_fwd_launch<kBf16, true, D>(err, tq, tk, tv, o, p, grid, (static_cast<int64_t>(kv_len) + at::kBKV - 1) / at::kBKV, s);
+  return attention_fwd_launch<kBf16, true, D>(err, tq, tk, tv, o, p, grid, static_cast<int64_t>(kv_len), s);
 }
 
 inline int32_t attention_prefill(std::string* err, const tsm100_attention_prefill_desc* d, const void* q, const void* k,
@@ -1669,7 +1666,7 @@ inline int32_t attention_tc_launch(std::string* err, const tsm100_attention_desc
   p.head_dim = d->head_dim;
   const int64_t grid = static_cast<int64_t>(p.q_blocks) * nq;
   if (grid > 0x7fffffff) return op_fail(err, TSM100_ERR_INVALID, "attention: too many tiles for one launch");
-  return attention_fwd_launch<kBf16, false, D>(err, tq, tk, tv, o, p, grid, (d->seq + at::kBKV - 1) / at::kBKV, s);
+  return attention_fwd_launch<kBf16, false, D>(err, tq, tk, tv, o, p, grid, d->seq, s);
 }
 
 inline int32_t attention(std::string* err, const tsm100_attention_desc* d, const void* q, const void* k,

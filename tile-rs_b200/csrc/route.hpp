@@ -22,6 +22,14 @@ inline bool attention_narrow_on_tcgen05(int32_t head_dim, int64_t seq_kv, int64_
   return seq_kv > (query_blocks > sms ? 128 : 448);
 }
 
+// 16-bit attention on tcgen05: how many CTAs share the KV steps of a query block.  One CTA fills an SM, so the steps are dealt out when
+// there are blocks for at most half of the SMs, 2048 keys or more to each.  512 tokens on 15872, 32 heads (64 blocks): 212 unsplit, 122
+// split.  Below 4096 keys a call is never split, so that a prompt in chunks gives the bits of the whole one.
+constexpr int64_t kAttentionSplitKeys = 2048;
+inline int attention_splits(int64_t blocks, int64_t keys, int sms) {
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(sms / blocks, keys / kAttentionSplitKeys)));
+}
+
 // 16-bit GEMM on the tensor cores: CTA pairs (256 x 256 tiles, gemm_tc2.cuh), single CTAs (128 x 256 tiles, gemm_tc.cuh; both
 // persistent) or the few-tiles kernel (128 columns x `rows` rows of C per CTA, K over `splits` CTAs of a cluster, gemm_skinny.cuh).
 struct Gemm16 {
