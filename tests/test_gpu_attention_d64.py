@@ -42,3 +42,18 @@ def test_prefill_heads_up_to_64(dev, pkg, oracle, s, hq, hkv, d, start, max_seq)
     f = oracle.bf16_to_f32
     o = run_prefill(dev, capi, q, k, v, start, capi.BF16).view(np.uint16)
     util.assert_16bit_close(oracle, f(o), oracle.attention_prefill_f32(f(q), f(k), f(v), start))
+
+
+@pytest.mark.parametrize("s", [3000, 9000])
+def test_f16_a_long_tail_of_small_probabilities(dev, pkg, s):
+    """One key that outweighs each of the others 2^26 times, far below f16's smallest number, but carries no value: the
+    others decide.  Their probabilities are taken to 2^-32 of the largest, that is to 2^-6 of themselves."""
+    capi = pkg.capi
+    q, k, v = (np.zeros((1, 1, s, 64), np.float32) for _ in range(3))
+    q[..., 0] = 8                       # scores: q . k / 8
+    k[0, 0, 1:, 0] = -26 * np.log(2)
+    v[0, 0, 1:] = 100
+    got = run_attention(dev, capi, *(util.f32_to_f16_bits(t) for t in (q, k, v)), capi.F16, False).view(np.float16).astype(np.float64)
+    p = np.exp(np.float64(k.astype(np.float16)[0, 0, 1, 0]))
+    want = 100 * (s - 1) * p / (1 + (s - 1) * p)
+    assert (np.abs(got - want) <= 2.0 ** -6 * want).all(), (got.min(), got.max(), want)

@@ -59,12 +59,16 @@ constexpr int kPolyPairs = 2;  // of every 8 pairs of exponentials, how many avo
 
 // The two forms of the kernel.  D = 128: the probabilities are handed to P V rounded to the storage type.  D = 64: the
 // narrower Q, K and V tiles leave shared memory for a second P tile, and the probabilities are handed over as hi + lo,
-// two 16-bit numbers whose sum is the f32 value to 2^-17 (bf16) or better: P V is two products of 128 x 64 x 16, so a step
-// costs the tensor core what one 128-wide product does and the softmax chain stays the bound.  Its exponentials all
-// go through MUFU (the cubic of the wide form is good to 7e-5 only).
+// two 16-bit numbers whose sum is the f32 value to 2^-17 of it (bf16), or to 2^-22 of it or 2^-32 of the row's largest (f16).
+// P V is two products of 128 x 64 x 16, so a step costs the tensor core what one 128-wide product does and the softmax chain
+// stays the bound.  Its exponentials all go through MUFU (the cubic of the wide form is good to 7e-5 only).
 template <int D>
 struct Shape {
   static constexpr bool kSplitP = D == 64;
+  // f16 numbers end at 2^-24: the probabilities of the split form (2^8 at most, see kRescaleThreshold) and their sum are taken
+  // 2^7 times as large, so that a long tail of them down to 2^-32 of the largest counts in P V as it does in the sum
+  template <bool kIsBf16>
+  static constexpr float kPShift = kSplitP && !kIsBf16 ? 7.0f : 0.0f;
   static constexpr int kHalves = D / 64;                   // 64-wide swizzled column groups of a Q, K or V tile
   static constexpr int kHalfBytes = 128 * 64 * 2;          // one 128-row x 64-column group: 16 KiB
   static constexpr int kTileBytes = kHalves * kHalfBytes;  // a 128 x D tile of Q, K or V
@@ -473,7 +477,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       // f32 probabilities before they are rounded (packed adds, two per instruction).
       // A row whose scores so far are all -inf (a step, or in kSplit a whole range, may lie behind the row's last visible key):
       // taking them against 0 gives them no weight, against their maximum of -inf NaN.
-      const float ms = m_used == -INFINITY ? 0.f : m_used * sl2;
+      const float ms = m_used == -INFINITY ? 0.f : m_used * sl2 - Sh::template kPShift<kIsBf16>;
       const ptx::f32x2_t sl2x2 = ptx::pack_f32x2(sl2, sl2);
       const ptx::f32x2_t nmsx2 = ptx::pack_f32x2(-ms, -ms);
       ptx::f32x2_t lsum[2] = {0ull, 0ull};  // (+0.0f, +0.0f)
