@@ -208,7 +208,14 @@ int32_t tsm100_silu_mul(tsm100_device_t dev, const tsm100_silu_mul_desc* desc, c
  * B stored [N,K]); semantics linalg.fill 0 + linalg.matmul
  * (mlir_to_linalg.rs:1345-1393).  Replaces mlir_to_gpu.rs:1373-1397 (a TODO
  * comment) and :1584-1622.  16-bit inputs accumulate in f32 on the tensor
- * cores; out_dtype is the input dtype or TSM100_F32.  `batch` independent
+ * cores; out_dtype is the input dtype or TSM100_F32.  f32 problems take three
+ * tensor-core products of operands split into two TF32 numbers (22 bits and
+ * more of 24; the product of the two low parts, 2^-22 of the term, is left out),
+ * accumulated in f32: large ones and small aligned ones; the rest runs on the
+ * FP32 pipe.  Sums of integers stay exact where f32 sums are and the entries of
+ * one operand need at most 11 bits.  In problems whose rows do not start on
+ * 16-byte boundaries infinities and NaNs come out as the FP32 pipe gives them;
+ * in aligned ones an infinite operand may give NaN.  `batch` independent
  * problems are stored back to back (the per-block tile stride of
  * #[tile_kernel], tile_std_macros/src/lib.rs:237-254).
  * lda / ldb / ldc are row pitches in elements; 0 means "packed" (K for A; N, or K

@@ -108,3 +108,16 @@ def test_f32_an_infinite_row_of_a_long_product(dev, pkg, oracle, m, n, k, bt):
     truth = oracle.gemm_f32(np.ascontiguousarray(a[rows]), np.ascontiguousarray(b[keep] if bt else b[:, keep]), bt, f64_acc=True)
     mt = oracle.compare(np.ascontiguousarray(c[rows][:, keep]), truth)
     assert mt["rel_max"] <= util.F32_REL and mt["rel_fro"] <= util.F32_REL, mt
+
+
+@pytest.mark.parametrize("m,n,k,bt,wide_a", [(1025, 2051, 301, False, True), (1025, 2051, 1503, True, False)])
+def test_f32_whole_numbers_stay_exact(dev, pkg, m, n, k, bt, wide_a):
+    """Entries of 21 bits on one side, of 2 on the other, sums below 2^24: hi + lo holds them, and f32 adds them exactly."""
+    capi = pkg.capi
+    rng = np.random.default_rng(641)
+    wide = rng.integers(-(1 << 20), 1 << 20, (m, k) if wide_a else (n, k)).astype(np.float32)
+    small = np.zeros((n, k) if wide_a else (m, k), np.float32)
+    small[np.arange(len(small))[:, None], rng.integers(0, k, (len(small), 5))] = rng.integers(-3, 4, (len(small), 5))  # 5 * 3 * 2^20 < 2^24
+    a, b = (wide, small) if wide_a else (small, wide)
+    c = run(dev, capi, capi.F32, a, b if bt else np.ascontiguousarray(b.T), m, n, k, bt)[0]
+    assert np.array_equal(c, a.astype(np.float64) @ b.T.astype(np.float64))
