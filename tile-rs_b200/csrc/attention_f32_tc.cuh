@@ -7,7 +7,7 @@
 //
 // One streaming launch writes the hi / lo planes of K ([keys][D]) and of V, transposed ([D][keys]), so that both products
 // see K-major operands only.  Then one CTA owns 128 query rows of one head and walks the keys in steps of 32:
-//   warp 8       TMA producer: K_0, K_1, V_0, K_2, V_1, ... (hi and lo together, 256 * D bytes a unit) through a 3-deep
+//   warp 8       TMA producer: K_0, K_1, V_0, K_2, V_1, ... (hi and lo together, 256 * D bytes a unit) through a 5-deep
 //                ring.  No multicast.
 //   warp 9       S = Q K^T: the hi tile of Q stays in tensor memory for the CTA's life, the lo tile in shared memory.  A
 //                128 x 32 x 8 product reads 4 KiB of A against 1 KiB of B; from shared memory that takes 40 cycles, 16 of which
@@ -20,7 +20,8 @@
 // S and the chunk of O are double-buffered, so that the products of one step run during the softmax of the next; P is not
 // (tensor memory at D = 128: 2 * 128 of O, 2 * 32 of S, 32 + 32 of P, 128 of Q: all 512 columns).
 // Bound: tensor pipe at the TF32 rate / 3; shared-memory reads of Q by the 32-wide S products come close behind.  16 heads of
-// 4096 x 128: 170 TFLOP/s (0.63 of a third of the TF32 rate; 137 with both parts of Q in shared memory), 48 on the warp-level kernel.
+// 4096 x 128, causal: 170 TFLOP/s as graph replays (0.63 of a third of the TF32 rate; 137 with both parts of Q in shared memory), 156 per
+// call in a row of calls; 48 on the warp-level kernel.
 #pragma once
 
 #include "attention_simt.cuh"  // Params
@@ -59,8 +60,8 @@ struct alignas(8) Barriers {
   uint64_t s_full[2], s_free[2];
   uint64_t p_ready, pv_done;
   uint64_t o_full[2], o_empty[2];
-  uint64_t m_ready[3];   // the maximum of a chunk is in its row slot; the last one used after the last chunk: the row sums are
-  uint64_t l_ready;
+  uint64_t m_ready[3];   // the maximum of a chunk is in its row slot
+  uint64_t l_ready;      // the row sums are in the slot after the last chunk's
   uint32_t tmem_base;
   uint32_t abort_flag;
   uint32_t pv_steps;     // steps whose P V has been issued (only grows)
