@@ -53,16 +53,10 @@ def gemm16(lib, m, n, k, batch):
 
 # the few-tiles kernel, and how far it splits K
 @pytest.mark.parametrize("m,n,k,batch,kind,splits", [
-    (16, 16384, 4096, 1, FEW, 2), (16, 4096, 16384, 1, FEW, 8), (300, 4096, 16384, 1, FEW, 2), (1024, 1024, 4096, 1, FEW, 4),
-    # two CTAs only for a long K; short ones unsplit or on the persistent kernels
-    (1024, 1024, 512, 1, FEW, 1), (192, 64, 512, 1, SINGLES, 1), (192, 64, 1024, 1, FEW, 4), (100, 16384, 2048, 1, SINGLES, 1),
-    # many small problems: persistent kernels
-    (1, 4096, 128, 1024, SINGLES, 1), (16, 4096, 64, 64, SINGLES, 1), (16, 512, 2048, 64, FEW, 1), (16, 512, 4096, 64, SINGLES, 1), (32, 512, 64, 1024, SINGLES, 1), (128, 64, 64, 1024, SINGLES, 1),
-    (128, 64, 512, 1, SINGLES, 1), (64, 4096, 128, 64, SINGLES, 1), (256, 256, 256, 128, PAIRS, 1),
-    # many rows of few columns
-    (65536, 64, 64, 1, SINGLES, 1), (65536, 64, 4096, 1, FEW, 1), (65536, 8, 1024, 1, FEW, 1),
-    # pairs from 38 pair tiles on
-    (256 * 37, 256, 1024, 1, FEW, 1), (256 * 38, 256, 1024, 1, PAIRS, 1), (8192, 8192, 8192, 1, PAIRS, 1)])
+    (16, 16384, 4096, 1, FEW, 2), (16, 4096, 16384, 1, FEW, 8), (1, 20480, 5120, 1, FEW, 1), (1, 24576, 8192, 1, FEW, 1),
+    (65, 6144, 1536, 1, FEW, 4), (192, 64, 512, 1, SINGLES, 1), (192, 64, 4096, 1, FEW, 8), (4096, 4096, 64, 1, PAIRS, 1),
+    (1, 4096, 128, 1024, SINGLES, 1), (16, 4096, 64, 64, SINGLES, 1), (32, 512, 64, 1024, SINGLES, 1), (128, 64, 64, 1024, SINGLES, 1),
+    (256, 256, 256, 128, PAIRS, 1), (65536, 64, 64, 1, SINGLES, 1), (65536, 64, 4096, 1, FEW, 1), (8192, 8192, 8192, 1, PAIRS, 1)])
 def test_16_bit_products(lib, m, n, k, batch, kind, splits):
     plan = gemm16(lib, m, n, k, batch)
     assert plan[0] == kind and (kind != FEW or plan[2] == splits), plan

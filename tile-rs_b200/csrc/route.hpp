@@ -44,31 +44,30 @@ inline Gemm16 gemm16(int64_t m, int64_t n, int64_t k, int64_t batch, int sms) {
   Gemm16 r{Gemm16::kFewTiles, m <= 16 ? 16 : m <= 32 ? 32 : m <= 64 ? 64 : 128, 1, 0};
   const bool wide = r.rows == 128;
   const int64_t tiles = div_up(m, r.rows) * div_up(n, 128) * batch, kb = div_up(k, 64);
-  // K over a cluster while all CTAs fit the GPU at once, two per SM, and keep four k-blocks (128-row tiles: eight, once the
-  // second CTA of an SM is taken).  Two CTAs alone do not earn a cluster's launch while K is short: 192 x 64 x 512 7.5 unsplit,
-  // 9.3 in two; 300 x 4096 x 4096 24.0 / 21.6.
-  while (r.splits < kMaxGemmSplit && tiles * r.splits * 2 <= 2 * sms &&
-         kb / (2 * r.splits) >= (wide && tiles * r.splits * 2 > sms ? 8 : 4)) r.splits *= 2;
-  if (r.splits == 2 && kb < (wide ? 64 : 32)) r.splits = 1;
-  r.k_blocks_per_cta = div_up(kb, r.splits);
-  bool few;
-  if (m > 128 && n > 128) {
-    // pairs once 256 x 256 tiles are there for more than half of them: 24 .. 36 of them 0.83 .. 1.0 of the pairs' time at any K,
-    // 37 .. 48 0.99 .. 1.29
-    few = div_up(m, 256) * div_up(n, 256) * batch <= sms / 4;
-    if (!few) r.kind = Gemm16::kPairs;
-  } else {
-    // Unsplit, the few-tiles kernel starts a CTA per tile and hides nothing of its start and end but behind a second CTA; the
-    // persistent kernel loads the next tile meanwhile.  So it pays for tiles that are all there at once, and beyond that where a
-    // 256-wide tile would be half empty (n <= 128) and K long enough.  Persistent / few tiles: 16 x 4096 x
-    // 4096 23.3 / 8.4, 16 x 4096 x 128 of a batch of 256 48 / 93, 128 x 64 x 64 of 1024 11 / 21, 32 x 64 x 4096 of 1024 175 / 127.
-    if (r.splits > 1) few = true;
-    else if (m <= 16) few = tiles <= (kb < 64 ? 2 : 1) * sms || (n <= 128 && kb >= 8);
-    else if (m <= 32) few = tiles <= sms || (n <= 128 && (tiles <= 2 * sms || kb >= 16));
-    else if (m <= 64) few = n > 128 ? tiles <= sms : kb >= 16 || (kb >= 8 && tiles <= 2 * sms);
-    else few = n <= 128 && (kb >= 64 || (n <= 32 && tiles >= 2 * sms));
-    if (!few) r.kind = Gemm16::kSingles;
+  // K over a cluster while every CTA keeps four k-blocks and all clusters fit the GPU at once, two CTAs per SM (clusters of 8 leave a
+  // fifth of the SMs' places empty, of 4 a sixteenth; with 128 k-blocks or more a second wave pays all the same).  Two CTAs alone do
+  // not earn a cluster's launch while K is short.
+  while (r.splits < kMaxGemmSplit) {
+    const int to = 2 * r.splits;
+    const int64_t room = to == 2 || kb >= 128 ? 2 * sms : to == 4 ? sms * 15 / 8 : sms * 8 / 5;
+    if (tiles * to > room || kb / to < 4) break;
+    r.splits = to;
   }
+  if (r.splits == 2 && kb < (tiles * 2 > sms ? 48 : wide ? 16 : r.rows == 64 ? 12 : 9)) r.splits = 1;
+  r.k_blocks_per_cta = div_up(kb, r.splits);
+  // Unsplit, the few-tiles kernel starts a CTA per tile and hides nothing of its start and end but behind a second CTA; the persistent
+  // kernels load the next tile meanwhile.  So it pays for tiles that are all there at once, and beyond that for a long K where 256-wide
+  // tiles would leave SMs idle or be half empty.  Weights from HBM, persistent / few tiles: 1 x 20480 x 5120 54 / 37, 65 x 6144 x
+  // 1536 15 / 11, 20 x 4096 x 64 of a batch of 256 35 / 88.  Over 3038 sizes 0.6 % from the best choice of each, 7 more than 5 % slower
+  // than the persistent kernels alone.
+  bool few;
+  if (r.splits > 1) few = true;
+  else if (m > 128 && n > 128) few = tiles <= sms;
+  else if (m <= 16) few = tiles <= 2 * sms || (n <= 128 && kb >= 8);
+  else if (m <= 64) few = 2 * tiles <= 3 * sms || (kb >= 64 && tiles <= 2 * sms) || (n <= 128 && kb >= 8 && (tiles <= 2 * sms || kb >= 16));
+  else if (n > 128) few = tiles <= sms;
+  else few = (n % 32 != 0 && n > 32 && tiles <= sms) || (tiles > sms && kb >= 40) || (n <= 32 && tiles >= 2 * sms && kb >= 4);
+  if (!few) r.kind = m > 128 && n > 128 ? Gemm16::kPairs : Gemm16::kSingles;
   // one CTA per tile has to fit one launch
   if (few && tiles * r.splits > 0x7fffffff) r.kind = m > 128 && n > 128 ? Gemm16::kPairs : Gemm16::kSingles;
   return r;
