@@ -123,6 +123,7 @@ template <typename T, int G, int D>
 __global__ void __launch_bounds__(kThreads)
 attention_decode_kernel(const T* __restrict__ q, const T* __restrict__ kc, const T* __restrict__ vc, T* __restrict__ o,
                         const Params p) {
+  q = ptx::wait_prior_grid(q);
   constexpr int LPP = lanes_per_pos<T, D>();
   constexpr int GROUPS = 32 / LPP;          // positions a warp works on at a time
   constexpr int kSlots = slots<T, D>();
@@ -224,6 +225,7 @@ attention_decode_kernel(const T* __restrict__ q, const T* __restrict__ kc, const
     }
   }
 
+  ptx::launch_dependents();
   // slot records -> shared memory
 #pragma unroll
   for (int h = 0; h < G; ++h) {
@@ -282,6 +284,7 @@ namespace mma {
 // warps per CTA: 4 for large launches (several CTAs per SM), 8 when a launch has at most one CTA per SM
 constexpr int kTilePos = 16;   // positions per tile
 constexpr int kRows = 16;      // query heads per pass (rows of the MMA tile)
+constexpr int kAheadBytes = 128 << 10;  // of K and of V that a CTA of the kGlobal form fetches into the L2 before the kernel before it has ended
 
 template <int D>
 constexpr int pitch_bytes() { return D * 2 + 16; }
@@ -348,7 +351,7 @@ attention_decode_mma_kernel(const T* __restrict__ q, const T* __restrict__ kc, c
   float* part = reinterpret_cast<float*>(ring);                       // warp w's record at part + w * WARP_FLOATS
   float* mine = part + kRows * REC;                                   // the CTA's merged record [16][REC], behind warp 0's
 
-  if (kGlobal) ptx::launch_dependents();  // the merge kernel may be set up meanwhile
+  if (kGlobal) ptx::launch_dependents();  // one CTA per SM: the merge kernel may be placed meanwhile
   const uint32_t splits = kGlobal ? static_cast<uint32_t>(p.splits) : ptx::cluster_nctarank();
   const uint32_t rank = kGlobal ? blockIdx.x % splits : ptx::cluster_ctarank();
   const int unit = blockIdx.x / splits;
@@ -387,6 +390,18 @@ attention_decode_mma_kernel(const T* __restrict__ q, const T* __restrict__ kc, c
   float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;  // rows gr and gr + 8 (this thread's share of the sums)
   const float sl2 = p.scale_log2;
 
+  if constexpr (kGlobal) {
+    // while the kernel before this one runs: the start of this CTA's range
+    constexpr int kPiece = 4096;
+    const int64_t ahead = min(kAheadBytes, max(0, p_end - p_begin) * (D * 2));
+    const int64_t at = static_cast<int64_t>(p_begin) * (D * 2);
+    for (int64_t i = static_cast<int64_t>(tid) * kPiece; i < ahead; i += static_cast<int64_t>(kThreads) * kPiece) {
+      const uint32_t bytes = static_cast<uint32_t>(ahead - i < kPiece ? ahead - i : kPiece);
+      ptx::prefetch_l2(kbase + at + i, bytes);
+      ptx::prefetch_l2(vbase + at + i, bytes);
+    }
+  }
+  q = ptx::wait_prior_grid(q);
 #pragma unroll
   for (int i = 0; i < STAGES - 1; ++i) {  // the first tiles are on their way before anything else is read
     if (warp + i * kWarps < n_tiles) prefetch(warp + i * kWarps, i);
@@ -471,6 +486,7 @@ attention_decode_mma_kernel(const T* __restrict__ q, const T* __restrict__ kc, c
     }
     __syncwarp();  // the stage is refilled at the top of the next iteration; every lane is done reading it
   }
+  if (!kGlobal) ptx::launch_dependents();
   cp_async_wait<0>();
   __syncwarp();  // the warp's ring share is free: it now receives the warp's record
   // this thread's share of the row sums -> the whole row's
@@ -536,7 +552,8 @@ attention_decode_merge_kernel(T* __restrict__ o, const Params p) {
   const int unit = blockIdx.x / p.heads_here, hh = blockIdx.x % p.heads_here;
   const int b = unit / p.heads_kv, g = unit % p.heads_kv;
   const float* rec = p.part + (static_cast<int64_t>(unit) * p.splits * kRows + hh) * REC;
-  ptx::wait_prior_grid();
+  ptx::launch_dependents();
+  rec = ptx::wait_prior_grid(rec);
   for (int i = threadIdx.x; i < p.splits; i += D) {
     m[i] = rec[i * (kRows * REC) + D];
     l[i] = rec[i * (kRows * REC) + D + 1];

@@ -183,8 +183,6 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   volatile uint32_t* abort_flag = &bars->abort_flag;
-  if (kSplit) ptx::launch_dependents();  // the merge kernel may be set up meanwhile
-
   const int splits = kSplit ? p.splits : 1;
   const int rank = kSplit ? static_cast<int>(blockIdx.x) % splits : 0;
   const int block = kSplit ? static_cast<int>(blockIdx.x) / splits : static_cast<int>(blockIdx.x);
@@ -227,6 +225,8 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   __syncthreads();
   ptx::tcgen05_fence_after_thread_sync();
   const uint32_t tmem_base = bars->tmem_base;
+  ptx::launch_dependents();
+  ptx::wait_prior_grid();
   const uint32_t tmem_s = tmem_base;        // S_A at +0, S_B at +128
   const uint32_t tmem_o = tmem_base + 256;  // O_A at +256, O_B at +384
 
@@ -634,6 +634,7 @@ attention_merge_kernel(uint16_t* __restrict__ o, const Params p) {
   block_coords(p, block, bh, kvh, qb);
   const int row = threadIdx.x, qrow = qb * 2 * kBQ + row;
   const int cols = D == 64 ? p.head_dim : D;
+  ptx::launch_dependents();
   ptx::wait_prior_grid();
   if (qrow >= p.seq || c0 >= cols) return;
   const int64_t rec0 = static_cast<int64_t>(block) * p.splits;

@@ -103,6 +103,8 @@ template <typename T, int D>
 __global__ void __launch_bounds__(kThreads, (sizeof(T) == 2 && D <= 64) ? 2 : 1)
 attention_tf32x3_kernel(const T* __restrict__ q, const T* __restrict__ k, const T* __restrict__ v,
                         T* __restrict__ o, const Params p) {
+  ptx::launch_dependents();
+  q = ptx::wait_prior_grid(q);
   namespace cp = attn_decode::mma;
   using gemm_simt::from_f32;
   using gemm_simt::to_f32;

@@ -28,6 +28,7 @@ constexpr int kThreads = 128;
 constexpr int kMaxSplit = 8;
 constexpr int kWBytes = kBN * kBK * 2;   // 16 KiB of B per stage
 constexpr int kMaxStages = 6;
+constexpr int kAhead = 8;                // tiles of B that a CTA fetches into the L2 before the kernel before it has ended
 
 template <int NT>
 struct Shape {
@@ -112,11 +113,24 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   __syncthreads();
   ptx::tcgen05_fence_after_thread_sync();
   const uint32_t tmem_base = bars->tmem_base;
+  if (threadIdx.x == 0) {
+    ptx::prefetch_tensormap(&tmap_a);
+    ptx::prefetch_tensormap(&tmap_b);
+    // while the kernel before this one runs: its first tiles of B
+    for (int i = 0; i < min(num_kb, kAhead); ++i) {
+      const int k0 = (kb0 + i) * kBK;
+      if (kBTransposed) {
+        ptx::prefetch_l2_3d(&tmap_b, k0, nb * kBN, b);
+      } else {
+        ptx::prefetch_l2_3d(&tmap_b, nb * kBN, k0, b);
+        ptx::prefetch_l2_3d(&tmap_b, nb * kBN + 64, k0, b);
+      }
+    }
+  }
+  ptx::wait_prior_grid();
 
   if (warp == 0) {
     if (lane == 0) {
-      ptx::prefetch_tensormap(&tmap_a);
-      ptx::prefetch_tensormap(&tmap_b);
       int stage = 0;
       uint32_t phase = 0;
       for (int i = 0; i < num_kb; ++i) {
@@ -168,6 +182,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   // ------------------------------ accumulator -> C ------------------------------
   const bool ready = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->acc_full, 0, abort_flag, p.status, 53));
   ptx::tcgen05_fence_after_thread_sync();
+  // not before: 11 x 4104 x 2064 of a batch of 4 in a row of calls 16.8 us with this at the start of the kernel, 14.2 here
+  ptx::launch_dependents();
   const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
   constexpr int kStep = NT < 32 ? 16 : 32;  // rows of C (TMEM columns) per read
   OutT* cb = c + static_cast<int64_t>(b) * p.c_batch_stride;

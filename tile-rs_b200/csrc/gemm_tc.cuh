@@ -169,6 +169,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   __syncthreads();
   ptx::tcgen05_fence_after_thread_sync();
   const uint32_t tmem_base = bars->tmem_base;
+  ptx::launch_dependents();
+  ptx::wait_prior_grid();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------

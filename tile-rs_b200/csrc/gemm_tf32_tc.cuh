@@ -159,6 +159,8 @@ __device__ __forceinline__ void split_transposed(const SplitOperand& p, int bloc
 template <bool kVec, bool kTransposeB>
 __global__ void __launch_bounds__(256)
 split_operands_kernel(const SplitOperand a, const SplitOperand b, uint32_t* zero, int64_t n_zero) {
+  ptx::launch_dependents();
+  ptx::wait_prior_grid();
   if (blockIdx.y == 0)
     for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n_zero; i += static_cast<int64_t>(gridDim.x) * blockDim.x) zero[i] = 0u;
   __shared__ float tile[kTransposeB ? 32 : 1][33];
@@ -417,6 +419,8 @@ gemm_tf32_tc_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_
   __syncthreads();
   ptx::tcgen05_fence_after_thread_sync();
   const uint32_t tmem_base = bars->tmem_base;
+  ptx::launch_dependents();
+  ptx::wait_prior_grid();
 
   if (warp == 0) {
     // ------------------------------ TMA producer ------------------------------
@@ -678,6 +682,8 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
   ptx::cluster_sync_all();  // the peer's barriers are initialised before anything signals them
   ptx::tcgen05_fence_after_thread_sync();
   const uint32_t tmem_base = bars->tmem_base;
+  ptx::launch_dependents();
+  ptx::wait_prior_grid();
 
   if (warp == 0) {
     // ------------------------------ TMA producer (both CTAs) ------------------

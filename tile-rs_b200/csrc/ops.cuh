@@ -21,6 +21,7 @@
 #include <string>
 #include <tuple>
 #include <type_traits>
+#include <utility>
 
 #include "../../include/tile_sm100.h"
 #include "attention_decode.cuh"
@@ -130,6 +131,59 @@ inline cudaError_t allow_wide_clusters_once(K kern) {
     return e == cudaSuccess;
   });
   return e;
+}
+// Launches a kernel in clusters of `cluster` CTAs where that is not 0; chained: as a programmatic dependent of the one before it in
+// the stream (the rules that such kernels keep are in ptx.cuh).  What that saves is the time between two kernels of a chain of calls:
+// the end of one grid, the launch of the next and its set-up run side by side.  bf16 MLP of 16 tokens, 4096 x 16384: 95.6 us, 83.0
+// chained and with the weights' first tiles fetched meanwhile; decode of one sequence of 32768, four kernels after each other:
+// 40.3 / 32.5; 16 x 4096 x 4096 in a row of calls 12.2 / 9.0.
+template <bool kChained, typename... P, typename... A>
+inline cudaError_t launch_kernel(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, unsigned cluster, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = kChained ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster ? 2 : 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  return cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, unsigned cluster, A&&... args) {
+  return launch_kernel<true>(kern, grid, threads, smem, s, cluster, std::forward<A>(args)...);
+}
+// How many clusters of `cluster` CTAs of a kernel the GPU holds at once, asked once per kernel and device; `fallback` if it cannot tell.
+template <typename K>
+inline int resident_clusters(K kern, unsigned threads, size_t smem, unsigned cluster, unsigned grid, int fallback) {
+  int answer = fallback;
+  kernel_fact(reinterpret_cast<const void*>(kern), kFactClusters, &answer, [&](int* out) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = cluster;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
+      (void)cudaGetLastError();
+      return false;
+    }
+    *out = n;
+    return true;
+  });
+  return answer;
 }
 // Resident CTAs per SM of a kernel launched with `threads` threads and no dynamic shared memory (at least 1).
 template <typename K>
@@ -258,25 +312,14 @@ template <typename T, int CHUNKS>
 inline cudaError_t launch_softmax_warp(const T* x, T* y, int64_t rows, int32_t cols, cudaStream_t s) {
   constexpr int WARPS = 4;
   const int64_t grid = (rows + WARPS - 1) / WARPS;
-  softmax::softmax_rows_warp<T, CHUNKS, WARPS><<<static_cast<unsigned>(grid), WARPS * 32, 0, s>>>(x, y, rows, cols);
-  return cudaGetLastError();
+  return launch_chained(softmax::softmax_rows_warp<T, CHUNKS, WARPS>, static_cast<unsigned>(grid), WARPS * 32, 0, s, 0, x, y, rows, cols);
 }
 
 // As many CTAs per row as its vectors need, one cluster per row.
 template <typename T, int VPT, int THREADS>
 inline int32_t softmax_cluster_launch(std::string* err, const T* x, T* y, int64_t rows, int64_t cols, int64_t ctas, cudaStream_t s) {
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(ctas);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cfg.blockDim = dim3(THREADS);
-  cfg.stream = s;
-  cfg.gridDim = dim3(static_cast<unsigned>(rows * ctas));
-  return cuda_ok(err, cudaLaunchKernelEx(&cfg, softmax::softmax_rows_cluster<T, VPT, THREADS>, x, y, rows, static_cast<int32_t>(cols)),
+  return cuda_ok(err, launch_chained(softmax::softmax_rows_cluster<T, VPT, THREADS>, static_cast<unsigned>(rows * ctas), THREADS, 0, s,
+                                     static_cast<unsigned>(ctas), x, y, rows, static_cast<int32_t>(cols)),
                  "softmax_rows_cluster launch");
 }
 
@@ -303,12 +346,12 @@ inline int32_t softmax_typed(std::string* err, const T* x, T* y, int64_t rows, i
     auto launch = [&](auto kern, int threads) {
       const int per_sm = blocks_per_sm(kern, threads);
       const unsigned grid = static_cast<unsigned>(std::min<int64_t>(rows, static_cast<int64_t>(sms_cta) * per_sm));
-      kern<<<grid, threads, 0, s>>>(x, y, rows, c);
+      e = launch_chained(kern, grid, threads, 0, s, 0, x, y, rows, c);
     };
     if (nvec <= 128 * 4) launch(softmax::softmax_rows_cta<T, 4, 128>, 128);
     else if (nvec <= 128 * 8) launch(softmax::softmax_rows_cta<T, 8, 128>, 128);
     else launch(softmax::softmax_rows_cta<T, 8, 256>, 256);
-    return cuda_ok(err, cudaGetLastError(), "softmax_rows_cta launch");
+    return cuda_ok(err, e, "softmax_rows_cta launch");
   }
   int sms = 0;
   int32_t st = sm_count(err, &sms);
@@ -322,20 +365,21 @@ inline int32_t softmax_typed(std::string* err, const T* x, T* y, int64_t rows, i
     if (route::softmax_row_per_warp(span, rows, sms) && rows <= 4ll * 0x7fffffff) {
       constexpr int WARPS = 4;
       const unsigned grid = static_cast<unsigned>((rows + WARPS - 1) / WARPS);
-      if (span <= 32 * 2) softmax::softmax_rows_warp_any<T, 2, WARPS><<<grid, WARPS * 32, 0, s>>>(x, y, rows, c);
-      else if (span <= 32 * 4) softmax::softmax_rows_warp_any<T, 4, WARPS><<<grid, WARPS * 32, 0, s>>>(x, y, rows, c);
-      else softmax::softmax_rows_warp_any<T, 8, WARPS><<<grid, WARPS * 32, 0, s>>>(x, y, rows, c);
-      return cuda_ok(err, cudaGetLastError(), "softmax_rows_warp_any launch");
+      if (span <= 32 * 2) e = launch_chained(softmax::softmax_rows_warp_any<T, 2, WARPS>, grid, WARPS * 32, 0, s, 0, x, y, rows, c);
+      else if (span <= 32 * 4) e = launch_chained(softmax::softmax_rows_warp_any<T, 4, WARPS>, grid, WARPS * 32, 0, s, 0, x, y, rows, c);
+      else e = launch_chained(softmax::softmax_rows_warp_any<T, 8, WARPS>, grid, WARPS * 32, 0, s, 0, x, y, rows, c);
+      return cuda_ok(err, e, "softmax_rows_warp_any launch");
     }
     // up to 1024 vectors a row stays in registers: 8000 rows of 3501 bf16 78 us scalar, 66 read twice, 27 here; 3000 of 1111
     // f32 17 / 23 / 8.5; 4000 of 8001 bf16 70 / 32 / 29
     if (span <= 256 * 4) {
       auto launch = [&](auto kern, int threads) {
-        kern<<<static_cast<unsigned>(std::min<int64_t>(rows, static_cast<int64_t>(sms) * blocks_per_sm(kern, threads))), threads, 0, s>>>(x, y, rows, c);
+        const unsigned grid = static_cast<unsigned>(std::min<int64_t>(rows, static_cast<int64_t>(sms) * blocks_per_sm(kern, threads)));
+        e = launch_chained(kern, grid, threads, 0, s, 0, x, y, rows, c);
       };
       if (span <= 128 * 4) launch(softmax::softmax_rows_cta_any<T, 4, 128>, 128);
       else launch(softmax::softmax_rows_cta_any<T, 4, 256>, 256);
-      return cuda_ok(err, cudaGetLastError(), "softmax_rows_cta_any launch");
+      return cuda_ok(err, e, "softmax_rows_cta_any launch");
     }
     if (const int ctas = route::softmax_cluster(span, rows, sms)) {
       if (span <= 8 * 1024) return softmax_cluster_launch<T, 4, 256>(err, x, y, rows, cols, ctas, s);
@@ -344,7 +388,8 @@ inline int32_t softmax_typed(std::string* err, const T* x, T* y, int64_t rows, i
     // one CTA per row.  1000 rows of 50001 bf16: 97 us scalar, 49 here; 1212 of 97648 f32 286 / 214; 2000 of 16392 bf16 (in shared
     // memory) 45 / 31
     const int threads = route::softmax_twice_threads(cols * static_cast<int64_t>(sizeof(T)), rows, sms);
-    auto launch = [&](auto kern) { kern<<<static_cast<unsigned>(std::min<int64_t>(rows, sms * (1024ll / threads))), threads, 0, s>>>(x, y, rows, c); };
+    const unsigned grid = static_cast<unsigned>(std::min<int64_t>(rows, sms * (1024ll / threads)));
+    auto launch = [&](auto kern) { e = launch_chained(kern, grid, threads, 0, s, 0, x, y, rows, c); };
     if (route::softmax_twice_skip((cols + PV - 1) / PV, threads, softmax::kTwiceUnroll)) {
       if (threads == 256) launch(softmax::softmax_rows_twice<T, 256, true>);
       else if (threads == 512) launch(softmax::softmax_rows_twice<T, 512, true>);
@@ -354,12 +399,12 @@ inline int32_t softmax_typed(std::string* err, const T* x, T* y, int64_t rows, i
       else if (threads == 512) launch(softmax::softmax_rows_twice<T, 512, false>);
       else launch(softmax::softmax_rows_twice<T, 1024, false>);
     }
-    return cuda_ok(err, cudaGetLastError(), "softmax_rows_twice launch");
+    return cuda_ok(err, e, "softmax_rows_twice launch");
   }
   constexpr int THREADS = 512;
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>(rows, static_cast<int64_t>(sms) * 4));
-  softmax::softmax_rows_stream<T, THREADS><<<grid, THREADS, 0, s>>>(x, y, rows, cols);
-  return cuda_ok(err, cudaGetLastError(), "softmax_rows_stream launch");
+  e = launch_chained(softmax::softmax_rows_stream<T, THREADS>, grid, THREADS, 0, s, 0, x, y, rows, cols);
+  return cuda_ok(err, e, "softmax_rows_stream launch");
 }
 
 inline int32_t softmax(std::string* err, const tsm100_softmax_desc* d, const void* x, void* y, void* stream) {
@@ -391,30 +436,31 @@ inline int32_t row_op_typed(std::string* err, const T* x, T* y, int64_t rows, in
   int sms = 0;
   int32_t st = sm_count(err, &sms);
   if (st != TSM100_OK) return st;
+  cudaError_t e = cudaSuccess;
   // persistent CTAs: exactly as many as are resident at once, each striding over the rows
   auto launch = [&](auto kern, int threads, int rows_per_cta) {
     const int per_sm = blocks_per_sm(kern, threads);
     const int64_t want = (rows + rows_per_cta - 1) / rows_per_cta;
     const unsigned grid = static_cast<unsigned>(std::min<int64_t>(want, static_cast<int64_t>(sms) * per_sm));
-    kern<<<grid, threads, 0, s>>>(x, y, rows, static_cast<int32_t>(cols), eps);
+    e = launch_chained(kern, grid, threads, 0, s, 0, x, y, rows, static_cast<int32_t>(cols), eps);
   };
   if (vec_ok && nvec <= 32 * 8) {  // one warp per row, four rows per CTA
     if (nvec <= 32 * 1) launch(ro::row_op_kernel<T, OP, 1, 32, 128>, 128, 4);
     else if (nvec <= 32 * 2) launch(ro::row_op_kernel<T, OP, 2, 32, 128>, 128, 4);
     else if (nvec <= 32 * 4) launch(ro::row_op_kernel<T, OP, 4, 32, 128>, 128, 4);
     else launch(ro::row_op_kernel<T, OP, 8, 32, 128>, 128, 4);
-    return cuda_ok(err, cudaGetLastError(), "row_op_kernel (warp per row) launch");
+    return cuda_ok(err, e, "row_op_kernel (warp per row) launch");
   }
   if (vec_ok && nvec <= 256 * 8) {  // 128 or 256 threads per row, 32 values each
     if (nvec <= 128 * 4) launch(ro::row_op_kernel<T, OP, 4, 128, 128>, 128, 1);
     else if (nvec <= 128 * 8) launch(ro::row_op_kernel<T, OP, 8, 128, 128>, 128, 1);
     else launch(ro::row_op_kernel<T, OP, 8, 256, 256>, 256, 1);
-    return cuda_ok(err, cudaGetLastError(), "row_op_kernel (CTA per row) launch");
+    return cuda_ok(err, e, "row_op_kernel (CTA per row) launch");
   }
   constexpr int THREADS = 512;
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>(rows, static_cast<int64_t>(sms) * 4));
-  ro::row_op_stream_kernel<T, OP, THREADS><<<grid, THREADS, 0, s>>>(x, y, rows, cols, eps);
-  return cuda_ok(err, cudaGetLastError(), "row_op_stream_kernel launch");
+  e = launch_chained(ro::row_op_stream_kernel<T, OP, THREADS>, grid, THREADS, 0, s, 0, x, y, rows, cols, eps);
+  return cuda_ok(err, e, "row_op_stream_kernel launch");
 }
 
 template <int OP>
@@ -466,15 +512,13 @@ inline int32_t silu_mul_typed(std::string* err, const T* gate, const T* up, T* y
     const int64_t nvec = n / PV;
     const int64_t want = (nvec + THREADS * UNROLL - 1) / (THREADS * UNROLL);
     const unsigned grid = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(want, static_cast<int64_t>(sms) * 8)));
-    if (up) ro::silu_mul_kernel<T, true, UNROLL, THREADS><<<grid, THREADS, 0, s>>>(gate, up, y, nvec);
-    else ro::silu_mul_kernel<T, false, UNROLL, THREADS><<<grid, THREADS, 0, s>>>(gate, up, y, nvec);
-    return cuda_ok(err, cudaGetLastError(), "silu_mul_kernel launch");
+    auto kern = up ? ro::silu_mul_kernel<T, true, UNROLL, THREADS> : ro::silu_mul_kernel<T, false, UNROLL, THREADS>;
+    return cuda_ok(err, launch_chained(kern, grid, THREADS, 0, s, 0, gate, up, y, nvec), "silu_mul_kernel launch");
   }
   const int64_t want = (n + THREADS - 1) / THREADS;
   const unsigned grid = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>(want, static_cast<int64_t>(sms) * 8)));
-  if (up) ro::silu_mul_scalar_kernel<T, true, THREADS><<<grid, THREADS, 0, s>>>(gate, up, y, n);
-  else ro::silu_mul_scalar_kernel<T, false, THREADS><<<grid, THREADS, 0, s>>>(gate, up, y, n);
-  return cuda_ok(err, cudaGetLastError(), "silu_mul_scalar_kernel launch");
+  auto kern = up ? ro::silu_mul_scalar_kernel<T, true, THREADS> : ro::silu_mul_scalar_kernel<T, false, THREADS>;
+  return cuda_ok(err, launch_chained(kern, grid, THREADS, 0, s, 0, gate, up, y, n), "silu_mul_scalar_kernel launch");
 }
 
 inline int32_t silu_mul(std::string* err, const tsm100_silu_mul_desc* d, const void* gate, const void* up, void* y,
@@ -517,19 +561,19 @@ inline int32_t rope(std::string* err, const tsm100_rope_desc* d, void* x, void* 
   const bool vec = d->head_dim % pv == 0 && aligned16(x);
   const int64_t n = tokens * (vec ? d->head_dim / pv : d->head_dim / 2);
   const unsigned grid = static_cast<unsigned>(std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, static_cast<int64_t>(sms) * 8)));
-  auto launch = [&](auto* xt) {
+  auto launch = [&](auto* xt) -> cudaError_t {
     using T = std::remove_pointer_t<decltype(xt)>;
     if (vec) {
       const int32_t heads_per = route::rope_heads_per_thread(grid, d->heads, sms);
       const dim3 grid2(grid, static_cast<unsigned>((d->heads + heads_per - 1) / heads_per));
-      rowops::rope_vec_kernel<T><<<grid2, 256, 0, s>>>(xt, tokens, d->seq_len, d->heads, heads_per, d->head_dim, d->start_pos, d->theta);
+      return launch_chained(rowops::rope_vec_kernel<T>, grid2, 256, 0, s, 0, xt, tokens, d->seq_len, d->heads, heads_per, d->head_dim, d->start_pos, d->theta);
     }
-    else rowops::rope_kernel<T><<<grid, 256, 0, s>>>(xt, tokens, d->seq_len, d->heads, d->head_dim, d->start_pos, d->theta);
+    return launch_chained(rowops::rope_kernel<T>, grid, 256, 0, s, 0, xt, tokens, d->seq_len, d->heads, d->head_dim, d->start_pos, d->theta);
   };
-  if (d->dtype == TSM100_F32) launch(static_cast<float*>(x));
-  else if (d->dtype == TSM100_BF16) launch(static_cast<__nv_bfloat16*>(x));
-  else launch(static_cast<__half*>(x));
-  return cuda_ok(err, cudaGetLastError(), "rope_kernel launch");
+  const cudaError_t e = d->dtype == TSM100_F32    ? launch(static_cast<float*>(x))
+                        : d->dtype == TSM100_BF16 ? launch(static_cast<__nv_bfloat16*>(x))
+                                                  : launch(static_cast<__half*>(x));
+  return cuda_ok(err, e, "rope_kernel launch");
 }
 
 template <typename T>
@@ -542,14 +586,13 @@ inline cudaError_t kv_cache_update_typed(const tsm100_kv_cache_update_desc* d, c
   auto launch = [&](auto vec_tag, auto index_tag) {
     constexpr int V = decltype(vec_tag)::value;
     using I = decltype(index_tag);
-    rowops::kv_cache_update_kernel<T, V, I><<<grid, 256, 0, s>>>(static_cast<const T*>(src), static_cast<T*>(cache), d->batch,
-                                                                 d->seq_len, d->heads, d->head_dim, d->start_pos, d->max_seq);
+    return launch_chained(rowops::kv_cache_update_kernel<T, V, I>, grid, 256, 0, s, 0, static_cast<const T*>(src), static_cast<T*>(cache),
+                          static_cast<int64_t>(d->batch), d->seq_len, d->heads, d->head_dim, d->start_pos, d->max_seq);
   };
-  if (vec && small) launch(std::integral_constant<int, PV>{}, uint32_t{});
-  else if (vec) launch(std::integral_constant<int, PV>{}, int64_t{});
-  else if (small) launch(std::integral_constant<int, 1>{}, uint32_t{});
-  else launch(std::integral_constant<int, 1>{}, int64_t{});
-  return cudaGetLastError();
+  if (vec && small) return launch(std::integral_constant<int, PV>{}, uint32_t{});
+  if (vec) return launch(std::integral_constant<int, PV>{}, int64_t{});
+  if (small) return launch(std::integral_constant<int, 1>{}, uint32_t{});
+  return launch(std::integral_constant<int, 1>{}, int64_t{});
 }
 
 inline int32_t kv_cache_update(std::string* err, const tsm100_kv_cache_update_desc* d, const void* src, void* cache, void* stream) {
@@ -625,23 +668,12 @@ inline int32_t gemm_tf32x3_launch(std::string* err, const tsm100_gemm_desc* d, c
   p.k_per_cta = static_cast<int32_t>(((d->k + splits - 1) / splits + g::kBK - 1) / g::kBK * g::kBK);
   const GemmPitch ld = gemm_pitch(d);
   p.lda = ld.lda, p.ldb = ld.ldb, p.ldc = ld.ldc;
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(splits);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cfg.blockDim = dim3(g::kThreads);
   const int stages = splits > 1 ? g::kStagesSplit : g::kStages;
-  cfg.dynamicSmemBytes = static_cast<size_t>(stages) * g::kStageBytes;
-  cfg.stream = s;
-  cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
   auto launch = [&](auto kern) -> cudaError_t {
     cudaError_t e = set_dyn_smem_once(kern, g::kSmemBytes);
     if (e != cudaSuccess) return e;
-    return cudaLaunchKernelEx(&cfg, kern, static_cast<const float*>(a), static_cast<const float*>(b), static_cast<float*>(c), p);
+    return launch_chained(kern, static_cast<unsigned>(tiles * splits), g::kThreads, static_cast<size_t>(stages) * g::kStageBytes, s,
+                          static_cast<unsigned>(splits), static_cast<const float*>(a), static_cast<const float*>(b), static_cast<float*>(c), p);
   };
   cudaError_t e;
   if (d->b_transposed)
@@ -675,14 +707,9 @@ inline int32_t split_operands_launch(std::string* err, gemm_tf32_tc::SplitOperan
   if (transpose_b && tiles > 0x7fffffff - a.blocks) return op_fail(err, TSM100_ERR_INVALID, "operand split: too many tiles for one launch");
   b.blocks = transpose_b ? static_cast<int32_t>(tiles) : row_blocks(b);
   const dim3 grid(static_cast<unsigned>(a.blocks) + static_cast<unsigned>(b.blocks), static_cast<unsigned>(batch));
-  if (transpose_b) {
-    if (vec(a)) g::split_operands_kernel<true, true><<<grid, 256, 0, s>>>(a, b, zero, n_zero);
-    else g::split_operands_kernel<false, true><<<grid, 256, 0, s>>>(a, b, zero, n_zero);
-  } else {
-    if (vec(a) && vec(b)) g::split_operands_kernel<true, false><<<grid, 256, 0, s>>>(a, b, zero, n_zero);
-    else g::split_operands_kernel<false, false><<<grid, 256, 0, s>>>(a, b, zero, n_zero);
-  }
-  return cuda_ok(err, cudaGetLastError(), "split_operands_kernel launch");
+  auto kern = transpose_b ? (vec(a) ? g::split_operands_kernel<true, true> : g::split_operands_kernel<false, true>)
+                          : (vec(a) && vec(b) ? g::split_operands_kernel<true, false> : g::split_operands_kernel<false, false>);
+  return cuda_ok(err, launch_chained(kern, grid, 256, 0, s, 0, a, b, zero, n_zero), "split_operands_kernel launch");
 }
 
 // f32 inputs on the tcgen05 tensor cores: split pass (hi / lo planes, B's planes K-major), then the
@@ -750,31 +777,10 @@ inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, 
     auto launch_pairs = [&](auto kern, int smem) -> cudaError_t {
       cudaError_t pe = set_dyn_smem_once(kern, smem);
       if (pe != cudaSuccess) return pe;
-      cudaLaunchConfig_t cfg = {};
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 2;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.blockDim = dim3(g::kThreads);
-      cfg.dynamicSmemBytes = static_cast<size_t>(smem);
-      cfg.stream = s;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      cfg.gridDim = dim3(static_cast<unsigned>(sms & ~1));
-      int max_clusters = sms / 2;
-      kernel_fact(reinterpret_cast<const void*>(kern), kFactClusters, &max_clusters, [&](int* out) {
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
-          (void)cudaGetLastError();
-          return false;
-        }
-        *out = n;
-        return true;
-      });
+      const int max_clusters = resident_clusters(kern, g::kThreads, static_cast<size_t>(smem), 2, static_cast<unsigned>(sms & ~1), sms / 2);
       const int64_t npairs = std::min<int64_t>(tiles, std::min<int64_t>(max_clusters, sms / 2));
-      cfg.gridDim = dim3(static_cast<unsigned>(2 * npairs));
-      return cudaLaunchKernelEx(&cfg, kern, ta_hi, ta_lo, tb_hi, tb_lo, static_cast<float*>(c), p);
+      return launch_chained(kern, static_cast<unsigned>(2 * npairs), g::kThreads, static_cast<size_t>(smem), s, 2, ta_hi, ta_lo, tb_hi, tb_lo,
+                            static_cast<float*>(c), p);
     };
     if (pairs) {
       if (rows_aligned)
@@ -789,8 +795,7 @@ inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, 
       e = set_dyn_smem_once(kern, g::kSmemBytes);
       if (e == cudaSuccess) {
         const unsigned grid = static_cast<unsigned>(std::min<int64_t>(tiles, sms));
-        kern<<<grid, g::kThreads, g::kSmemBytes, s>>>(ta_hi, ta_lo, tb_hi, tb_lo, static_cast<float*>(c), p);
-        e = cudaGetLastError();
+        e = launch_chained(kern, grid, g::kThreads, g::kSmemBytes, s, 0, ta_hi, ta_lo, tb_hi, tb_lo, static_cast<float*>(c), p);
       }
       st = cuda_ok(err, e, "gemm_tf32_tc_kernel launch");
     }
@@ -833,8 +838,7 @@ inline int32_t gemm_tc_launch(std::string* err, const tsm100_gemm_desc* d, const
   cudaError_t e = set_dyn_smem_once(kern, g::kSmemBytes);
   if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(gemm_tc_kernel)");
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>(tiles, sms));
-  kern<<<grid, g::kThreads, g::kSmemBytes, s>>>(ta, tb, static_cast<OutT*>(c), p);
-  return cuda_ok(err, cudaGetLastError(), "gemm_tc_kernel launch");
+  return cuda_ok(err, launch_chained(kern, grid, g::kThreads, g::kSmemBytes, s, 0, ta, tb, static_cast<OutT*>(c), p), "gemm_tc_kernel launch");
 }
 
 // Few output tiles: 128 columns x NT rows of C per CTA, K split over clusters (gemm_skinny.cuh).
@@ -871,19 +875,8 @@ inline int32_t gemm_skinny_launch_nt(std::string* err, const tsm100_gemm_desc* d
   constexpr int smem = g::smem_bytes<NT>();
   cudaError_t e = set_dyn_smem_once(kern, smem);
   if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(gemm_skinny_kernel)");
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(splits);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cfg.blockDim = dim3(g::kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.gridDim = dim3(static_cast<unsigned>(tiles * splits));
-  e = cudaLaunchKernelEx(&cfg, kern, ta, tb, static_cast<OutT*>(c), p);
+  e = launch_chained(kern, static_cast<unsigned>(tiles * splits), g::kThreads, smem, s, static_cast<unsigned>(splits), ta, tb,
+                     static_cast<OutT*>(c), p);
   return cuda_ok(err, e, "gemm_skinny_kernel launch");
 }
 template <typename OutT, bool kBT, bool kBf16>
@@ -929,32 +922,10 @@ inline int32_t gemm_tc2_launch(std::string* err, const tsm100_gemm_desc* d, cons
   int sms = 0;
   st = sm_count(err, &sms);
   if (st != TSM100_OK) return st;
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.blockDim = dim3(g::kThreads);
-  cfg.dynamicSmemBytes = g::kSmemBytes;
-  cfg.stream = s;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cfg.gridDim = dim3(static_cast<unsigned>(sms & ~1));
-  int max_clusters = sms / 2;  // how many pairs the GPU holds at once: asked once per kernel and device
-  kernel_fact(reinterpret_cast<const void*>(kern), kFactClusters, &max_clusters, [&](int* out) {
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n < 1) {
-      (void)cudaGetLastError();
-      return false;
-    }
-    *out = n;
-    return true;
-  });
+  const int max_clusters = resident_clusters(kern, g::kThreads, g::kSmemBytes, 2, static_cast<unsigned>(sms & ~1), sms / 2);
   const int64_t tiles = static_cast<int64_t>(p.m_blocks) * p.n_blocks * p.batch;
   const int64_t pairs = std::min<int64_t>(tiles, std::min<int64_t>(max_clusters, sms / 2));
-  cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs));
-  e = cudaLaunchKernelEx(&cfg, kern, ta, tb, static_cast<OutT*>(c), p);
+  e = launch_chained(kern, static_cast<unsigned>(2 * pairs), g::kThreads, g::kSmemBytes, s, 2, ta, tb, static_cast<OutT*>(c), p);
   return cuda_ok(err, e, "gemm_tc2_kernel launch");
 }
 
@@ -988,9 +959,9 @@ inline int32_t gemm_padded(std::string* err, const tsm100_gemm_desc* d, const vo
   auto pad = [&](const void* src, int64_t pitch, int64_t rows, int64_t cols, uint16_t* dst, int64_t drows, int64_t dcols) {
     const int64_t items = drows * (dcols / 8);
     const dim3 grid(static_cast<unsigned>(std::min<int64_t>((items + g::kThreads - 1) / g::kThreads, 16ll * sms)), static_cast<unsigned>(batch));
-    g::pad_kernel<<<grid, g::kThreads, 0, s>>>(static_cast<const uint16_t*>(src), pitch, rows * pitch, static_cast<int32_t>(rows),
-                                              static_cast<int32_t>(cols), reinterpret_cast<uint4*>(dst), static_cast<int32_t>(drows),
-                                              static_cast<int32_t>(dcols));
+    if (e == cudaSuccess)
+      e = launch_chained(g::pad_kernel, grid, g::kThreads, 0, s, 0, static_cast<const uint16_t*>(src), pitch, rows * pitch, static_cast<int32_t>(rows),
+                         static_cast<int32_t>(cols), reinterpret_cast<uint4*>(dst), static_cast<int32_t>(drows), static_cast<int32_t>(dcols));
   };
   tsm100_gemm_desc t = *d;
   t.n = np, t.k = kp;
@@ -999,13 +970,13 @@ inline int32_t gemm_padded(std::string* err, const tsm100_gemm_desc* d, const vo
   if (pad_a) pad(a, ld.lda, d->m, d->k, ws, d->m, kp), ta = ws, t.lda = kp;
   if (pad_b) pad(b, ld.ldb, b_rows, b_cols, ws + a_elems, bp_rows, bp_cols), tb = ws + a_elems, t.ldb = bp_cols;
   if (pad_c) tc = ws + a_elems + b_elems, t.ldc = np;
-  st = cuda_ok(err, cudaGetLastError(), "gemm operand padding launch");
+  st = cuda_ok(err, e, "gemm operand padding launch");
   if (st == TSM100_OK) st = gemm(err, &t, ta, tb, tc, status, s);
   if (st == TSM100_OK && pad_c) {
     const dim3 grid(static_cast<unsigned>((d->n + g::kThreads - 1) / g::kThreads), static_cast<unsigned>(std::min<int64_t>(d->m, 4096)), static_cast<unsigned>(batch));
-    g::unpad_kernel<<<grid, g::kThreads, 0, s>>>(static_cast<const uint16_t*>(tc), static_cast<int32_t>(np), static_cast<uint16_t*>(c), ld.ldc,
-                                                d->m * ld.ldc, static_cast<int32_t>(d->m), static_cast<int32_t>(d->n));
-    st = cuda_ok(err, cudaGetLastError(), "gemm result copy launch");
+    e = launch_chained(g::unpad_kernel, grid, g::kThreads, 0, s, 0, static_cast<const uint16_t*>(tc), static_cast<int32_t>(np),
+                       static_cast<uint16_t*>(c), ld.ldc, d->m * ld.ldc, static_cast<int32_t>(d->m), static_cast<int32_t>(d->n));
+    st = cuda_ok(err, e, "gemm result copy launch");
   }
   e = cudaFreeAsync(ws, s);
   if (st == TSM100_OK && e != cudaSuccess) st = cuda_ok(err, e, "cudaFreeAsync");
@@ -1113,8 +1084,7 @@ inline int32_t attention_tf32x3_launch_d(std::string* err, const attn_simt::Para
   constexpr int smem = at::smem_bytes<T, D>();
   cudaError_t e = set_dyn_smem_once(kern, smem);
   if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(attention_tf32x3_kernel)");
-  kern<<<static_cast<unsigned>(grid), at::kThreads, smem, s>>>(q, k, v, o, p);
-  return cuda_ok(err, cudaGetLastError(), "attention_tf32x3_kernel launch");
+  return cuda_ok(err, launch_chained(kern, static_cast<unsigned>(grid), at::kThreads, smem, s, 0, q, k, v, o, p), "attention_tf32x3_kernel launch");
 }
 template <typename T>
 inline int32_t attention_tf32x3_launch(std::string* err, const attn_simt::Params& p, const void* q, const void* k,
@@ -1168,6 +1138,7 @@ inline int32_t attention_f32_tc_launch_d(std::string* err, const attn_simt::Para
       pp.a = p;
       pp.status = status;
       const int64_t grid = static_cast<int64_t>((p.seq + at::kBQ - 1) / at::kBQ) * p.batch * p.heads_q;
+      // not chained: it fills every SM by itself, and 16 heads of 4096 took 0.7 % longer that way
       kern<<<static_cast<unsigned>(grid), at::kThreads, at::smem_bytes<D>(), s>>>(tk_hi, tk_lo, tv_hi, tv_lo, q, o, pp);
       e = cudaGetLastError();
     }
@@ -1281,29 +1252,15 @@ inline int32_t attention_fwd_launch(std::string* err, const CUtensorMap& tq, con
     auto kern = at::attention_fwd_kernel<kBf16, kCache, D>;
     e = set_dyn_smem_once(kern, smem);
     if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(attention_fwd_kernel)");
-    kern<<<static_cast<unsigned>(blocks), at::kThreads, smem, s>>>(tq, tk, tv, out, p);
-    return cuda_ok(err, cudaGetLastError(), "attention_fwd_kernel launch");
+    return cuda_ok(err, launch_chained(kern, static_cast<unsigned>(blocks), at::kThreads, smem, s, 0, tq, tk, tv, out, p), "attention_fwd_kernel launch");
   }
   p.part = reinterpret_cast<float4*>(ws);
   p.part_ml = reinterpret_cast<float2*>(ws + rows * D);
   auto kern = at::attention_fwd_kernel<kBf16, kCache, D, true>;
   e = set_dyn_smem_once(kern, smem);
-  if (e == cudaSuccess) {
-    kern<<<static_cast<unsigned>(blocks * p.splits), at::kThreads, smem, s>>>(tq, tk, tv, out, p);
-    e = cudaGetLastError();
-  }
-  if (e == cudaSuccess) {
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cfg.blockDim = dim3(2 * at::kBQ);
-    cfg.stream = s;
-    cfg.gridDim = dim3(static_cast<unsigned>(blocks * (D / 16)));
-    e = cudaLaunchKernelEx(&cfg, at::attention_merge_kernel<kBf16, kCache, D>, out, p);
-  }
+  if (e == cudaSuccess) e = launch_chained(kern, static_cast<unsigned>(blocks * p.splits), at::kThreads, smem, s, 0, tq, tk, tv, out, p);
+  if (e == cudaSuccess)
+    e = launch_chained(at::attention_merge_kernel<kBf16, kCache, D>, static_cast<unsigned>(blocks * (D / 16)), 2 * at::kBQ, 0, s, 0, out, p);
   st = cuda_ok(err, e, "attention_fwd_kernel (split) launch");
   e = cudaFreeAsync(ws, s);
   if (st == TSM100_OK && e != cudaSuccess) st = cuda_ok(err, e, "cudaFreeAsync");
@@ -1402,19 +1359,8 @@ inline int32_t attention_decode_launch(std::string* err, const tsm100_attention_
   constexpr int smem = ad::smem_floats<T, G, D>() * static_cast<int>(sizeof(float));
   cudaError_t e = set_dyn_smem_once(kern, smem);
   if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(attention_decode_kernel)");
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(splits);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cfg.blockDim = dim3(ad::kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.gridDim = dim3(static_cast<unsigned>(static_cast<int64_t>(d->batch) * d->heads_kv * splits));
-  e = cudaLaunchKernelEx(&cfg, kern, q, k, v, o, p);
+  e = launch_chained(kern, static_cast<unsigned>(static_cast<int64_t>(d->batch) * d->heads_kv * splits), ad::kThreads, smem, s,
+                     static_cast<unsigned>(splits), q, k, v, o, p);
   return cuda_ok(err, e, "attention_decode_kernel launch");
 }
 
@@ -1453,19 +1399,10 @@ inline int32_t attention_decode_mma_launch(std::string* err, const tsm100_attent
     e = allow_wide_clusters_once(kern);
     if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(attention_decode_mma_kernel, wide clusters)");
   }
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = static_cast<unsigned>(splits);
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cfg.blockDim = dim3(WARPS * 32);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cfg.gridDim = dim3(static_cast<unsigned>(static_cast<int64_t>(d->batch) * d->heads_kv * splits));
-  e = cudaLaunchKernelEx(&cfg, kern, q, k, v, o, p);
+  // f32 caches are bound by the arithmetic, so an uneven placement beside the kernel before costs more than the early start gives:
+  // 24 caches of 10449 x 64, 8 heads each, 52.3 us, 53.5 chained
+  e = launch_kernel<sizeof(T) == 2>(kern, static_cast<unsigned>(static_cast<int64_t>(d->batch) * d->heads_kv * splits), WARPS * 32, smem, s,
+                                    static_cast<unsigned>(splits), q, k, v, o, p);
   return cuda_ok(err, e, "attention_decode_mma_kernel launch");
 }
 
@@ -1498,19 +1435,9 @@ inline int32_t attention_decode_global_launch(std::string* err, const tsm100_att
   for (int base = 0; base < p.group && e == cudaSuccess; base += ad::mma::kRows) {
     p.head_base = base;
     p.heads_here = std::min(ad::mma::kRows, p.group - base);
-    kern<<<static_cast<unsigned>(units * splits), WARPS * 32, smem, s>>>(q, k, v, o, p);
-    e = cudaGetLastError();
+    e = launch_chained(kern, static_cast<unsigned>(units * splits), WARPS * 32, smem, s, 0, q, k, v, o, p);
     if (e != cudaSuccess) break;
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cfg.blockDim = dim3(D);
-    cfg.stream = s;
-    cfg.gridDim = dim3(static_cast<unsigned>(units * p.heads_here));
-    e = cudaLaunchKernelEx(&cfg, ad::mma::attention_decode_merge_kernel<T, D>, o, p);
+    e = launch_chained(ad::mma::attention_decode_merge_kernel<T, D>, static_cast<unsigned>(units * p.heads_here), D, 0, s, 0, o, p);
   }
   int32_t st = cuda_ok(err, e, "attention_decode_mma_kernel (partial results) launch");
   e = cudaFreeAsync(ws, s);

@@ -275,10 +275,33 @@ __device__ __forceinline__ void cluster_sync_all() {
   __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// Programmatic dependent launch: a kernel launched with that attribute starts while the kernel before it in the stream still
-// runs, and waits here before it touches memory; the other call lets the next such kernel be set up from now on.
+// Programmatic dependent launch.  The CTAs of kernels launched with that attribute (ops.cuh: launch_chained) are placed and set up
+// while the kernel before them in the stream still runs.  Such kernels keep to these rules:
+//   * every thread waits here before it reads or writes memory that other kernels may share, and before the first barrier of its
+//     own whose wait is bounded (the kernel before may run for any time).  What comes earlier: barrier and tensor-memory set-up,
+//     arithmetic on the parameters, prefetches into the L2 (where all writes meet, so a line fetched too early is not stale);
+//   * every CTA waits before it ends, so a grid is over after the one before it, and waiting for one is waiting for all;
+//   * launch_dependents, which lets the next kernel of the stream be placed, comes after the CTA has its tensor memory: the next
+//     kernel's CTAs hold theirs while they wait, and would keep this one from ever getting its own;
+//   * where a grid fills the SMs only in part, or several CTAs to an SM, it comes after the main loop: the next such grid would take
+//     the places that become free first and leave other SMs without work;
+//   * pointers read through the read-only path go through the second form: such loads may be moved across the wait itself, but not
+//     before the value they depend on.
 __device__ __forceinline__ void wait_prior_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename T>
+__device__ __forceinline__ T* wait_prior_grid(T* p) {
+  asm volatile("griddepcontrol.wait;" : "+l"(p) : : "memory");
+  return p;
+}
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Fetches what a TMA load with the same map and coordinates would read, or `bytes` (a multiple of 16) from a 16-byte aligned
+// address, into the L2.
+__device__ __forceinline__ void prefetch_l2_3d(const CUtensorMap* map, int32_t x, int32_t y, int32_t z) {
+  asm volatile("cp.async.bulk.prefetch.tensor.3d.L2.global.tile [%0, {%1, %2, %3}];" ::"l"(map), "r"(x), "r"(y), "r"(z) : "memory");
+}
+__device__ __forceinline__ void prefetch_l2(const void* p, uint32_t bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
 // shared::cluster address of `smem_addr` (a shared::cta address) in CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t mapa_shared(uint32_t smem_addr, uint32_t rank) {
   uint32_t r;

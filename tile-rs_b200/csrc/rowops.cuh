@@ -45,6 +45,8 @@ enum : int { kRmsNorm = 0, kReduceSum = 1, kReduceMax = 2 };
 template <typename T, int OP, int VPT, int LANES, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 row_op_kernel(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t cols, float eps) {
+  ptx::launch_dependents();
+  ptx::wait_prior_grid();
   constexpr int PV = Elem<T>::kPerVec;
   constexpr int GROUPS = THREADS / LANES;  // rows in flight per CTA
   constexpr int NW = LANES / 32;           // warps per row
@@ -131,6 +133,8 @@ row_op_kernel(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t 
 template <typename T, int OP, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 row_op_stream_kernel(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int64_t cols, float eps) {
+  ptx::launch_dependents();
+  x = ptx::wait_prior_grid(x);
   __shared__ float red[32];
   constexpr bool kIsMax = OP == kReduceMax;
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -170,6 +174,8 @@ __device__ __forceinline__ float silu(float x) {
 template <typename T, bool HAS_UP, int UNROLL, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 silu_mul_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __restrict__ y, int64_t nvec) {
+  ptx::launch_dependents();
+  ptx::wait_prior_grid();
   constexpr int PV = Elem<T>::kPerVec;
   const Vec16* g = reinterpret_cast<const Vec16*>(gate);
   const Vec16* u = reinterpret_cast<const Vec16*>(up);
@@ -203,6 +209,9 @@ silu_mul_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __restr
 template <typename T, bool HAS_UP, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 silu_mul_scalar_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __restrict__ y, int64_t n) {
+  ptx::launch_dependents();
+  gate = ptx::wait_prior_grid(gate);
+  up = ptx::wait_prior_grid(up);
   const int64_t step = static_cast<int64_t>(gridDim.x) * THREADS;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * THREADS + threadIdx.x; i < n; i += step) {
     const float s = silu<T>(Elem<T>::load1(gate + i));
@@ -234,6 +243,8 @@ namespace rowops {
 template <typename T>
 __global__ void __launch_bounds__(256)
 rope_kernel(T* __restrict__ x, int64_t tokens, int32_t seq_len, int32_t heads, int32_t d, int32_t start_pos, float theta) {
+  ptx::launch_dependents();
+  ptx::wait_prior_grid();
   const int half = d / 2;
   const int64_t n = tokens * half;
   for (int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < n;
@@ -263,6 +274,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 rope_vec_kernel(T* __restrict__ x, int64_t tokens, int32_t seq_len, int32_t heads, int32_t heads_per, int32_t d, int32_t start_pos,
                 float theta) {
+  ptx::launch_dependents();
   constexpr int PV = Elem<T>::kPerVec;
   constexpr int HU = 4;
   const int dv = d / PV;
@@ -281,6 +293,7 @@ rope_vec_kernel(T* __restrict__ x, int64_t tokens, int32_t seq_len, int32_t head
       const float angle = static_cast<float>(pos) * freq;
       sincosf(angle, &s[e], &c[e]);
     }
+    ptx::wait_prior_grid();  // the angles are computed meanwhile
     Vec16* p = reinterpret_cast<Vec16*>(x + tok * heads * d) + j;
     auto rotate = [&](const Vec16& raw) -> Vec16 {
       float f[PV], r[PV];
@@ -303,6 +316,7 @@ rope_vec_kernel(T* __restrict__ x, int64_t tokens, int32_t seq_len, int32_t head
     }
     for (; h < h1; ++h) p[static_cast<int64_t>(h) * dv] = rotate(p[static_cast<int64_t>(h) * dv]);
   }
+  ptx::wait_prior_grid();
 }
 
 // VEC = elements per access (16 bytes when rows allow it, else 1); I = index arithmetic type: 32-bit when the
@@ -311,6 +325,8 @@ template <typename T, int VEC, typename I>
 __global__ void __launch_bounds__(256)
 kv_cache_update_kernel(const T* __restrict__ src, T* __restrict__ cache, int64_t batch, int32_t seq_len, int32_t heads,
                        int32_t d, int32_t start_pos, int32_t max_seq) {
+  ptx::launch_dependents();
+  src = ptx::wait_prior_grid(src);
   const I dv = static_cast<I>(d / VEC);
   const I n = static_cast<I>(batch * seq_len * heads) * dv;
   const I stride = static_cast<I>(gridDim.x) * blockDim.x;
@@ -324,7 +340,7 @@ kv_cache_update_kernel(const T* __restrict__ src, T* __restrict__ cache, int64_t
     const T* s = src + ((b * seq_len + static_cast<int64_t>(si)) * heads + static_cast<int64_t>(h)) * d + dd;
     T* c = cache + ((b * heads + static_cast<int64_t>(h)) * max_seq + start_pos + static_cast<int64_t>(si)) * d + dd;
     if (VEC == 1) *c = *s;
-    else *reinterpret_cast<Vec16*>(c) = *reinterpret_cast<const Vec16*>(s);
+    else *reinterpret_cast<Vec16*>(c) = softmax::ld_keep(reinterpret_cast<const Vec16*>(s));
   }
 }
 

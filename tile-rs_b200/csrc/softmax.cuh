@@ -153,6 +153,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 template <typename T, int CHUNKS, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
 softmax_rows_warp(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t cols) {
+  ptx::launch_dependents();
+  ptx::wait_prior_grid();
   constexpr int PV = Elem<T>::kPerVec;
   const int lane = threadIdx.x & 31;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
@@ -223,6 +225,8 @@ __device__ __forceinline__ float exp_shifted(float x, float m_log2e) {
 template <typename T, int VPT, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 softmax_rows_cta(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t cols) {
+  ptx::launch_dependents();
+  ptx::wait_prior_grid();
   constexpr int PV = Elem<T>::kPerVec;
   constexpr int NW = THREADS / 32;
   __shared__ float red_max[NW];
@@ -377,6 +381,8 @@ __device__ __forceinline__ float exp_diff(float x, float m) {
 template <typename T, int CHUNKS, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
 softmax_rows_warp_any(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t cols) {
+  ptx::launch_dependents();
+  x = ptx::wait_prior_grid(x);
   constexpr int PV = Elem<T>::kPerVec;
   const int lane = threadIdx.x & 31;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * WARPS + (threadIdx.x >> 5);
@@ -415,6 +421,8 @@ softmax_rows_warp_any(const T* __restrict__ x, T* __restrict__ y, int64_t rows, 
 template <typename T, int VPT, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 softmax_rows_cta_any(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t cols) {
+  ptx::launch_dependents();
+  x = ptx::wait_prior_grid(x);
   constexpr int PV = Elem<T>::kPerVec;
   constexpr int NW = THREADS / 32;
   __shared__ float2 slots[2][NW];  // alternating: a slot is rewritten after the next row's barrier at the earliest
@@ -484,6 +492,8 @@ constexpr int kTwiceUnroll = 4;
 template <typename T, int THREADS, bool kSkip>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 softmax_rows_twice(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t cols) {
+  ptx::launch_dependents();
+  x = ptx::wait_prior_grid(x);
   constexpr int PV = Elem<T>::kPerVec;
   constexpr int NW = THREADS / 32;
   constexpr int UNROLL = kTwiceUnroll;
@@ -551,6 +561,8 @@ softmax_rows_twice(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int
 template <typename T, int VPT, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 softmax_rows_cluster(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t cols) {
+  ptx::launch_dependents();
+  x = ptx::wait_prior_grid(x);
   constexpr int PV = Elem<T>::kPerVec;
   constexpr int NW = THREADS / 32;
   __shared__ float2 slots[NW];
@@ -627,6 +639,8 @@ __device__ __forceinline__ float block_reduce(float v, float* red, bool is_max) 
 template <typename T, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 softmax_rows_stream(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int64_t cols) {
+  ptx::launch_dependents();
+  x = ptx::wait_prior_grid(x);
   __shared__ float red[32];
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
     const T* xr = x + row * cols;
