@@ -1,0 +1,130 @@
+"""f32 GEMM with the operands split on the way in: tile edges, both widths, splits of K, several tiles per CTA, rows that start anywhere,
+pitches, batches, and values that a split cannot represent."""
+
+import pytest
+
+import util
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def rnd(*shape, seed=1, sigma=1.0):
+    g = torch.Generator(device="cuda:0")
+    g.manual_seed(seed)
+    return torch.randn(shape, generator=g, device="cuda:0") * sigma
+
+
+def product(dev, capi, a, b, m, n, k, bt, batch=1, lda=0, ldb=0, ldc=0, c=None):
+    c = torch.full((batch, m, ldc or n), float("nan"), device="cuda:0") if c is None else c
+    dev.gemm(capi.F32, m, n, k, a.data_ptr(), b.data_ptr(), c.data_ptr(), b_transposed=bt, batch=batch, lda=lda, ldb=ldb, ldc=ldc,
+             stream=util.cur_stream(torch))
+    torch.cuda.synchronize()
+    assert dev.status() == 0
+    return c
+
+
+# An accumulator rounds toward zero, at most 2^-24 of what it holds (half of that in the mean) at each of the 12 instructions per 32
+# of K: 1.4e-6 of the result for a chunk of 128.  Sums the warp-level kernel took in one go are kept within 384 of K of that.
+def bound(m, n, k, aligned):
+    if not aligned:
+        return 1e-6
+    tiles = -(-m // 64) * -(-n // 64)
+    s = 1
+    while s < 4 and tiles * s * 2 <= 296 and k // (2 * s) >= 128:
+        s *= 2
+    return max(2e-6, 7.5e-9 * (k / s - 300))
+
+
+@pytest.mark.parametrize("bt", [False, True])
+@pytest.mark.parametrize("m,n,k", [
+    (1, 1, 64), (1, 1, 65), (128, 64, 64), (129, 65, 95), (127, 63, 97), (100, 70, 2501), (301, 301, 1000), (512, 512, 512), (130, 129, 1024),
+    (1024, 1024, 1024), (600, 2401, 201), (600, 2400, 200), (1001, 1003, 333), (2400, 1900, 161), (2401, 1901, 65), (3000, 5000, 160), (5, 4000, 777)])
+def test_against_64_bits(dev, pkg, m, n, k, bt):
+    s = k ** -0.25
+    a, b = rnd(m, k, sigma=s), rnd(*((n, k) if bt else (k, n)), seed=2, sigma=s)
+    c = product(dev, pkg.capi, a, b, m, n, k, bt)[0]
+    want = a.double() @ (b.double().T if bt else b.double())
+    err = float((c - want).norm() / want.norm())
+    assert err <= bound(m, n, k, k % 4 == 0 and n % 4 == 0), err
+
+
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+@pytest.mark.parametrize("bt", [False, True])
+def test_rows_that_start_anywhere_pitches_and_batches(dev, pkg, shift, bt):
+    """Column blocks of larger matrices, `shift` elements from a 16-byte boundary; what lies around C stays."""
+    m, n, k, batch = 150, 203, 300, 3
+    lda, ldb, ldc = 309, 331, 223
+    rows_b, cols_b = (n, k) if bt else (k, n)
+    big_a, big_b = rnd(batch * m * lda + 8), rnd(batch * rows_b * ldb + 8, seed=2)
+    big_c = torch.full((batch * m * ldc + 8,), 7.0, device="cuda:0")
+    a, b, c = big_a[shift:], big_b[shift:], big_c[shift:]
+    product(dev, pkg.capi, a, b, m, n, k, bt, batch, lda, ldb, ldc, c)
+    av = a[:batch * m * lda].view(batch, m, lda)[:, :, :k].double()
+    bv = b[:batch * rows_b * ldb].view(batch, rows_b, ldb)[:, :, :cols_b].double()
+    want = av @ (bv.transpose(1, 2) if bt else bv)
+    got = c[:batch * m * ldc].view(batch, m, ldc)
+    assert float((got[:, :, :n] - want).norm() / want.norm()) <= 1e-6
+    assert bool((got[:, :, n:] == 7.0).all()) and bool((big_c[:shift] == 7.0).all()) and bool((c[batch * m * ldc:] == 7.0).all())
+
+
+@pytest.mark.parametrize("m,n,k,bt", [(300, 301, 2001, False), (200, 131, 333, True), (1700, 1501, 97, False), (2401, 2301, 129, True)])
+def test_infinities_nans_and_the_largest_numbers_as_on_the_fp32_pipe(dev, pkg, m, n, k, bt):
+    """Split K, one tile and several tiles per CTA: outputs infinite or NaN where plain f32 sums are, finite where those are finite."""
+    a, b = rnd(m, k, sigma=0.1), rnd(*((n, k) if bt else (k, n)), seed=2, sigma=0.1)
+    bv = b.T if bt else b
+    all_ones = torch.tensor([-1], dtype=torch.int32, device="cuda:0").view(torch.float32)[0]  # a NaN whose rounding carries
+    a[0, 5], a[m // 2, 0], a[m - 1, k - 1] = float("inf"), float("-inf"), all_ones
+    a[1, 3], a[2, 4] = 3.4e38, -3.4028234e38   # the second rounds up to infinity as a TF32 number
+    bv[3, :], bv[4, :] = 0.25, 0.5
+    bv[5, n - 1] = 0.0                           # 0 * inf
+    bv[k - 2, 1] = float("nan")
+    c = product(dev, pkg.capi, a, b, m, n, k, bt)[0]
+    want = a.double() @ bv.double()  # finite ones stay far below the largest f32 number
+    want32 = want.float()
+    assert torch.equal(torch.isnan(c), torch.isnan(want32))
+    assert torch.equal(torch.isinf(c), torch.isinf(want32)) and torch.equal(c[torch.isinf(c)] > 0, want32[torch.isinf(c)] > 0)
+    ok = torch.isfinite(want32)
+    # sums of k products of 0.1 x 0.1 stand beside terms of up to 1.7e38
+    scale = a.abs().nan_to_num(0, 0, 0).double() @ bv.abs().nan_to_num(0, 0, 0).double()
+    assert float(((c - want).abs()[ok] / scale[ok]).max()) <= 4e-6
+    whole = product(dev, pkg.capi, a, b, m, n, k, bt)[0]
+    assert torch.equal(whole.view(torch.int32), c.view(torch.int32))  # the second pass has one order too
+
+
+def test_every_output_infinite(dev, pkg):
+    m, n, k = 1500, 1301, 301
+    a, b = rnd(m, k).abs() + 0.1, rnd(k, n, seed=2).abs() + 0.1
+    a[:, 7] = float("inf")
+    assert bool(torch.isposinf(product(dev, pkg.capi, a, b, m, n, k, False)).all())
+
+
+def test_whole_numbers_stay_exact(dev, pkg):
+    """Products and partial sums below 2^24 (factors of up to 13 bits: hi and lo both in use)."""
+    for (m, n, k, bt) in ((200, 301, 401, False), (600, 600, 1024, True), (129, 500, 64, False)):
+        g = torch.Generator(device="cuda:0")
+        g.manual_seed(3)
+        a = torch.randint(-8191, 8192, (m, k), generator=g, device="cuda:0").float()
+        b = torch.randint(-1, 2, (n, k) if bt else (k, n), generator=g, device="cuda:0").float()
+        want = a.double() @ (b.double().T if bt else b.double())
+        assert float(want.abs().max()) < 2 ** 24
+        assert torch.equal(product(dev, pkg.capi, a, b, m, n, k, bt)[0].double(), want)
+
+
+def test_captured_and_on_two_streams(dev, pkg):
+    m, n, k = 300, 333, 1111
+    a, b = rnd(m, k), rnd(k, n, seed=2)
+    want = product(dev, pkg.capi, a, b, m, n, k, False)
+    streams, outs = [torch.cuda.Stream() for _ in range(2)], [torch.zeros(m, n, device="cuda:0") for _ in range(3)]
+    torch.cuda.synchronize()
+    for s, o in zip(streams, outs):
+        for _ in range(10):
+            dev.gemm(pkg.capi.F32, m, n, k, a.data_ptr(), b.data_ptr(), o.data_ptr(), stream=s.cuda_stream)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        dev.gemm(pkg.capi.F32, m, n, k, a.data_ptr(), b.data_ptr(), outs[2].data_ptr(), stream=torch.cuda.current_stream().cuda_stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want[0]) for o in outs)
+    del graph

@@ -15,6 +15,10 @@ extern "C" void gemm16_plan(long long m, long long n, long long k, long long bat
   const Gemm16 r = gemm16(m, n, k, batch, sms);
   out[0] = r.kind, out[1] = r.rows, out[2] = r.splits, out[3] = r.k_blocks_per_cta;
 }
+extern "C" void gemm_f32_plan(long long m, long long n, long long k, long long batch, int aligned, int sms, long long* out) {
+  const GemmF32 r = gemm_f32(m, n, k, batch, aligned != 0, sms);
+  out[0] = r.kind, out[1] = r.bn, out[2] = r.splits, out[3] = r.chunk_kb;
+}
 extern "C" int padding_pays(long long m, long long n, long long k, long long batch) { return gemm16_padding_pays(m, n, k, batch); }
 extern "C" int row_per_warp(long long span, long long rows, int sms) { return softmax_row_per_warp(span, rows, sms); }
 extern "C" int cluster(long long span, long long rows, int sms) { return softmax_cluster(span, rows, sms); }
@@ -122,3 +126,24 @@ def test_rotary_head_groups(lib, blocks, heads, per):
     (1, 1, 1), (1, 3969, 1), (1, 4095, 1), (1, 4096, 2), (64, 16384, 2), (74, 1 << 20, 2), (75, 1 << 20, 1), (9, 34000, 16), (1, 1 << 20, 148), (1 << 20, 8192, 1)])
 def test_attention_steps_over_several_ctas(lib, blocks, keys, ctas):
     assert lib.splits(C.c_longlong(blocks), C.c_longlong(keys), SMS) == ctas
+
+
+PLANES, FUSED, WARP, FP32 = 0, 1, 2, 3
+
+
+@pytest.mark.parametrize("m,n,k,batch,aligned,kind,splits,chunk", [
+    (4096, 4096, 4096, 1, 1, PLANES, None, None), (1999, 3001, 1501, 1, 0, PLANES, None, None), (1999, 3001, 255, 1, 0, FUSED, 1, 1),
+    (512, 512, 512, 1, 1, FUSED, 4, 4), (512, 512, 512, 1, 0, FUSED, 4, 2), (64, 64, 64, 1, 1, WARP, None, None), (64, 64, 63, 1, 0, FP32, None, None),
+    (64, 64, 64, 1, 0, FUSED, 1, 1), (1024, 1024, 156, 1, 1, FUSED, 1, 4), (300, 300, 156, 1, 1, WARP, None, None),
+    # the warp-level kernel sums 1024 in one go, the fused kernel 640 of them (20 k-blocks), in one CTA
+    (1024, 1024, 1024, 1, 1, FUSED, 1, 20), (1024, 1024, 1024, 1, 0, FUSED, 2, 2), (64, 64, 100000, 1, 0, FUSED, 8, 2),
+    (1419, 372, 680, 1, 1, FUSED, 2, 4), (64, 64, 200, 149, 1, WARP, None, None), (64, 64, 200, 148, 1, FUSED, 1, 4), (65, 64, 200, 149, 1, FUSED, 1, 4)])
+def test_f32_products(lib, m, n, k, batch, aligned, kind, splits, chunk):
+    out = (C.c_longlong * 4)()
+    lib.gemm_f32_plan(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch), aligned, SMS, out)
+    assert out[0] == kind
+    if kind == FUSED:
+        assert out[1] in (64, 128) and (out[2], out[3]) == (splits, chunk)
+        # every CTA of a cluster has work, and all clusters fit the GPU at once
+        tiles = -(-m // 128) * -(-n // out[1]) * batch
+        assert out[2] == 1 or tiles * out[2] <= SMS

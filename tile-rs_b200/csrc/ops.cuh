@@ -35,6 +35,7 @@
 #include "gemm_skinny.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_tc2.cuh"
+#include "gemm_tf32_fused.cuh"
 #include "gemm_tf32_tc.cuh"
 #include "gemm_tf32x3.cuh"
 #include "route.hpp"
@@ -656,10 +657,8 @@ inline int32_t gemm_tf32x3_launch(std::string* err, const tsm100_gemm_desc* d, c
   if (st != TSM100_OK) return st;
   const int64_t tiles = ((d->m + g::kBM - 1) / g::kBM) * ((d->n + g::kBN - 1) / g::kBN) * d->batch;
   if (tiles * g::kMaxSplit > 0x7fffffff) return op_fail(err, TSM100_ERR_INVALID, "gemm: too many tiles for one launch");
-  // fewer tiles than SMs: a cluster splits K while all CTAs still fit the GPU at once (two per SM) and every CTA
-  // keeps at least four 32-deep slices
-  int splits = 1;
-  while (splits < g::kMaxSplit && tiles * splits * 2 <= 2 * sms && d->k / (2 * splits) >= 4 * g::kBK) splits *= 2;
+  static_assert(g::kBM == 64 && g::kBN == 64 && g::kBK == 32 && g::kMaxSplit == route::kMaxWarpF32Split, "route.hpp plans in these units");
+  const int splits = route::gemm_f32_warp_splits(tiles, d->k, sms);
   g::Params p;
   p.m = static_cast<int32_t>(d->m);
   p.n = static_cast<int32_t>(d->n);
@@ -803,6 +802,54 @@ inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, 
   e = cudaFreeAsync(ws, s);  // stream-ordered: after the kernel that reads the planes
   if (st == TSM100_OK && e != cudaSuccess) st = cuda_ok(err, e, "cudaFreeAsync");
   return st;
+}
+
+// f32 inputs on the tcgen05 tensor cores, split on the way in (gemm_tf32_fused.cuh).
+inline int32_t gemm_tf32_fused_launch(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
+                                      const route::GemmF32& plan, uint32_t* status, bool redo, cudaStream_t s) {
+  namespace g = gemm_tf32_fused;
+  const int bn = plan.bn;
+  const GemmPitch ld = gemm_pitch(d);
+  int sms = 0;
+  int32_t st = sm_count(err, &sms);
+  if (st != TSM100_OK) return st;
+  g::Params p = {};
+  p.g.m = static_cast<int32_t>(d->m);
+  p.g.n = static_cast<int32_t>(d->n);
+  p.g.k = static_cast<int32_t>(d->k);
+  p.g.batch = d->batch;
+  p.g.m_blocks = static_cast<int32_t>((d->m + g::kBM - 1) / g::kBM);
+  p.g.n_blocks = static_cast<int32_t>((d->n + bn - 1) / bn);
+  p.g.c_batch_stride = d->m * ld.ldc;
+  p.g.ldc = ld.ldc;
+  p.g.status = status;
+  p.g.vec_store = aligned16(c) && ld.ldc % 4 == 0 ? 1 : 0;
+  p.g.chunk_kb = plan.chunk_kb;
+  p.g.b_transposed = d->b_transposed;
+  p.g.a = static_cast<const float*>(a);
+  p.g.b = static_cast<const float*>(b);
+  p.g.lda = ld.lda, p.g.ldb = ld.ldb;
+  p.g.a_batch_stride = d->m * ld.lda;
+  p.g.b_batch_stride = (d->b_transposed ? d->n : d->k) * ld.ldb;
+  p.vec_a = aligned16(a) && d->k % 4 == 0 && ld.lda % 4 == 0;
+  p.vec_b = aligned16(b) && d->k % 4 == 0 && ld.ldb % 4 == 0;
+  const int64_t kb = (d->k + g::kBK - 1) / g::kBK;
+  p.kb_per_cta = static_cast<int32_t>((kb + plan.splits - 1) / plan.splits);
+  const int splits = static_cast<int>((kb + p.kb_per_cta - 1) / p.kb_per_cta);  // a last CTA without work is dropped
+  const int64_t tiles = static_cast<int64_t>(p.g.m_blocks) * p.g.n_blocks * p.g.batch;
+  const unsigned grid = static_cast<unsigned>(splits > 1 ? tiles * splits : std::min<int64_t>(tiles, sms));
+  auto launch = [&](auto kern, int smem) -> cudaError_t {
+    cudaError_t e = set_dyn_smem_once(kern, smem);
+    if (e != cudaSuccess) return e;
+    return launch_chained(kern, grid, g::kThreads, static_cast<size_t>(smem), s, static_cast<unsigned>(splits > 1 ? splits : 0), static_cast<float*>(c), p);
+  };
+  auto pick = [&](auto bn_tag) -> cudaError_t {
+    constexpr int BN = decltype(bn_tag)::value;
+    auto kern = d->b_transposed ? (redo ? g::gemm_tf32_fused_kernel<BN, true, true> : g::gemm_tf32_fused_kernel<BN, true, false>)
+                                : (redo ? g::gemm_tf32_fused_kernel<BN, false, true> : g::gemm_tf32_fused_kernel<BN, false, false>);
+    return launch(kern, g::smem_bytes<BN>());
+  };
+  return cuda_ok(err, bn == 64 ? pick(std::integral_constant<int, 64>{}) : pick(std::integral_constant<int, 128>{}), "gemm_tf32_fused_kernel launch");
 }
 
 template <typename OutT, bool kBT, bool kBf16>
@@ -1009,14 +1056,18 @@ inline int32_t gemm(std::string* err, const tsm100_gemm_desc* d, const void* a, 
   if (d->dtype == TSM100_F32) {
     const bool vec_ok = aligned16(a) && aligned16(b) && aligned16(c) && d->k % 4 == 0 && (d->b_transposed || d->n % 4 == 0) &&
                         d->n % 2 == 0 && ld.lda % 4 == 0 && ld.ldb % 4 == 0 && ld.ldc % 2 == 0;
-    // enough work for the persistent tcgen05 kernels; their split pass takes rows of any alignment
-    const int64_t tiles = ((d->m + 127) / 128) * ((d->n + 255) / 256) * d->batch;
-    if (status != nullptr && tiles >= 64 && tiles < 0x7fffffff && d->k >= 256) {
-      const int32_t st = gemm_tf32_tc_launch(err, d, a, b, c, status, vec_ok, s);
-      if (st != kNoScratch) return st;
+    if (status != nullptr) {
+      int sms = 0;
+      int32_t st = sm_count(err, &sms);
+      if (st != TSM100_OK) return st;
+      const route::GemmF32 plan = route::gemm_f32(d->m, d->n, d->k, d->batch, vec_ok, sms);
+      const int64_t tiles = ((d->m + 127) / 128) * ((d->n + 255) / 256) * d->batch;
+      if (plan.kind == route::GemmF32::kPlanes && tiles < 0x7fffffff) {
+        st = gemm_tf32_tc_launch(err, d, a, b, c, status, vec_ok, s);
+        if (st != kNoScratch) return st;
+      }
+      if (plan.kind == route::GemmF32::kFused) return gemm_tf32_fused_launch(err, d, a, b, c, plan, status, !vec_ok, s);
     }
-    // fewer tiles (the 512^3 configuration has 8): the warp-level kernel, whose 64 x 64 tiles and cluster split-K
-    // spread a small problem over the SMs, if rows start on 16-byte boundaries, else the FP32 pipe
     if (vec_ok) return gemm_tf32x3_launch(err, d, a, b, c, s);
     return gemm_simt_launch<float, float>(err, d, a, b, c, s);
   }
