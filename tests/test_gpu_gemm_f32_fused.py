@@ -92,6 +92,21 @@ def test_infinities_nans_and_the_largest_numbers_as_on_the_fp32_pipe(dev, pkg, m
     assert torch.equal(whole.view(torch.int32), c.view(torch.int32))  # the second pass has one order too
 
 
+@pytest.mark.parametrize("n", [512, 511])
+def test_the_largest_numbers_stay_finite(dev, pkg, n):
+    """Factors up to the largest one whose hi part is finite, also where rows are aligned and no second pass looks after them."""
+    m, k = 200, 512
+    a, b = rnd(m, k), rnd(k, n, seed=2, sigma=1e-3)
+    for i, x in enumerate((8.6e37, 1.2345678e38, 1.7014e38, 2.9876543e38, 3.4011e38, -3.4011e38, 3.3999999e38)):
+        a[i * 20, :] *= 1e-3
+        a[i * 20, 17 * i] = x
+    c = product(dev, pkg.capi, a, b, m, n, k, False)[0]
+    want = a.double() @ b.double()
+    assert bool(torch.isfinite(c).all())
+    scale = a.abs().double() @ b.abs().double()
+    assert float(((c - want).abs() / scale).max()) <= 2e-6
+
+
 def test_every_output_infinite(dev, pkg):
     m, n, k = 1500, 1301, 301
     a, b = rnd(m, k).abs() + 0.1, rnd(k, n, seed=2).abs() + 0.1

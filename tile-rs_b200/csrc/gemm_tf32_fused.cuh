@@ -75,21 +75,16 @@ __device__ __forceinline__ void load4(float (&v)[4], const float* src, int64_t l
     for (int j = 0; j < 4; ++j) v[j] = row < rows && k + j < k_end ? p[j] : 0.f;
   }
 }
-// hi = x rounded to TF32, ties away from zero, as an add on the bits: the conversion instruction runs at 8 a cycle and SM, which made
-// the two of every value the bound of this kernel (1.2 us per 32 of K and 128 x 128 tile).  A NaN of all ones carries into a zero
-// here, but x - hi is NaN then.  lo = x - hi (exact) rounded to TF32 by multiplying it with 2^13 + 1 and cancelling: |lo| <= 2^-11 |x|,
-// so that overflows only where hi did, and a NaN stays one.
+// hi = x rounded to TF32, lo = x - hi (exact) rounded again, without the conversion instruction (two of them for every value made 1.2 us
+// per 32 of K and 128 x 128 tile, 1.04 this way).  A NaN stays one in hi.
 __device__ __forceinline__ void split_store(uint32_t hi, uint32_t lo, const float (&v)[4]) {
-  uint32_t h[4];
-  float l[4];
+  float h[4], l[4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
-    h[j] = (__float_as_uint(v[j]) + 0x1000u) & 0xffffe000u;
-    const float d = v[j] - __uint_as_float(h[j]);
-    const float e = __fmul_rn(d, 8193.0f);
-    l[j] = __fsub_rn(e, __fsub_rn(e, d));
+    h[j] = tc::tf32_rn_fast(v[j]);
+    l[j] = tc::tf32_rn_finite(v[j] - h[j]);
   }
-  ptx::st_shared_v4(hi, h[0], h[1], h[2], h[3]);
+  ptx::st_shared_v4(hi, __float_as_uint(h[0]), __float_as_uint(h[1]), __float_as_uint(h[2]), __float_as_uint(h[3]));
   ptx::st_shared_v4(lo, __float_as_uint(l[0]), __float_as_uint(l[1]), __float_as_uint(l[2]), __float_as_uint(l[3]));
 }
 // A tile that came out infinite or NaN somewhere: those outputs are summed again in plain f32, in the order of k (an infinity split

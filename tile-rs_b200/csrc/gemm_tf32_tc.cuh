@@ -88,6 +88,12 @@ __device__ __forceinline__ float tf32_rn(float x) {
 // ---------------------------------------------------------------------------
 // One launch splits both operands (two launches cost a ramp and a tail more).
 // rows: src [rows][cols] with row pitch ld -> hi, lo [rows][cols] with row pitch kp, a multiple of 4 >= cols, so that every
+// The same as an add on the bits, for kernels where the conversion instruction, 8 a cycle and SM, would be the bound: finite numbers and
+// infinities alike, but a NaN whose bits are all ones carries into a zero.  `tf32_rn_fast` keeps a NaN, tf32_rn_finite is for what is none
+// or where another part carries it.
+__device__ __forceinline__ float tf32_rn_finite(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
+__device__ __forceinline__ float tf32_rn_fast(float x) { return x == x ? tf32_rn_finite(x) : x; }
+
 // plane row starts on a 16-byte boundary whatever cols is (the columns from cols to kp are never read: the tensor maps
 // end at cols).  One thread per four values; kVec: rows of src start on 16-byte boundaries and cols % 4 == 0, else the
 // four values are loaded one by one.
