@@ -19,6 +19,10 @@ extern "C" void gemm_f32_plan(long long m, long long n, long long k, long long b
   const GemmF32 r = gemm_f32(m, n, k, batch, aligned != 0, sms);
   out[0] = r.kind, out[1] = r.bn, out[2] = r.splits, out[3] = r.chunk_kb;
 }
+extern "C" void pair_tiles(long long m, long long n, long long k, long long batch, int sms, long long* out) {
+  const PairTiles r = gemm_f32_pair_tiles(m, n, k, batch, sms);
+  out[0] = r.bn, out[1] = r.whole_tiles, out[2] = r.splits;
+}
 extern "C" int padding_pays(long long m, long long n, long long k, long long batch) { return gemm16_padding_pays(m, n, k, batch); }
 extern "C" int row_per_warp(long long span, long long rows, int sms) { return softmax_row_per_warp(span, rows, sms); }
 extern "C" int cluster(long long span, long long rows, int sms) { return softmax_cluster(span, rows, sms); }
@@ -147,3 +151,17 @@ def test_f32_products(lib, m, n, k, batch, aligned, kind, splits, chunk):
         # every CTA of a cluster has work, and all clusters fit the GPU at once
         tiles = -(-m // 128) * -(-n // out[1]) * batch
         assert out[2] == 1 or tiles * out[2] <= SMS
+
+
+# columns of a tile, whole tiles, pairs to each of the rest
+@pytest.mark.parametrize("m,n,k,batch,want", [
+    (1999, 3001, 1501, 1, (256, 74, 3)), (2048, 2048, 2048, 1, (256, 64, 1)), (512, 10880, 999, 1, (256, 74, 4)), (4096, 4096, 4096, 1, (256, 222, 2)),
+    (1536, 1536, 1536, 1, (128, 72, 1)), (512, 9472, 1500, 1, (256, 74, 1)), (1999, 3001, 256, 1, (256, 96, 1)), (256, 256, 100000, 75, (256, 74, 4))])
+def test_shared_tiles(lib, m, n, k, batch, want):
+    out = (C.c_longlong * 3)()
+    lib.pair_tiles(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch), SMS, out)
+    assert tuple(out) == want
+    kb, splits = -(-k // 32), out[2]
+    assert (splits - 1) * -(-kb // splits) < kb  # every share has k-blocks
+    tiles = -(-m // 256) * -(-n // out[0]) * batch
+    assert (tiles - out[1]) * splits <= SMS // 2

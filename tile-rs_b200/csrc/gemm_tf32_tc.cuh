@@ -73,6 +73,11 @@ struct Params {
   int32_t b_transposed;
   const float *a, *b;
   int64_t lda, ldb, a_batch_stride, b_batch_stride;
+  // pair kernels: tiles from whole_tiles on are worked on by `splits` pairs each (see pair::Walk); their partial sums, and a counter
+  // per CTA's half of such a tile, zero at the start
+  int32_t whole_tiles, splits;
+  float4* part;
+  uint32_t* arrivals;
 };
 
 // x rounded to the nearest TF32 number (10 explicit mantissa bits; ties away from zero).  The conversion instruction, not
@@ -83,17 +88,17 @@ __device__ __forceinline__ float tf32_rn(float x) {
   return __uint_as_float(r & 0xffffe000u);
 }
 
-// ---------------------------------------------------------------------------
-// the split pass
-// ---------------------------------------------------------------------------
-// One launch splits both operands (two launches cost a ramp and a tail more).
-// rows: src [rows][cols] with row pitch ld -> hi, lo [rows][cols] with row pitch kp, a multiple of 4 >= cols, so that every
 // The same as an add on the bits, for kernels where the conversion instruction, 8 a cycle and SM, would be the bound: finite numbers and
 // infinities alike, but a NaN whose bits are all ones carries into a zero.  `tf32_rn_fast` keeps a NaN, tf32_rn_finite is for what is none
 // or where another part carries it.
 __device__ __forceinline__ float tf32_rn_finite(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
 __device__ __forceinline__ float tf32_rn_fast(float x) { return x == x ? tf32_rn_finite(x) : x; }
 
+// ---------------------------------------------------------------------------
+// the split pass
+// ---------------------------------------------------------------------------
+// One launch splits both operands (two launches cost a ramp and a tail more).
+// rows: src [rows][cols] with row pitch ld -> hi, lo [rows][cols] with row pitch kp, a multiple of 4 >= cols, so that every
 // plane row starts on a 16-byte boundary whatever cols is (the columns from cols to kp are never read: the tensor maps
 // end at cols).  One thread per four values; kVec: rows of src start on 16-byte boundaries and cols % 4 == 0, else the
 // four values are loaded one by one.
@@ -189,7 +194,7 @@ split_operands_kernel(const SplitOperand a, const SplitOperand b, uint32_t* zero
 // Columns of an accumulator read at a time.  16 leave the kRedo kernels, whose second pass holds registers too, without spills:
 // 1999 x 3001 x 1501 130.2 us with 32, 124.7 with 16; no difference for the others.
 template <bool kRedo>
-constexpr int kDrain = kRedo ? 16 : 32;
+constexpr int kDrain = 16;
 // kRedo (problems that the FP32 pipe could take as well): a block with an infinity or a NaN is marked for second_pass.
 template <bool kRedo>
 __device__ __forceinline__ void store_block_32x32(float* __restrict__ c, const Params& p, int batch, int row0, int col0,
@@ -543,8 +548,7 @@ gemm_tf32_tc_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_
 #pragma unroll
           for (int h = 0; h < 32; h += kDrain<kRedo>) {
             uint32_t v[kDrain<kRedo>];
-            if constexpr (kRedo) ptx::tmem_ld_32x32b_x16(lane_addr + acc * kBN + cc * 32 + h, v);
-            else ptx::tmem_ld_32x32b_x32(lane_addr + acc * kBN + cc * 32, v);
+            ptx::tmem_ld_32x32b_x16(lane_addr + acc * kBN + cc * 32 + h, v);
             ptx::tmem_ld_wait();
 #pragma unroll
             for (int i = 0; i < kDrain<kRedo>; ++i) sum[cc][h + i] += __uint_as_float(v[i]);  // round-to-nearest add of the chunk
@@ -632,6 +636,34 @@ __device__ __forceinline__ void tile_coords(const Params& p, int tile, int& b, i
   nb = t / rows_in_band;
 }
 
+// A pair's work, in order: whole tiles pair_id, pair_id + pairs, ... below whole_tiles, then a share of K of one of the tiles left, which
+// by themselves would occupy `splits` times fewer pairs.  (Dealing all their k-blocks out evenly gives a pair pieces of two tiles: the
+// sums of the first have to leave before the second goes on, and that cost more than the even shares gave.)
+struct Piece {
+  int tile, kb0, kb1;
+};
+struct Walk {
+  const Params& p;
+  const int pair, pairs, num_kb;
+  int next_tile;
+  bool shared;
+  __device__ __forceinline__ Walk(const Params& params, int pair_id, int num_pairs, int num_kb_)
+      : p(params), pair(pair_id), pairs(num_pairs), num_kb(num_kb_), next_tile(pair_id),
+        shared(pair_id < (params.batch * params.m_blocks * params.n_blocks - params.whole_tiles) * params.splits) {}
+  __device__ __forceinline__ bool next(Piece& w) {
+    if (next_tile < p.whole_tiles) {
+      w = Piece{next_tile, 0, num_kb};
+      next_tile += pairs;
+      return true;
+    }
+    if (!shared) return false;
+    shared = false;
+    const int t = pair / p.splits, i = pair - t * p.splits, per = (num_kb + p.splits - 1) / p.splits;
+    w = Piece{p.whole_tiles + t, i * per, min(num_kb, (i + 1) * per)};
+    return true;
+  }
+};
+
 __device__ __forceinline__ void tcgen05_mma_tf32_ss_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                          uint32_t accumulate) {
   asm volatile(
@@ -662,9 +694,7 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
   const uint32_t rank = ptx::cluster_ctarank();  // 0 = leader
   const int pair_id = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
-  const int num_tiles = p.batch * p.m_blocks * p.n_blocks;
   const int num_kb = (p.k + kBK - 1) / kBK;
-  const int num_chunks = (num_kb + p.chunk_kb - 1) / p.chunk_kb;
   volatile uint32_t* abort_flag = &bars->abort_flag;
 
   if (threadIdx.x == 0) {
@@ -701,12 +731,13 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = pair_id; tile < num_tiles && ok; tile += num_pairs) {
+      Walk walk(p, pair_id, num_pairs, num_kb);
+      for (Piece w; ok && walk.next(w);) {
         int b, mb, nb;
-        pair::tile_coords(p, tile, b, mb, nb);
+        pair::tile_coords(p, w.tile, b, mb, nb);
         const int row0 = mb * kPairM + static_cast<int>(rank) * kCtaM;
         const int col0 = nb * BN + static_cast<int>(rank) * kCtaN;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        for (int kb = w.kb0; kb < w.kb1; ++kb) {
           if (!ptx::mbar_wait(&bars->empty[stage], phase ^ 1u, abort_flag, p.status, 45)) {
             ok = false;
             break;
@@ -735,8 +766,9 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
       uint32_t phase = 0;
       bool ok = true;
       uint32_t chunk_count = 0;
-      for (int tile = pair_id; tile < num_tiles && ok; tile += num_pairs) {
-        for (int ch = 0; ch < num_chunks && ok; ++ch, ++chunk_count) {
+      Walk walk(p, pair_id, num_pairs, num_kb);
+      for (Piece w; ok && walk.next(w);) {
+        for (int kb_begin = w.kb0; kb_begin < w.kb1 && ok; kb_begin += p.chunk_kb, ++chunk_count) {
           const uint32_t acc = chunk_count & 1u;
           const uint32_t acc_phase = (chunk_count >> 1) & 1u;
           if (!ptx::mbar_wait_relaxed(&bars->acc_empty[acc], acc_phase ^ 1u, abort_flag, p.status, 46)) {
@@ -745,8 +777,8 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
           }
           ptx::tcgen05_fence_after_thread_sync();
           const uint32_t d_tmem = tmem_base + acc * BN;
-          const int kb_end = min(num_kb, (ch + 1) * p.chunk_kb);
-          for (int kb = ch * p.chunk_kb; kb < kb_end; ++kb) {
+          const int kb_end = min(w.kb1, kb_begin + p.chunk_kb);
+          for (int kb = kb_begin; kb < kb_end; ++kb) {
             if (!ptx::mbar_wait_relaxed(&bars->full[stage], phase, abort_flag, p.status, 47)) {
               ok = false;
               break;
@@ -754,7 +786,7 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
             ptx::tcgen05_fence_after_thread_sync();
             const uint32_t a_hi = ptx::smem_u32(smem + stage * kStageBytes);
             const uint32_t a_lo = a_hi + kAPlane, b_hi = a_lo + kAPlane, b_lo = b_hi + kBPlane;
-            const bool first_kb = kb == ch * p.chunk_kb;
+            const bool first_kb = kb == kb_begin;
 #pragma unroll
             for (int kk = 0; kk < kBK / kUmmaK; ++kk) {
               const uint32_t off = kk * kstep;
@@ -784,15 +816,14 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
     float* staging = reinterpret_cast<float*>(smem + kStages * kStageBytes) + (warp - 2) * kStagingFloats;
     uint32_t chunk_count = 0;
     bool alive = true;
-    for (int tile = pair_id; tile < num_tiles && alive; tile += num_pairs) {
-      int b, mb, nb;
-      pair::tile_coords(p, tile, b, mb, nb);
+    Walk walk(p, pair_id, num_pairs, num_kb);
+    for (Piece w; walk.next(w);) {
       float sum[kChunks][32];
 #pragma unroll
       for (int cc = 0; cc < kChunks; ++cc)
 #pragma unroll
         for (int i = 0; i < 32; ++i) sum[cc][i] = 0.f;
-      for (int ch = 0; ch < num_chunks; ++ch, ++chunk_count) {
+      for (int kb = w.kb0; kb < w.kb1 && alive; kb += p.chunk_kb, ++chunk_count) {
         const uint32_t acc = chunk_count & 1u;
         const uint32_t acc_phase = (chunk_count >> 1) & 1u;
         const bool ready = ptx::mbar_wait(&bars->acc_full[acc], acc_phase, abort_flag, p.status, 48);
@@ -806,8 +837,7 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
 #pragma unroll
           for (int h = 0; h < 32; h += kDrain<kRedo>) {
             uint32_t v[kDrain<kRedo>];
-            if constexpr (kRedo) ptx::tmem_ld_32x32b_x16(lane_addr + acc * BN + cc * 32 + h, v);
-            else ptx::tmem_ld_32x32b_x32(lane_addr + acc * BN + cc * 32, v);
+            ptx::tmem_ld_32x32b_x16(lane_addr + acc * BN + cc * 32 + h, v);
             ptx::tmem_ld_wait();
 #pragma unroll
             for (int i = 0; i < kDrain<kRedo>; ++i) sum[cc][h + i] += __uint_as_float(v[i]);
@@ -817,7 +847,46 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa_shared(ptx::smem_u32(&bars->acc_empty[acc]), 0));
       }
-      if (!alive) break;
+      if (w.kb1 - w.kb0 != num_kb) {
+        // every warp comes here, also one whose wait gave up: the barrier is for all eight
+        if (epilogue_any(!alive)) {
+          alive = false;
+          continue;
+        }
+        const int tid = static_cast<int>(threadIdx.x) - 64;
+        constexpr int kVecs = BN / 8;  // float4 per thread
+        float4* mine = p.part + (static_cast<int64_t>(pair_id) * 2 + rank) * (kVecs * kEpilogueThreads) + tid;
+#pragma unroll
+        for (int cc = 0; cc < kChunks; ++cc)
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+            __stcg(mine + (cc * 8 + i) * kEpilogueThreads, make_float4(sum[cc][4 * i], sum[cc][4 * i + 1], sum[cc][4 * i + 2], sum[cc][4 * i + 3]));
+        __threadfence();
+        epilogue_sync();
+        const int first = (w.tile - p.whole_tiles) * p.splits;
+        if (tid == 0) bars->redo.got = atomicAdd(&p.arrivals[2 * (w.tile - p.whole_tiles) + rank], 1u);
+        epilogue_sync();
+        if (bars->redo.got + 1u != static_cast<uint32_t>(p.splits)) continue;
+        // the last one here adds all pieces, in order
+        __threadfence();
+#pragma unroll
+        for (int cc = 0; cc < kChunks; ++cc)
+#pragma unroll
+          for (int i = 0; i < 32; ++i) sum[cc][i] = 0.f;
+        for (int q = first; q < first + p.splits; ++q) {
+          const float4* from = p.part + (static_cast<int64_t>(q) * 2 + rank) * (kVecs * kEpilogueThreads) + tid;
+#pragma unroll
+          for (int cc = 0; cc < kChunks; ++cc)
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float4 x = __ldcg(from + (cc * 8 + i) * kEpilogueThreads);
+              sum[cc][4 * i] += x.x, sum[cc][4 * i + 1] += x.y, sum[cc][4 * i + 2] += x.z, sum[cc][4 * i + 3] += x.w;
+            }
+        }
+      }
+      if (!alive) continue;
+      int b, mb, nb;
+      pair::tile_coords(p, w.tile, b, mb, nb);
       const int row0 = mb * kPairM + static_cast<int>(rank) * kCtaM + quad * 32;
 #pragma unroll
       for (int cc = 0; cc < kChunks; ++cc)

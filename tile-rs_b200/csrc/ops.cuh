@@ -682,15 +682,6 @@ inline int32_t gemm_tf32x3_launch(std::string* err, const tsm100_gemm_desc* d, c
   return cuda_ok(err, e, "gemm_tf32x3_kernel launch");
 }
 
-// Columns of a pair's tile: the width whose waves of tiles over the SM pairs take the least time.  A 128-wide tile
-// costs two thirds of a 256-wide one, not half (its operand traffic per product is 4/3 and a chunk's drain overlaps
-// half the products): 4096^3 655 us in 4 wide waves, 757 in 7 narrow ones; 1536^3 79 us in one wide wave, 56 in one narrow.
-inline int gemm_tf32_pair_width(uint64_t m, uint64_t n, uint64_t batch, int sms) {
-  const uint64_t pairs = static_cast<uint64_t>(std::max(1, sms / 2)), rows = (m + 255) / 256 * batch;
-  const uint64_t wide = (rows * ((n + 255) / 256) + pairs - 1) / pairs, narrow = (rows * ((n + 127) / 128) + pairs - 1) / pairs;
-  return 67 * narrow < 100 * wide ? 128 : 256;
-}
-
 // The hi / lo planes of two operands (gemm_tf32_tc.cuh), `batch` of them; `transpose_b`: b comes as [cols][rows].  The same
 // launch clears zero[0 .. n_zero).
 inline int32_t split_operands_launch(std::string* err, gemm_tf32_tc::SplitOperand a, gemm_tf32_tc::SplitOperand b, bool transpose_b,
@@ -723,27 +714,31 @@ inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, 
   if (st != TSM100_OK) return st;
   cudaError_t e = cudaSuccess;
   const uint64_t kp = (K + 3) / 4 * 4;  // row pitch of the planes: every row starts on a 16-byte boundary
+  // Problems with more than one 128-row and 128-column block run on CTA pairs (256 x 256 or 256 x 128 tiles); the rest
+  // on single CTAs (128 x 256 tiles).
+  const bool pairs = M > 128 && N > 128;
+  const route::PairTiles plan = pairs ? route::gemm_f32_pair_tiles(d->m, d->n, d->k, d->batch, sms) : route::PairTiles{g::kBN, 0, 1};
+  const int bn = plan.bn;
   const size_t a_plane = static_cast<size_t>(B) * M * kp, b_plane = static_cast<size_t>(B) * N * kp;  // elements
   // rows that start anywhere: a flag per 128 x 128 block of C, behind the planes
   const int64_t flags = rows_aligned ? 0 : static_cast<int64_t>(B * ((M + 127) / 128) * ((N + 127) / 128));
   float* ws = nullptr;
+  // tiles that several pairs share: partial sums of each of them, in front, and two counters per tile behind the flags
+  const int64_t shared_tiles = plan.splits > 1 ? static_cast<int64_t>((M + 255) / 256) * ((N + bn - 1) / bn) * B - plan.whole_tiles : 0;
+  const size_t part = static_cast<size_t>(shared_tiles) * plan.splits * 256 * bn;  // elements
   {
-    const int32_t got = take_scratch(err, reinterpret_cast<void**>(&ws), (2 * (a_plane + b_plane) + flags) * sizeof(float), s);
+    const int32_t got = take_scratch(err, reinterpret_cast<void**>(&ws), (part + 2 * (a_plane + b_plane) + flags + 2 * shared_tiles) * sizeof(float), s);
     if (got != TSM100_OK) return got;
   }
-  float *a_hi = ws, *a_lo = ws + a_plane, *b_hi = ws + 2 * a_plane, *b_lo = b_hi + b_plane;
+  float *a_hi = ws + part, *a_lo = a_hi + a_plane, *b_hi = a_lo + a_plane, *b_lo = b_hi + b_plane;
   uint32_t* flag_words = reinterpret_cast<uint32_t*>(b_lo + b_plane);
   const float* af = static_cast<const float*>(a);
   const float* bf = static_cast<const float*>(b);
   st = split_operands_launch(err, {af, a_hi, a_lo, ld.lda, static_cast<int64_t>(M) * ld.lda, static_cast<int64_t>(M), static_cast<int32_t>(K), static_cast<int32_t>(kp), 0},
                              {bf, b_hi, b_lo, ld.ldb, static_cast<int64_t>(d->b_transposed ? N : K) * ld.ldb, static_cast<int64_t>(N), static_cast<int32_t>(K), static_cast<int32_t>(kp), 0},
-                             !d->b_transposed, d->batch, sms, s, flag_words, flags);
+                             !d->b_transposed, d->batch, sms, s, flag_words, flags + 2 * shared_tiles);
   CUtensorMap ta_hi, ta_lo, tb_hi, tb_lo;
   const CUtensorMapDataType f32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  // Problems with more than one 128-row and 128-column block run on CTA pairs (256 x 256 or 256 x 128 tiles); the rest
-  // on single CTAs (128 x 256 tiles).
-  const bool pairs = M > 128 && N > 128;
-  const int bn = pairs ? gemm_tf32_pair_width(M, N, B, sms) : g::kBN;
   const uint32_t box_b = pairs ? bn / 2 : g::kBN;
   if (st == TSM100_OK) st = make_tmap_3d(err, &ta_hi, a_hi, K, M, B, kp, M * kp, g::kBK, g::kBM, f32, 4);
   if (st == TSM100_OK) st = make_tmap_3d(err, &ta_lo, a_lo, K, M, B, kp, M * kp, g::kBK, g::kBM, f32, 4);
@@ -774,10 +769,15 @@ inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, 
     p.b_batch_stride = static_cast<int64_t>(d->b_transposed ? N : K) * ld.ldb;
     const int64_t tiles = static_cast<int64_t>(p.m_blocks) * p.n_blocks * p.batch;
     auto launch_pairs = [&](auto kern, int smem) -> cudaError_t {
+    p.whole_tiles = static_cast<int32_t>(tiles - shared_tiles);
+    p.splits = plan.splits;
+    p.part = reinterpret_cast<float4*>(ws);
+    p.arrivals = flag_words + flags;
       cudaError_t pe = set_dyn_smem_once(kern, smem);
       if (pe != cudaSuccess) return pe;
       const int max_clusters = resident_clusters(kern, g::kThreads, static_cast<size_t>(smem), 2, static_cast<unsigned>(sms & ~1), sms / 2);
-      const int64_t npairs = std::min<int64_t>(tiles, std::min<int64_t>(max_clusters, sms / 2));
+      // as many pairs as the GPU holds at once, but one for every share (nobody waits for another pair)
+      const int64_t npairs = std::max<int64_t>(shared_tiles * plan.splits, std::min<int64_t>(tiles, std::min<int64_t>(max_clusters, sms / 2)));
       return launch_chained(kern, static_cast<unsigned>(2 * npairs), g::kThreads, static_cast<size_t>(smem), s, 2, ta_hi, ta_lo, tb_hi, tb_lo,
                             static_cast<float*>(c), p);
     };

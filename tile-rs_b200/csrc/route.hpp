@@ -139,6 +139,37 @@ inline GemmF32 gemm_f32(int64_t m, int64_t n, int64_t k, int64_t batch, bool ali
   return r;
 }
 
+// The tiles of the planes' kernel over SM pairs: columns of a tile (256 or 128, of 256 rows), how many tiles are worked on whole, and how
+// many pairs share each of the rest.
+struct PairTiles {
+  int bn;
+  int64_t whole_tiles;
+  int splits;
+};
+inline PairTiles gemm_f32_pair_tiles(int64_t m, int64_t n, int64_t k, int64_t batch, int sms) {
+  const int64_t pairs = sms / 2 > 0 ? sms / 2 : 1, kb = div_up(k, 32);
+  PairTiles best{256, 0, 1};
+  int64_t best_cost = INT64_MAX;
+  for (int bn = 256; bn >= 128; bn -= 128) {
+    const int64_t tiles = div_up(m, 256) * div_up(n, bn) * batch, rest = tiles % pairs;
+    // A 128-wide tile costs two thirds of a 256-wide one, not half (its operand traffic per product is 4/3 and a chunk's drain overlaps
+    // half the products): 4096^3 655 us in 4 wide waves, 757 in 7 narrow ones; 1536^3 79 us in one wide wave, 56 in one narrow.
+    const int64_t per_kb = bn == 256 ? 100 : 67;
+    int64_t cost = div_up(tiles, pairs) * kb * per_kb;
+    int splits = 1;
+    for (int s = 2; rest > 0 && s <= 4 && rest * s <= pairs && kb / s >= 8; ++s) {
+      // partial sums on their way through the L2 and back cost what 14 k-blocks do, and two for each of them
+      const int64_t shared = (tiles / pairs * kb + div_up(kb, s) + 14 + 2 * s) * per_kb;
+      if (shared < cost) cost = shared, splits = s;
+    }
+    if (cost < best_cost) best_cost = cost, best = PairTiles{bn, splits > 1 ? tiles - rest : tiles, splits};
+  }
+  // the last share has to have k-blocks of its own
+  while (best.splits > 1 && (best.splits - 1) * div_up(kb, best.splits) >= kb) --best.splits;
+  if (best.splits == 1) best.whole_tiles = div_up(m, 256) * div_up(n, best.bn) * batch;
+  return best;
+}
+
 // Row softmax whose rows start anywhere or are too wide for one CTA's registers (softmax.cuh); `span`: the most 16-byte vectors a row
 // can touch.
 // 129 .. 256 vectors: a warp per row while there are rows for all warps, else a CTA.  1111 bf16, 200 rows 3.7 a warp, 2.9 a CTA, 600
