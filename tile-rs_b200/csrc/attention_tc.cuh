@@ -12,8 +12,7 @@
 // (mlir_to_gpu.rs:1976-1979) and the GQA form recomputes every q.k dot product
 // three times per output element (mlir_to_gpu.rs:1624-1711).
 //
-// Layout: Q,O [batch*heads_q][seq][d], K,V [batch*heads_kv][seq][d], 16-bit; d = 128, or any multiple of 8 up to 64
-// (the D = 64 form of the kernel; the tensor maps end at d and fill the rest of a 64-wide row with zeros).
+// Layout: Q,O [batch*heads_q][seq][d], K,V [batch*heads_kv][seq][d], 16-bit, d = 128; narrower heads: attention_narrow.cuh.
 //
 // One CTA owns 256 query rows of one (batch, head): two 128-row tiles A and B.
 //   warp 8      TMA producer: Q once, then K_0,K_1,V_0,K_2,V_1,... (128 x 128 tiles,
@@ -47,7 +46,7 @@
 namespace tsm100 {
 namespace attn {
 
-constexpr int kD = 128;          // head_dim of the wide form
+constexpr int kD = 128;          // head_dim
 constexpr int kBQ = 128;         // query rows per tile (two tiles per CTA)
 constexpr int kBKV = 128;        // key/value rows per step
 constexpr int kThreads = 384;         // warps 0..3 softmax A, 4..7 softmax B, 8 TMA, 9 QK MMAs, 10 PV MMAs, 11 idle
@@ -57,33 +56,16 @@ constexpr int kTmemCols = 512;
 constexpr float kRescaleThreshold = 8.0f;  // log2 units
 constexpr int kPolyPairs = 2;  // of every 8 pairs of exponentials, how many avoid MUFU
 
-// The two forms of the kernel.  D = 128: the probabilities are handed to P V rounded to the storage type.  D = 64: the
-// narrower Q, K and V tiles leave shared memory for a second P tile, and the probabilities are handed over as hi + lo,
-// two 16-bit numbers whose sum is the f32 value to 2^-17 of it (bf16), or to 2^-22 of it or 2^-32 of the row's largest (f16).
-// P V is two products of 128 x 64 x 16, so a step costs the tensor core what one 128-wide product does and the softmax chain
-// stays the bound.  Its exponentials all go through MUFU (the cubic of the wide form is good to 7e-5 only).
-template <int D>
-struct Shape {
-  static constexpr bool kSplitP = D == 64;
-  // f16 numbers end at 2^-24: the probabilities of the split form (2^8 at most, see kRescaleThreshold) and their sum are taken
-  // 2^7 times as large, so that a long tail of them down to 2^-32 of the largest counts in P V as it does in the sum
-  template <bool kIsBf16>
-  static constexpr float kPShift = kSplitP && !kIsBf16 ? 7.0f : 0.0f;
-  static constexpr int kHalves = D / 64;                   // 64-wide swizzled column groups of a Q, K or V tile
-  static constexpr int kHalfBytes = 128 * 64 * 2;          // one 128-row x 64-column group: 16 KiB
-  static constexpr int kTileBytes = kHalves * kHalfBytes;  // a 128 x D tile of Q, K or V
-  static constexpr int kPTile = 2 * kHalfBytes;            // 128 rows x 128 keys
-  static constexpr int kPBytes = (kSplitP ? 2 : 1) * kPTile;
-  static constexpr int kRing = D == 64 ? 4 : 3;
-  static constexpr int kQOff = 0, kPOff = 2 * kTileBytes, kRingOff = kPOff + 2 * kPBytes;  // Q_A, Q_B, P_A, P_B, ring
-  static constexpr int kBarsOff = kRingOff + kRing * kTileBytes;
-};
-constexpr int kMaxRing = 4;
+constexpr int kHalfBytes = 128 * 64 * 2;   // a 128-row x 64-column swizzled group: 16 KiB
+constexpr int kTileBytes = 2 * kHalfBytes;  // a 128 x 128 tile of Q, K, V or P
+constexpr int kRing = 3;
+constexpr int kQOff = 0, kPOff = 2 * kTileBytes, kRingOff = kPOff + 2 * kTileBytes;  // Q_A, Q_B, P_A, P_B, ring
+constexpr int kBarsOff = kRingOff + kRing * kTileBytes;
 
 struct alignas(8) Barriers {
   uint64_t q_full;
-  uint64_t kv_full[kMaxRing];
-  uint64_t kv_empty[kMaxRing];
+  uint64_t kv_full[kRing];
+  uint64_t kv_empty[kRing];
   uint64_t s_full[2];
   uint64_t s_free[2];
   uint64_t p_ready[2];
@@ -94,11 +76,8 @@ struct alignas(8) Barriers {
 };
 
 
-template <int D>
-constexpr int smem_bytes() {
-  return Shape<D>::kBarsOff + static_cast<int>(sizeof(Barriers)) + 1024;
-}
-static_assert(smem_bytes<128>() <= 227 * 1024 && smem_bytes<64>() <= 227 * 1024, "shared memory budget of one CTA");
+constexpr int kSmemBytes = kBarsOff + static_cast<int>(sizeof(Barriers)) + 1024;
+static_assert(kSmemBytes <= 227 * 1024, "shared memory budget of one CTA");
 
 struct Params {
   int32_t seq;
@@ -112,7 +91,7 @@ struct Params {
   // filled positions; O is token-major, row and head strides in elements
   int32_t seq_kv, q_offset;
   int64_t o_row_stride, o_head_stride;
-  int32_t head_dim;        // D = 64 form: columns of Q, K, V and O that exist (a multiple of 8)
+  int32_t head_dim;        // attention_narrow.cuh: columns of Q, K, V and O that exist (a multiple of 8)
   int32_t blocks;          // query blocks of the launch: q_blocks * heads_q * batch
   // kSplit: CTAs per query block, and their records.  part: [block][split][D / 4][256 rows] of four columns each, so that
   // the lanes of a warp, which hold rows, write and read contiguous memory; part_ml: [block][split][256 rows] (max, sum)
@@ -166,19 +145,16 @@ __device__ __forceinline__ void block_coords(const Params& p, int block, int& bh
 // kCache = false: plain attention, Q, O [batch*heads_q][seq][128], K, V [batch*heads_kv][seq][128] (the tensor
 // maps say so).  kCache = true: causal prefill against a KV cache - the tensor maps describe token-major Q and the
 // filled part of the caches, query rows are offset by q_offset, O is written with the strides of Params.
-template <bool kIsBf16, bool kCache = false, int D = 128, bool kSplit = false>
+template <bool kIsBf16, bool kCache = false, bool kSplit = false>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                      const __grid_constant__ CUtensorMap tmap_v, uint16_t* __restrict__ o, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  using Sh = Shape<D>;
-  constexpr int kRing = Sh::kRing, kTileBytes = Sh::kTileBytes, kHalfBytes = Sh::kHalfBytes;
-  constexpr bool kSplitP = Sh::kSplitP;
-  uint8_t* smem_q = smem + Sh::kQOff;             // 2 tiles
-  uint8_t* smem_p = smem + Sh::kPOff;             // the probabilities of tile A and of tile B (split: hi, then lo, of each)
-  uint8_t* smem_kv = smem + Sh::kRingOff;         // ring
-  Barriers* bars = reinterpret_cast<Barriers*>(smem + Sh::kBarsOff);
+  uint8_t* smem_q = smem + kQOff;             // 2 tiles
+  uint8_t* smem_p = smem + kPOff;             // the probabilities of tile A and of tile B
+  uint8_t* smem_kv = smem + kRingOff;         // ring
+  Barriers* bars = reinterpret_cast<Barriers*>(smem + kBarsOff);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -244,7 +220,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 #pragma unroll
       for (int g = 0; g < 2; ++g)
 #pragma unroll
-        for (int c = 0; c < Sh::kHalves; ++c)
+        for (int c = 0; c < kD / 64; ++c)
           ptx::tma_load_3d(smem_q + g * kTileBytes + c * kHalfBytes, &tmap_q, &bars->q_full, c * 64,
                            q0 + g * kBQ, bh);
       // ring order = the order the tensor core first needs the tiles in: K_0, K_1, V_0, K_2, V_1, ..., K_{n-1}, V_{n-2}, V_{n-1}
@@ -260,7 +236,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         const CUtensorMap* tm = is_v ? &tmap_v : &tmap_k;
         const int row0 = (j0 + step) * kBKV;
 #pragma unroll
-        for (int c = 0; c < Sh::kHalves; ++c)
+        for (int c = 0; c < kD / 64; ++c)
           ptx::tma_load_3d(smem_kv + slot * kTileBytes + c * kHalfBytes, tm, &bars->kv_full[slot], c * 64,
                            row0, kvh);
       }
@@ -274,7 +250,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     ptx::setmaxnreg_dec<kRegsOther>();
     {  // the whole warp runs the loop (uniform control flow, uniform operands); one elected lane issues
       constexpr uint32_t idesc_qk = ptx::make_idesc_f16(kBQ, kBKV, false, false, kIsBf16);
-      constexpr uint32_t idesc_pv = ptx::make_idesc_f16(kBQ, D, false, true, kIsBf16);
+      constexpr uint32_t idesc_pv = ptx::make_idesc_f16(kBQ, kD, false, true, kIsBf16);
       constexpr uint64_t kmajor = ptx::make_smem_desc_base(16, 1024);
       constexpr uint64_t v_mnmajor = ptx::make_smem_desc_base(kHalfBytes, 1024);
 
@@ -304,7 +280,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           const uint32_t d = tmem_s + g * 128;
           if (ptx::elect_one_sync()) {
 #pragma unroll
-            for (int kk = 0; kk < D / 16; ++kk) {
+            for (int kk = 0; kk < kD / 16; ++kk) {
               constexpr int kHalf16 = kHalfBytes >> 4;
               const uint32_t off = (kk >> 2) * kHalf16 + (kk & 3) * 2;  // in 16-byte units
               ptx::tcgen05_mma_f16_ss(d, desc64(k_hi, a_lo + off), desc64(k_hi, b_lo + off), idesc_qk, kk != 0 ? 1u : 0u);
@@ -339,10 +315,10 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         }
       } else {
         // ---- O_g (+)= P_g V : P K-major from its shared-memory tile (keys in two 64-wide halves), V MN-major
-        const uint32_t p_lo = k_lo_base | (ptx::smem_u32(smem_p) >> 4);       // + g * (kPBytes >> 4)
+        const uint32_t p_lo = k_lo_base | (ptx::smem_u32(smem_p) >> 4);       // + g * (kTileBytes >> 4)
         const uint32_t ring_v_lo = v_lo_base | (ptx::smem_u32(smem_kv) >> 4);
         auto issue_pv = [&](int g, int idx, bool accumulate) {
-          const uint32_t a_lo = p_lo + g * (Sh::kPBytes >> 4);
+          const uint32_t a_lo = p_lo + g * (kTileBytes >> 4);
           const uint32_t b_lo = ring_v_lo + (idx % kRing) * (kTileBytes >> 4);
           const uint32_t d = tmem_o + g * 128;
           if (ptx::elect_one_sync()) {
@@ -352,9 +328,6 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
               const uint32_t a_off = (kk >> 2) * kHalf16 + (kk & 3) * 2;
               ptx::tcgen05_mma_f16_ss(d, desc64(k_hi, a_lo + a_off), desc64(v_hi, b_lo + kk * (2048 >> 4)), idesc_pv,
                                       (accumulate || kk != 0) ? 1u : 0u);
-              if (kSplitP)
-                ptx::tcgen05_mma_f16_ss(d, desc64(k_hi, a_lo + (Sh::kPTile >> 4) + a_off), desc64(v_hi, b_lo + kk * (2048 >> 4)),
-                                        idesc_pv, 1u);
             }
             ptx::tcgen05_commit(&bars->pv_done[g]);
           }
@@ -396,7 +369,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     const uint32_t ts = tmem_s + g * 128 + lane_base;
     const uint32_t to = tmem_o + g * 128 + lane_base;
     const float sl2 = p.scale_log2;
-    const uint32_t p_row = ptx::smem_u32(smem_p) + g * Sh::kPBytes + r * 128;  // this row in the first 64-key half of P_g
+    const uint32_t p_row = ptx::smem_u32(smem_p) + g * kTileBytes + r * 128;  // this row in the first 64-key half of P_g
 
     float m_used = -INFINITY;  // running max in raw score units
     float l = 0.f;
@@ -456,7 +429,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           if (need) m_used = m_new;
           l *= alpha;
 #pragma unroll 1
-          for (int c = 0; c < D / 32; ++c) {
+          for (int c = 0; c < kD / 32; ++c) {
             uint32_t ov[32];
             ptx::tmem_ld_32x32b_x32(to + c * 32, ov);
             ptx::tmem_ld_wait();
@@ -477,46 +450,10 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       // f32 probabilities before they are rounded (packed adds, two per instruction).
       // A row whose scores so far are all -inf (a step, or in kSplit a whole range, may lie behind the row's last visible key):
       // taking them against 0 gives them no weight, against their maximum of -inf NaN.
-      const float ms = m_used == -INFINITY ? 0.f : m_used * sl2 - Sh::template kPShift<kIsBf16>;
+      const float ms = m_used == -INFINITY ? 0.f : m_used * sl2;
       const ptx::f32x2_t sl2x2 = ptx::pack_f32x2(sl2, sl2);
       const ptx::f32x2_t nmsx2 = ptx::pack_f32x2(-ms, -ms);
       ptx::f32x2_t lsum[2] = {0ull, 0ull};  // (+0.0f, +0.0f)
-      if constexpr (kSplitP) {
-        // 32 keys at a time: hi = p rounded to the storage type, lo = p - hi rounded again
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t hi[16], lo[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const ptx::f32x2_t t2 = ptx::fma_f32x2(
-                ptx::pack_f32x2(__uint_as_float(v[c][2 * i]), __uint_as_float(v[c][2 * i + 1])), sl2x2, nmsx2);
-            float t0, t1;
-            ptx::unpack_f32x2(t2, t0, t1);
-            const float p0 = ptx::ex2_approx(t0), p1 = ptx::ex2_approx(t1);  // 2^(-inf) = 0
-            const ptx::f32x2_t p2 = ptx::pack_f32x2(p0, p1);
-            hi[i] = pack16x2<kIsBf16>(p0, p1);
-            float d0, d1;
-            ptx::unpack_f32x2(ptx::fma_f32x2(ptx::pack_f32x2(unpack16_lo<kIsBf16>(hi[i]), unpack16_hi<kIsBf16>(hi[i])),
-                                             ptx::pack_f32x2(-1.0f, -1.0f), p2), d0, d1);
-            lo[i] = pack16x2<kIsBf16>(d0, d1);
-            lsum[i & 1] = ptx::add_f32x2(lsum[i & 1], p2);
-          }
-          if (c == 0 && j > 0) {  // P_g is free once the previous step's P V has read it
-            ready = ptx::mbar_wait(&bars->pv_done[g], (j - 1) & 1u, abort_flag, p.status, 24 + g);
-            if (!__all_sync(0xffffffffu, ready)) {
-              alive = false;
-              break;
-            }
-          }
-          const uint32_t prow = p_row + (c >> 1) * kHalfBytes;
-#pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
-            const uint32_t at = prow + ((((c & 1) * 4 + q4) ^ (r & 7)) << 4);
-            ptx::st_shared_v4(at, hi[4 * q4], hi[4 * q4 + 1], hi[4 * q4 + 2], hi[4 * q4 + 3]);
-            ptx::st_shared_v4(at + Sh::kPTile, lo[4 * q4], lo[4 * q4 + 1], lo[4 * q4 + 2], lo[4 * q4 + 3]);
-          }
-        }
-      } else {
 #pragma unroll
       for (int h2 = 0; h2 < 2; ++h2) {
         uint32_t pk[32];
@@ -550,7 +487,6 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         for (int c = 0; c < 8; ++c)
           ptx::st_shared_v4(prow + ((c ^ (r & 7)) << 4), pk[4 * c], pk[4 * c + 1], pk[4 * c + 2], pk[4 * c + 3]);
       }
-      }
       if (!alive) break;
       float l4[4];
       ptx::unpack_f32x2(lsum[0], l4[0], l4[1]);
@@ -566,9 +502,9 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       ptx::tcgen05_fence_after_thread_sync();
       const int64_t rec = static_cast<int64_t>(block) * splits + rank;
       const int row = g * kBQ + r;
-      float4* part = p.part + rec * (D / 4) * (2 * kBQ) + row;
+      float4* part = p.part + rec * (kD / 4) * (2 * kBQ) + row;
 #pragma unroll 1
-      for (int c = 0; c < D / 32; ++c) {
+      for (int c = 0; c < kD / 32; ++c) {
         uint32_t ov[32];
         ptx::tmem_ld_32x32b_x32(to + c * 32, ov);
         ptx::tmem_ld_wait();
@@ -585,11 +521,10 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         ptx::tcgen05_fence_after_thread_sync();
         // all scores -inf (or NaN): softmax is NaN there, l a stand-in (the wide form's cubic ends at 2^-125)
         const float inv = m_used == -INFINITY ? NAN : 1.0f / l;
-        const int cols = D == 64 ? p.head_dim : D;
         uint16_t* orow = kCache ? o + bh * p.o_head_stride + qrow * p.o_row_stride
-                                : o + (static_cast<int64_t>(bh) * p.seq + qrow) * cols;
+                                : o + (static_cast<int64_t>(bh) * p.seq + qrow) * kD;
 #pragma unroll 1
-        for (int c = 0; c < D / 32; ++c) {
+        for (int c = 0; c < kD / 32; ++c) {
           uint32_t ov[32];
           ptx::tmem_ld_32x32b_x32(to + c * 32, ov);
           ptx::tmem_ld_wait();
@@ -601,7 +536,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
               w.y = pack16x2<kIsBf16>(__uint_as_float(ov[8 * t + 2]) * inv, __uint_as_float(ov[8 * t + 3]) * inv);
               w.z = pack16x2<kIsBf16>(__uint_as_float(ov[8 * t + 4]) * inv, __uint_as_float(ov[8 * t + 5]) * inv);
               w.w = pack16x2<kIsBf16>(__uint_as_float(ov[8 * t + 6]) * inv, __uint_as_float(ov[8 * t + 7]) * inv);
-              if (D != 64 || c * 32 + t * 8 < cols) reinterpret_cast<uint4*>(orow + c * 32)[t] = w;
+              reinterpret_cast<uint4*>(orow + c * 32)[t] = w;
             }
           }
         }

@@ -1000,8 +1000,8 @@ Kernel lower(const Func& f) {
              << "], args[" << store_arg << "], status, stream);\n";
         if (out_dt != qt->dtype) reject("kernel " + f.name + ": attention input and output storage types differ");
         if (qt->dtype != Dt::F32 && (dim == 128 || dim == 64 || dim == 32))
-          inst << "template __global__ void tsm100::attn::attention_fwd_kernel<" << (qt->dtype == Dt::BF16 ? "true" : "false")
-               << (dim == 128 ? "" : ", false, 64") << ">(const __grid_constant__ CUtensorMap, const __grid_constant__ CUtensorMap, const __grid_constant__ CUtensorMap, uint16_t*, const tsm100::attn::Params);\n";
+          inst << "template __global__ void tsm100::" << (dim == 128 ? "attn::attention_fwd_kernel<" : "attn_narrow::attention_narrow_kernel<") << (qt->dtype == Dt::BF16 ? "true" : "false")
+               << (dim == 128 ? "" : ", false, false") << ">(const __grid_constant__ CUtensorMap, const __grid_constant__ CUtensorMap, const __grid_constant__ CUtensorMap, uint16_t*, const tsm100::attn::Params);\n";
         else
           inst << "template __global__ void tsm100::attn_simt::attention_simt_kernel<" << cxx_type(qt->dtype) << ">(const "
                << cxx_type(qt->dtype) << "*, const " << cxx_type(qt->dtype) << "*, const " << cxx_type(qt->dtype) << "*, "
@@ -1058,8 +1058,8 @@ Kernel lower(const Func& f) {
          << "  st = tsm100::ops::attention(&msg, &d, args[" << q.arg << "], args[" << kk.arg << "], args[" << v.arg << "], args["
          << store_arg << "], status, stream);\n";
     if (q.dtype != Dt::F32 && (root.dim == 128 || root.dim == 64 || root.dim == 32))
-      inst << "template __global__ void tsm100::attn::attention_fwd_kernel<" << (q.dtype == Dt::BF16 ? "true" : "false")
-           << (root.dim == 128 ? "" : ", false, 64") << ">(const __grid_constant__ CUtensorMap, const __grid_constant__ CUtensorMap, const __grid_constant__ CUtensorMap, uint16_t*, const tsm100::attn::Params);\n";
+      inst << "template __global__ void tsm100::" << (root.dim == 128 ? "attn::attention_fwd_kernel<" : "attn_narrow::attention_narrow_kernel<") << (q.dtype == Dt::BF16 ? "true" : "false")
+           << (root.dim == 128 ? "" : ", false, false") << ">(const __grid_constant__ CUtensorMap, const __grid_constant__ CUtensorMap, const __grid_constant__ CUtensorMap, uint16_t*, const tsm100::attn::Params);\n";
     else
       inst << "template __global__ void tsm100::attn_simt::attention_simt_kernel<" << cxx_type(q.dtype) << ">(const "
            << cxx_type(q.dtype) << "*, const " << cxx_type(q.dtype) << "*, const " << cxx_type(q.dtype) << "*, " << cxx_type(q.dtype)

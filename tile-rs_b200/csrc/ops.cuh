@@ -26,6 +26,7 @@
 #include "../../include/tile_sm100.h"
 #include "attention_decode.cuh"
 #include "attention_f32_tc.cuh"
+#include "attention_narrow.cuh"
 #include "attention_simt.cuh"
 #include "attention_tc.cuh"
 #include "attention_tf32x3.cuh"
@@ -713,19 +714,19 @@ inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, 
   int32_t st = sm_count(err, &sms);
   if (st != TSM100_OK) return st;
   cudaError_t e = cudaSuccess;
-  const uint64_t kp = (K + 3) / 4 * 4;  // row pitch of the planes: every row starts on a 16-byte boundary
   // Problems with more than one 128-row and 128-column block run on CTA pairs (256 x 256 or 256 x 128 tiles); the rest
   // on single CTAs (128 x 256 tiles).
   const bool pairs = M > 128 && N > 128;
   const route::PairTiles plan = pairs ? route::gemm_f32_pair_tiles(d->m, d->n, d->k, d->batch, sms) : route::PairTiles{g::kBN, 0, 1};
   const int bn = plan.bn;
+  const uint64_t kp = (K + 3) / 4 * 4;  // row pitch of the planes: every row starts on a 16-byte boundary
   const size_t a_plane = static_cast<size_t>(B) * M * kp, b_plane = static_cast<size_t>(B) * N * kp;  // elements
   // rows that start anywhere: a flag per 128 x 128 block of C, behind the planes
   const int64_t flags = rows_aligned ? 0 : static_cast<int64_t>(B * ((M + 127) / 128) * ((N + 127) / 128));
-  float* ws = nullptr;
   // tiles that several pairs share: partial sums of each of them, in front, and two counters per tile behind the flags
   const int64_t shared_tiles = plan.splits > 1 ? static_cast<int64_t>((M + 255) / 256) * ((N + bn - 1) / bn) * B - plan.whole_tiles : 0;
   const size_t part = static_cast<size_t>(shared_tiles) * plan.splits * 256 * bn;  // elements
+  float* ws = nullptr;
   {
     const int32_t got = take_scratch(err, reinterpret_cast<void**>(&ws), (part + 2 * (a_plane + b_plane) + flags + 2 * shared_tiles) * sizeof(float), s);
     if (got != TSM100_OK) return got;
@@ -768,11 +769,11 @@ inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, 
     p.a_batch_stride = static_cast<int64_t>(M) * ld.lda;
     p.b_batch_stride = static_cast<int64_t>(d->b_transposed ? N : K) * ld.ldb;
     const int64_t tiles = static_cast<int64_t>(p.m_blocks) * p.n_blocks * p.batch;
-    auto launch_pairs = [&](auto kern, int smem) -> cudaError_t {
     p.whole_tiles = static_cast<int32_t>(tiles - shared_tiles);
     p.splits = plan.splits;
     p.part = reinterpret_cast<float4*>(ws);
     p.arrivals = flag_words + flags;
+    auto launch_pairs = [&](auto kern, int smem) -> cudaError_t {
       cudaError_t pe = set_dyn_smem_once(kern, smem);
       if (pe != cudaSuccess) return pe;
       const int max_clusters = resident_clusters(kern, g::kThreads, static_cast<size_t>(smem), 2, static_cast<unsigned>(sms & ~1), sms / 2);
@@ -1276,13 +1277,27 @@ inline int32_t attention_kv_band(uint64_t kv_len, int64_t kv_heads, uint64_t hea
   return static_cast<int32_t>(std::max<int64_t>(1, std::min<int64_t>(band, std::max<int64_t>(kv_heads, 1))));
 }
 
+// The tcgen05 attention kernels: heads of 128, and of 64 and less.
+template <bool kBf16, bool kCache, int D, bool kSplit>
+struct AttentionFwd {
+  static auto kernel() {
+    if constexpr (D == 64) return attn_narrow::attention_narrow_kernel<kBf16, kCache, kSplit>;
+    else return attn::attention_fwd_kernel<kBf16, kCache, kSplit>;
+  }
+  static constexpr int smem() {
+    if constexpr (D == 64) return attn_narrow::kSmemBytes;
+    else return attn::kSmemBytes;
+  }
+};
+
 // Launches the tcgen05 attention kernel over `blocks` query blocks that see at most `keys` keys, the KV steps of a block dealt to
 // several CTAs and merged by a second kernel where route.hpp says so.
 template <bool kBf16, bool kCache, int D>
 inline int32_t attention_fwd_launch(std::string* err, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, void* o,
                                     attn::Params p, int64_t blocks, int64_t keys, cudaStream_t s) {
   namespace at = attn;
-  constexpr int smem = at::smem_bytes<D>();
+  constexpr int smem = AttentionFwd<kBf16, kCache, D, false>::smem();
+  static_assert(attn_narrow::kThreads == at::kThreads, "one launch for both");
   int sms = 0;
   int32_t st = sm_count(err, &sms);
   if (st != TSM100_OK) return st;
@@ -1300,14 +1315,14 @@ inline int32_t attention_fwd_launch(std::string* err, const CUtensorMap& tq, con
   }
   cudaError_t e = cudaSuccess;
   if (p.splits == 1) {
-    auto kern = at::attention_fwd_kernel<kBf16, kCache, D>;
+    auto kern = AttentionFwd<kBf16, kCache, D, false>::kernel();
     e = set_dyn_smem_once(kern, smem);
     if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(attention_fwd_kernel)");
     return cuda_ok(err, launch_chained(kern, static_cast<unsigned>(blocks), at::kThreads, smem, s, 0, tq, tk, tv, out, p), "attention_fwd_kernel launch");
   }
   p.part = reinterpret_cast<float4*>(ws);
   p.part_ml = reinterpret_cast<float2*>(ws + rows * D);
-  auto kern = at::attention_fwd_kernel<kBf16, kCache, D, true>;
+  auto kern = AttentionFwd<kBf16, kCache, D, true>::kernel();
   e = set_dyn_smem_once(kern, smem);
   if (e == cudaSuccess) e = launch_chained(kern, static_cast<unsigned>(blocks * p.splits), at::kThreads, smem, s, 0, tq, tk, tv, out, p);
   if (e == cudaSuccess)
