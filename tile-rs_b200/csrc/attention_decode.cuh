@@ -554,6 +554,11 @@ attention_decode_merge_kernel(T* __restrict__ o, const Params p) {
   const float* rec = p.part + (static_cast<int64_t>(unit) * p.splits * kRows + hh) * REC;
   ptx::launch_dependents();
   rec = ptx::wait_prior_grid(rec);
+  // this thread's column of the first records, on its way while the weights are worked out
+  constexpr int kFirst = 20;
+  float first[kFirst];
+#pragma unroll
+  for (int i = 0; i < kFirst; ++i) first[i] = i < p.splits ? rec[i * (kRows * REC) + threadIdx.x] : 0.f;
   for (int i = threadIdx.x; i < p.splits; i += D) {
     m[i] = rec[i * (kRows * REC) + D];
     l[i] = rec[i * (kRows * REC) + D + 1];
@@ -564,8 +569,11 @@ attention_decode_merge_kernel(T* __restrict__ o, const Params p) {
   for (int i = threadIdx.x; i < p.splits; i += D) w[i] = m[i] == -INFINITY ? 0.f : ptx::ex2_approx(m[i] - mm);
   __syncthreads();
   float ll = 0.f, oo = 0.f;
+#pragma unroll
+  for (int i = 0; i < kFirst; ++i)
+    if (i < p.splits) ll = fmaf(l[i], w[i], ll), oo = fmaf(first[i], w[i], oo);
 #pragma unroll 8
-  for (int i = 0; i < p.splits; ++i) {
+  for (int i = kFirst; i < p.splits; ++i) {
     ll = fmaf(l[i], w[i], ll);
     oo = fmaf(rec[i * (kRows * REC) + threadIdx.x], w[i], oo);
   }
