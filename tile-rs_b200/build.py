@@ -12,6 +12,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -20,6 +21,8 @@ CSRC = PKG_DIR / "csrc"
 INCLUDE = PKG_DIR.parent / "include"
 BUILD_DIR = PKG_DIR / "_build"
 LIB_PATH = PKG_DIR / "libtile_sm100.so"
+# the operators for CPython without ctypes (csrc/python.cpp); absent where there are no CPython headers
+FAST_PATH = PKG_DIR / ("_tile_sm100" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 CUDA_SOURCES = ["runtime.cu", "capi_ops.cu", "multi.cu"]
 CXX_SOURCES = ["inputs.cpp", "emit.cpp"]
@@ -63,6 +66,17 @@ def _compile(src: str) -> Path:
     return obj
 
 
+def _compile_fast() -> None:
+    include = Path(sysconfig.get_paths()["include"])
+    FAST_PATH.unlink(missing_ok=True)
+    if not (include / "Python.h").exists():
+        return
+    cmd = [shutil.which("g++") or "g++", "-std=c++17", "-O2", "-Wall", "-shared", "-fPIC", f"-I{include}", str(CSRC / "python.cpp"), "-o", str(FAST_PATH)]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on python.cpp:\n{r.stdout}\n{r.stderr}")
+
+
 def build_library(force: bool = False, verbose: bool = False) -> Path:
     """Compiles the library unless an up-to-date one exists. Returns its path."""
     BUILD_DIR.mkdir(exist_ok=True)
@@ -76,6 +90,7 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
+    _compile_fast()
     stamp.write_text(digest)
     if verbose:
         for src in CUDA_SOURCES:

@@ -7,6 +7,7 @@ wrong argument count or type fails in Python instead of corrupting a call.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 from typing import Optional
 
 from . import build as _build
@@ -163,6 +164,34 @@ def lib() -> C.CDLL:
             fn.argtypes = args
         _LIB = handle
     return _LIB
+
+
+class _ThroughCtypes:
+    """Stands in where there is no extension for this interpreter: None asks the caller to go through ctypes."""
+
+    def __getattr__(self, name):
+        return lambda *args: None
+
+
+_FAST = None
+FAST_ENTRIES = ("softmax", "rms_norm", "silu_mul", "gemm", "attention", "rope", "kv_cache_update", "attention_prefill", "attention_decode")
+
+
+def fast():
+    """The operators as functions of plain integers (csrc/python.cpp).  Each answers a status, or None for arguments that ctypes has to
+    convert."""
+    global _FAST
+    if _FAST is None:
+        handle = lib()
+        if _build.FAST_PATH.exists():
+            spec = importlib.util.spec_from_file_location("_tile_sm100", _build.FAST_PATH)
+            module = importlib.util.module_from_spec(spec)
+            spec.loader.exec_module(module)
+            module.bind(*(C.cast(getattr(handle, "tsm100_" + name), C.c_void_p).value for name in FAST_ENTRIES))
+            _FAST = module
+        else:
+            _FAST = _ThroughCtypes()
+    return _FAST
 
 
 def last_error() -> str:
