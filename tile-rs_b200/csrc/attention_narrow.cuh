@@ -44,7 +44,10 @@ struct alignas(8) Barriers {
   uint64_t s_full[kBuffers];    // the scores of a job are in its buffer
   uint64_t p_ready[kBuffers];   // its probabilities have taken their place
   uint64_t buf_free[kBuffers];  // its product has read them
-  uint64_t pv_done[2];          // per tile: the product of a step has retired
+  // Per tile, of even and of odd steps: the product of a step has retired.  A softmax thread may be two products ahead of the tensor
+  // core when it waits for the last one, and the parity of one barrier cannot tell a phase from the one two before it.  With the steps
+  // on two barriers the phase before on the same barrier is of step j - 2 or earlier, which the scores of step j have waited for.
+  uint64_t pv_done[2][2];
   uint32_t tmem_base;
   uint32_t abort_flag;
 };
@@ -98,7 +101,8 @@ attention_narrow_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       ptx::mbar_init(&bars->p_ready[b], 128);
       ptx::mbar_init(&bars->buf_free[b], 1);
     }
-    for (int g = 0; g < 2; ++g) ptx::mbar_init(&bars->pv_done[g], 1);
+    for (int g = 0; g < 2; ++g)
+      for (int e = 0; e < 2; ++e) ptx::mbar_init(&bars->pv_done[g][e], 1);
     bars->abort_flag = 0;
     ptx::fence_mbar_init();
   }
@@ -195,7 +199,7 @@ attention_narrow_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
               ptx::tcgen05_mma_f16_ts(d, a + 64 + kk * 8, b, idesc, 1u);
             }
             ptx::tcgen05_commit(&bars->buf_free[buf]);
-            ptx::tcgen05_commit(&bars->pv_done[g]);
+            ptx::tcgen05_commit(&bars->pv_done[g][j & 1]);
             if (g == 1) ptx::tcgen05_commit(&bars->kv_empty[v_pos(j) % kRing]);  // last reader of V_j
           }
           __syncwarp();
@@ -263,7 +267,7 @@ attention_narrow_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         const bool need = (m_new - m_used) * sl2 > attn::kRescaleThreshold;
         if (__any_sync(0xffffffffu, need)) {
           // once the previous step's product has retired (the next one is not issued before this step's probabilities are handed over)
-          ready = ptx::mbar_wait(&bars->pv_done[g], (j - 1) & 1u, abort_flag, p.status, 108 + g);
+          ready = ptx::mbar_wait(&bars->pv_done[g][(j - 1) & 1], ((j - 1) >> 1) & 1u, abort_flag, p.status, 108 + g);
           if (!__all_sync(0xffffffffu, ready)) {
             alive = false;
             break;
@@ -324,7 +328,7 @@ attention_narrow_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
 
     if constexpr (kSplit) {
       bool have = alive && n_g > 0;  // a range may be empty for this tile: weight 0, O zero
-      if (have) have = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done[g], (n_g - 1) & 1u, abort_flag, p.status, 110 + g));
+      if (have) have = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done[g][(n_g - 1) & 1], ((n_g - 1) >> 1) & 1u, abort_flag, p.status, 110 + g));
       ptx::tcgen05_fence_after_thread_sync();
       const int64_t rec = static_cast<int64_t>(block) * splits + rank;
       const int row = g * kBQ + r;
@@ -342,7 +346,7 @@ attention_narrow_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       }
       p.part_ml[rec * (2 * kBQ) + row] = have ? make_float2(m_used, l) : make_float2(-INFINITY, 0.f);
     } else if (alive && n_g > 0) {
-      const bool ready = ptx::mbar_wait(&bars->pv_done[g], (n_g - 1) & 1u, abort_flag, p.status, 112 + g);
+      const bool ready = ptx::mbar_wait(&bars->pv_done[g][(n_g - 1) & 1], ((n_g - 1) >> 1) & 1u, abort_flag, p.status, 112 + g);
       if (__all_sync(0xffffffffu, ready)) {
         ptx::tcgen05_fence_after_thread_sync();
         // all scores -inf (or NaN): softmax is NaN there
