@@ -492,7 +492,8 @@ constexpr int kTwiceUnroll = 4;
 template <typename T, int THREADS, bool kSkip>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 softmax_rows_twice(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t cols) {
-  ptx::launch_dependents();
+  // no launch_dependents: the CTAs of a next call would take the places that become free while others still have a row to go (2000 x
+  // 16392 bf16 in a row of calls 33.3 us with it, 31.4 without)
   x = ptx::wait_prior_grid(x);
   constexpr int PV = Elem<T>::kPerVec;
   constexpr int NW = THREADS / 32;
