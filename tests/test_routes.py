@@ -132,6 +132,11 @@ def test_attention_steps_over_several_ctas(lib, blocks, keys, ctas):
     assert lib.splits(C.c_longlong(blocks), C.c_longlong(keys), SMS) == ctas
 
 
+@pytest.mark.parametrize("blocks,keys,ctas", [(1, 8191, 3), (1, 8192, 8), (4, 9030, 8), (16, 10200, 9), (64, 16384, 2), (75, 16384, 1)])
+def test_attention_steps_of_long_caches(lib, blocks, keys, ctas):
+    assert lib.splits(C.c_longlong(blocks), C.c_longlong(keys), SMS) == ctas
+
+
 PLANES, FUSED, WARP, FP32 = 0, 1, 2, 3
 
 

@@ -574,10 +574,12 @@ attention_merge_kernel(uint16_t* __restrict__ o, const Params p) {
   if (qrow >= p.seq || c0 >= cols) return;
   const int64_t rec0 = static_cast<int64_t>(block) * p.splits;
   float gm = -INFINITY;
+#pragma unroll 8
   for (int q = 0; q < p.splits; ++q) gm = fmaxf(gm, p.part_ml[(rec0 + q) * (2 * kBQ) + row].x);
   float acc[16], gl = 0.f;
 #pragma unroll
   for (int i = 0; i < 16; ++i) acc[i] = 0.f;
+#pragma unroll 4
   for (int q = 0; q < p.splits; ++q) {
     const float2 ml = p.part_ml[(rec0 + q) * (2 * kBQ) + row];
     // a range without a visible key weighs 0; it is added all the same, because a range of NaN scores has that maximum too

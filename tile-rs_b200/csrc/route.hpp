@@ -23,11 +23,13 @@ inline bool attention_narrow_on_tcgen05(int32_t head_dim, int64_t seq_kv, int64_
 }
 
 // 16-bit attention on tcgen05: how many CTAs share the KV steps of a query block.  One CTA fills an SM, so the steps are dealt out when
-// there are blocks for at most half of the SMs, 2048 keys or more to each.  512 tokens on 15872, 32 heads (64 blocks): 212 unsplit, 122
-// split.  Below 4096 keys a call is never split, so that a prompt in chunks gives the bits of the whole one.
-constexpr int64_t kAttentionSplitKeys = 2048;
+// there are blocks for at most half of the SMs, 2048 keys or more to each, 1024 from 8192 keys on, where the merge of more records is
+// short beside the steps saved.  512 tokens on 15872, 32 heads (64 blocks): 212 unsplit, 122 split; the whole step of 30 tokens on 9000, 4 heads,
+// 52 us with 2048 keys to a CTA, 38 with 1024, 36 with 512; on 16000 56 / 44 / 48; 200 on 16000, 8 heads, 60 / 50 / 52.  Below 4096 keys a
+// call is never split, so that a prompt in chunks gives the bits of the whole one.
+constexpr int64_t kAttentionSplitKeys = 2048, kAttentionSplitKeysLong = 1024;
 inline int attention_splits(int64_t blocks, int64_t keys, int sms) {
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(sms / blocks, keys / kAttentionSplitKeys)));
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(sms / blocks, keys / (keys < 8192 ? kAttentionSplitKeys : kAttentionSplitKeysLong))));
 }
 
 // 16-bit GEMM on the tensor cores: CTA pairs (256 x 256 tiles, gemm_tc2.cuh), single CTAs (128 x 256 tiles, gemm_tc.cuh; both
