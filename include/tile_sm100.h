@@ -211,8 +211,8 @@ int32_t tsm100_silu_mul(tsm100_device_t dev, const tsm100_silu_mul_desc* desc, c
  * cores; out_dtype is the input dtype or TSM100_F32.  f32 problems take three
  * tensor-core products of operands split into two TF32 numbers (22 bits and
  * more of 24; the product of the two low parts, 2^-22 of the term, is left out),
- * accumulated in f32: large ones and small aligned ones; the rest runs on the
- * FP32 pipe.  Sums of integers stay exact where f32 sums are and the entries of
+ * accumulated in f32: all with a K of 64 or more, and aligned ones; the rest
+ * runs on the FP32 pipe.  Sums of integers stay exact where f32 sums are and the entries of
  * one operand need at most 11 bits.  In problems whose rows do not start on
  * 16-byte boundaries infinities and NaNs come out as the FP32 pipe gives them;
  * in aligned ones an infinite operand may give NaN.  `batch` independent

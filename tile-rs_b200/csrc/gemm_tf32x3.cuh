@@ -8,10 +8,11 @@
 // tensor-core products  hi*hi + hi*lo + lo*hi  accumulated in f32; the dropped lo*lo term and
 // the truncation of lo are below 2^-21 of |a||b|, the size of f32 rounding itself.
 //
+// What is small in every way runs here (route.hpp: gemm_f32): a launch has less to start than on tcgen05.
+//
 // 64 x 64 output tile per CTA, 4 warps of 32 x 32 (2 x 4 mma.sync.m16n8k8.tf32 tiles), 32-deep
 // K slices through a three- or four-stage cp.async ring; rows padded so that fragment loads are
-// conflict-free.  A CTA cluster may split K (the 512^3 configuration has only 64 output tiles
-// for 148 SMs): every CTA of a cluster accumulates its share of K and the partial tiles are
+// conflict-free.  A CTA cluster may split K (fewer output tiles than SMs): every CTA of a cluster accumulates its share of K and the partial tiles are
 // added through distributed shared memory in rank order (every CTA its share of the tile), so the result
 // does not depend on timing.
 // Needs 16-byte aligned rows: K % 4 == 0, and N % 4 == 0 for row-major B.
