@@ -137,6 +137,13 @@ def test_attention_steps_of_long_caches(lib, blocks, keys, ctas):
     assert lib.splits(C.c_longlong(blocks), C.c_longlong(keys), SMS) == ctas
 
 
+@pytest.mark.parametrize("m,n,k,batch,pays", [
+    (20, 320, 693, 4, True), (3, 1001, 5003, 1, True), (64, 301, 129, 1, True), (2, 4097, 129, 1, False), (64, 301, 127, 1, False), (25, 99, 501, 1, True),
+    (3, 171, 8001, 1, True), (1, 511, 100001, 1, False), (10, 60, 1001, 1, False)])
+def test_16_bit_products_of_odd_sizes_and_a_longer_k(lib, m, n, k, batch, pays):
+    assert lib.padding_pays(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch)) == pays
+
+
 PLANES, FUSED, WARP, FP32 = 0, 1, 2, 3
 
 
