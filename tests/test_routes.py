@@ -151,8 +151,9 @@ PLANES, FUSED, WARP, FP32 = 0, 1, 2, 3
     (4096, 4096, 4096, 1, 1, PLANES, None, None), (1999, 3001, 1501, 1, 0, PLANES, None, None), (1999, 3001, 255, 1, 0, FUSED, 1, 1),
     (512, 512, 512, 1, 1, FUSED, 4, 4), (512, 512, 512, 1, 0, FUSED, 4, 2), (64, 64, 64, 1, 1, WARP, None, None), (64, 64, 63, 1, 0, FP32, None, None),
     (64, 64, 64, 1, 0, FUSED, 1, 1), (1024, 1024, 156, 1, 1, FUSED, 1, 4), (300, 300, 156, 1, 1, WARP, None, None),
-    # the warp-level kernel sums 1024 in one go, the fused kernel 640 of them (20 k-blocks), in one CTA
-    (1024, 1024, 1024, 1, 1, FUSED, 1, 20), (1024, 1024, 1024, 1, 0, FUSED, 2, 2), (64, 64, 100000, 1, 0, FUSED, 8, 2),
+    # 128 of K to an accumulator, however long K is
+    (1024, 1024, 1024, 1, 1, FUSED, 2, 4), (1000, 1000, 4096, 1, 1, FUSED, 2, 4), (900, 900, 20000, 1, 1, FUSED, 2, 4), (64, 64, 100000, 1, 1, FUSED, 8, 4),
+    (1024, 1024, 1024, 1, 0, FUSED, 2, 2), (64, 64, 100000, 1, 0, FUSED, 8, 2),
     (1419, 372, 680, 1, 1, FUSED, 2, 4), (64, 64, 200, 149, 1, WARP, None, None), (64, 64, 200, 148, 1, FUSED, 1, 4), (65, 64, 200, 149, 1, FUSED, 1, 4)])
 def test_f32_products(lib, m, n, k, batch, aligned, kind, splits, chunk):
     out = (C.c_longlong * 4)()

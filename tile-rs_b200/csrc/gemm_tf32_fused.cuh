@@ -8,9 +8,9 @@
 // tensor maps to build.  Tiles are 128 x BN, BN = 64 or 128, and where they are fewer than the SMs a cluster of up to 8 CTAs splits K;
 // the partial tiles are summed in rank order through distributed shared memory.
 //
-// 512^3 12.9 us on the warp-level kernel, 9.1 here (as graph replays); 1024^3 51 / 30; rows that start anywhere, FP32 pipe / here:
+// 512^3 12.9 us on the warp-level kernel, 9.1 here (as graph replays); 1024^3 51 / 23; rows that start anywhere, FP32 pipe / here:
 // 1001 x 1003 x 1005 133 / 25, 301 x 301 x 2501 199 / 15, 601 x 2401 x 201 40 / 16.  Error against 64 bits 8.2e-7 of the result in
-// chunks of 128 (warp level 9.1e-7 at K = 512, 7.2e-6 at 1024), 3.7e-7 and 1.4e-7 in chunks of 64 and 32 (FP32 pipe 5.7e-7 at 1005).
+// chunks of 128, whatever K is (warp level 9.1e-7 at K = 512, 7.2e-6 at 1024, 1.4e-4 at 20000), 3.7e-7 and 1.4e-7 in chunks of 64 and 32 (FP32 pipe 5.7e-7 at 1005).
 //
 // Per CTA (one per SM): warps 8..15 load, split and store; warps 0..7 drain the chunks, keep the sums in registers and write C; warp
 // 0 also issues the products.  Bound, per 32 of K and 128 x 128 tile: shared memory, 768 cycles to feed the tensor core (which needs

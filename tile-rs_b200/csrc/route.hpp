@@ -117,15 +117,9 @@ inline GemmF32 gemm_f32(int64_t m, int64_t n, int64_t k, int64_t batch, bool ali
   if (aligned ? (k < 160 && tiles64 <= sms) || (m <= 64 && tiles64 > sms) : k < 64) return r;
   if (div_up(m, 128) * div_up(n, 64) * batch >= 0x7fffffff) return r;
   // Chunks: 128 of K, and shorter ones for the problems of the FP32 pipe, whose error is smaller at short K (relative to the 64-bit
-  // result: FP32 pipe 1.5e-7 at K = 65, 3.2e-7 at 333, 5.7e-7 at 1005; chunks of 32 1.4e-7 .. 1.8e-7, of 64 3.7e-7, of 128 8.2e-7).
-  // Sums that the warp-level kernel took over more than 512 of K in one go are 7e-9 of the result times that length below the 64-bit
-  // one; callers may rely on results within 4e-6 of those, so there the chunk is shorter by 384 of K only.
-  int64_t least_kb = 1;
+  // result: FP32 pipe 1.5e-7 at K = 65, 3.2e-7 at 333, 5.7e-7 at 1005; chunks of 32 1.4e-7 .. 1.8e-7, of 64 3.7e-7, of 128 8.2e-7).  An
+  // accumulator rounds toward zero, so the error grows with the chunk and not with K.
   r.chunk_kb = aligned ? 4 : k >= 512 ? 2 : 1;
-  if (aligned) {
-    const int64_t kb_warp = div_up(kb, gemm_f32_warp_splits(tiles64, k, sms));
-    if (kb_warp > 16) least_kb = kb_warp - 12, r.chunk_kb = static_cast<int>(least_kb);
-  }
   // Tile width and split by the time they take, in nanoseconds (fitted to 134 sizes between 64 and 2600, 10 % off in the mean): a k-block
   // costs 0.84 us on 64 columns, 1.06 on 128, a launch 4.4 and 5.5, a further wave 1.4 and 2.3.  All clusters have to fit the GPU at
   // once, one CTA per SM: 74 of two, 33 of four, 14 of eight (1419 x 372 x 680 as 36 clusters of four 23 us, in two waves, of two 16).
@@ -134,7 +128,7 @@ inline GemmF32 gemm_f32(int64_t m, int64_t n, int64_t k, int64_t batch, bool ali
     for (int s = 1; s <= 8; s *= 2) {
       const int64_t tiles = div_up(m, 128) * div_up(n, bn) * batch, per = div_up(kb, s);
       const int64_t room = s == 2 ? sms / 2 : s == 4 ? sms * 9 / 40 : sms / 10;
-      if (s > 1 && (tiles > room || per < 2 || per < least_kb)) break;
+      if (s > 1 && (tiles > room || per < 2)) break;
       const int64_t waves = s > 1 ? 1 : div_up(tiles, sms);
       const int64_t ns = bn == 64 ? 4350 + waves * per * 840 + (waves > 1 ? waves * 1400 : 0) + (s > 1 ? 860 + 80 * s : 0)
                                   : 5550 + waves * per * 1060 + (waves > 1 ? waves * 2300 : 0) + (s > 1 ? 440 + 110 * s : 0);
