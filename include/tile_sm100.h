@@ -208,14 +208,20 @@ int32_t tsm100_silu_mul(tsm100_device_t dev, const tsm100_silu_mul_desc* desc, c
  * B stored [N,K]); semantics linalg.fill 0 + linalg.matmul
  * (mlir_to_linalg.rs:1345-1393).  Replaces mlir_to_gpu.rs:1373-1397 (a TODO
  * comment) and :1584-1622.  16-bit inputs accumulate in f32 on the tensor
- * cores; out_dtype is the input dtype or TSM100_F32.  f32 problems take three
+ * cores; out_dtype is the input dtype or TSM100_F32.  f32 problems accumulate
+ * in f32.  With 64 tiles of 128 x 256 and a K of 256 or more they take three
  * tensor-core products of operands split into two TF32 numbers (22 bits and
- * more of 24; the product of the two low parts, 2^-22 of the term, is left out),
- * accumulated in f32: all with a K of 64 or more, and aligned ones; the rest
- * runs on the FP32 pipe.  Sums of integers stay exact where f32 sums are and the entries of
- * one operand need at most 11 bits.  In problems whose rows do not start on
- * 16-byte boundaries infinities and NaNs come out as the FP32 pipe gives them;
- * in aligned ones an infinite operand may give NaN.  `batch` independent
+ * more of 24; the product of the two low parts, 2^-22 of the term, is left
+ * out), and so do small aligned ones with a K below 160: sums of integers stay
+ * exact where f32 sums are and the entries of one operand need at most 11 bits.
+ * The others with a K of 64 or more, and other aligned ones, take six products
+ * of operands split into three bf16 numbers, all 24 bits (2^-24 of the term is
+ * left out): a one-hot row or column picks values bit for bit.  The rest runs
+ * on the FP32 pipe.  In problems whose rows do not start on 16-byte boundaries,
+ * and in all that take six products, infinities and NaNs come out as the FP32
+ * pipe gives them, and with six products so do outputs beside which what bf16
+ * numbers lose below 2^-133 would count; elsewhere an infinite operand may
+ * give NaN.  `batch` independent
  * problems are stored back to back (the per-block tile stride of
  * #[tile_kernel], tile_std_macros/src/lib.rs:237-254).
  * lda / ldb / ldc are row pitches in elements; 0 means "packed" (K for A; N, or K

@@ -17,7 +17,7 @@ extern "C" void gemm16_plan(long long m, long long n, long long k, long long bat
 }
 extern "C" void gemm_f32_plan(long long m, long long n, long long k, long long batch, int aligned, int sms, long long* out) {
   const GemmF32 r = gemm_f32(m, n, k, batch, aligned != 0, sms);
-  out[0] = r.kind, out[1] = r.bn, out[2] = r.splits, out[3] = r.chunk_kb;
+  out[0] = r.kind, out[1] = r.bn, out[2] = r.splits;
 }
 extern "C" void pair_tiles(long long m, long long n, long long k, long long batch, int sms, long long* out) {
   const PairTiles r = gemm_f32_pair_tiles(m, n, k, batch, sms);
@@ -147,20 +147,19 @@ def test_16_bit_products_of_odd_sizes_and_a_longer_k(lib, m, n, k, batch, pays):
 PLANES, FUSED, WARP, FP32 = 0, 1, 2, 3
 
 
-@pytest.mark.parametrize("m,n,k,batch,aligned,kind,splits,chunk", [
-    (4096, 4096, 4096, 1, 1, PLANES, None, None), (1999, 3001, 1501, 1, 0, PLANES, None, None), (1999, 3001, 255, 1, 0, FUSED, 1, 1),
-    (512, 512, 512, 1, 1, FUSED, 4, 4), (512, 512, 512, 1, 0, FUSED, 4, 2), (64, 64, 64, 1, 1, WARP, None, None), (64, 64, 63, 1, 0, FP32, None, None),
-    (64, 64, 64, 1, 0, FUSED, 1, 1), (1024, 1024, 156, 1, 1, FUSED, 1, 4), (300, 300, 156, 1, 1, WARP, None, None),
-    # 128 of K to an accumulator, however long K is
-    (1024, 1024, 1024, 1, 1, FUSED, 2, 4), (1000, 1000, 4096, 1, 1, FUSED, 2, 4), (900, 900, 20000, 1, 1, FUSED, 2, 4), (64, 64, 100000, 1, 1, FUSED, 8, 4),
-    (1024, 1024, 1024, 1, 0, FUSED, 2, 2), (64, 64, 100000, 1, 0, FUSED, 8, 2),
-    (1419, 372, 680, 1, 1, FUSED, 2, 4), (64, 64, 200, 149, 1, WARP, None, None), (64, 64, 200, 148, 1, FUSED, 1, 4), (65, 64, 200, 149, 1, FUSED, 1, 4)])
-def test_f32_products(lib, m, n, k, batch, aligned, kind, splits, chunk):
-    out = (C.c_longlong * 4)()
+@pytest.mark.parametrize("m,n,k,batch,aligned,kind,splits", [
+    (4096, 4096, 4096, 1, 1, PLANES, None), (1999, 3001, 1501, 1, 0, PLANES, None), (1999, 3001, 255, 1, 0, FUSED, 1),
+    (512, 512, 512, 1, 1, FUSED, 4), (512, 512, 512, 1, 0, FUSED, 4), (64, 64, 64, 1, 1, WARP, None), (64, 64, 63, 1, 0, FP32, None),
+    (64, 64, 64, 1, 0, FUSED, 1), (1024, 1024, 156, 1, 1, FUSED, 1), (300, 300, 156, 1, 1, WARP, None),
+    (1024, 1024, 1024, 1, 1, FUSED, 2), (1000, 1000, 4096, 1, 1, FUSED, 2), (900, 900, 20000, 1, 1, FUSED, 2), (64, 64, 100000, 1, 1, FUSED, 8),
+    (1024, 1024, 1024, 1, 0, FUSED, 2), (64, 64, 100000, 1, 0, FUSED, 8),
+    (1419, 372, 680, 1, 1, FUSED, 2), (64, 64, 200, 149, 1, WARP, None), (64, 64, 200, 148, 1, FUSED, 1), (65, 64, 200, 149, 1, FUSED, 1)])
+def test_f32_products(lib, m, n, k, batch, aligned, kind, splits):
+    out = (C.c_longlong * 3)()
     lib.gemm_f32_plan(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch), aligned, SMS, out)
     assert out[0] == kind
     if kind == FUSED:
-        assert out[1] in (64, 128) and (out[2], out[3]) == (splits, chunk)
+        assert out[1] in (64, 128) and out[2] == splits
         # every CTA of a cluster has work, and all clusters fit the GPU at once
         tiles = -(-m // 128) * -(-n // out[1]) * batch
         assert out[2] == 1 or tiles * out[2] <= SMS

@@ -31,12 +31,12 @@
 #include "attention_tc.cuh"
 #include "attention_tf32x3.cuh"
 #include "ewise.cuh"
+#include "gemm_f32_fused.cuh"
 #include "gemm_pad.cuh"
 #include "gemm_simt.cuh"
 #include "gemm_skinny.cuh"
 #include "gemm_tc.cuh"
 #include "gemm_tc2.cuh"
-#include "gemm_tf32_fused.cuh"
 #include "gemm_tf32_tc.cuh"
 #include "gemm_tf32x3.cuh"
 #include "route.hpp"
@@ -805,10 +805,10 @@ inline int32_t gemm_tf32_tc_launch(std::string* err, const tsm100_gemm_desc* d, 
   return st;
 }
 
-// f32 inputs on the tcgen05 tensor cores, split on the way in (gemm_tf32_fused.cuh).
-inline int32_t gemm_tf32_fused_launch(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
-                                      const route::GemmF32& plan, uint32_t* status, bool redo, cudaStream_t s) {
-  namespace g = gemm_tf32_fused;
+// f32 inputs on the tcgen05 tensor cores, split on the way in (gemm_f32_fused.cuh).
+inline int32_t gemm_f32_fused_launch(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
+                                      const route::GemmF32& plan, uint32_t* status, bool rows_aligned, cudaStream_t s) {
+  namespace g = gemm_f32_fused;
   const int bn = plan.bn;
   const GemmPitch ld = gemm_pitch(d);
   int sms = 0;
@@ -825,7 +825,7 @@ inline int32_t gemm_tf32_fused_launch(std::string* err, const tsm100_gemm_desc* 
   p.g.ldc = ld.ldc;
   p.g.status = status;
   p.g.vec_store = aligned16(c) && ld.ldc % 4 == 0 ? 1 : 0;
-  p.g.chunk_kb = plan.chunk_kb;
+  p.g.chunk_kb = rows_aligned ? g::kChunkKbAligned : g::kChunkKb;
   p.g.b_transposed = d->b_transposed;
   p.g.a = static_cast<const float*>(a);
   p.g.b = static_cast<const float*>(b);
@@ -846,11 +846,11 @@ inline int32_t gemm_tf32_fused_launch(std::string* err, const tsm100_gemm_desc* 
   };
   auto pick = [&](auto bn_tag) -> cudaError_t {
     constexpr int BN = decltype(bn_tag)::value;
-    auto kern = d->b_transposed ? (redo ? g::gemm_tf32_fused_kernel<BN, true, true> : g::gemm_tf32_fused_kernel<BN, true, false>)
-                                : (redo ? g::gemm_tf32_fused_kernel<BN, false, true> : g::gemm_tf32_fused_kernel<BN, false, false>);
+    auto kern = p.kb_per_cta <= g::kStages ? (d->b_transposed ? g::gemm_f32_fused_kernel<BN, true, true> : g::gemm_f32_fused_kernel<BN, false, true>)
+                                           : (d->b_transposed ? g::gemm_f32_fused_kernel<BN, true, false> : g::gemm_f32_fused_kernel<BN, false, false>);
     return launch(kern, g::smem_bytes<BN>());
   };
-  return cuda_ok(err, bn == 64 ? pick(std::integral_constant<int, 64>{}) : pick(std::integral_constant<int, 128>{}), "gemm_tf32_fused_kernel launch");
+  return cuda_ok(err, bn == 64 ? pick(std::integral_constant<int, 64>{}) : pick(std::integral_constant<int, 128>{}), "gemm_f32_fused_kernel launch");
 }
 
 template <typename OutT, bool kBT, bool kBf16>
@@ -1071,7 +1071,7 @@ inline int32_t gemm(std::string* err, const tsm100_gemm_desc* d, const void* a, 
         st = gemm_tf32_tc_launch(err, d, a, b, c, status, vec_ok, s);
         if (st != kNoScratch) return st;
       }
-      if (plan.kind == route::GemmF32::kFused) return gemm_tf32_fused_launch(err, d, a, b, c, plan, status, !vec_ok, s);
+      if (plan.kind == route::GemmF32::kFused) return gemm_f32_fused_launch(err, d, a, b, c, plan, status, vec_ok, s);
     }
     if (vec_ok) return gemm_tf32x3_launch(err, d, a, b, c, s);
     return gemm_simt_launch<float, float>(err, d, a, b, c, s);

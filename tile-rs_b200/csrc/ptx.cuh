@@ -69,6 +69,10 @@ __device__ __forceinline__ void st_shared_v4(uint32_t smem_addr, uint32_t a, uin
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(smem_addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
+__device__ __forceinline__ void st_shared_v2(uint32_t smem_addr, uint32_t a, uint32_t b) {
+  asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(smem_addr), "r"(a), "r"(b) : "memory");
+}
+
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
                "r"(bytes)
@@ -308,6 +312,9 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t smem_addr, uint32_t ran
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr), "r"(rank));
   return r;
 }
+__device__ __forceinline__ void st_shared_cluster_u32(uint32_t cluster_addr, uint32_t v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
+}
 __device__ __forceinline__ float ld_shared_cluster_f32(uint32_t cluster_addr) {
   float v;
   asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr) : "memory");
@@ -395,12 +402,13 @@ __device__ __forceinline__ void tcgen05_mma_f16_ss_pair(uint32_t d_tmem, uint64_
 //      LBO = byte distance between 64-element chunks along MN,
 //      SBO = byte distance between 8-row groups along K (1024 when packed).
 //      A K step of 16 advances the start address by 2 * SBO.
-constexpr uint64_t kSwizzle128B = 2ull;
+//    64-byte swizzle, K-major: one 64 B row = 32 bf16 of K, 16-byte unit u of row r at u ^ ((r >> 1) & 3), SBO = 512 when packed.
+constexpr uint64_t kSwizzle128B = 2ull, kSwizzle64B = 4ull;
 
-__host__ __device__ constexpr uint64_t make_smem_desc_base(uint32_t lbo_bytes, uint32_t sbo_bytes) {
+__host__ __device__ constexpr uint64_t make_smem_desc_base(uint32_t lbo_bytes, uint32_t sbo_bytes, uint64_t swizzle = kSwizzle128B) {
   return (static_cast<uint64_t>((lbo_bytes >> 4) & 0x3fffu) << 16) |
          (static_cast<uint64_t>((sbo_bytes >> 4) & 0x3fffu) << 32) | (1ull << 46) |
-         (kSwizzle128B << 61);
+         (swizzle << 61);
 }
 __device__ __forceinline__ uint64_t smem_desc(uint64_t base, uint32_t smem_addr) {
   return base | static_cast<uint64_t>((smem_addr >> 4) & 0x3fffu);

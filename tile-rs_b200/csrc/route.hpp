@@ -86,7 +86,7 @@ inline bool gemm16_padding_pays(int64_t m, int64_t n, int64_t k, int64_t batch) 
   return outputs * k >= 67108864.0 && (k >= 64 || (k >= 32 && outputs >= 7340032.0));
 }
 
-// f32 GEMM: operand planes and CTA pairs (gemm_tf32_tc.cuh), operands split on the way in (gemm_tf32_fused.cuh), the warp-level kernel
+// f32 GEMM: operand planes and CTA pairs (gemm_tf32_tc.cuh), operands split on the way in (gemm_f32_fused.cuh), the warp-level kernel
 // (gemm_tf32x3.cuh; `aligned`: rows start on 16-byte boundaries, the only ones it takes) or the FP32 pipe.
 constexpr int kMaxWarpF32Split = 4;
 inline int gemm_f32_warp_splits(int64_t tiles64, int64_t k, int sms) {
@@ -99,10 +99,9 @@ inline int gemm_f32_warp_splits(int64_t tiles64, int64_t k, int sms) {
 struct GemmF32 {
   enum Kind { kPlanes, kFused, kWarp, kFp32 } kind;
   int bn, splits;   // fused: columns per tile, CTAs that share K
-  int chunk_kb;     // fused: 32-deep k-blocks per accumulation chunk
 };
 inline GemmF32 gemm_f32(int64_t m, int64_t n, int64_t k, int64_t batch, bool aligned, int sms) {
-  GemmF32 r{aligned ? GemmF32::kWarp : GemmF32::kFp32, 0, 1, 0};
+  GemmF32 r{aligned ? GemmF32::kWarp : GemmF32::kFp32, 0, 1};
   // The fused kernel moves 32 KiB of operands from the L2 for every 128 x 128 x 32 products, the planes' 256 x 256 tiles half of that:
   // planes / fused 1552 x 2281 x 1827 82 / 141, 1533 x 1448 x 968 (72 tiles of 128 x 256) 31 / 36, 1500 x 1036 x 1723 (60) 43 / 41.
   if (div_up(m, 128) * div_up(n, 256) * batch >= 64 && k >= 256) {
@@ -111,15 +110,11 @@ inline GemmF32 gemm_f32(int64_t m, int64_t n, int64_t k, int64_t batch, bool ali
   }
   const int64_t tiles64 = div_up(m, 64) * div_up(n, 64) * batch, kb = div_up(k, 32);
   // What is small in every way: warp level 3.9, fused 5.3 (650 x 80 x 64), 5.1 / 6.3 (1670 x 124 x 68), 6.4 / 6.9 (1268 x 228 x 100); but
-  // 7.1 / 6.4 (878 x 984 x 68) and 9.5 / 8.4 (1523 x 120 x 220).  Below 64 of K the FP32 pipe is the more exact one.
+  // 7.1 / 6.4 (878 x 984 x 68) and 9.5 / 8.4 (1523 x 120 x 220).  Below 64 of K rows that start anywhere stay on the FP32 pipe.
   // Many tiles of 64 rows or less: the fused kernel's are half empty.  300 problems of 64 x 64 x 128 13.8 / 15.3, 1000 of 32 x 32 x 200
   // 39 / 50 (of 33 x 33 x 201, FP32 pipe, 110 / 64).
   if (aligned ? (k < 160 && tiles64 <= sms) || (m <= 64 && tiles64 > sms) : k < 64) return r;
   if (div_up(m, 128) * div_up(n, 64) * batch >= 0x7fffffff) return r;
-  // Chunks: 128 of K, and shorter ones for the problems of the FP32 pipe, whose error is smaller at short K (relative to the 64-bit
-  // result: FP32 pipe 1.5e-7 at K = 65, 3.2e-7 at 333, 5.7e-7 at 1005; chunks of 32 1.4e-7 .. 1.8e-7, of 64 3.7e-7, of 128 8.2e-7).  An
-  // accumulator rounds toward zero, so the error grows with the chunk and not with K.
-  r.chunk_kb = aligned ? 4 : k >= 512 ? 2 : 1;
   // Tile width and split by the time they take, in nanoseconds (fitted to 134 sizes between 64 and 2600, 10 % off in the mean): a k-block
   // costs 0.84 us on 64 columns, 1.06 on 128, a launch 4.4 and 5.5, a further wave 1.4 and 2.3.  All clusters have to fit the GPU at
   // once, one CTA per SM: 74 of two, 33 of four, 14 of eight (1419 x 372 x 680 as 36 clusters of four 23 us, in two waves, of two 16).
