@@ -20,7 +20,7 @@ constexpr int kThreads = 256;
 __global__ void __launch_bounds__(kThreads)
 pad_kernel(const uint16_t* __restrict__ src, int64_t ld, int64_t src_batch, int32_t rows, int32_t cols,
            uint4* __restrict__ dst, int32_t drows, int32_t dcols) {
-  ptx::launch_dependents();
+  ptx::launch_dependents_if_few();
   src = ptx::wait_prior_grid(src);
   const uint16_t* s = src + blockIdx.y * src_batch;
   const int64_t per_row = dcols / 8, total = drows * per_row;
@@ -44,7 +44,7 @@ pad_kernel(const uint16_t* __restrict__ src, int64_t ld, int64_t src_batch, int3
 __global__ void __launch_bounds__(kThreads)
 unpad_kernel(const uint16_t* __restrict__ src, int32_t scols, uint16_t* __restrict__ dst, int64_t ld, int64_t dst_batch,
              int32_t rows, int32_t cols) {
-  ptx::launch_dependents();
+  ptx::launch_dependents_if_few();
   src = ptx::wait_prior_grid(src);
   const int32_t c = blockIdx.x * kThreads + threadIdx.x;
   if (c >= cols) return;

@@ -165,7 +165,7 @@ gemm_tf32x3_kernel(const float* __restrict__ a, const float* __restrict__ b, flo
   }
   cp::cp_async_wait<0>();
   // not before: 512^3 in a row of calls 14.5 us with this at the start of the kernel, 13.2 here, 14.3 without early placement
-  ptx::launch_dependents();
+  ptx::launch_dependents_if_few();
 
   if (splits > 1) {
     // every CTA parks its partial tile in its own shared memory; rank 0 adds them in rank order

@@ -136,21 +136,28 @@ inline cudaError_t allow_wide_clusters_once(K kern) {
 }
 // Launches a kernel in clusters of `cluster` CTAs where that is not 0; chained: as a programmatic dependent of the one before it in
 // the stream (the rules that such kernels keep are in ptx.cuh).  What that saves is the time between two kernels of a chain of calls:
-// the end of one grid, the launch of the next and its set-up run side by side.  bf16 MLP of 16 tokens, 4096 x 16384: 95.6 us, 83.0
-// chained and with the weights' first tiles fetched meanwhile; decode of one sequence of 32768, four kernels after each other:
-// 40.3 / 32.5; 16 x 4096 x 4096 in a row of calls 12.2 / 9.0.
-template <bool kChained, typename... P, typename... A>
-inline cudaError_t launch_kernel(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, unsigned cluster, A&&... args) {
+// the end of one grid, the launch of the next and its set-up run side by side.  bf16 MLP of 16 tokens, 4096 x 16384: 84.1 us, 78.1
+// chained and with the weights' first tiles fetched meanwhile; one token of one sequence of 32768, with rotation and appends: 38.1 / 36.3, of
+// 1000 18.8 / 14.1; 16 x 4096 x 4096 in a row of calls 8.9 / 8.4 (all as graph replays).
+template <typename... P, typename... A>
+inline cudaError_t launch_kernel(bool chained, void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, unsigned cluster, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = kChained ? 1 : 0;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = cluster;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
+  unsigned n = 0;
+  if (cluster) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster;
+    attr[n].val.clusterDim.y = 1;
+    attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  if (chained) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
+  }
   cfg.attrs = attr;
-  cfg.numAttrs = cluster ? 2 : 1;
+  cfg.numAttrs = n;
   cfg.gridDim = grid;
   cfg.blockDim = dim3(threads);
   cfg.dynamicSmemBytes = smem;
@@ -159,7 +166,7 @@ inline cudaError_t launch_kernel(void (*kern)(P...), dim3 grid, unsigned threads
 }
 template <typename... P, typename... A>
 inline cudaError_t launch_chained(void (*kern)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, unsigned cluster, A&&... args) {
-  return launch_kernel<true>(kern, grid, threads, smem, s, cluster, std::forward<A>(args)...);
+  return launch_kernel(true, kern, grid, threads, smem, s, cluster, std::forward<A>(args)...);
 }
 // How many clusters of `cluster` CTAs of a kernel the GPU holds at once, asked once per kernel and device; `fallback` if it cannot tell.
 template <typename K>
@@ -1429,8 +1436,11 @@ inline int32_t attention_decode_launch(std::string* err, const tsm100_attention_
   constexpr int smem = ad::smem_floats<T, G, D>() * static_cast<int>(sizeof(float));
   cudaError_t e = set_dyn_smem_once(kern, smem);
   if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(attention_decode_kernel)");
-  e = launch_chained(kern, static_cast<unsigned>(static_cast<int64_t>(d->batch) * d->heads_kv * splits), ad::kThreads, smem, s,
-                     static_cast<unsigned>(splits), q, k, v, o, p);
+  int sms = 0;
+  const int32_t st = sm_count(err, &sms);
+  if (st != TSM100_OK) return st;
+  const unsigned grid = static_cast<unsigned>(static_cast<int64_t>(d->batch) * d->heads_kv * splits);
+  e = launch_kernel(route::decode_is_chained(grid, sms), kern, grid, ad::kThreads, smem, s, static_cast<unsigned>(splits), q, k, v, o, p);
   return cuda_ok(err, e, "attention_decode_kernel launch");
 }
 
@@ -1469,10 +1479,13 @@ inline int32_t attention_decode_mma_launch(std::string* err, const tsm100_attent
     e = allow_wide_clusters_once(kern);
     if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(attention_decode_mma_kernel, wide clusters)");
   }
-  // f32 caches are bound by the arithmetic, so an uneven placement beside the kernel before costs more than the early start gives:
-  // 24 caches of 10449 x 64, 8 heads each, 52.3 us, 53.5 chained
-  e = launch_kernel<sizeof(T) == 2>(kern, static_cast<unsigned>(static_cast<int64_t>(d->batch) * d->heads_kv * splits), WARPS * 32, smem, s,
-                                    static_cast<unsigned>(splits), q, k, v, o, p);
+  int sms = 0;
+  const int32_t st = sm_count(err, &sms);
+  if (st != TSM100_OK) return st;
+  const unsigned grid = static_cast<unsigned>(static_cast<int64_t>(d->batch) * d->heads_kv * splits);
+  // the kernel for f32 caches does not wait for the one before it: bound by the arithmetic, it took longer beside its last CTAs (24 caches
+  // of 10449 x 64, 8 heads each, 52.3 us, 53.5 chained)
+  e = launch_kernel(sizeof(T) == 2 && route::decode_is_chained(grid, sms), kern, grid, WARPS * 32, smem, s, static_cast<unsigned>(splits), q, k, v, o, p);
   return cuda_ok(err, e, "attention_decode_mma_kernel launch");
 }
 

@@ -164,6 +164,12 @@ inline PairTiles gemm_f32_pair_tiles(int64_t m, int64_t n, int64_t k, int64_t ba
   return best;
 }
 
+// Decode attention in clusters, as a programmatic dependent of the kernel before it?  Where there are more CTAs than SMs an uneven
+// placement beside that kernel's last CTAs costs more than the early start gives: in a row of calls, plain / chained, 10 caches of 18800 x 128
+// with 2 KV heads (160 CTAs) 42.7 / 48.3 us, 4 of 8000 with 8 (256) 28.9 / 33.0, 4 f32 ones of 5000 x 64 28.0 / 29.9; but one cache of 1000 with its
+// rotation and appends (16 CTAs) 17.4 / 14.1.
+inline bool decode_is_chained(int64_t ctas, int sms) { return ctas <= sms; }
+
 // Row softmax whose rows start anywhere or are too wide for one CTA's registers (softmax.cuh); `span`: the most 16-byte vectors a row
 // can touch.
 // 129 .. 256 vectors: a warp per row while there are rows for all warps, else a CTA.  1111 bf16, 200 rows 3.7 a warp, 2.9 a CTA, 600

@@ -45,7 +45,7 @@ enum : int { kRmsNorm = 0, kReduceSum = 1, kReduceMax = 2 };
 template <typename T, int OP, int VPT, int LANES, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 row_op_kernel(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t cols, float eps) {
-  ptx::launch_dependents();
+  ptx::launch_dependents_if_few();
   ptx::wait_prior_grid();
   constexpr int PV = Elem<T>::kPerVec;
   constexpr int GROUPS = THREADS / LANES;  // rows in flight per CTA
@@ -128,12 +128,12 @@ row_op_kernel(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t 
 
 // ---------------------------------------------------------------------------
 // Any width, any alignment: one CTA per row, scalar accesses, the row is read
-// twice for rms_norm (once for the reductions).
+// twice for rms_norm (once for the reductions).  The next kernel is placed at its end: 100 rows of 20001 bf16 in a row of calls 4.8 us,
+// 7.7 with the next call's CTAs placed on some of the SMs from the start.
 // ---------------------------------------------------------------------------
 template <typename T, int OP, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 row_op_stream_kernel(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int64_t cols, float eps) {
-  ptx::launch_dependents();
   x = ptx::wait_prior_grid(x);
   __shared__ float red[32];
   constexpr bool kIsMax = OP == kReduceMax;
@@ -174,7 +174,7 @@ __device__ __forceinline__ float silu(float x) {
 template <typename T, bool HAS_UP, int UNROLL, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 silu_mul_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __restrict__ y, int64_t nvec) {
-  ptx::launch_dependents();
+  ptx::launch_dependents_if_few();
   ptx::wait_prior_grid();
   constexpr int PV = Elem<T>::kPerVec;
   const Vec16* g = reinterpret_cast<const Vec16*>(gate);
@@ -209,7 +209,7 @@ silu_mul_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __restr
 template <typename T, bool HAS_UP, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 silu_mul_scalar_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __restrict__ y, int64_t n) {
-  ptx::launch_dependents();
+  ptx::launch_dependents_if_few();
   gate = ptx::wait_prior_grid(gate);
   up = ptx::wait_prior_grid(up);
   const int64_t step = static_cast<int64_t>(gridDim.x) * THREADS;
@@ -243,7 +243,7 @@ namespace rowops {
 template <typename T>
 __global__ void __launch_bounds__(256)
 rope_kernel(T* __restrict__ x, int64_t tokens, int32_t seq_len, int32_t heads, int32_t d, int32_t start_pos, float theta) {
-  ptx::launch_dependents();
+  ptx::launch_dependents_if_few();
   ptx::wait_prior_grid();
   const int half = d / 2;
   const int64_t n = tokens * half;
@@ -274,7 +274,7 @@ template <typename T>
 __global__ void __launch_bounds__(256)
 rope_vec_kernel(T* __restrict__ x, int64_t tokens, int32_t seq_len, int32_t heads, int32_t heads_per, int32_t d, int32_t start_pos,
                 float theta) {
-  ptx::launch_dependents();
+  ptx::launch_dependents_if_few();
   constexpr int PV = Elem<T>::kPerVec;
   constexpr int HU = 4;
   const int dv = d / PV;
@@ -325,7 +325,7 @@ template <typename T, int VEC, typename I>
 __global__ void __launch_bounds__(256)
 kv_cache_update_kernel(const T* __restrict__ src, T* __restrict__ cache, int64_t batch, int32_t seq_len, int32_t heads,
                        int32_t d, int32_t start_pos, int32_t max_seq) {
-  ptx::launch_dependents();
+  ptx::launch_dependents_if_few();
   src = ptx::wait_prior_grid(src);
   const I dv = static_cast<I>(d / VEC);
   const I n = static_cast<I>(batch * seq_len * heads) * dv;

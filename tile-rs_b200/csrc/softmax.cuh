@@ -153,7 +153,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 template <typename T, int CHUNKS, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
 softmax_rows_warp(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t cols) {
-  ptx::launch_dependents();
+  ptx::launch_dependents_if_few();
   ptx::wait_prior_grid();
   constexpr int PV = Elem<T>::kPerVec;
   const int lane = threadIdx.x & 31;
@@ -225,7 +225,7 @@ __device__ __forceinline__ float exp_shifted(float x, float m_log2e) {
 template <typename T, int VPT, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 softmax_rows_cta(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t cols) {
-  ptx::launch_dependents();
+  ptx::launch_dependents_if_few();
   ptx::wait_prior_grid();
   constexpr int PV = Elem<T>::kPerVec;
   constexpr int NW = THREADS / 32;
@@ -381,7 +381,7 @@ __device__ __forceinline__ float exp_diff(float x, float m) {
 template <typename T, int CHUNKS, int WARPS>
 __global__ void __launch_bounds__(WARPS * 32)
 softmax_rows_warp_any(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t cols) {
-  ptx::launch_dependents();
+  ptx::launch_dependents_if_few();
   x = ptx::wait_prior_grid(x);
   constexpr int PV = Elem<T>::kPerVec;
   const int lane = threadIdx.x & 31;
@@ -421,7 +421,7 @@ softmax_rows_warp_any(const T* __restrict__ x, T* __restrict__ y, int64_t rows, 
 template <typename T, int VPT, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 softmax_rows_cta_any(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t cols) {
-  ptx::launch_dependents();
+  ptx::launch_dependents_if_few();
   x = ptx::wait_prior_grid(x);
   constexpr int PV = Elem<T>::kPerVec;
   constexpr int NW = THREADS / 32;
@@ -562,7 +562,7 @@ softmax_rows_twice(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int
 template <typename T, int VPT, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 softmax_rows_cluster(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t cols) {
-  ptx::launch_dependents();
+  ptx::launch_dependents_if_few();
   x = ptx::wait_prior_grid(x);
   constexpr int PV = Elem<T>::kPerVec;
   constexpr int NW = THREADS / 32;
@@ -640,7 +640,6 @@ __device__ __forceinline__ float block_reduce(float v, float* red, bool is_max) 
 template <typename T, int THREADS>
 __global__ void __launch_bounds__(THREADS)
 softmax_rows_stream(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int64_t cols) {
-  ptx::launch_dependents();
   x = ptx::wait_prior_grid(x);
   __shared__ float red[32];
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
