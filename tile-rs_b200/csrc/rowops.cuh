@@ -132,25 +132,54 @@ row_op_kernel(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int32_t 
 // 7.7 with the next call's CTAs placed on some of the SMs from the start.
 // ---------------------------------------------------------------------------
 template <typename T, int OP, int THREADS>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 2048 / THREADS)
 row_op_stream_kernel(const T* __restrict__ x, T* __restrict__ y, int64_t rows, int64_t cols, float eps) {
   x = ptx::wait_prior_grid(x);
   __shared__ float red[32];
   constexpr bool kIsMax = OP == kReduceMax;
+  // Loads of a thread that are in flight together.  Through a pointer that has been through the wait the compiler cannot tell loads from stores
+  // to y, and moves none across the other: 765 rows of 39384 f16 49.4 us one by one, 33.9 this way (35.3 with read-only loads, not chained).
+  constexpr int UNROLL = 8;
+  const bool narrow = cols <= THREADS;  // one value a thread, kept for the second use: 3000 rows of 333 f32 9.1 us read twice, 6.2 this way
   for (int64_t row = blockIdx.x; row < rows; row += gridDim.x) {
     const T* xr = x + row * cols;
     float a = kIsMax ? -INFINITY : 0.f;
-    for (int64_t i = threadIdx.x; i < cols; i += THREADS) {
-      const float f = Elem<T>::load1(xr + i);
+    int64_t i = threadIdx.x;
+    auto add = [&](float f) {
       if (OP == kRmsNorm) a = fmaf(f, f, a);
       else if (OP == kReduceSum) a += f;
       else a = fmaxf(a, f);
+    };
+    float only = 0.f;
+    if (narrow) {
+      if (i < cols) add(only = Elem<T>::load1(xr + i));
+    } else {
+      for (; i + (UNROLL - 1) * THREADS < cols; i += UNROLL * THREADS) {
+        float f[UNROLL];
+#pragma unroll
+        for (int k = 0; k < UNROLL; ++k) f[k] = Elem<T>::load1(xr + i + k * THREADS);
+#pragma unroll
+        for (int k = 0; k < UNROLL; ++k) add(f[k]);
+      }
+      for (; i < cols; i += THREADS) add(Elem<T>::load1(xr + i));
     }
     a = softmax::block_reduce<THREADS>(a, red, kIsMax);
     if (OP == kRmsNorm) {
       const float scale = rsqrtf(a / static_cast<float>(cols) + eps);
       T* yr = y + row * cols;
-      for (int64_t i = threadIdx.x; i < cols; i += THREADS) Elem<T>::store1(yr + i, Elem<T>::load1(xr + i) * scale);
+      i = threadIdx.x;
+      if (narrow) {
+        if (i < cols) Elem<T>::store1(yr + i, only * scale);
+        continue;
+      }
+      for (; i + (UNROLL - 1) * THREADS < cols; i += UNROLL * THREADS) {
+        float f[UNROLL];
+#pragma unroll
+        for (int k = 0; k < UNROLL; ++k) f[k] = Elem<T>::load1(xr + i + k * THREADS);
+#pragma unroll
+        for (int k = 0; k < UNROLL; ++k) Elem<T>::store1(yr + i + k * THREADS, f[k] * scale);
+      }
+      for (; i < cols; i += THREADS) Elem<T>::store1(yr + i, Elem<T>::load1(xr + i) * scale);
     } else if (threadIdx.x == 0) {
       Elem<T>::store1(y + row, a);
     }
@@ -207,13 +236,25 @@ silu_mul_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __restr
 }
 
 template <typename T, bool HAS_UP, int THREADS>
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(THREADS, 2048 / THREADS)
 silu_mul_scalar_kernel(const T* __restrict__ gate, const T* __restrict__ up, T* __restrict__ y, int64_t n) {
   ptx::launch_dependents_if_few();
   gate = ptx::wait_prior_grid(gate);
   up = ptx::wait_prior_grid(up);
+  constexpr int UNROLL = 8;  // loads of a thread that are in flight together: 3775 x 3631 bf16 18.9 us one by one
   const int64_t step = static_cast<int64_t>(gridDim.x) * THREADS;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * THREADS + threadIdx.x; i < n; i += step) {
+  int64_t i = static_cast<int64_t>(blockIdx.x) * THREADS + threadIdx.x;
+  for (; i + (UNROLL - 1) * step < n; i += UNROLL * step) {
+    float f[UNROLL], u[UNROLL];
+#pragma unroll
+    for (int k = 0; k < UNROLL; ++k) {
+      f[k] = Elem<T>::load1(gate + i + k * step);
+      if (HAS_UP) u[k] = Elem<T>::load1(up + i + k * step);
+    }
+#pragma unroll
+    for (int k = 0; k < UNROLL; ++k) Elem<T>::store1(y + i + k * step, HAS_UP ? silu<T>(f[k]) * u[k] : silu<T>(f[k]));
+  }
+  for (; i < n; i += step) {
     const float s = silu<T>(Elem<T>::load1(gate + i));
     Elem<T>::store1(y + i, HAS_UP ? s * Elem<T>::load1(up + i) : s);
   }
