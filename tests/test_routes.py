@@ -24,6 +24,7 @@ extern "C" void pair_tiles(long long m, long long n, long long k, long long batc
   out[0] = r.bn, out[1] = r.whole_tiles, out[2] = r.splits;
 }
 extern "C" int padding_pays(long long m, long long n, long long k, long long batch) { return gemm16_padding_pays(m, n, k, batch); }
+extern "C" int rope_is_few(long long blocks, int heads_per, int sms) { return rope_few(blocks, heads_per, sms); }
 extern "C" int decode_chained(long long ctas, int sms) { return decode_is_chained(ctas, sms); }
 extern "C" int row_per_warp(long long span, long long rows, int sms) { return softmax_row_per_warp(span, rows, sms); }
 extern "C" int cluster(long long span, long long rows, int sms) { return softmax_cluster(span, rows, sms); }
@@ -143,6 +144,11 @@ def test_attention_steps_of_long_caches(lib, blocks, keys, ctas):
     (3, 171, 8001, 1, True), (1, 511, 100001, 1, False), (10, 60, 1001, 1, False)])
 def test_16_bit_products_of_odd_sizes_and_a_longer_k(lib, m, n, k, batch, pays):
     assert lib.padding_pays(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch)) == pays
+
+
+@pytest.mark.parametrize("blocks,heads_per,few", [(1, 4, True), (296, 4, True), (297, 4, False), (250, 8, False), (1, 32, False)])
+def test_little_rotary_work(lib, blocks, heads_per, few):
+    assert lib.rope_is_few(C.c_longlong(blocks), heads_per, SMS) == few
 
 
 @pytest.mark.parametrize("ctas,chained", [(1, True), (148, True), (149, False), (512, False)])

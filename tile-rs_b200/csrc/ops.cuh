@@ -575,7 +575,8 @@ inline int32_t rope(std::string* err, const tsm100_rope_desc* d, void* x, void* 
     if (vec) {
       const int32_t heads_per = route::rope_heads_per_thread(grid, d->heads, sms);
       const dim3 grid2(grid, static_cast<unsigned>((d->heads + heads_per - 1) / heads_per));
-      return launch_chained(rowops::rope_vec_kernel<T>, grid2, 256, 0, s, 0, xt, tokens, d->seq_len, d->heads, heads_per, d->head_dim, d->start_pos, d->theta);
+      auto kern = route::rope_few(static_cast<int64_t>(grid2.x) * grid2.y, heads_per, sms) ? rowops::rope_vec_kernel<T, true> : rowops::rope_vec_kernel<T, false>;
+      return launch_chained(kern, grid2, 256, 0, s, 0, xt, tokens, d->seq_len, d->heads, heads_per, d->head_dim, d->start_pos, d->theta);
     }
     return launch_chained(rowops::rope_kernel<T>, grid, 256, 0, s, 0, xt, tokens, d->seq_len, d->heads, d->head_dim, d->start_pos, d->theta);
   };

@@ -216,6 +216,8 @@ inline int rope_heads_per_thread(int64_t blocks, int heads, int sms) {
   const int64_t groups = std::max<int64_t>(1, std::min<int64_t>(div_up(2 * sms, blocks), heads / 4));
   return static_cast<int>(div_up(div_up(heads, groups), 4) * 4);
 }
+// Little work: one round of loads to a thread, and room for all blocks at once beside those of the kernel before (rowops.cuh: kFew).
+inline bool rope_few(int64_t blocks, int heads_per, int sms) { return heads_per <= 4 && blocks <= 2 * sms; }
 
 }  // namespace route
 }  // namespace tsm100

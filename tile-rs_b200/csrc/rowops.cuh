@@ -311,11 +311,15 @@ rope_kernel(T* __restrict__ x, int64_t tokens, int32_t seq_len, int32_t heads, i
 // them, and the loads of four heads are in flight together.  Same formula per pair as above.  Few tokens: with all heads on
 // one thread, 512 tokens of 32 x 128 bf16 were 32 blocks walking eight times through four heads; blockIdx.y deals the heads
 // out instead (the angles are then computed once per group).
-template <typename T>
+// kFew: little work, mostly the start of a launch; the angles are computed while the kernel before this one ends, and the next is placed from the
+// start (1 token of 32 heads 2.6 us without either, 1.6 with both, 512 tokens 3.3 / 2.5).  Otherwise the loads are issued beside the angles: with
+// the wait between them 4000 tokens of 32 x 128 took 12.7 us and 20000 took 62, 8.5 and 56 this way.
+template <typename T, bool kFew>
 __global__ void __launch_bounds__(256)
 rope_vec_kernel(T* __restrict__ x, int64_t tokens, int32_t seq_len, int32_t heads, int32_t heads_per, int32_t d, int32_t start_pos,
                 float theta) {
-  ptx::launch_dependents_if_few();
+  if (kFew) ptx::launch_dependents();
+  else ptx::wait_prior_grid();
   constexpr int PV = Elem<T>::kPerVec;
   constexpr int HU = 4;
   const int dv = d / PV;
@@ -334,7 +338,7 @@ rope_vec_kernel(T* __restrict__ x, int64_t tokens, int32_t seq_len, int32_t head
       const float angle = static_cast<float>(pos) * freq;
       sincosf(angle, &s[e], &c[e]);
     }
-    ptx::wait_prior_grid();  // the angles are computed meanwhile
+    if (kFew) ptx::wait_prior_grid();  // the angles are computed meanwhile
     Vec16* p = reinterpret_cast<Vec16*>(x + tok * heads * d) + j;
     auto rotate = [&](const Vec16& raw) -> Vec16 {
       float f[PV], r[PV];
@@ -357,7 +361,7 @@ rope_vec_kernel(T* __restrict__ x, int64_t tokens, int32_t seq_len, int32_t head
     }
     for (; h < h1; ++h) p[static_cast<int64_t>(h) * dv] = rotate(p[static_cast<int64_t>(h) * dv]);
   }
-  ptx::wait_prior_grid();
+  if (kFew) ptx::wait_prior_grid();
 }
 
 // VEC = elements per access (16 bytes when rows allow it, else 1); I = index arithmetic type: 32-bit when the
