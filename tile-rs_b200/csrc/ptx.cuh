@@ -303,8 +303,8 @@ __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontr
 // Two CTAs to an SM at most: what is won is the start of the next kernel beside this one (MLP of 16 tokens 78.1 us, 80.5 without; the silu of
 // 200 tokens has 200 CTAs, that MLP 111.4 / 112.7).
 constexpr uint32_t kFewCtas = 256;
-__device__ __forceinline__ void launch_dependents_if_few() {
-  if (static_cast<uint64_t>(gridDim.x) * gridDim.y * gridDim.z <= kFewCtas) launch_dependents();
+__device__ __forceinline__ void launch_dependents_if_few(uint32_t few = kFewCtas) {
+  if (static_cast<uint64_t>(gridDim.x) * gridDim.y * gridDim.z <= few) launch_dependents();
 }
 // Fetches what a TMA load with the same map and coordinates would read, or `bytes` (a multiple of 16) from a 16-byte aligned
 // address, into the L2.
