@@ -165,6 +165,9 @@ PLANES, FUSED, WARP, FP32 = 0, 1, 2, 3
     (64, 64, 64, 1, 0, FUSED, 1), (1024, 1024, 156, 1, 1, FUSED, 1), (300, 300, 156, 1, 1, WARP, None),
     (1024, 1024, 1024, 1, 1, FUSED, 2), (1000, 1000, 4096, 1, 1, FUSED, 2), (900, 900, 20000, 1, 1, FUSED, 2), (64, 64, 100000, 1, 1, FUSED, 8),
     (1024, 1024, 1024, 1, 0, FUSED, 2), (64, 64, 100000, 1, 0, FUSED, 8),
+    # one block of K, and one column of tiles
+    (1000, 1000, 32, 1, 1, WARP, None), (1000, 1000, 36, 1, 1, FUSED, 1), (2000, 2000, 20, 1, 1, WARP, None), (4000, 4000, 32, 1, 1, FUSED, 1),
+    (1029, 140, 20, 300, 1, WARP, None), (931, 16, 64, 60, 1, WARP, None), (931, 16, 68, 60, 1, FUSED, 1), (931, 68, 64, 60, 1, FUSED, 1), (931, 17, 65, 60, 0, FUSED, 1),
     (1419, 372, 680, 1, 1, FUSED, 2), (64, 64, 200, 149, 1, WARP, None), (64, 64, 200, 148, 1, FUSED, 1), (65, 64, 200, 149, 1, FUSED, 1)])
 def test_f32_products(lib, m, n, k, batch, aligned, kind, splits):
     out = (C.c_longlong * 3)()

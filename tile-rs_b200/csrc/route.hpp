@@ -25,7 +25,8 @@ inline bool attention_narrow_on_tcgen05(int32_t head_dim, int64_t seq_kv, int64_
 // 16-bit attention on tcgen05: how many CTAs share the KV steps of a query block.  One CTA fills an SM, so the steps are dealt out when
 // there are blocks for at most half of the SMs, 2048 keys or more to each, 1024 from 8192 keys on, where the merge of more records is
 // short beside the steps saved.  512 tokens on 15872, 32 heads (64 blocks): 212 unsplit, 122 split; the whole step of 30 tokens on 9000, 4 heads,
-// 52 us with 2048 keys to a CTA, 38 with 1024, 36 with 512; on 16000 56 / 44 / 48; 200 on 16000, 8 heads, 60 / 50 / 52.  Below 4096 keys a
+// 45 us with 2048 keys to a CTA, 32 with 1024, 30 with 512; on 16000 48 / 37 / 39; 200 on 16000, 8 heads, 51 / 43 / 46.  Between 4096 and 8191
+// keys 1024 or 512 to a CTA would do as well (30 tokens on 5000 47 / 32 / 26, 512 on 7000, 8 heads, 50 / 38 / 39).  Below 4096 keys a
 // call is never split, so that a prompt in chunks gives the bits of the whole one.
 constexpr int64_t kAttentionSplitKeys = 2048, kAttentionSplitKeysLong = 1024;
 inline int attention_splits(int64_t blocks, int64_t keys, int sms) {
@@ -109,11 +110,21 @@ inline GemmF32 gemm_f32(int64_t m, int64_t n, int64_t k, int64_t batch, bool ali
     return r;
   }
   const int64_t tiles64 = div_up(m, 64) * div_up(n, 64) * batch, kb = div_up(k, 32);
-  // What is small in every way: warp level 3.9, fused 5.3 (650 x 80 x 64), 5.1 / 6.3 (1670 x 124 x 68), 6.4 / 6.9 (1268 x 228 x 100); but
-  // 7.1 / 6.4 (878 x 984 x 68) and 9.5 / 8.4 (1523 x 120 x 220).  Below 64 of K rows that start anywhere stay on the FP32 pipe.
-  // Many tiles of 64 rows or less: the fused kernel's are half empty.  300 problems of 64 x 64 x 128 13.8 / 15.3, 1000 of 32 x 32 x 200
-  // 39 / 50 (of 33 x 33 x 201, FP32 pipe, 110 / 64).
-  if (aligned ? (k < 160 && tiles64 <= sms) || (m <= 64 && tiles64 > sms) : k < 64) return r;
+  if (!aligned && k < 64) return r;
+  if (aligned) {
+    // What is small in every way: warp level / fused 3.9 / 5.3 (650 x 80 x 64), 5.1 / 6.3 (1670 x 124 x 68), 6.4 / 6.9 (1268 x 228 x 100); but
+    // 7.1 / 6.4 (878 x 984 x 68) and 9.5 / 8.4 (1523 x 120 x 220).
+    if (k < 160 && tiles64 <= sms) return r;
+    // Many tiles of 64 rows or less: the fused kernel's are half empty.  300 problems of 64 x 64 x 128 13.8 / 15.3, 1000 of 32 x 32 x 200
+    // 39 / 50 (of 33 x 33 x 201, FP32 pipe, 110 / 64).
+    if (m <= 64 && tiles64 > sms) return r;
+    // A K of one block: a tile is little more than its start and its stores, and smaller ones overlap better, unless there are very many and
+    // the fused kernel's are full: 1000 x 1000 x 32 3.8 / 4.9, 2000 x 2000 8.0 / 8.8, 40 of 1029 x 140 14.8 / 20.9, but 4000 x 4000 27.2 / 24.6.
+    if (k <= 32 && (tiles64 <= 10 * sms || 2 * tiles64 <= 7 * div_up(m, 128) * div_up(n, 128) * batch)) return r;
+    // One column of tiles: 60 of 931 x 16 x 64 12.4 / 15.8, x 96 17.3 / 18.7, x 128 22.4 / 21.8; 20 of 2000 x 64 x 64 10.0 / 11.2, x 96 13.5 / 13.6;
+    // 400 of 128 x 64 x 64 11.7 / 11.5, x 96 16.0 / 13.8.
+    if (k <= 64 && n <= 64) return r;
+  }
   if (div_up(m, 128) * div_up(n, 64) * batch >= 0x7fffffff) return r;
   // Tile width and split by the time they take, in nanoseconds (fitted to 134 sizes between 64 and 2600, 10 % off in the mean): a k-block
   // costs 0.84 us on 64 columns, 1.06 on 128, a launch 4.4 and 5.5, a further wave 1.4 and 2.3.  All clusters have to fit the GPU at
