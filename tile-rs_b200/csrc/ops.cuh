@@ -924,10 +924,6 @@ inline int32_t gemm_skinny_launch_nt(std::string* err, const tsm100_gemm_desc* d
   p.c_batch_stride = static_cast<int64_t>(M) * ld.ldc;
   p.ldc = ld.ldc;
   p.status = status;
-  // A large B keeps HBM busy to the end, however the next kernel's CTAs lie, and the next one's first tiles can follow at once: the bf16 MLP of 16
-  // tokens (three B of 134 MB) 88.8 us with the next kernel placed after the main loop, 81.9 from the start; one such product in a row
-  // of calls 23.9 / 24.4
-  p.early = B * N * K * 2 >= (96ull << 20) ? 1 : 0;
   const int64_t tiles = static_cast<int64_t>(p.m_blocks) * p.n_blocks * p.batch;
   p.kb_per_cta = static_cast<int32_t>(plan.k_blocks_per_cta);
   const int64_t kb = (K + g::kBK - 1) / g::kBK, splits = (kb + p.kb_per_cta - 1) / p.kb_per_cta;  // a last CTA without work is dropped
