@@ -13,6 +13,7 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+import warnings
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -66,15 +67,25 @@ def _compile(src: str) -> Path:
     return obj
 
 
-def _compile_fast() -> None:
+def _compile_fast(digest: str) -> None:
+    """Compiles csrc/python.cpp for this interpreter unless that is up to date.  Without it calls go through ctypes, so that nothing here
+    keeps the library from being used."""
     include = Path(sysconfig.get_paths()["include"])
-    FAST_PATH.unlink(missing_ok=True)
-    if not (include / "Python.h").exists():
+    stamp = BUILD_DIR / (FAST_PATH.name + ".txt")
+    if not (include / "Python.h").exists() or (FAST_PATH.exists() and stamp.exists() and stamp.read_text() == digest):
         return
+    FAST_PATH.unlink(missing_ok=True)
     cmd = [shutil.which("g++") or "g++", "-std=c++17", "-O2", "-Wall", "-shared", "-fPIC", f"-I{include}", str(CSRC / "python.cpp"), "-o", str(FAST_PATH)]
-    r = subprocess.run(cmd, capture_output=True, text=True)
-    if r.returncode != 0:
-        raise RuntimeError(f"g++ failed on python.cpp:\n{r.stdout}\n{r.stderr}")
+    try:
+        r = subprocess.run(cmd, capture_output=True, text=True)
+        why = r.stderr if r.returncode else ""
+    except OSError as e:
+        why = str(e)
+    if why or not FAST_PATH.exists():
+        FAST_PATH.unlink(missing_ok=True)
+        warnings.warn(f"python.cpp was not compiled, calls go through ctypes: {why}")
+        return
+    stamp.write_text(digest)
 
 
 def build_library(force: bool = False, verbose: bool = False) -> Path:
@@ -83,6 +94,7 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
     stamp = BUILD_DIR / "digest.txt"
     digest = _digest()
     if not force and LIB_PATH.exists() and stamp.exists() and stamp.read_text() == digest:
+        _compile_fast(digest)
         return LIB_PATH
     with ThreadPoolExecutor(max_workers=4) as pool:
         objs = list(pool.map(_compile, CUDA_SOURCES + CXX_SOURCES))
@@ -90,7 +102,7 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"link failed:\n{r.stdout}\n{r.stderr}")
-    _compile_fast()
+    _compile_fast(digest)
     stamp.write_text(digest)
     if verbose:
         for src in CUDA_SOURCES:

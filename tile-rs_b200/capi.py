@@ -8,6 +8,7 @@ from __future__ import annotations
 
 import ctypes as C
 import importlib.util
+import warnings
 from typing import Optional
 
 from . import build as _build
@@ -183,14 +184,16 @@ def fast():
     global _FAST
     if _FAST is None:
         handle = lib()
+        _FAST = _ThroughCtypes()
         if _build.FAST_PATH.exists():
-            spec = importlib.util.spec_from_file_location("_tile_sm100", _build.FAST_PATH)
-            module = importlib.util.module_from_spec(spec)
-            spec.loader.exec_module(module)
-            module.bind(*(C.cast(getattr(handle, "tsm100_" + name), C.c_void_p).value for name in FAST_ENTRIES))
-            _FAST = module
-        else:
-            _FAST = _ThroughCtypes()
+            try:
+                spec = importlib.util.spec_from_file_location("_tile_sm100", _build.FAST_PATH)
+                module = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(module)
+                module.bind(*(C.cast(getattr(handle, "tsm100_" + name), C.c_void_p).value for name in FAST_ENTRIES))
+                _FAST = module
+            except (ImportError, OSError, TypeError, AttributeError) as e:
+                warnings.warn(f"{_build.FAST_PATH.name} cannot be used, calls go through ctypes: {e}")
     return _FAST
 
 
