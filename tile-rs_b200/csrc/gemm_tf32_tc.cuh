@@ -88,12 +88,6 @@ __device__ __forceinline__ float tf32_rn(float x) {
   return __uint_as_float(r & 0xffffe000u);
 }
 
-// The same as an add on the bits, for kernels where the conversion instruction, 8 a cycle and SM, would be the bound: finite numbers and
-// infinities alike, but a NaN whose bits are all ones carries into a zero.  `tf32_rn_fast` keeps a NaN, tf32_rn_finite is for what is none
-// or where another part carries it.
-__device__ __forceinline__ float tf32_rn_finite(float x) { return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u); }
-__device__ __forceinline__ float tf32_rn_fast(float x) { return x == x ? tf32_rn_finite(x) : x; }
-
 // ---------------------------------------------------------------------------
 // the split pass
 // ---------------------------------------------------------------------------
@@ -191,9 +185,8 @@ split_operands_kernel(const SplitOperand a, const SplitOperand b, uint32_t* zero
 // `staging`: 16-byte unit u of row r lies at unit u ^ (r & 7), so neither side has bank conflicts.  vec_store: 16-byte
 // stores, four rows at a time, otherwise 4-byte stores of one row.  Writing rows from the lanes that hold them costs more
 // even where they are aligned: every store then touches 32 rows (2000 x 3000 x 1500 on 256 x 128 tiles: 127 us against 117).
-// Columns of an accumulator read at a time.  16 leave the kRedo kernels, whose second pass holds registers too, without spills:
-// 1999 x 3001 x 1501 130.2 us with 32, 124.7 with 16; no difference for the others.
-template <bool kRedo>
+// Columns of an accumulator read at a time.  32 leave the kRedo kernels, whose second pass holds registers too, with spills: 1999 x 3001 x
+// 1501 130.2 us with 32, 124.7 with 16; no difference for the others.
 constexpr int kDrain = 16;
 // kRedo (problems that the FP32 pipe could take as well): a block with an infinity or a NaN is marked for second_pass.
 template <bool kRedo>
@@ -546,12 +539,12 @@ gemm_tf32_tc_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid_
 #pragma unroll
         for (int cc = 0; cc < 4; ++cc) {
 #pragma unroll
-          for (int h = 0; h < 32; h += kDrain<kRedo>) {
-            uint32_t v[kDrain<kRedo>];
+          for (int h = 0; h < 32; h += kDrain) {
+            uint32_t v[kDrain];
             ptx::tmem_ld_32x32b_x16(lane_addr + acc * kBN + cc * 32 + h, v);
             ptx::tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < kDrain<kRedo>; ++i) sum[cc][h + i] += __uint_as_float(v[i]);  // round-to-nearest add of the chunk
+            for (int i = 0; i < kDrain; ++i) sum[cc][h + i] += __uint_as_float(v[i]);  // round-to-nearest add of the chunk
           }
         }
         ptx::tcgen05_fence_before_thread_sync();
@@ -835,12 +828,12 @@ gemm_tf32_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a_hi, const __grid
 #pragma unroll
         for (int cc = 0; cc < kChunks; ++cc) {
 #pragma unroll
-          for (int h = 0; h < 32; h += kDrain<kRedo>) {
-            uint32_t v[kDrain<kRedo>];
+          for (int h = 0; h < 32; h += kDrain) {
+            uint32_t v[kDrain];
             ptx::tmem_ld_32x32b_x16(lane_addr + acc * BN + cc * 32 + h, v);
             ptx::tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < kDrain<kRedo>; ++i) sum[cc][h + i] += __uint_as_float(v[i]);
+            for (int i = 0; i < kDrain; ++i) sum[cc][h + i] += __uint_as_float(v[i]);
           }
         }
         ptx::tcgen05_fence_before_thread_sync();
