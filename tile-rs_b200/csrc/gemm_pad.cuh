@@ -15,14 +15,16 @@ namespace gemm_pad {
 
 constexpr int kThreads = 256;
 constexpr int kUnpadRows = 8;
-constexpr uint32_t kFewCtas = 1024;  // 300 x 1301 x 1203 bf16, whole call, 15.5 us with the 256 of other kernels, 14.7 this way
+// Up to how many CTAs the next kernel of the call is placed from the start: 300 x 1301 x 1203 bf16, whole call, 15.5 us with the 256 of other kernels,
+// 14.7 this way; 3 of 22 x 1923 x 1267 18.7 with 1024 for the copies in, 17.0 this way.
+constexpr uint32_t kFewCtasIn = 8192, kFewCtasOut = 1024;
 
 // src [rows][cols] with row pitch ld (problems src_batch apart) -> dst [drows][dcols] packed, zeros beyond rows and cols.
 // dcols is a multiple of 8 and dst 16-byte aligned: one thread per eight values.  blockIdx.y = problem.
 __global__ void __launch_bounds__(kThreads)
 pad_kernel(const uint16_t* __restrict__ src, int64_t ld, int64_t src_batch, int32_t rows, int32_t cols,
            uint4* __restrict__ dst, int32_t drows, int32_t dcols) {
-  ptx::launch_dependents_if_few(kFewCtas);
+  ptx::launch_dependents_if_few(kFewCtasIn);
   src = ptx::wait_prior_grid(src);
   const uint16_t* s = src + blockIdx.y * src_batch;
   const int64_t per_row = dcols / 8, total = drows * per_row;
@@ -42,24 +44,26 @@ pad_kernel(const uint16_t* __restrict__ src, int64_t ld, int64_t src_batch, int3
 }
 
 // src [rows][scols] packed -> dst [rows][cols] with row pitch ld (problems dst_batch apart), cols <= scols.
-// One thread per column of eight rows, a warp's stores are contiguous; the eight loads are in flight together (2000 x 3001 x 65 bf16, whole
-// call, 31.5 us row by row, 24 this way).  grid (x, eights of rows in strides, problem).
+// One thread per column of ROWS rows, a warp's stores are contiguous and the loads of a thread in flight together: eight rows where there are
+// CTAs for all SMs (2000 x 3001 x 65 bf16, whole call, 31.5 us row by row, 24 this way), one where there are few.  grid (x, groups of rows in
+// strides, problem).
+template <int ROWS>
 __global__ void __launch_bounds__(kThreads)
 unpad_kernel(const uint16_t* __restrict__ src, int32_t scols, uint16_t* __restrict__ dst, int64_t ld, int64_t dst_batch,
              int32_t rows, int32_t cols) {
-  ptx::launch_dependents_if_few(kFewCtas);
+  ptx::launch_dependents_if_few(kFewCtasOut);
   src = ptx::wait_prior_grid(src);
   const int32_t c = blockIdx.x * kThreads + threadIdx.x;
   if (c >= cols) return;
   const uint16_t* s = src + blockIdx.z * static_cast<int64_t>(rows) * scols + c;
   uint16_t* d = dst + blockIdx.z * dst_batch + c;
-  for (int64_t r = static_cast<int64_t>(blockIdx.y) * kUnpadRows; r < rows; r += static_cast<int64_t>(gridDim.y) * kUnpadRows) {
-    uint16_t v[kUnpadRows];
+  for (int64_t r = static_cast<int64_t>(blockIdx.y) * ROWS; r < rows; r += static_cast<int64_t>(gridDim.y) * ROWS) {
+    uint16_t v[ROWS];
 #pragma unroll
-    for (int k = 0; k < kUnpadRows; ++k)
+    for (int k = 0; k < ROWS; ++k)
       if (r + k < rows) v[k] = s[(r + k) * scols];
 #pragma unroll
-    for (int k = 0; k < kUnpadRows; ++k)
+    for (int k = 0; k < ROWS; ++k)
       if (r + k < rows) d[(r + k) * ld] = v[k];
   }
 }

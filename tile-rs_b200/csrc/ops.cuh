@@ -1029,9 +1029,11 @@ inline int32_t gemm_padded(std::string* err, const tsm100_gemm_desc* d, const vo
   st = cuda_ok(err, e, "gemm operand padding launch");
   if (st == TSM100_OK) st = gemm(err, &t, ta, tb, tc, status, s);
   if (st == TSM100_OK && pad_c) {
-    const dim3 grid(static_cast<unsigned>((d->n + g::kThreads - 1) / g::kThreads), static_cast<unsigned>(std::min<int64_t>((d->m + g::kUnpadRows - 1) / g::kUnpadRows, 4096)), static_cast<unsigned>(batch));
-    e = launch_chained(g::unpad_kernel, grid, g::kThreads, 0, s, 0, static_cast<const uint16_t*>(tc), static_cast<int32_t>(np),
-                       static_cast<uint16_t*>(c), ld.ldc, d->m * ld.ldc, static_cast<int32_t>(d->m), static_cast<int32_t>(d->n));
+    const int64_t across = (d->n + g::kThreads - 1) / g::kThreads;
+    const int rows_each = across * d->m * batch >= 16ll * sms ? g::kUnpadRows : 1;
+    const dim3 grid(static_cast<unsigned>(across), static_cast<unsigned>(std::min<int64_t>((d->m + rows_each - 1) / rows_each, 4096)), static_cast<unsigned>(batch));
+    e = launch_chained(rows_each == 1 ? g::unpad_kernel<1> : g::unpad_kernel<g::kUnpadRows>, grid, g::kThreads, 0, s, 0, static_cast<const uint16_t*>(tc),
+                       static_cast<int32_t>(np), static_cast<uint16_t*>(c), ld.ldc, d->m * ld.ldc, static_cast<int32_t>(d->m), static_cast<int32_t>(d->n));
     st = cuda_ok(err, e, "gemm result copy launch");
   }
   e = cudaFreeAsync(ws, s);
