@@ -25,7 +25,8 @@ extern "C" void pair_tiles(long long m, long long n, long long k, long long batc
 }
 extern "C" int padding_pays(long long m, long long n, long long k, long long batch) { return gemm16_padding_pays(m, n, k, batch); }
 extern "C" int rope_is_few(long long blocks, int heads_per, int sms) { return rope_few(blocks, heads_per, sms); }
-extern "C" int decode_chained(long long ctas, int sms) { return decode_is_chained(ctas, sms); }
+extern "C" int decode_chained(long long ctas, long long bytes, int sms) { return decode_is_chained(ctas, bytes, sms); }
+extern "C" int early(long long b_bytes, long long ctas, int sms) { return skinny_places_early(b_bytes, ctas, sms); }
 extern "C" int row_per_warp(long long span, long long rows, int sms) { return softmax_row_per_warp(span, rows, sms); }
 extern "C" int cluster(long long span, long long rows, int sms) { return softmax_cluster(span, rows, sms); }
 extern "C" int splits(long long blocks, long long keys, int sms) { return attention_splits(blocks, keys, sms); }
@@ -146,14 +147,19 @@ def test_16_bit_products_of_odd_sizes_and_a_longer_k(lib, m, n, k, batch, pays):
     assert lib.padding_pays(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch)) == pays
 
 
-@pytest.mark.parametrize("blocks,heads_per,few", [(1, 4, True), (296, 4, True), (297, 4, False), (250, 8, False), (1, 32, False)])
+@pytest.mark.parametrize("blocks,heads_per,few", [(1, 4, True), (296, 8, True), (297, 4, False), (250, 9, False), (1, 32, False)])
 def test_little_rotary_work(lib, blocks, heads_per, few):
     assert lib.rope_is_few(C.c_longlong(blocks), heads_per, SMS) == few
 
 
-@pytest.mark.parametrize("ctas,chained", [(1, True), (148, True), (149, False), (512, False)])
-def test_decode_is_placed_early_where_every_cta_has_an_sm(lib, ctas, chained):
-    assert lib.decode_chained(C.c_longlong(ctas), SMS) == chained
+@pytest.mark.parametrize("ctas,kib,chained", [(1, 500, True), (148, 500, True), (149, 500, False), (296, 200, False), (296, 199, True), (297, 500, True)])
+def test_decode_is_placed_early_unless_some_sms_have_two_long_ctas(lib, ctas, kib, chained):
+    assert lib.decode_chained(C.c_longlong(ctas), C.c_longlong(kib * 1024), SMS) == chained
+
+
+@pytest.mark.parametrize("mib,ctas,early", [(128, 256, True), (256, 256, True), (126, 252, True), (125, 256, False), (256, 251, False), (200, 160, False), (64, 256, False)])
+def test_few_rows_products_that_place_the_next_kernel_early(lib, mib, ctas, early):
+    assert lib.early(C.c_longlong(mib << 20), C.c_longlong(ctas), SMS) == early
 
 
 PLANES, FUSED, WARP, FP32 = 0, 1, 2, 3

@@ -63,6 +63,7 @@ struct Params {
   int64_t c_batch_stride;
   int64_t ldc;
   uint32_t* status;
+  int32_t early;            // the next kernel may be placed from the start
 };
 
 template <typename OutT>
@@ -113,6 +114,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   __syncthreads();
   ptx::tcgen05_fence_after_thread_sync();
   const uint32_t tmem_base = bars->tmem_base;
+  if (p.early) ptx::launch_dependents();
   if (threadIdx.x == 0) {
     ptx::prefetch_tensormap(&tmap_a);
     ptx::prefetch_tensormap(&tmap_b);
@@ -182,8 +184,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
   // ------------------------------ accumulator -> C ------------------------------
   const bool ready = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->acc_full, 0, abort_flag, p.status, 53));
   ptx::tcgen05_fence_after_thread_sync();
-  // not before: 11 x 4104 x 2064 of a batch of 4 in a row of calls 16.8 us with this at the start of the kernel, 14.2 here; the MLP of one token,
-  // 5120 x 20480, 123 / 107, of 16 tokens, 4096 x 12288, 67 / 64, 4096 x 16384 78 / 80, 8192 x 16384 140 / 142
+  // not before, unless the host says so (route.hpp: skinny_places_early): 11 x 4104 x 2064 of a batch of 4 in a row of calls 16.8 us with this at
+  // the start of the kernel, 14.2 here
   ptx::launch_dependents();
   const uint32_t lane_addr = tmem_base + (static_cast<uint32_t>(warp * 32) << 16);
   constexpr int kStep = NT < 32 ? 16 : 32;  // rows of C (TMEM columns) per read

@@ -927,6 +927,9 @@ inline int32_t gemm_skinny_launch_nt(std::string* err, const tsm100_gemm_desc* d
   const int64_t tiles = static_cast<int64_t>(p.m_blocks) * p.n_blocks * p.batch;
   p.kb_per_cta = static_cast<int32_t>(plan.k_blocks_per_cta);
   const int64_t kb = (K + g::kBK - 1) / g::kBK, splits = (kb + p.kb_per_cta - 1) / p.kb_per_cta;  // a last CTA without work is dropped
+  int sms = 0;
+  if (const int32_t got = sm_count(err, &sms); got != TSM100_OK) return got;
+  p.early = route::skinny_places_early(B * N * K * 2, tiles * splits, sms) ? 1 : 0;
   auto kern = g::gemm_skinny_kernel<OutT, kBT, kBf16, NT>;
   constexpr int smem = g::smem_bytes<NT>();
   cudaError_t e = set_dyn_smem_once(kern, smem);
@@ -1439,7 +1442,7 @@ inline int32_t attention_decode_launch(std::string* err, const tsm100_attention_
   const int32_t st = sm_count(err, &sms);
   if (st != TSM100_OK) return st;
   const unsigned grid = static_cast<unsigned>(static_cast<int64_t>(d->batch) * d->heads_kv * splits);
-  e = launch_kernel(route::decode_is_chained(grid, sms), kern, grid, ad::kThreads, smem, s, static_cast<unsigned>(splits), q, k, v, o, p);
+  e = launch_kernel(route::decode_is_chained(grid, static_cast<int64_t>(d->seq_len) * D * 2 * static_cast<int64_t>(sizeof(T)) / splits, sms), kern, grid, ad::kThreads, smem, s, static_cast<unsigned>(splits), q, k, v, o, p);
   return cuda_ok(err, e, "attention_decode_kernel launch");
 }
 
@@ -1484,7 +1487,7 @@ inline int32_t attention_decode_mma_launch(std::string* err, const tsm100_attent
   const unsigned grid = static_cast<unsigned>(static_cast<int64_t>(d->batch) * d->heads_kv * splits);
   // the kernel for f32 caches does not wait for the one before it: bound by the arithmetic, it took longer beside its last CTAs (24 caches
   // of 10449 x 64, 8 heads each, 52.3 us, 53.5 chained)
-  e = launch_kernel(sizeof(T) == 2 && route::decode_is_chained(grid, sms), kern, grid, WARPS * 32, smem, s, static_cast<unsigned>(splits), q, k, v, o, p);
+  e = launch_kernel(sizeof(T) == 2 && route::decode_is_chained(grid, static_cast<int64_t>(d->seq_len) * D * 2 * static_cast<int64_t>(sizeof(T)) / splits, sms), kern, grid, WARPS * 32, smem, s, static_cast<unsigned>(splits), q, k, v, o, p);
   return cuda_ok(err, e, "attention_decode_mma_kernel launch");
 }
 

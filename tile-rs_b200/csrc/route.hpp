@@ -175,11 +175,21 @@ inline PairTiles gemm_f32_pair_tiles(int64_t m, int64_t n, int64_t k, int64_t ba
   return best;
 }
 
-// Decode attention in clusters, as a programmatic dependent of the kernel before it?  Where there are more CTAs than SMs an uneven
-// placement beside that kernel's last CTAs costs more than the early start gives: in a row of calls, plain / chained, 10 caches of 18800 x 128
-// with 2 KV heads (160 CTAs) 42.7 / 48.3 us, 4 of 8000 with 8 (256) 28.9 / 33.0, 4 f32 ones of 5000 x 64 28.0 / 29.9; but one cache of 1000 with its
-// rotation and appends (16 CTAs) 17.4 / 14.1.
-inline bool decode_is_chained(int64_t ctas, int sms) { return ctas <= sms; }
+// Decode attention in clusters, as a programmatic dependent of the kernel before it?  That is worth 1.5 to 2.5 us of a call (not replayed from a
+// graph), but with one CTA on some SMs and two on others an uneven placement beside the last CTAs of that kernel may cost the time of a CTA:
+// in a row of calls, plain / chained, 10 caches of 18800 x 128 with 2 KV heads (160 CTAs) 42.7 / 48.3 us, 4 of 8000 with 8 (256) 28.9 / 33.0, 60 of
+// 1000 with 2 (240, 250 KB each) 19.3 / 21.3; but one cache of 1000 with its rotation and appends (16) 17.4 / 14.1, 55 of 182 with 8 (440) 16.6 /
+// 14.6, 5 of 8000 with 8 (320) 40.8 / 37.6, 10 of 3000 with 2 (160, 184 KB each) 16.5 / 13.8.
+inline bool decode_is_chained(int64_t ctas, int64_t bytes_per_cta, int sms) {
+  return ctas <= sms || ctas > 2 * sms || bytes_per_cta < 200 * 1024;
+}
+
+// Few-rows GEMM: is the next kernel placed from the start, or after the main loop?  From the start its first tiles follow at once where B is
+// larger than the L2 and the CTAs leave few of the places of two to an SM; with more places free the next grid piles up on them.  MLP,
+// off / on, where all three products are such (256 CTAs): 4096 x 16384 (128 MB) 1 token 71.8 / 73.6 us, 4 73.9 / 76.8, 16 80.3 / 78.0, 32 83.1 / 80.4,
+// 8192 x 16384 137.2 / 135.0, 138.8 / 136.9, 141.8 / 139.6, 143.8 / 142.5; 3072 x 16384 (96 MB) 57.3 / 57.9, 62.2 / 62.6 (16 tokens).  With 160 CTAs 5120 x
+// 20480 106 / 126 and, 16 tokens, 110 / 119, with 192 8192 x 12288 102 / 108 and 4096 x 12288 57 / 60.
+inline bool skinny_places_early(uint64_t b_bytes, int64_t ctas, int sms) { return b_bytes >= (126ull << 20) && 10 * ctas >= 17 * sms; }
 
 // Row softmax whose rows start anywhere or are too wide for one CTA's registers (softmax.cuh); `span`: the most 16-byte vectors a row
 // can touch.
@@ -227,8 +237,8 @@ inline int rope_heads_per_thread(int64_t blocks, int heads, int sms) {
   const int64_t groups = std::max<int64_t>(1, std::min<int64_t>(div_up(2 * sms, blocks), heads / 4));
   return static_cast<int>(div_up(div_up(heads, groups), 4) * 4);
 }
-// Little work: one round of loads to a thread, and room for all blocks at once beside those of the kernel before (rowops.cuh: kFew).
-inline bool rope_few(int64_t blocks, int heads_per, int sms) { return heads_per <= 4 && blocks <= 2 * sms; }
+// Little work: one or two rounds of loads to a thread, and room for all blocks at once beside those of the kernel before (rowops.cuh: kFew).
+inline bool rope_few(int64_t blocks, int heads_per, int sms) { return heads_per <= 8 && blocks <= 2 * sms; }
 
 }  // namespace route
 }  // namespace tsm100
