@@ -22,6 +22,7 @@
 // 36.1 / 32.5; 1024^3 24 us.
 #pragma once
 
+#include "attention_decode.cuh"  // cp.async helpers
 #include "attention_tc.cuh"  // 16-bit pairs
 #include "gemm_tf32_tc.cuh"
 #include "ptx.cuh"
@@ -120,11 +121,12 @@ __device__ __forceinline__ void split_store8(uint32_t at, uint32_t plane, const 
   ptx::st_shared_v4(at + plane, mid[0], mid[1], mid[2], mid[3]);
   ptx::st_shared_v4(at + 2 * plane, lo[0], lo[1], lo[2], lo[3]);
 }
-// The largest finite magnitude among rows [row0, row_end) x columns [0, cols) of `src`, over all 256 threads; `red`: 8 floats.
+// The largest finite magnitude among rows [row0, row_end) x columns [col0, col_end) of `src`, over all 256 threads; `red`: 8 floats.
 __device__ __forceinline__ float largest(const float* src, int64_t ld, int row0, int row_end, int col0, int col_end, float* red, int tid) {
   float most = 0.f;
-  for (int r = row0 + (tid >> 5); r < row_end; r += 8)
-    for (int i = col0 + (tid & 31); i < col_end; i += 32) {
+  for (int i = col0 + (tid & 31); i < col_end; i += 32)
+#pragma unroll 8
+    for (int r = row0 + (tid >> 5); r < row_end; r += 8) {
       const float v = fabsf(src[r * ld + i]);
       if (v < INFINITY) most = fmaxf(most, v);
     }
@@ -136,67 +138,90 @@ __device__ __forceinline__ float largest(const float* src, int64_t ld, int row0,
   return most;
 }
 // The outputs of rows [row_begin, row_end) of a tile that the parts of the operands do not give are summed again in plain f32, in the
-// order of k.  Infinities and NaNs always (an infinity split into parts is infinity + NaN).  Where an operand's parts miss bits, which are
-// below 2^-133, outputs beside which K times those bits and the largest operand are more than 2^-25.  256 threads, 64 x 64 outputs at a
-// time, 4 x 4 each.
-constexpr int kPanelK = 16, kPanelPitch = 68;
+// order of k.  Infinities and NaNs always (an infinity split into parts is infinity + NaN).  Where an operand's parts miss bits (`lost`), which
+// are below 2^-133, outputs beside which K times those bits and the largest operand are more than 2^-25; all, if there are infinities or NaNs too
+// (`odd`).  256 threads, 64 x 64 outputs at a time, 4 x 4 each (with what more registers take, the whole kernel spills), the next 32 of k copied
+// meanwhile.  1001 x 1003 x 1005, 29 us, with one infinity 235 us, all outputs infinite 437, a hundredth of A
+// 1e-36 102 (FP32 pipe 137).
+constexpr int kPanelK = 32, kPanelPitch = 68, kPanelBytes = 2 * kPanelK * kPanelPitch * 4;
+static_assert(2 * kPanelBytes <= kStages * Shape<64>::kStageBytes, "two panels of both operands take the place of the stages");
 template <int BN>
-__device__ __noinline__ void redo_tile(const Params& p, float* c, float* panels, int tile, int row_begin, int row_end, bool lost, int tid) {
+__device__ __noinline__ void redo_tile(const Params& p, float* c, float* panels, int tile, int row_begin, int row_end, bool lost, bool odd, int tid) {
   const tc::Params& g = p.g;
   int bz, mb, nb;
   tc::tile_coords(g, tile, bz, mb, nb);
-  const float* a = g.a + bz * g.a_batch_stride;
-  const float* b = g.b + bz * g.b_batch_stride;
-  float *sa = panels, *sb = panels + kPanelK * kPanelPitch;
-  const int tx = tid & 15, ty = tid >> 4;
   row_begin += mb * kBM, row_end = min(row_end + mb * kBM, g.m);
-  float least = 0.f;
-  if (lost) {
+  const bool bt = g.b_transposed != 0;
+  float least = lost ? INFINITY : 0.f;
+  if (lost && !odd) {
+    const float* a = g.a + bz * g.a_batch_stride;
+    const float* b = g.b + bz * g.b_batch_stride;
     const int col0 = nb * BN, col_end = min(col0 + BN, g.n);
     const float most_a = largest(a, g.lda, row_begin, row_end, 0, g.k, panels, tid);
-    const float most_b = g.b_transposed ? largest(b, g.ldb, col0, col_end, 0, g.k, panels, tid) : largest(b, g.ldb, 0, g.k, col0, col_end, panels, tid);
+    const float most_b = bt ? largest(b, g.ldb, col0, col_end, 0, g.k, panels, tid) : largest(b, g.ldb, 0, g.k, col0, col_end, panels, tid);
     least = static_cast<float>(g.k) * 0x1p-108f * (most_a + most_b);
   }
+  const int tx = tid & 15, ty = tid >> 4;
+  // this thread's eight values of a panel of A: k = tid & 31, rows (tid >> 5) + 8 i; of B the same, or, stored [K][N], column tid & 63, k = (tid >>
+  // 6) + 4 i
+  const int ak = tid & 31, ar = tid >> 5, bk = bt ? ak : tid >> 6, bn = bt ? ar : tid & 63, bk_step = bt ? 0 : 4, bn_step = bt ? 8 : 0;
   for (int block = 0; block < 2 * (BN / 64); ++block) {
     const int row0 = mb * kBM + (block & 1) * 64, col0 = nb * BN + (block >> 1) * 64;
     if (row0 >= row_end || row0 + 64 <= row_begin || col0 >= g.n) continue;
+    float* out = c + bz * g.c_batch_stride + (row0 + ty * 4) * g.ldc + col0 + tx * 4;
     uint32_t again = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const int row = row0 + ty * 4 + i, col = col0 + tx * 4 + j;
-        if (row < row_begin || row >= row_end || col >= g.n) continue;
-        const float v = fabsf(__ldcg(c + bz * g.c_batch_stride + row * g.ldc + col));
+        const int row = row0 + ty * 4 + i;
+        if (row < row_begin || row >= row_end || col0 + tx * 4 + j >= g.n) continue;
+        const float v = fabsf(__ldcg(out + i * g.ldc + j));
         if (!(v < INFINITY) || v < least) again |= 1u << (i * 4 + j);
       }
     if (!tc::epilogue_any(again != 0u)) continue;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < g.k; k0 += kPanelK) {
-      tc::epilogue_sync();
-      for (int i = tid; i < 64 * kPanelK; i += 256) {
-        const int r = i / kPanelK, kk = i % kPanelK;
-        sa[kk * kPanelPitch + r] = row0 + r < g.m && k0 + kk < g.k ? a[(row0 + r) * g.lda + k0 + kk] : 0.f;
-        const int n = g.b_transposed ? r : i % 64, kb = g.b_transposed ? kk : i / 64;
-        sb[kb * kPanelPitch + n] = col0 + n < g.n && k0 + kb < g.k ? b[g.b_transposed ? (col0 + n) * g.ldb + k0 + kb : (k0 + kb) * g.ldb + col0 + n] : 0.f;
+    const float* a = g.a + bz * g.a_batch_stride + (row0 + ar) * g.lda + ak;
+    const float* b = g.b + bz * g.b_batch_stride + (bt ? (col0 + bn) * g.ldb + bk : bk * g.ldb + col0 + bn);
+    const int64_t b_step = (bt ? 8 : 4) * g.ldb;
+    auto copy = [&](int k0, uint32_t to) {
+#pragma unroll 1
+      for (int i = 0; i < 8; ++i) {
+        const bool in_a = row0 + ar + 8 * i < g.m && k0 + ak < g.k, in_b = col0 + bn + i * bn_step < g.n && k0 + bk + i * bk_step < g.k;
+        ptx::cp_async_4(to + (ak * kPanelPitch + ar + 8 * i) * 4, in_a ? a + i * 8 * g.lda : g.a, in_a);
+        ptx::cp_async_4(to + kPanelBytes / 2 + ((bk + i * bk_step) * kPanelPitch + bn + i * bn_step) * 4, in_b ? b + i * b_step : g.b, in_b);
       }
+      a += kPanelK;
+      b += bt ? kPanelK : kPanelK * g.ldb;
+      attn_decode::mma::cp_async_commit();
+    };
+    float acc[4][4] = {};
+    uint32_t second = 0;
+    copy(0, ptx::smem_u32(panels));
+    for (int k0 = 0; k0 < g.k; k0 += kPanelK, second ^= 1u) {
+      copy(k0 + kPanelK, ptx::smem_u32(panels) + (second ^ 1u) * kPanelBytes);
+      attn_decode::mma::cp_async_wait<1>();
       tc::epilogue_sync();
-#pragma unroll 4
-      for (int kk = 0; kk < kPanelK; ++kk) {
-        const float4 x = *reinterpret_cast<const float4*>(sa + kk * kPanelPitch + ty * 4);
-        const float4 w = *reinterpret_cast<const float4*>(sb + kk * kPanelPitch + tx * 4);
+      const float* sa = panels + second * (kPanelBytes / 4) + ty * 4;
+      const float* sb = panels + second * (kPanelBytes / 4) + kPanelBytes / 8 + tx * 4;
+#pragma unroll 2
+      for (int kk = 0; kk < kPanelK; ++kk, sa += kPanelPitch, sb += kPanelPitch) {
+        const float4 x = *reinterpret_cast<const float4*>(sa);
+        const float4 w = *reinterpret_cast<const float4*>(sb);
         const float xs[4] = {x.x, x.y, x.z, x.w}, ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(xs[i], ws[j], acc[i][j]);
       }
+      tc::epilogue_sync();
     }
+    attn_decode::mma::cp_async_wait<0>();
+    tc::epilogue_sync();
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int j = 0; j < 4; ++j)
-        if ((again >> (i * 4 + j)) & 1u) c[bz * g.c_batch_stride + (row0 + ty * 4 + i) * g.ldc + col0 + tx * 4 + j] = acc[i][j];
+        if ((again >> (i * 4 + j)) & 1u) out[i * g.ldc + j] = acc[i][j];
   }
 }
 
@@ -463,8 +488,8 @@ gemm_f32_fused_kernel(float* __restrict__ c, const __grid_constant__ Params p) {
         seq = 0;
         for (int tile = first_tile; tile < num_tiles; tile += tile_step, ++seq) {
           const int bit = min(seq, kRedoTiles - 1);
-          const bool lost = (bars->marks[kLost][bit >> 5] >> (bit & 31)) & 1u;
-          if (lost || ((bars->marks[kOdd][bit >> 5] >> (bit & 31)) & 1u)) redo_tile<BN>(p, c, reinterpret_cast<float*>(smem), tile, 0, kBM, lost, threadIdx.x);
+          const bool lost = (bars->marks[kLost][bit >> 5] >> (bit & 31)) & 1u, odd = (bars->marks[kOdd][bit >> 5] >> (bit & 31)) & 1u;
+          if (lost || odd) redo_tile<BN>(p, c, reinterpret_cast<float*>(smem), tile, 0, kBM, lost, odd, threadIdx.x);
         }
       }
     }
@@ -510,9 +535,9 @@ gemm_f32_fused_kernel(float* __restrict__ c, const __grid_constant__ Params p) {
     }
     if (odd) bars->marks[kOdd][0] = 1u;
     ptx::cluster_sync_all();  // nobody's partial tile goes while a peer reads it; all of the tile is in memory
-    const bool lost = bars->marks[kLost][0] != 0u;
-    if ((lost || bars->marks[kOdd][0] != 0u) && *abort_flag == 0u && threadIdx.x < 256)
-      redo_tile<BN>(p, c, reinterpret_cast<float*>(smem), first_tile, rank * per, row_end, lost, threadIdx.x);
+    const bool lost = bars->marks[kLost][0] != 0u, any_odd = bars->marks[kOdd][0] != 0u;
+    if ((lost || any_odd) && *abort_flag == 0u && threadIdx.x < 256)
+      redo_tile<BN>(p, c, reinterpret_cast<float*>(smem), first_tile, rank * per, row_end, lost, any_odd, threadIdx.x);
   }
 
   // ------------------------------ teardown ------------------------------------

@@ -69,6 +69,10 @@ __device__ __forceinline__ void st_shared_v4(uint32_t smem_addr, uint32_t a, uin
   asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(smem_addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
 }
 
+// Four bytes to shared memory, zeros if not `ok` (then nothing is read).
+__device__ __forceinline__ void cp_async_4(uint32_t smem_addr, const void* src, bool ok) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr), "l"(src), "r"(ok ? 4 : 0) : "memory");
+}
 __device__ __forceinline__ void st_shared_v2(uint32_t smem_addr, uint32_t a, uint32_t b) {
   asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(smem_addr), "r"(a), "r"(b) : "memory");
 }
