@@ -1346,9 +1346,9 @@ inline int32_t attention_fwd_launch(std::string* err, const CUtensorMap& tq, con
   return st;
 }
 
-// Which 16-bit problems run on the tcgen05 kernel: head_dim 128, and 32 and 64 on its 64-wide form.  96 stays on the TF32
-// kernel: the second P tile that keeps the probabilities' precision does not fit beside 128-wide tiles.  b4, 32 / 8 heads of
-// 64, 2000 tokens, causal: 724 us on the TF32 kernel, 171 here; both 1.6e-3 from the 64-bit result, the rounding of bf16.  Short
+// Which 16-bit problems run on the tcgen05 kernels: head_dim 128 (attention_tc.cuh), 32 and 64 (attention_narrow.cuh).  96 stays on the TF32
+// kernel: in tensor memory three score buffers of 128 columns leave room for two O of 64, not of 96.  b4, 32 / 8 heads of
+// 64, 2000 tokens, causal: 724 us on the TF32 kernel, 132 here (graph replays); both 1.6e-3 from the 64-bit result, the rounding of bf16.  Short
 // sequences of 32 and 64 stay there too (route.hpp).  rows: query rows per head, heads: of all problems.
 inline bool attention_tc_ok(int32_t dtype, int32_t head_dim, int64_t rows, int64_t heads, int64_t seq_kv, const uint32_t* status,
                             const void* q, const void* k, const void* v, const void* o) {
