@@ -198,3 +198,12 @@ def test_shared_tiles(lib, m, n, k, batch, want):
     assert (splits - 1) * -(-kb // splits) < kb  # every share has k-blocks
     tiles = -(-m // 256) * -(-n // out[0]) * batch
     assert (tiles - out[1]) * splits <= SMS // 2
+
+
+# clusters of any size: tiles x CTAs at once, and every share has k-blocks
+@pytest.mark.parametrize("m,n,k,aligned,splits", [(1900, 261, 2591, 0, 3), (549, 1064, 900, 1, 3), (341, 412, 796, 1, 5), (234, 2177, 1525, 0, 2), (330, 180, 388, 1, 7)])
+def test_f32_shares_of_k(lib, m, n, k, aligned, splits):
+    out = (C.c_longlong * 3)()
+    lib.gemm_f32_plan(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(1), aligned, SMS, out)
+    kb, tiles = -(-k // 32), -(-m // 128) * -(-n // out[1])
+    assert out[0] == FUSED and out[2] == splits and tiles * splits <= SMS and (splits - 1) * -(-kb // splits) < kb

@@ -1074,7 +1074,7 @@ inline int32_t gemm(std::string* err, const tsm100_gemm_desc* d, const void* a, 
       int sms = 0;
       int32_t st = sm_count(err, &sms);
       if (st != TSM100_OK) return st;
-      const route::GemmF32 plan = route::gemm_f32(d->m, d->n, d->k, d->batch, vec_ok, sms);
+      const route::GemmF32 plan = route::gemm_f32(d->m, d->n, d->k, d->batch, vec_ok, sms, d->b_transposed != 0);
       const int64_t tiles = ((d->m + 127) / 128) * ((d->n + 255) / 256) * d->batch;
       if (plan.kind == route::GemmF32::kPlanes && tiles < 0x7fffffff) {
         st = gemm_tf32_tc_launch(err, d, a, b, c, status, vec_ok, s);

@@ -91,7 +91,7 @@ inline bool gemm16_padding_pays(int64_t m, int64_t n, int64_t k, int64_t batch) 
 
 // f32 GEMM: operand planes and CTA pairs (gemm_tf32_tc.cuh), operands split on the way in (gemm_f32_fused.cuh), the warp-level kernel
 // (gemm_tf32x3.cuh; `aligned`: rows start on 16-byte boundaries, the only ones it takes) or the FP32 pipe.
-constexpr int kMaxWarpF32Split = 4;
+constexpr int kMaxWarpF32Split = 4, kMaxF32FusedSplit = 8;
 inline int gemm_f32_warp_splits(int64_t tiles64, int64_t k, int sms) {
   // fewer 64 x 64 tiles than SMs: a cluster splits K while all CTAs still fit the GPU at once (two per SM) and every CTA keeps at least
   // four 32-deep slices
@@ -103,7 +103,7 @@ struct GemmF32 {
   enum Kind { kPlanes, kFused, kWarp, kFp32 } kind;
   int bn, splits;   // fused: columns per tile, CTAs that share K
 };
-inline GemmF32 gemm_f32(int64_t m, int64_t n, int64_t k, int64_t batch, bool aligned, int sms) {
+inline GemmF32 gemm_f32(int64_t m, int64_t n, int64_t k, int64_t batch, bool aligned, int sms, bool b_transposed = false) {
   GemmF32 r{aligned ? GemmF32::kWarp : GemmF32::kFp32, 0, 1};
   // The fused kernel moves 32 KiB of operands from the L2 for every 128 x 128 x 32 products, the planes' 256 x 256 tiles half of that:
   // planes / fused 1552 x 2281 x 1827 82 / 141, 1533 x 1448 x 968 (72 tiles of 128 x 256) 31 / 36, 1500 x 1036 x 1723 (60) 43 / 41.
@@ -128,18 +128,22 @@ inline GemmF32 gemm_f32(int64_t m, int64_t n, int64_t k, int64_t batch, bool ali
     if (k <= 64 && n <= 64) return r;
   }
   if (div_up(m, 128) * div_up(n, 64) * batch >= 0x7fffffff) return r;
-  // Tile width and split by the time they take, in nanoseconds (fitted to 134 sizes between 64 and 2600, 10 % off in the mean): a k-block
-  // costs 0.84 us on 64 columns, 1.06 on 128, a launch 4.4 and 5.5, a further wave 1.4 and 2.3.  All clusters have to fit the GPU at
-  // once, one CTA per SM: 74 of two, 33 of four, 14 of eight (1419 x 372 x 680 as 36 clusters of four 23 us, in two waves, of two 16).
+  // Tile width and split by the time they take, in nanoseconds (fitted to 200 sizes between 64 and 2600, 8 % off in the mean): a launch costs
+  // 4.4 us on 64 columns, 5.5 on 128, a further wave 1.4 and 2.3, a k-block what stands below: rows that start anywhere are loaded value by
+  // value, B stored [K][N] in columns, and both cost more where a CTA loads 128 columns.  All clusters have to fit the GPU at
+  // once, one CTA per SM (1419 x 372 x 680 as 36 clusters of four 23 us, in two waves, of two 16); of clusters of 2, 3, ... 8 a B200
+  // holds 74, 45, 33, 26, 22, 15 and 15.  Any size of cluster, not powers of two alone: 2410 x 108 x 2256 26.8 -> 20.1, 549 x 1064 x 900 23.2 -> 19.8,
+  // 1900 x 261 x 2591 58 -> 48, 267 x 724 x 792 13.2 -> 11.6.
+  const int64_t kb64 = aligned ? 810 : 880, kb128 = aligned ? (b_transposed ? 1020 : 1170) : (b_transposed ? 1200 : 1270);
   int64_t best = INT64_MAX;
   for (int bn = 64; bn <= 128; bn += 64)
-    for (int s = 1; s <= 8; s *= 2) {
+    for (int s = 1; s <= kMaxF32FusedSplit; ++s) {
       const int64_t tiles = div_up(m, 128) * div_up(n, bn) * batch, per = div_up(kb, s);
-      const int64_t room = s == 2 ? sms / 2 : s == 4 ? sms * 9 / 40 : sms / 10;
-      if (s > 1 && (tiles > room || per < 2)) break;
+      const int64_t room = s == 2 ? sms / 2 : s == 3 ? sms * 9 / 29 : s == 4 ? sms * 9 / 40 : s == 5 ? sms * 7 / 40 : s == 6 ? sms * 3 / 20 : sms / 10;
+      if (s > 1 && (tiles > room || per < 2 || (s - 1) * per >= kb)) continue;
       const int64_t waves = s > 1 ? 1 : div_up(tiles, sms);
-      const int64_t ns = bn == 64 ? 4350 + waves * per * 840 + (waves > 1 ? waves * 1400 : 0) + (s > 1 ? 860 + 80 * s : 0)
-                                  : 5550 + waves * per * 1060 + (waves > 1 ? waves * 2300 : 0) + (s > 1 ? 440 + 110 * s : 0);
+      const int64_t ns = bn == 64 ? 4350 + waves * per * kb64 + (waves > 1 ? waves * 1400 : 0) + (s > 1 ? 860 + 80 * s : 0)
+                                  : 5550 + waves * per * kb128 + (waves > 1 ? waves * 2300 : 0) + (s > 1 ? 440 + 110 * s : 0);
       if (ns < best) best = ns, r.bn = bn, r.splits = s;
     }
   r.kind = GemmF32::kFused;
