@@ -30,6 +30,7 @@ extern "C" int early(long long b_bytes, long long ctas, int sms) { return skinny
 extern "C" int row_per_warp(long long span, long long rows, int sms) { return softmax_row_per_warp(span, rows, sms); }
 extern "C" int cluster(long long span, long long rows, int sms) { return softmax_cluster(span, rows, sms); }
 extern "C" int splits(long long blocks, long long keys, int sms) { return attention_splits(blocks, keys, sms); }
+extern "C" int attention_f32(int d, long long keys) { return attention_f32_on_tcgen05(d, keys); }
 extern "C" int rope_heads(long long blocks, int heads, int sms) { return rope_heads_per_thread(blocks, heads, sms); }
 extern "C" int twice_skip(long long vectors, int threads) { return softmax_twice_skip(vectors, threads, 4); }
 extern "C" int twice_threads(long long bytes, long long rows, int sms) { return softmax_twice_threads(bytes, rows, sms); }
@@ -207,3 +208,8 @@ def test_f32_shares_of_k(lib, m, n, k, aligned, splits):
     lib.gemm_f32_plan(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(1), aligned, SMS, out)
     kb, tiles = -(-k // 32), -(-m // 128) * -(-n // out[1])
     assert out[0] == FUSED and out[2] == splits and tiles * splits <= SMS and (splits - 1) * -(-kb // splits) < kb
+
+
+@pytest.mark.parametrize("d,keys,tc", [(128, 1, True), (96, 64, False), (96, 65, True), (64, 64, False), (64, 65, True), (32, 160, False), (32, 161, True)])
+def test_f32_attention(lib, d, keys, tc):
+    assert lib.attention_f32(d, C.c_longlong(keys)) == tc

@@ -1,103 +1,117 @@
-// Fused attention forward for f32 tensors on the 5th-generation tensor cores (tcgen05, kind::tf32), f32-grade results.
+// Fused attention forward for f32 tensors on the 5th-generation tensor cores (tcgen05, kind::f16), f32-grade results.
 //
 // Semantics as attention_tf32x3.cuh (__tile_attention_f32, crates/tile_std/src/tile.rs:218-224;
 // crates/rustc_codegen_tile/src/mlir_to_linalg.rs:1781-1902, :1191-1244; grouped heads
-// crates/rustc_codegen_tile/src/mlir_to_gpu.rs:1657-1673); the scheme of three TF32 products per product on hi / lo
-// parts, and of accumulating in short chunks, is that of gemm_tf32_tc.cuh.
+// crates/rustc_codegen_tile/src/mlir_to_gpu.rs:1657-1673).  Every operand, Q, K, V and the probabilities, is split into three bf16 numbers, 24 bits
+// together, and six of the nine products are taken, as in gemm_f32_fused.cuh.
 //
-// One streaming launch writes the hi / lo planes of K ([keys][D]) and of V, transposed ([D][keys]), so that both products
-// see K-major operands only.  Then one CTA owns 128 query rows of one head and walks the keys in steps of 32:
-//   warp 8       TMA producer: K_0, K_1, V_0, K_2, V_1, ... (hi and lo together, 256 * D bytes a unit) through a 5-deep
-//                ring.  No multicast.
-//   warp 9       S = Q K^T: the hi tile of Q stays in tensor memory for the CTA's life, the lo tile in shared memory.  A
-//                128 x 32 x 8 product reads 4 KiB of A against 1 KiB of B; from shared memory that takes 40 cycles, 16 of which
-//                the tensor core needs, so two of the three products take A from tensor memory.
-//   warp 10      O += P V: P_hi, P_lo are read from tensor memory.
-//   warps 0..3   softmax, one thread per query row; the running maximum is raised freely where a chunk of O begins and
-//                otherwise only when it grows by more than 2^8 (the chunk in tensor memory is then rescaled).
-//   warps 4..7   drain: the tensor core rounds its accumulator toward zero, so O is accumulated over kChunkSteps steps
-//                (128 keys) from zero and then added, round to nearest, to running sums in registers (D per thread).
-// S and the chunk of O are double-buffered, so that the products of one step run during the softmax of the next; P is not
-// (tensor memory at D = 128: 2 * 128 of O, 2 * 32 of S, 32 + 32 of P, 128 of Q: all 512 columns).
-// Bound: tensor pipe at the TF32 rate / 3; shared-memory reads of Q by the 32-wide S products come close behind.  16 heads of
-// 4096 x 128, causal: 170 TFLOP/s as graph replays (0.63 of a third of the TF32 rate; 137 with both parts of Q in shared memory), 156 per
-// call in a row of calls; 48 on the warp-level kernel.
+// One streaming launch writes the parts of K and of V, each as planes [3][heads][keys][D]; V is read MN-major as it lies.  Then one CTA owns 128
+// query rows of one head and walks the keys in steps of 64:
+//   warp 8       TMA producer: K_0, K_1, V_0, K_2, V_1, ... (three parts together, 384 * D bytes a unit) through a ring.  No multicast.
+//   warp 9       S = Q K^T, the parts of Q in tensor memory for the CTA's life.
+//   warp 10      O = P V of one step, from zero: the tensor core rounds its accumulator toward zero, and what that costs grows with what it holds.
+//   warps 0..3   softmax, one thread per query row; the parts of the probabilities take the place of the scores they were made from.
+//   warps 4..7   drain: the O of a step is added, round to nearest, to running sums in registers (D per thread), scaled by how far the
+//                step's maximum has grown.
+// Tensor memory at D = 128: 3 * 64 columns of Q, two buffers of 96 for scores (64) and then probabilities (3 * 32), 128 of O: all 512.  A step's softmax
+// runs during the scores of the next, and the drain too, so one O is enough.
+// Bound: the tensor pipe, 3072 cycles a step (48 products of 128 x 64 x 16, 24 of 128 x 128 x 16), and the board's power: 16 heads of 4096 x 128, causal,
+// 297 us at 1.6 GHz, 475 K cycles of which 350 K are products, and 26 us for the parts of K and V; 363 us a call in a row (189 TFLOP/s), 2.2e-7 off the
+// 64-bit result.  The form before this one took three products of two TF32 numbers in steps of 32 keys, whose scores spend most of a product on
+// reading Q, and wrote a third more for the parts, V transposed: 450 us, 9e-7; 2 heads of 1283 70 us, 48 here, 256 heads of 530 242 / 182.
+// What no bf16 number holds is bits below 2^-133, so that operands below 1e-34 have fewer: V of 1e-35 3.6e-6, of 1e-36 2.6e-5 (two TF32 numbers, whose
+// low part ends at 2^-126, 1.7e-6 and 7e-6).
 #pragma once
 
-#include "attention_simt.cuh"  // Params
-#include "gemm_tf32_tc.cuh"    // split passes, tf32_rn, descriptors
+#include "attention_simt.cuh"    // Params
+#include "gemm_f32_fused.cuh"    // split2
 #include "ptx.cuh"
 
 namespace tsm100 {
 namespace attn_f32_tc {
 
-using gemm_tf32_tc::tf32_rn;
-
 constexpr int kBQ = 128;           // query rows per CTA
-constexpr int kBKV = 32;           // keys per step: one 128-byte swizzle row of f32
-constexpr int kChunkSteps = 4;     // steps per accumulation chunk of O
+constexpr int kBKV = 64;           // keys per step
 constexpr int kThreads = 384;
-constexpr int kRing = 5;
-constexpr int kRegsOther = 56, kRegsSoftmax = 168, kRegsDrain = 224;
+constexpr int kRegsOther = 56, kRegsSoftmax = 200, kRegsDrain = 224;
 static_assert(128 * (kRegsOther + kRegsSoftmax + kRegsDrain) <= kThreads * 168, "setmaxnreg draws on the launch's registers");
 constexpr int kTmemCols = 512;
-constexpr int kTmemO = 0, kTmemS = 256, kTmemP = 320, kTmemQ = 384;  // two accumulators of 128, two of 32, 32 hi + 32 lo, 128
-constexpr float kRescaleThreshold = 8.0f;              // log2 units
-// its bounded waits report sites 71 .. 84
+constexpr int kTmemQ = 0, kQPart = 64, kTmemS = 192, kBuffer = 96, kPPart = 32, kTmemO = 384;
+// its bounded waits report sites 71 .. 83
 
 template <int D>
 struct Shape {
-  static constexpr int kQPlane = kBQ * D * 4;           // D / 32 groups of 128 rows x 128 bytes
-  static constexpr int kUnitPlane = kBKV * D * 4;       // K: D / 32 groups of 32 rows x 128 bytes; V: D rows x 128 bytes
-  static constexpr int kUnitBytes = 2 * kUnitPlane;     // hi, lo
-  static constexpr int kRingOff = kQPlane;              // behind the lo tile of Q
-  static constexpr int kRowsOff = kRingOff + kRing * kUnitBytes;  // float [3][128]: per chunk, the maximum it is scaled by
+  static constexpr int kGroup = D % 64 == 0 ? 64 : 32;   // columns of a swizzled row
+  static constexpr int kRow = kGroup * 2;                // bytes: the swizzle
+  static constexpr int kGroups = D / kGroup;
+  static constexpr int kGroupBytes = kBKV * kRow;
+  static constexpr int kPart = kBKV * D * 2;             // one part of 64 rows of K or V
+  static constexpr int kUnitBytes = 3 * kPart;
+  static constexpr int kRing = D == 128 ? 4 : D == 96 ? 5 : 8;
+  static constexpr int kRowsOff = kRing * kUnitBytes;    // float [3][128]: per step, the maximum it is scaled by
   static constexpr int kBarsOff = kRowsOff + 3 * kBQ * 4;
 };
+constexpr int kMaxRing = 8;
 struct alignas(8) Barriers {
   uint64_t q_ready;
-  uint64_t kv_full[kRing], kv_empty[kRing];
-  uint64_t s_full[2], s_free[2];
-  uint64_t p_ready, pv_done;
-  uint64_t o_full[2], o_empty[2];
-  uint64_t m_ready[3];   // the maximum of a chunk is in its row slot
-  uint64_t l_ready;      // the row sums are in the slot after the last chunk's
+  uint64_t kv_full[kMaxRing], kv_empty[kMaxRing];
+  uint64_t s_full[2];     // the scores of a step are in its buffer
+  uint64_t p_ready[2];    // its probabilities have taken their place
+  uint64_t buf_free[2];   // its product has read them
+  uint64_t o_full, o_empty;
+  uint64_t m_ready[3];    // the maximum of a step is in its row slot
+  uint64_t l_ready;       // the row sums are in the slot after the last step's
   uint32_t tmem_base;
   uint32_t abort_flag;
-  uint32_t pv_steps;     // steps whose P V has been issued (only grows)
 };
 template <int D>
 constexpr int smem_bytes() {
   return Shape<D>::kBarsOff + static_cast<int>(sizeof(Barriers)) + 1024;
 }
-static_assert(smem_bytes<128>() <= 227 * 1024, "shared memory budget of one CTA");
+static_assert(smem_bytes<128>() <= 227 * 1024 && smem_bytes<96>() <= 227 * 1024 && smem_bytes<64>() <= 227 * 1024, "shared memory budget of one CTA");
 
 struct Params {
   attn_simt::Params a;      // shapes, and the strides of Q and O
   uint32_t* status;
 };
 
-__device__ __forceinline__ void mma_tf32_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n"
-      ".reg .pred p;\n"
-      "setp.ne.b32 p, %4, 0;\n"
-      "tcgen05.mma.cta_group::1.kind::tf32 [%0], [%1], %2, %3, p;\n"
-      "}\n" ::"r"(d_tmem),
-      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
+// The parts of K and of V, bf16 [3][heads][rows * D]: grid (blocks, heads, 2), a thread per eight values.
+struct SplitParams {
+  const float* src[2];
+  uint16_t* dst[2];
+  int64_t head_stride;      // of src, in elements
+  int64_t head_vecs;        // rows * D / 8
+};
+__global__ void __launch_bounds__(256)
+split_kv_kernel(const SplitParams p) {
+  ptx::launch_dependents_if_few();
+  const int which = static_cast<int>(blockIdx.z);
+  const int64_t head = blockIdx.y, part = p.head_vecs * gridDim.y;
+  const float4* src = reinterpret_cast<const float4*>(ptx::wait_prior_grid((which ? p.src[1] : p.src[0]) + head * p.head_stride));
+  uint4* dst = reinterpret_cast<uint4*>(which ? p.dst[1] : p.dst[0]) + head * p.head_vecs;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < p.head_vecs; i += step) {
+    const float4 x = __ldcs(src + 2 * i), y = __ldcs(src + 2 * i + 1);
+    uint32_t hi[4], mid[4], lo[4], unused = 0;
+    gemm_f32_fused::split2(x.x, x.y, hi[0], mid[0], lo[0], unused);
+    gemm_f32_fused::split2(x.z, x.w, hi[1], mid[1], lo[1], unused);
+    gemm_f32_fused::split2(y.x, y.y, hi[2], mid[2], lo[2], unused);
+    gemm_f32_fused::split2(y.z, y.w, hi[3], mid[3], lo[3], unused);
+    dst[i] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+    dst[i + part] = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+    dst[i + 2 * part] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+  }
 }
 
 template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
-attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __grid_constant__ CUtensorMap tmap_k_lo,
-                        const __grid_constant__ CUtensorMap tmap_v_hi, const __grid_constant__ CUtensorMap tmap_v_lo,
-                        const float* __restrict__ q, float* __restrict__ o, const Params pp) {
+attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v, const float* __restrict__ q,
+                        float* __restrict__ o, const Params pp) {
   using Sh = Shape<D>;
+  constexpr int kRing = Sh::kRing;
   const attn_simt::Params& p = pp.a;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* ring = smem + Sh::kRingOff;
   float* row_slot = reinterpret_cast<float*>(smem + Sh::kRowsOff);
   Barriers* bars = reinterpret_cast<Barriers*>(smem + Sh::kBarsOff);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -111,28 +125,26 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
   const int qb_raw = static_cast<int>(blockIdx.x) / heads;
   const int q0 = (p.causal ? q_blocks - 1 - qb_raw : qb_raw) * kBQ;
   const int kvh = bh / p.heads_q * p.heads_kv + bh % p.heads_q / (p.heads_q / p.heads_kv);
+  const int all_kv = p.batch * p.heads_kv;
   const int n_all = (p.seq_kv + kBKV - 1) / kBKV;
   const int n = p.causal ? min(n_all, (min(q0 + kBQ, p.seq) - 1 + p.q_offset) / kBKV + 1) : n_all;  // steps, >= 1
-  const int chunks = (n + kChunkSteps - 1) / kChunkSteps;
 
   if (threadIdx.x == 0) {
     ptx::mbar_init(&bars->q_ready, 128);
-    ptx::mbar_init(&bars->p_ready, 128);
-    ptx::mbar_init(&bars->pv_done, 1);
     for (int s = 0; s < kRing; ++s) {
       ptx::mbar_init(&bars->kv_full[s], 1);
       ptx::mbar_init(&bars->kv_empty[s], 1);
     }
     for (int i = 0; i < 2; ++i) {
       ptx::mbar_init(&bars->s_full[i], 1);
-      ptx::mbar_init(&bars->s_free[i], 128);
-      ptx::mbar_init(&bars->o_full[i], 1);
-      ptx::mbar_init(&bars->o_empty[i], 128);
+      ptx::mbar_init(&bars->p_ready[i], 128);
+      ptx::mbar_init(&bars->buf_free[i], 1);
     }
+    ptx::mbar_init(&bars->o_full, 1);
+    ptx::mbar_init(&bars->o_empty, 128);
     for (int i = 0; i < 3; ++i) ptx::mbar_init(&bars->m_ready[i], 128);
     ptx::mbar_init(&bars->l_ready, 128);
     bars->abort_flag = 0;
-    bars->pv_steps = 0;
     ptx::fence_mbar_init();
   }
   if (warp == 9) {
@@ -143,34 +155,33 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
   __syncthreads();
   ptx::tcgen05_fence_after_thread_sync();
   const uint32_t tmem = bars->tmem_base;
+  ptx::wait_prior_grid();
   // ring positions: K_0, K_1, V_0, K_2, V_1, ..., K_{n-1}, V_{n-2}, V_{n-1}
   auto k_pos = [&](int j) { return j == 0 ? 0 : 2 * j - 1; };
   auto v_pos = [&](int j) { return j == n - 1 ? 2 * n - 1 : 2 * j + 2; };
 
-  // Q, split (warps 0..3, one row each): hi to tensor memory, lo to the swizzled K-major tile in shared memory (16-byte unit u
-  // of row r at position u ^ (r & 7) of its group of 32 columns)
+  // Q, split, to tensor memory (warps 0..3, one row each)
   if (warp < 4) {
     const int r = warp * 32 + lane;
     const bool valid = q0 + r < p.seq;
     const float4* qr = reinterpret_cast<const float4*>(q + bh * p.q_head_stride + (q0 + r) * p.q_row_stride);
-    const uint32_t base = ptx::smem_u32(smem) + r * 128;
+    const uint32_t tq = tmem + (static_cast<uint32_t>(warp * 32) << 16) + kTmemQ;
 #pragma unroll
     for (int c = 0; c < D / 32; ++c) {
-      uint32_t hi[32];
+      uint32_t hi[16], mid[16], lo[16], unused = 0;
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const float4 x = valid ? qr[c * 8 + u] : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 h = make_float4(tf32_rn(x.x), tf32_rn(x.y), tf32_rn(x.z), tf32_rn(x.w));
-        hi[4 * u] = __float_as_uint(h.x), hi[4 * u + 1] = __float_as_uint(h.y), hi[4 * u + 2] = __float_as_uint(h.z), hi[4 * u + 3] = __float_as_uint(h.w);
-        ptx::st_shared_v4(base + c * (kBQ * 128) + ((u ^ (r & 7)) << 4), __float_as_uint(tf32_rn(x.x - h.x)), __float_as_uint(tf32_rn(x.y - h.y)),
-                          __float_as_uint(tf32_rn(x.z - h.z)), __float_as_uint(tf32_rn(x.w - h.w)));
+        gemm_f32_fused::split2(x.x, x.y, hi[2 * u], mid[2 * u], lo[2 * u], unused);
+        gemm_f32_fused::split2(x.z, x.w, hi[2 * u + 1], mid[2 * u + 1], lo[2 * u + 1], unused);
       }
       __syncwarp();
-      ptx::tmem_st_32x32b_x32(tmem + (static_cast<uint32_t>(warp * 32) << 16) + kTmemQ + c * 32, hi);
+      ptx::tmem_st_32x32b_x16(tq + c * 16, hi);
+      ptx::tmem_st_32x32b_x16(tq + kQPart + c * 16, mid);
+      ptx::tmem_st_32x32b_x16(tq + 2 * kQPart + c * 16, lo);
     }
     ptx::tmem_st_wait();
     ptx::tcgen05_fence_before_thread_sync();
-    ptx::fence_proxy_async_smem();
     ptx::mbar_arrive(&bars->q_ready);
   }
 
@@ -185,87 +196,86 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
         ptx::mbar_arrive_expect_tx(&bars->kv_full[slot], Sh::kUnitBytes);
         const bool is_v = idx == total - 1 || (idx >= 2 && (idx & 1) == 0);
         const int step = idx == 0 ? 0 : idx == total - 1 ? n - 1 : is_v ? (idx >> 1) - 1 : (idx + 1) >> 1;
-        uint8_t* dst = ring + slot * Sh::kUnitBytes;
-        if (is_v) {
-          ptx::tma_load_3d(dst, &tmap_v_hi, &bars->kv_full[slot], step * kBKV, 0, kvh);
-          ptx::tma_load_3d(dst + Sh::kUnitPlane, &tmap_v_lo, &bars->kv_full[slot], step * kBKV, 0, kvh);
-        } else {
+        uint8_t* dst = smem + slot * Sh::kUnitBytes;
+        const CUtensorMap* map = is_v ? &tmap_v : &tmap_k;
 #pragma unroll
-          for (int c = 0; c < D / 32; ++c) {
-            ptx::tma_load_3d(dst + c * (kBKV * 128), &tmap_k_hi, &bars->kv_full[slot], c * 32, step * kBKV, kvh);
-            ptx::tma_load_3d(dst + Sh::kUnitPlane + c * (kBKV * 128), &tmap_k_lo, &bars->kv_full[slot], c * 32, step * kBKV, kvh);
-          }
-        }
+        for (int part = 0; part < 3; ++part)
+#pragma unroll
+          for (int c = 0; c < Sh::kGroups; ++c)
+            ptx::tma_load_3d(dst + part * Sh::kPart + c * Sh::kGroupBytes, map, &bars->kv_full[slot], c * Sh::kGroup, step * kBKV, part * all_kv + kvh);
       }
     }
   } else if (warp == 9 || warp == 10) {
     // ------------------------------ MMA issuers --------------------------------
     ptx::setmaxnreg_dec<kRegsOther>();
-    constexpr uint64_t kmajor = ptx::make_smem_desc_base(16, 1024);
-    constexpr uint32_t k_hi32 = static_cast<uint32_t>(kmajor >> 32), k_lo32 = static_cast<uint32_t>(kmajor);
-    auto desc = [](uint32_t lo) -> uint64_t { return (static_cast<uint64_t>(k_hi32) << 32) | lo; };
-    const uint32_t ring_lo = k_lo32 | (ptx::smem_u32(ring) >> 4);
+    constexpr uint64_t swizzle = Sh::kRow == 128 ? ptx::kSwizzle128B : ptx::kSwizzle64B;
+    constexpr uint64_t k_base = ptx::make_smem_desc_base(16, 8 * Sh::kRow, swizzle);
+    constexpr uint64_t v_base = ptx::make_smem_desc_base(Sh::kGroupBytes, 8 * Sh::kRow, swizzle);
     auto wait_kv = [&](int idx) -> bool {
       const bool r = ptx::mbar_wait_relaxed(&bars->kv_full[idx % kRing], (idx / kRing) & 1u, abort_flag, status, 72);
       return __all_sync(0xffffffffu, r);
     };
+    auto desc = [](uint64_t base, uint32_t lo) -> uint64_t { return (base & 0xffffffff00000000ull) | lo; };
+    const uint32_t ring16 = ptx::smem_u32(smem) >> 4;
+    constexpr uint32_t kPart16 = Sh::kPart >> 4;
     bool ok = true;
     if (warp == 9) {
-      constexpr uint32_t idesc = gemm_tf32_tc::make_idesc_tf32(kBQ, kBKV);
-      const uint32_t q_lo32 = k_lo32 | (ptx::smem_u32(smem) >> 4);
+      constexpr uint32_t idesc = ptx::make_idesc_f16(kBQ, kBKV, false, false, true);
       ok = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->q_ready, 0, abort_flag, status, 73));
-      ptx::tcgen05_fence_after_thread_sync();
-      volatile uint32_t* pv_steps = &bars->pv_steps;
       for (int j = 0; j < n && ok; ++j) {
-        // not before the P V of step j - 2 is queued: the tensor core would take this product first
-        if (j >= 2 && !(ok = __all_sync(0xffffffffu, ptx::wait_counter_ge(pv_steps, static_cast<uint32_t>(j - 1), abort_flag, status, 74)))) break;
+        const int b = j & 1;
         if (!(ok = wait_kv(k_pos(j)))) break;
-        if (j >= 2 && !(ok = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&bars->s_free[j & 1], ((j - 2) >> 1) & 1u, abort_flag, status, 75)))) break;
+        // the product of step j - 2 has read the probabilities in this buffer
+        if (j >= 2 && !(ok = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&bars->buf_free[b], ((j - 2) >> 1) & 1u, abort_flag, status, 74)))) break;
         ptx::tcgen05_fence_after_thread_sync();
-        const uint32_t d = tmem + kTmemS + (j & 1) * kBKV;
-        const uint32_t b_hi = ring_lo + (k_pos(j) % kRing) * (Sh::kUnitBytes >> 4), b_lo = b_hi + (Sh::kUnitPlane >> 4);
+        const uint32_t d = tmem + kTmemS + b * kBuffer, a = tmem + kTmemQ;
+        const uint32_t k_lo = static_cast<uint32_t>(k_base) | (ring16 + (k_pos(j) % kRing) * (Sh::kUnitBytes >> 4));
         if (ptx::elect_one_sync()) {
-          // the small products first, then the large ones: the accumulator is rounded toward zero at every product, and
-          // what that costs grows with what it holds
+          auto products = [&](int x, int y, bool first) {
 #pragma unroll
-          for (int kk = 0; kk < D / 8; ++kk) {
-            const uint32_t a_off = (kk >> 2) * ((kBQ * 128) >> 4) + (kk & 3) * 2, b_off = (kk >> 2) * ((kBKV * 128) >> 4) + (kk & 3) * 2;
-            gemm_tf32_tc::tcgen05_mma_tf32_ss(d, desc(q_lo32 + a_off), desc(b_hi + b_off), idesc, kk != 0 ? 1u : 0u);
-            mma_tf32_ts(d, tmem + kTmemQ + kk * 8, desc(b_lo + b_off), idesc, 1u);
-          }
-#pragma unroll
-          for (int kk = 0; kk < D / 8; ++kk) {
-            const uint32_t b_off = (kk >> 2) * ((kBKV * 128) >> 4) + (kk & 3) * 2;
-            mma_tf32_ts(d, tmem + kTmemQ + kk * 8, desc(b_hi + b_off), idesc, 1u);
-          }
-          ptx::tcgen05_commit(&bars->s_full[j & 1]);
+            for (int kk = 0; kk < D / 16; ++kk) {
+              constexpr int kPerGroup = Sh::kGroup / 16;
+              const uint32_t off = y * kPart16 + (kk / kPerGroup) * (Sh::kGroupBytes >> 4) + (kk % kPerGroup) * 2;
+              ptx::tcgen05_mma_f16_ts(d, a + x * kQPart + kk * 8, desc(k_base, k_lo + off), idesc, first && kk == 0 ? 0u : 1u);
+            }
+          };
+          // the small products first: the accumulator cuts every term off at its own last place
+          products(2, 0, true);
+          products(0, 2, false);
+          products(1, 1, false);
+          products(1, 0, false);
+          products(0, 1, false);
+          products(0, 0, false);
+          ptx::tcgen05_commit(&bars->s_full[b]);
           ptx::tcgen05_commit(&bars->kv_empty[k_pos(j) % kRing]);
         }
         __syncwarp();
       }
     } else {
-      constexpr uint32_t idesc = gemm_tf32_tc::make_idesc_tf32(kBQ, D);
+      constexpr uint32_t idesc = ptx::make_idesc_f16(kBQ, D, false, true, true);
       for (int j = 0; j < n && ok; ++j) {
-        const int c = j / kChunkSteps, acc = c & 1;
-        const bool first = j % kChunkSteps == 0, last = j % kChunkSteps == kChunkSteps - 1 || j == n - 1;
+        const int b = j & 1;
         if (!(ok = wait_kv(v_pos(j)))) break;
-        if (first && c >= 2 && !(ok = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&bars->o_empty[acc], ((c - 2) >> 1) & 1u, abort_flag, status, 76)))) break;
-        if (!(ok = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->p_ready, j & 1u, abort_flag, status, 77)))) break;
+        if (j >= 1 && !(ok = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&bars->o_empty, (j - 1) & 1u, abort_flag, status, 76)))) break;
+        if (!(ok = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->p_ready[b], (j >> 1) & 1u, abort_flag, status, 77)))) break;
         ptx::tcgen05_fence_after_thread_sync();
-        const uint32_t d = tmem + kTmemO + acc * 128;
-        const uint32_t a_hi = tmem + kTmemP, a_lo = a_hi + kBKV;
-        const uint32_t b_hi = ring_lo + (v_pos(j) % kRing) * (Sh::kUnitBytes >> 4), b_lo = b_hi + (Sh::kUnitPlane >> 4);
+        const uint32_t d = tmem + kTmemO, a = tmem + kTmemS + b * kBuffer;
+        const uint32_t v_lo = static_cast<uint32_t>(v_base) | (ring16 + (v_pos(j) % kRing) * (Sh::kUnitBytes >> 4));
         if (ptx::elect_one_sync()) {
+          auto products = [&](int x, int y, bool first) {
 #pragma unroll
-          for (int kk = 0; kk < kBKV / 8; ++kk) {
-            mma_tf32_ts(d, a_lo + kk * 8, desc(b_hi + kk * 2), idesc, (first && kk == 0) ? 0u : 1u);
-            mma_tf32_ts(d, a_hi + kk * 8, desc(b_lo + kk * 2), idesc, 1u);
-            mma_tf32_ts(d, a_hi + kk * 8, desc(b_hi + kk * 2), idesc, 1u);
-          }
-          ptx::tcgen05_commit(&bars->pv_done);
+            for (int kk = 0; kk < kBKV / 16; ++kk)
+              ptx::tcgen05_mma_f16_ts(d, a + x * kPPart + kk * 8, desc(v_base, v_lo + y * kPart16 + kk * (16 * Sh::kRow >> 4)), idesc, first && kk == 0 ? 0u : 1u);
+          };
+          products(2, 0, true);
+          products(0, 2, false);
+          products(1, 1, false);
+          products(1, 0, false);
+          products(0, 1, false);
+          products(0, 0, false);
+          ptx::tcgen05_commit(&bars->buf_free[b]);
+          ptx::tcgen05_commit(&bars->o_full);
           ptx::tcgen05_commit(&bars->kv_empty[v_pos(j) % kRing]);
-          if (last) ptx::tcgen05_commit(&bars->o_full[acc]);
-          *const_cast<volatile uint32_t*>(&bars->pv_steps) = static_cast<uint32_t>(j + 1);
         }
         __syncwarp();
       }
@@ -284,95 +294,69 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
     bool alive = true;
     for (int j = 0; j < n; ++j) {
       const int b = j & 1;
+      const uint32_t ts = lane_base + kTmemS + b * kBuffer;
       if (!__all_sync(0xffffffffu, ptx::mbar_wait(&bars->s_full[b], (j >> 1) & 1u, abort_flag, status, 78))) {
         alive = false;
         break;
       }
       ptx::tcgen05_fence_after_thread_sync();
-      uint32_t v[32];
-      ptx::tmem_ld_32x32b_x32(lane_base + kTmemS + b * kBKV, v);
+      uint32_t v[2][32];
+      ptx::tmem_ld_32x32b_x32(ts, v[0]);
+      ptx::tmem_ld_32x32b_x32(ts + 32, v[1]);
       ptx::tmem_ld_wait();
-      ptx::tcgen05_fence_before_thread_sync();
-      ptx::mbar_arrive(&bars->s_free[b]);
       const int key0 = j * kBKV;
       if (key0 + kBKV - 1 > limit) {
 #pragma unroll
-        for (int i = 0; i < 32; ++i)
-          if (key0 + i > limit) v[i] = 0xff800000u;  // -inf
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (key0 + h * 32 + i > limit) v[h][i] = 0xff800000u;  // -inf
       }
       float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-      for (int i = 0; i < 32; i += 2)
-        mx4[(i >> 1) & 3] = ptx::fmax3(mx4[(i >> 1) & 3], __uint_as_float(v[i]), __uint_as_float(v[i + 1]));
+      for (int i = 0; i < 64; i += 2)
+        mx4[(i >> 1) & 3] = ptx::fmax3(mx4[(i >> 1) & 3], __uint_as_float(v[i >> 5][i & 31]), __uint_as_float(v[i >> 5][(i & 31) + 1]));
       const float m_new = fmaxf(m_used, fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])));
-      const bool chunk_start = j % kChunkSteps == 0;
-      if (chunk_start) {
-        // nothing of this chunk is in tensor memory yet; the drain warps rescale their sums
-        if (m_new != m_used) {
-          l *= ptx::ex2_approx((m_used - m_new) * sl2);  // l = 0 while m_used = -inf
-          m_used = m_new;
-        }
-      } else if (__any_sync(0xffffffffu, (m_new - m_used) * sl2 > kRescaleThreshold)) {
-        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done, (j - 1) & 1u, abort_flag, status, 79))) {
-          alive = false;
-          break;
-        }
-        ptx::tcgen05_fence_after_thread_sync();
-        const bool need = (m_new - m_used) * sl2 > kRescaleThreshold;
-        const float alpha = need ? ptx::ex2_approx((m_used - m_new) * sl2) : 1.0f;
-        if (need) m_used = m_new;
-        l *= alpha;
-        const uint32_t to = lane_base + kTmemO + ((j / kChunkSteps) & 1) * 128;
-#pragma unroll 1
-        for (int c = 0; c < D / 32; ++c) {
-          uint32_t ov[32];
-          ptx::tmem_ld_32x32b_x32(to + c * 32, ov);
-          ptx::tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) ov[i] = __float_as_uint(__uint_as_float(ov[i]) * alpha);
-          ptx::tmem_st_32x32b_x32(to + c * 32, ov);
-        }
-        ptx::tmem_st_wait();
-        ptx::tcgen05_fence_before_thread_sync();
+      // nothing of this step is in tensor memory yet; the drain warps rescale their sums
+      if (m_new != m_used) {
+        l *= ptx::ex2_approx((m_used - m_new) * sl2);  // l = 0 while m_used = -inf
+        m_used = m_new;
       }
       // a row that has seen nothing but -inf so far: probabilities 0, not NaN
       const float nms = m_used == -INFINITY ? 0.f : -m_used * sl2;
-      uint32_t hi[32], lo[32];
-      float ls[4] = {0.f, 0.f, 0.f, 0.f};
+      const ptx::f32x2_t sl2x2 = ptx::pack_f32x2(sl2, sl2), nmsx2 = ptx::pack_f32x2(nms, nms);
+      ptx::f32x2_t ls[2] = {0ull, 0ull};
+      // The parts of the probabilities take the place of the scores.
 #pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        const float e = ptx::ex2_approx(fmaf(__uint_as_float(v[i]), sl2, nms));
-        ls[i & 3] += e;
-        const float h = tf32_rn(e);
-        hi[i] = __float_as_uint(h);
-        lo[i] = __float_as_uint(e - h);  // exact; the tensor core reads its top 11 bits
+      for (int h = 0; h < 2; ++h) {
+        uint32_t hi[16], mid[16], lo[16], unused = 0;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          float t0, t1;
+          ptx::unpack_f32x2(ptx::fma_f32x2(ptx::pack_f32x2(__uint_as_float(v[h][2 * i]), __uint_as_float(v[h][2 * i + 1])), sl2x2, nmsx2), t0, t1);
+          const float e0 = ptx::ex2_approx(t0), e1 = ptx::ex2_approx(t1);
+          ls[i & 1] = ptx::add_f32x2(ls[i & 1], ptx::pack_f32x2(e0, e1));
+          gemm_f32_fused::split2(e0, e1, hi[i], mid[i], lo[i], unused);
+        }
+        ptx::tmem_st_32x32b_x16(ts + h * 16, hi);
+        ptx::tmem_st_32x32b_x16(ts + kPPart + h * 16, mid);
+        ptx::tmem_st_32x32b_x16(ts + 2 * kPPart + h * 16, lo);
       }
-      l += (ls[0] + ls[1]) + (ls[2] + ls[3]);
-      // P of step j - 1 has been read
-      if (j >= 1 && !__all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done, (j - 1) & 1u, abort_flag, status, 80))) {
-        alive = false;
-        break;
-      }
-      __syncwarp();
-      ptx::tcgen05_fence_after_thread_sync();
-      const uint32_t tp = lane_base + kTmemP;
-      ptx::tmem_st_32x32b_x32(tp, hi);
-      ptx::tmem_st_32x32b_x32(tp + kBKV, lo);
+      float l4[4];
+      ptx::unpack_f32x2(ls[0], l4[0], l4[1]);
+      ptx::unpack_f32x2(ls[1], l4[2], l4[3]);
+      l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
       ptx::tmem_st_wait();
       ptx::tcgen05_fence_before_thread_sync();
-      ptx::mbar_arrive(&bars->p_ready);
-      if (j % kChunkSteps == kChunkSteps - 1 || j == n - 1) {
-        // slot c % 3: the wait above says that P V of step j - 1 was issued, which (accumulators alternate) says that
-        // the drain warps are done with chunk c - 3
-        const int c3 = (j / kChunkSteps) % 3;
-        row_slot[c3 * kBQ + r] = m_used;
-        ptx::mbar_arrive(&bars->m_ready[c3]);
-      }
+      ptx::mbar_arrive(&bars->p_ready[b]);
+      // slot j % 3: the scores of step j were issued after the product of step j - 2 had retired, which was issued after step j - 3 was drained
+      row_slot[j % 3 * kBQ + r] = m_used;
+      ptx::mbar_arrive(&bars->m_ready[j % 3]);
     }
-    // the row sum takes the slot after the last chunk's, once the last product has retired: by then the chunk that had it
-    // (chunks - 3) is drained
-    if (alive && __all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done, (n - 1) & 1u, abort_flag, status, 81))) {
-      row_slot[(chunks % 3) * kBQ + r] = l;
+    // the row sum takes the slot after the last step's, once the last product has retired: by then step n - 3, which had it, is drained
+    // (the product of step n - 1 was issued after step n - 2 was)
+    if (alive && __all_sync(0xffffffffu, ptx::mbar_wait(&bars->buf_free[(n - 1) & 1], ((n - 1) >> 1) & 1u, abort_flag, status, 79))) {
+      row_slot[n % 3 * kBQ + r] = l;
       ptx::mbar_arrive(&bars->l_ready);
     }
   } else {
@@ -380,38 +364,37 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k_hi, const __g
     ptx::setmaxnreg_inc<kRegsDrain>();
     const int quad = warp & 3;
     const int r = quad * 32 + lane;
-    const uint32_t lane_base = tmem + (static_cast<uint32_t>(quad * 32) << 16);
+    const uint32_t to = tmem + (static_cast<uint32_t>(quad * 32) << 16) + kTmemO;
     const float sl2 = p.scale * 1.4426950408889634f;
     float sum[D];
 #pragma unroll
     for (int i = 0; i < D; ++i) sum[i] = 0.f;
     float m_prev = -INFINITY;
     bool alive = true;
-    for (int c = 0; c < chunks; ++c) {
-      const int acc = c & 1;
-      bool ready = ptx::mbar_wait(&bars->m_ready[c % 3], (c / 3) & 1u, abort_flag, status, 82);
-      ready = ready && ptx::mbar_wait(&bars->o_full[acc], (c >> 1) & 1u, abort_flag, status, 83);
+    for (int j = 0; j < n; ++j) {
+      bool ready = ptx::mbar_wait(&bars->m_ready[j % 3], (j / 3) & 1u, abort_flag, status, 80);
+      ready = ready && ptx::mbar_wait(&bars->o_full, j & 1u, abort_flag, status, 81);
       if (!__all_sync(0xffffffffu, ready)) {
         alive = false;
         break;
       }
       ptx::tcgen05_fence_after_thread_sync();
-      const float m_c = row_slot[(c % 3) * kBQ + r];
-      const float alpha = m_c == m_prev ? 1.0f : ptx::ex2_approx((m_prev - m_c) * sl2);  // 0 before the first chunk
-      m_prev = m_c;
+      const float m_j = row_slot[j % 3 * kBQ + r];
+      const float alpha = m_j == m_prev ? 1.0f : ptx::ex2_approx((m_prev - m_j) * sl2);  // 0 before the first step
+      m_prev = m_j;
 #pragma unroll
       for (int cc = 0; cc < D / 32; ++cc) {
         uint32_t ov[32];
-        ptx::tmem_ld_32x32b_x32(lane_base + kTmemO + acc * 128 + cc * 32, ov);
+        ptx::tmem_ld_32x32b_x32(to + cc * 32, ov);
         ptx::tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 32; ++i) sum[cc * 32 + i] = fmaf(sum[cc * 32 + i], alpha, __uint_as_float(ov[i]));
       }
       ptx::tcgen05_fence_before_thread_sync();
-      ptx::mbar_arrive(&bars->o_empty[acc]);
+      ptx::mbar_arrive(&bars->o_empty);
     }
-    if (alive && __all_sync(0xffffffffu, ptx::mbar_wait(&bars->l_ready, 0, abort_flag, status, 84))) {
-      const float inv = 1.0f / row_slot[(chunks % 3) * kBQ + r];
+    if (alive && __all_sync(0xffffffffu, ptx::mbar_wait(&bars->l_ready, 0, abort_flag, status, 82))) {
+      const float inv = 1.0f / row_slot[n % 3 * kBQ + r];
       if (q0 + r < p.seq) {
         float4* orow = reinterpret_cast<float4*>(o + bh * p.o_head_stride + (q0 + r) * p.o_row_stride);
 #pragma unroll

@@ -245,8 +245,8 @@ struct TmapSlot {
   bool used = false;
 };
 
-// dims (x contiguous, y, z), strides in elements of `elem_bytes`, box (box_x, box_y, 1), 128-byte swizzle,
-// out-of-range elements read as zero.
+// dims (x contiguous, y, z), strides in elements of `elem_bytes`, box (box_x, box_y, 1), 128-byte swizzle (64-byte where a row of the
+// box has 64 bytes), out-of-range elements read as zero.
 inline int32_t make_tmap_3d(std::string* err, CUtensorMap* out, const void* base, uint64_t dim_x, uint64_t dim_y,
                             uint64_t dim_z, uint64_t stride_y, uint64_t stride_z, uint32_t box_x, uint32_t box_y,
                             CUtensorMapDataType dtype, uint32_t elem_bytes) {
@@ -275,7 +275,8 @@ inline int32_t make_tmap_3d(std::string* err, CUtensorMap* out, const void* base
   if ((strides[0] & 15u) || (strides[1] & 15u) || !aligned16(base))
     return op_fail(err, TSM100_ERR_INVALID, "tensor map needs a 16-byte aligned base and 16-byte-multiple strides");
   CUresult r = fn(out, dtype, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                  box_x * elem_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     char buf[96];
     snprintf(buf, sizeof buf, "cuTensorMapEncodeTiled failed: CUresult %d", static_cast<int>(r));
@@ -1167,34 +1168,30 @@ inline int32_t attention_tf32x3_launch(std::string* err, const attn_simt::Params
   }
 }
 
-// f32 on the tcgen05 kernel: one launch writes the hi / lo planes of K and of V transposed into stream-ordered scratch.
-// kv_row 0 of every (batch, KV head) is kv_head_stride elements after the one before.
+// f32 on the tcgen05 kernel: one launch writes the parts of K and of V into stream-ordered scratch.  Row 0 of every (batch, KV head) is
+// kv_head_stride elements after the one before.
 template <int D>
 inline int32_t attention_f32_tc_launch_d(std::string* err, const attn_simt::Params& p, const float* q, const float* k,
                                          const float* v, float* o, uint32_t* status, cudaStream_t s) {
   namespace at = attn_f32_tc;
-  namespace g = gemm_tf32_tc;
+  using Sh = at::Shape<D>;
   int sms = 0;
   int32_t st = sm_count(err, &sms);
   if (st != TSM100_OK) return st;
-  cudaError_t e = cudaSuccess;
-  const uint64_t n_kv = static_cast<uint64_t>(p.batch) * p.heads_kv, len = p.seq_kv, len4 = (len + 3) / 4 * 4;
-  const size_t k_plane = n_kv * len * D, v_plane = n_kv * len4 * D;
-  float* ws = nullptr;
+  const uint64_t n_kv = static_cast<uint64_t>(p.batch) * p.heads_kv, len = p.seq_kv;
+  const size_t plane = n_kv * len * D;
+  uint16_t* ws = nullptr;
   {
-    const int32_t got = take_scratch(err, reinterpret_cast<void**>(&ws), 2 * (k_plane + v_plane) * sizeof(float), s);
+    const int32_t got = take_scratch(err, reinterpret_cast<void**>(&ws), 6 * plane * sizeof(uint16_t), s);
     if (got != TSM100_OK) return got;
   }
-  float *k_hi = ws, *k_lo = ws + k_plane, *v_hi = ws + 2 * k_plane, *v_lo = v_hi + v_plane;
-  st = split_operands_launch(err, {k, k_hi, k_lo, D, p.kv_head_stride, static_cast<int64_t>(len), D, D, 0},
-                             {v, v_hi, v_lo, D, p.kv_head_stride, D, static_cast<int32_t>(len), static_cast<int32_t>(len4), 0}, true,
-                             static_cast<int32_t>(n_kv), sms, s);
-  CUtensorMap tk_hi, tk_lo, tv_hi, tv_lo;
-  const CUtensorMapDataType f32 = CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
-  if (st == TSM100_OK) st = make_tmap_3d(err, &tk_hi, k_hi, D, len, n_kv, D, len * D, 32, at::kBKV, f32, 4);
-  if (st == TSM100_OK) st = make_tmap_3d(err, &tk_lo, k_lo, D, len, n_kv, D, len * D, 32, at::kBKV, f32, 4);
-  if (st == TSM100_OK) st = make_tmap_3d(err, &tv_hi, v_hi, len, D, n_kv, len4, len4 * D, at::kBKV, D, f32, 4);
-  if (st == TSM100_OK) st = make_tmap_3d(err, &tv_lo, v_lo, len, D, n_kv, len4, len4 * D, at::kBKV, D, f32, 4);
+  at::SplitParams sp = {{k, v}, {ws, ws + 3 * plane}, p.kv_head_stride, static_cast<int64_t>(len * D / 8)};
+  const int64_t per_head = std::max<int64_t>(1, std::min<int64_t>((sp.head_vecs + 255) / 256, 4ll * sms / static_cast<int64_t>(n_kv)));
+  cudaError_t e = launch_chained(at::split_kv_kernel, dim3(static_cast<unsigned>(per_head), static_cast<unsigned>(n_kv), 2), 256, 0, s, 0, sp);
+  st = cuda_ok(err, e, "split_kv_kernel launch");
+  CUtensorMap tk, tv;
+  if (st == TSM100_OK) st = make_tmap_16bit_3d(err, &tk, ws, D, len, 3 * n_kv, D, len * D, Sh::kGroup, at::kBKV, true);
+  if (st == TSM100_OK) st = make_tmap_16bit_3d(err, &tv, ws + 3 * plane, D, len, 3 * n_kv, D, len * D, Sh::kGroup, at::kBKV, true);
   if (st == TSM100_OK) {
     auto kern = at::attention_f32_tc_kernel<D>;
     e = set_dyn_smem_once(kern, at::smem_bytes<D>());
@@ -1203,9 +1200,7 @@ inline int32_t attention_f32_tc_launch_d(std::string* err, const attn_simt::Para
       pp.a = p;
       pp.status = status;
       const int64_t grid = static_cast<int64_t>((p.seq + at::kBQ - 1) / at::kBQ) * p.batch * p.heads_q;
-      // not chained: it fills every SM by itself, and 16 heads of 4096 took 0.7 % longer that way
-      kern<<<static_cast<unsigned>(grid), at::kThreads, at::smem_bytes<D>(), s>>>(tk_hi, tk_lo, tv_hi, tv_lo, q, o, pp);
-      e = cudaGetLastError();
+      e = launch_chained(kern, static_cast<unsigned>(grid), at::kThreads, at::smem_bytes<D>(), s, 0, tk, tv, q, o, pp);
     }
     st = cuda_ok(err, e, "attention_f32_tc_kernel launch");
   }
@@ -1224,13 +1219,11 @@ inline int32_t attention_f32_tc_launch(std::string* err, const attn_simt::Params
     default: return attention_f32_tc_launch_d<32>(err, p, qf, kf, vf, of, status, s);
   }
 }
-// The problems that attention_tf32x3_ok takes, with enough work to pay for the split passes and a kernel's start: 16 heads of
-// 4096 x 128, causal, 1446 us on the warp-level kernel, 406 here; 4 heads of 256 x 128 44 / 30; 2 heads of 512 x 64 43 / 27.
-// Error against the 64-bit result 8.6e-6 / 9e-7 at 4096 keys (the warp-level kernel accumulates all keys in one go).
+// Of the problems that attention_tf32x3_ok takes, those for the tcgen05 kernel.
 inline bool attention_f32_tc_ok(const attn_simt::Params& p, const uint32_t* status) {
   const int64_t blocks = static_cast<int64_t>((p.seq + 127) / 128) * p.batch * p.heads_q;
   const int64_t n_kv = static_cast<int64_t>(p.batch) * p.heads_kv;
-  return status != nullptr && p.seq >= 64 && p.seq_kv >= 256 && blocks <= 0x7fffffff && n_kv <= 65535 && p.seq_kv <= 1 << 20;
+  return status != nullptr && route::attention_f32_on_tcgen05(p.head_dim, p.seq_kv) && blocks <= 0x7fffffff && n_kv <= 65535 && p.seq_kv <= 1 << 20;
 }
 
 template <typename T>

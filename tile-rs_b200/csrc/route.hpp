@@ -22,6 +22,13 @@ inline bool attention_narrow_on_tcgen05(int32_t head_dim, int64_t seq_kv, int64_
   return seq_kv > (query_blocks > sms ? 128 : 448);
 }
 
+// f32 attention: the tcgen05 kernel (attention_f32_tc.cuh, 128 query rows and 64 keys at a time, behind a launch that splits K and V), or the
+// warp-level one (128 rows, 64 keys).  A step of 64 keys takes the one 1.9 us and the other 3 (heads of 32) to 11 us, the second launch 3.5 us of a
+// call in a row and 1.5 as graph replays.  Calls in a row, causal, warp level / tcgen05: 2 heads of 16 x 128 11.6 / 10.3, of 64 x 128 13.2 / 10.5, of 200
+// x 128 40.9 / 14.6, 128 heads of 128 x 128 25.9 / 19.2; heads of 96 16 of 64 11.0 / 10.4, of 128 19.8 / 12.3; of 64 16 of 64 7.9 / 10.4, of 65 12.6 /
+// 10.4, 128 of 128 13.8 / 12.1; of 32 16 of 128 8.1 / 10.4, of 200 12.9 / 10.6, 128 of 200 24.8 / 16.1.
+inline bool attention_f32_on_tcgen05(int32_t head_dim, int64_t seq_kv) { return head_dim == 128 || seq_kv > (head_dim == 32 ? 160 : 64); }
+
 // 16-bit attention on tcgen05: how many CTAs share the KV steps of a query block.  One CTA fills an SM, so the steps are dealt out when
 // there are blocks for at most half of the SMs, 2048 keys or more to each, 1024 from 8192 keys on, where the merge of more records is
 // short beside the steps saved.  512 tokens on 15872, 32 heads (64 blocks): 212 unsplit, 122 split; the whole step of 30 tokens on 9000, 4 heads,
