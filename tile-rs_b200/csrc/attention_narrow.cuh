@@ -81,14 +81,15 @@ attention_narrow_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
   const int n_kv_all = (seq_kv + kBKV - 1) / kBKV;
   // number of KV steps each tile needs (causal: up to and including the step of its last row's own position)
   const int n_a_all = p.causal ? min(n_kv_all, (q0 + kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
-  const int n_b_all = p.causal ? min(n_kv_all, (q0 + 2 * kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
+  const bool lone = q0 + kBQ >= p.seq;  // no tile B, as in attention_tc.cuh
+  const int n_b_all = lone ? n_a_all : p.causal ? min(n_kv_all, (q0 + 2 * kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
   // kSplit: this CTA's range [j0, j0 + n_b) of them, possibly empty
   const int per_rank = kSplit ? (n_b_all + splits - 1) / splits : n_b_all;
   const int j0 = kSplit ? min(rank * per_rank, n_b_all) : 0;
   const int n_b = kSplit ? min(per_rank, n_b_all - j0) : n_b_all;
   const int n_a = kSplit ? max(0, min(n_a_all - j0, n_b)) : n_a_all;
-  // the place of step j of tile g among the jobs: A_0, B_0, A_1, B_1, ... and B alone once A has no step any more
-  auto job = [&](int g, int j) { return j < n_a ? 2 * j + g : n_a + j; };
+  // the place of step j of tile g among the jobs: A_0, B_0, A_1, B_1, ... and one tile alone once the other has no step any more
+  auto job = [&](int g, int j) { return lone ? j : j < n_a ? 2 * j + g : n_a + j; };
 
   if (threadIdx.x == 0) {
     ptx::mbar_init(&bars->q_full, 1);
@@ -159,7 +160,7 @@ attention_narrow_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         const uint32_t b_lo = ring_lo + (k_pos(j) % kRing) * (kTileBytes >> 4);
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
-          if (g == 0 && j >= n_a) continue;
+          if (g == 0 ? j >= n_a : lone) continue;
           const int q = job(g, j), buf = q % kBuffers, use = q / kBuffers;
           // the product of the job that had this buffer has read it
           if (use > 0) ok = __all_sync(0xffffffffu, ptx::mbar_wait_relaxed(&bars->buf_free[buf], (use - 1) & 1u, abort_flag, p.status, 104));
@@ -171,7 +172,7 @@ attention_narrow_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
               ptx::tcgen05_mma_f16_ss(tmem_base + buf * 128, desc(k_hi, q_lo + g * (kTileBytes >> 4) + kk * 2), desc(k_hi, b_lo + kk * 2), idesc,
                                       kk != 0 ? 1u : 0u);
             ptx::tcgen05_commit(&bars->s_full[buf]);
-            if (g == 1) ptx::tcgen05_commit(&bars->kv_empty[k_pos(j) % kRing]);  // last reader of K_j
+            if (g == 1 || lone) ptx::tcgen05_commit(&bars->kv_empty[k_pos(j) % kRing]);  // last reader of K_j
           }
           __syncwarp();
         }
@@ -185,7 +186,7 @@ attention_narrow_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
         const uint32_t b_lo = ring_lo + (v_pos(j) % kRing) * (kTileBytes >> 4);
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
-          if (g == 0 && j >= n_a) continue;
+          if (g == 0 ? j >= n_a : lone) continue;
           const int q = job(g, j), buf = q % kBuffers;
           ok = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->p_ready[buf], (q / kBuffers) & 1u, abort_flag, p.status, 105));
           if (!ok) break;
@@ -200,7 +201,7 @@ attention_narrow_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
             }
             ptx::tcgen05_commit(&bars->buf_free[buf]);
             ptx::tcgen05_commit(&bars->pv_done[g][j & 1]);
-            if (g == 1) ptx::tcgen05_commit(&bars->kv_empty[v_pos(j) % kRing]);  // last reader of V_j
+            if (g == 1 || lone) ptx::tcgen05_commit(&bars->kv_empty[v_pos(j) % kRing]);  // last reader of V_j
           }
           __syncwarp();
         }
@@ -214,7 +215,7 @@ attention_narrow_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
     const int g = warp >> 2;                // 0: tile A, 1: tile B
     const int quad = warp & 3;              // tensor-memory lanes this warp may touch
     const int r = quad * 32 + lane;         // row inside the tile == lane
-    const int n_g = g == 0 ? n_a : n_b;
+    const int n_g = g == 0 ? n_a : lone ? 0 : n_b;
     const int qrow = q0 + g * kBQ + r;
     const int limit = p.causal ? min(qrow + q_off, seq_kv - 1) : (seq_kv - 1);  // last visible column
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
@@ -326,7 +327,9 @@ attention_narrow_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
       ptx::mbar_arrive(&bars->p_ready[buf]);
     }
 
-    if constexpr (kSplit) {
+    if (kSplit && g == 1 && lone) {
+      // nobody reads the records of rows that do not exist
+    } else if constexpr (kSplit) {
       bool have = alive && n_g > 0;  // a range may be empty for this tile: weight 0, O zero
       if (have) have = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done[g][(n_g - 1) & 1], ((n_g - 1) >> 1) & 1u, abort_flag, p.status, 110 + g));
       ptx::tcgen05_fence_after_thread_sync();

@@ -170,7 +170,10 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   const int n_kv_all = (seq_kv + kBKV - 1) / kBKV;
   // number of KV steps each tile needs (causal: up to and including the step of its last row's own position)
   const int n_a_all = p.causal ? min(n_kv_all, (q0 + kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
-  const int n_b_all = p.causal ? min(n_kv_all, (q0 + 2 * kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
+  // A block of 128 rows or fewer (a short prompt, the end of a sequence) has no tile B, whose products and exponentials would slow tile A down:
+  // 2060 cycles a step instead of 3240.  Rotation, appends and attention of 30 tokens on 3000, 4 heads, 49.9 -> 39.0 us, of 100 on 12000, 32 heads, 65.4 -> 51.7.
+  const bool lone = q0 + kBQ >= p.seq;
+  const int n_b_all = lone ? n_a_all : p.causal ? min(n_kv_all, (q0 + 2 * kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
   // kSplit: this CTA's range [j0, j0 + n_b) of them, possibly empty
   const int per_rank = kSplit ? (n_b_all + splits - 1) / splits : n_b_all;
   const int j0 = kSplit ? min(rank * per_rank, n_b_all) : 0;
@@ -309,8 +312,11 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             if (j > 0 && !(ok = wait_s_free(0, j - 1))) break;
             issue_qk(0, k_pos(j));
           }
-          if (j > 0 && !(ok = wait_s_free(1, j - 1))) break;
-          issue_qk(1, k_pos(j));  // last reader of K_j
+          if (!lone) {
+            if (j > 0 && !(ok = wait_s_free(1, j - 1))) break;
+            issue_qk(1, k_pos(j));
+          }
+          // the last reader of K_j has been issued
           if (ptx::elect_one_sync()) ptx::tcgen05_commit(&bars->kv_empty[k_pos(j) % kRing]);
         }
       } else {
@@ -345,8 +351,11 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             if (!(ok = wait_p(0, j))) break;
             issue_pv(0, v_pos(j), j > 0);
           }
-          if (!(ok = wait_p(1, j))) break;
-          issue_pv(1, v_pos(j), j > 0);  // last reader of V_j
+          if (!lone) {
+            if (!(ok = wait_p(1, j))) break;
+            issue_pv(1, v_pos(j), j > 0);
+          }
+          // the last reader of V_j has been issued
           if (ptx::elect_one_sync()) {
             ptx::tcgen05_commit(&bars->kv_empty[v_pos(j) % kRing]);
             *const_cast<volatile uint32_t*>(&bars->pv_steps) = static_cast<uint32_t>(j + 1);
@@ -362,7 +371,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     const int g = warp >> 2;          // 0: tile A, 1: tile B
     const int quad = warp & 3;              // TMEM lanes this warp may touch
     const int r = quad * 32 + lane;         // row inside the tile == TMEM lane
-    const int n_g = g == 0 ? n_a : n_b;
+    const int n_g = g == 0 ? n_a : lone ? 0 : n_b;
     const int qrow = q0 + g * kBQ + r;
     const int limit = p.causal ? min(qrow + q_off, seq_kv - 1) : (seq_kv - 1);  // last visible column
     const uint32_t lane_base = static_cast<uint32_t>(quad * 32) << 16;
@@ -496,7 +505,9 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       ptx::mbar_arrive(&bars->p_ready[g]);
     }
 
-    if constexpr (kSplit) {
+    if (kSplit && g == 1 && lone) {
+      // nobody reads the records of rows that do not exist
+    } else if constexpr (kSplit) {
       bool have = alive && n_g > 0;  // a range may be empty for this tile: weight 0, O zero
       if (have) have = __all_sync(0xffffffffu, ptx::mbar_wait(&bars->pv_done[g], (n_g - 1) & 1u, abort_flag, p.status, 20 + g));
       ptx::tcgen05_fence_after_thread_sync();
