@@ -30,6 +30,7 @@ extern "C" int early(long long b_bytes, long long ctas, int sms) { return skinny
 extern "C" int row_per_warp(long long span, long long rows, int sms) { return softmax_row_per_warp(span, rows, sms); }
 extern "C" int cluster(long long span, long long rows, int sms) { return softmax_cluster(span, rows, sms); }
 extern "C" int splits(long long blocks, long long keys, int sms) { return attention_splits(blocks, keys, sms); }
+extern "C" int block_rows(long long rows, long long heads, long long keys, long long offset, int causal, int sms) { return attention_block_rows(rows, heads, keys, offset, causal != 0, sms); }
 extern "C" int attention_f32(int d, long long keys) { return attention_f32_on_tcgen05(d, keys); }
 extern "C" int rope_heads(long long blocks, int heads, int sms) { return rope_heads_per_thread(blocks, heads, sms); }
 extern "C" int twice_skip(long long vectors, int threads) { return softmax_twice_skip(vectors, threads, 4); }
@@ -213,3 +214,11 @@ def test_f32_shares_of_k(lib, m, n, k, aligned, splits):
 @pytest.mark.parametrize("d,keys,tc", [(128, 1, True), (96, 64, False), (96, 65, True), (64, 64, False), (64, 65, True), (32, 160, False), (32, 161, True)])
 def test_f32_attention(lib, d, keys, tc):
     assert lib.attention_f32(d, C.c_longlong(keys)) == tc
+
+
+# query rows of a block: one tile where all blocks of 128 rows find an SM, or the longest chain of a causal call is what counts
+@pytest.mark.parametrize("rows,heads,keys,offset,causal,want", [
+    (1, 1, 1, 0, 1, 128), (128, 1000, 128, 0, 1, 128), (129, 1, 129, 0, 1, 128), (256, 74, 256, 0, 0, 128), (256, 75, 256, 0, 0, 256), (838, 16, 838, 0, 1, 128),
+    (512, 32, 4000, 3488, 1, 128), (2048, 12, 2048, 0, 1, 128), (4096, 256, 4096, 0, 1, 256), (300, 64, 300, 0, 0, 256), (2777, 8, 2777, 0, 0, 256), (1430, 16, 8206, 6776, 1, 256), (2482, 8, 2482, 0, 1, 128), (938, 32, 938, 0, 1, 256), (0x7fffffff, 1, 0x7fffffff, 0, 1, 256)])
+def test_attention_block_rows(lib, rows, heads, keys, offset, causal, want):
+    assert lib.block_rows(C.c_longlong(rows), C.c_longlong(heads), C.c_longlong(keys), C.c_longlong(offset), causal, SMS) == want

@@ -1296,11 +1296,11 @@ struct AttentionFwd {
   }
 };
 
-// Launches the tcgen05 attention kernel over `blocks` query blocks that see at most `keys` keys, the KV steps of a block dealt to
+// Launches the tcgen05 attention kernel over the rows of `heads` heads that see at most `keys` keys, the KV steps of a block dealt to
 // several CTAs and merged by a second kernel where route.hpp says so.
 template <bool kBf16, bool kCache, int D>
 inline int32_t attention_fwd_launch(std::string* err, const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, void* o,
-                                    attn::Params p, int64_t blocks, int64_t keys, cudaStream_t s) {
+                                    attn::Params p, int64_t heads, int64_t keys, cudaStream_t s) {
   namespace at = attn;
   constexpr int smem = AttentionFwd<kBf16, kCache, D, false>::smem();
   static_assert(attn_narrow::kThreads == at::kThreads, "one launch for both");
@@ -1308,8 +1308,13 @@ inline int32_t attention_fwd_launch(std::string* err, const CUtensorMap& tq, con
   int32_t st = sm_count(err, &sms);
   if (st != TSM100_OK) return st;
   uint16_t* out = static_cast<uint16_t*>(o);
+  p.block_rows = 2 * at::kBQ;
+  p.splits = route::attention_splits(route::div_up(p.seq, 2 * at::kBQ) * heads, keys, sms);
+  if (p.splits == 1) p.block_rows = route::attention_block_rows(p.seq, heads, keys, p.q_offset, p.causal != 0, sms);
+  p.q_blocks = static_cast<int32_t>(route::div_up(p.seq, p.block_rows));
+  const int64_t blocks = p.q_blocks * heads;
+  if (blocks > 0x7fffffff) return op_fail(err, TSM100_ERR_INVALID, "attention: too many tiles for one launch");
   p.blocks = static_cast<int32_t>(blocks);
-  p.splits = route::attention_splits(blocks, keys, sms);
   p.part = nullptr;
   p.part_ml = nullptr;
   const size_t rows = static_cast<size_t>(blocks) * p.splits * (2 * at::kBQ);
@@ -1371,7 +1376,6 @@ inline int32_t attention_prefill_tc_launch(std::string* err, const tsm100_attent
   p.heads_kv = d->heads_kv;
   p.batch = 1;
   p.causal = 1;
-  p.q_blocks = (d->seq_len + 2 * at::kBQ - 1) / (2 * at::kBQ);
   p.kv_band = attention_kv_band(kv_len, d->heads_kv, d_row);
   p.scale_log2 = static_cast<float>((1.0 / std::sqrt(static_cast<double>(d->head_dim))) * 1.4426950408889634);
   p.status = status;
@@ -1380,9 +1384,7 @@ inline int32_t attention_prefill_tc_launch(std::string* err, const tsm100_attent
   p.o_row_stride = static_cast<int64_t>(hq * d_row);
   p.o_head_stride = static_cast<int64_t>(d_row);
   p.head_dim = d->head_dim;
-  const int64_t grid = static_cast<int64_t>(p.q_blocks) * d->heads_q;
-  if (grid > 0x7fffffff) return op_fail(err, TSM100_ERR_INVALID, "attention_prefill: too many tiles for one launch");
-  return attention_fwd_launch<kBf16, true, D>(err, tq, tk, tv, o, p, grid, static_cast<int64_t>(kv_len), s);
+  return attention_fwd_launch<kBf16, true, D>(err, tq, tk, tv, o, p, d->heads_q, static_cast<int64_t>(kv_len), s);
 }
 
 inline int32_t attention_prefill(std::string* err, const tsm100_attention_prefill_desc* d, const void* q, const void* k,
@@ -1661,7 +1663,6 @@ inline int32_t attention_tc_launch(std::string* err, const tsm100_attention_desc
   p.heads_kv = d->heads_kv;
   p.batch = d->batch;
   p.causal = d->causal ? 1 : 0;
-  p.q_blocks = (d->seq + 2 * at::kBQ - 1) / (2 * at::kBQ);
   p.kv_band = attention_kv_band(S, static_cast<int64_t>(nkv), d_row);
   p.scale_log2 = static_cast<float>((1.0 / std::sqrt(static_cast<double>(d->head_dim))) * 1.4426950408889634);
   p.status = status;
@@ -1669,9 +1670,7 @@ inline int32_t attention_tc_launch(std::string* err, const tsm100_attention_desc
   p.q_offset = 0;
   p.o_row_stride = p.o_head_stride = 0;
   p.head_dim = d->head_dim;
-  const int64_t grid = static_cast<int64_t>(p.q_blocks) * nq;
-  if (grid > 0x7fffffff) return op_fail(err, TSM100_ERR_INVALID, "attention: too many tiles for one launch");
-  return attention_fwd_launch<kBf16, false, D>(err, tq, tk, tv, o, p, grid, d->seq, s);
+  return attention_fwd_launch<kBf16, false, D>(err, tq, tk, tv, o, p, static_cast<int64_t>(nq), d->seq, s);
 }
 
 inline int32_t attention(std::string* err, const tsm100_attention_desc* d, const void* q, const void* k,

@@ -29,6 +29,31 @@ inline bool attention_narrow_on_tcgen05(int32_t head_dim, int64_t seq_kv, int64_
 // 10.4, 128 of 128 13.8 / 12.1; of 32 16 of 128 8.1 / 10.4, of 200 12.9 / 10.6, 128 of 200 24.8 / 16.1.
 inline bool attention_f32_on_tcgen05(int32_t head_dim, int64_t seq_kv) { return head_dim == 128 || seq_kv > (head_dim == 32 ? 160 : 64); }
 
+// 16-bit attention on tcgen05, unsplit: query rows of a block, 256 (two tiles) or 128.  Two tiles share K and V, and a step of both takes the SM
+// 3240 cycles, of one 2060; but blocks of one tile are twice as many, and the longest chain of steps is shorter.  `rows` per head, which see
+// `offset` keys before their own where `causal`, all `keys` otherwise; a block's start and end take 9000 cycles, once more where there is a second wave, and a
+// wave as long as its lightest block at least.
+// 256 rows / 128: causal 8 heads of 2482 37.3 / 27.7 us, 16 of 838 15.6 / 12.6, 32 of 938 18.4 / 19.8; all keys 16 of 640 13.7 / 10.8; heads of 64 8 of 764 13.9 /
+// 10.7; with rotation and appends 131 tokens on 3677, 16 heads, 62.9 / 49.1, 581 on 11, 32 heads, 26.4 / 28.1.
+inline int attention_block_rows(int64_t rows, int64_t heads, int64_t keys, int64_t offset, bool causal, int sms) {
+  if (rows <= 128) return 128;
+  if (div_up(rows, 256) * heads > 4 * sms) return 256;
+  int64_t best = 0, best_cost = INT64_MAX;
+  for (int64_t block = 256; block >= 128; block -= 128) {
+    const int64_t blocks = div_up(rows, block);
+    auto time = [&](int64_t i) {  // of the block that is i-th from the end, the heaviest first
+      const int64_t r = (blocks - 1 - i) * block, end = std::min(rows, r + block);
+      return 9000 + div_up(causal ? std::min(keys, end + offset) : keys, 128) * (end - r > 128 ? 3240 : 2060);
+    };
+    int64_t longest = 0, all = 0, waves = 0;
+    for (int64_t i = 0; i < blocks; ++i) longest = std::max(longest, time(i)), all += time(i) * heads;
+    for (int64_t done = 0; done < blocks * heads; done += sms) waves += time((std::min(blocks * heads, done + sms) - 1) / heads);  // the lightest of each
+    const int64_t cost = blocks * heads <= sms ? longest : std::max({longest, waves, all / sms + 9000});
+    if (cost < best_cost) best_cost = cost, best = block;
+  }
+  return static_cast<int>(best);
+}
+
 // 16-bit attention on tcgen05: how many CTAs share the KV steps of a query block.  One CTA fills an SM, so the steps are dealt out when
 // there are blocks for at most half of the SMs, 2048 keys or more to each, 1024 from 8192 keys on, where the merge of more records is
 // short beside the steps saved.  512 tokens on 15872, 32 heads (64 blocks): 212 unsplit, 122 split; the whole step of 30 tokens on 9000, 4 heads,
