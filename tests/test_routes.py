@@ -30,6 +30,7 @@ extern "C" int early(long long b_bytes, long long ctas, int sms) { return skinny
 extern "C" int row_per_warp(long long span, long long rows, int sms) { return softmax_row_per_warp(span, rows, sms); }
 extern "C" int cluster(long long span, long long rows, int sms) { return softmax_cluster(span, rows, sms); }
 extern "C" int splits(long long blocks, long long keys, int sms) { return attention_splits(blocks, keys, sms); }
+extern "C" int boxes(long long k, long long tiles, int sms) { return gemm16_pairs_store_boxes(k, tiles, sms); }
 extern "C" int block_rows(long long rows, long long heads, long long keys, long long offset, int causal, int sms) { return attention_block_rows(rows, heads, keys, offset, causal != 0, sms); }
 extern "C" int attention_f32(int d, long long keys) { return attention_f32_on_tcgen05(d, keys); }
 extern "C" int rope_heads(long long blocks, int heads, int sms) { return rope_heads_per_thread(blocks, heads, sms); }
@@ -222,3 +223,8 @@ def test_f32_attention(lib, d, keys, tc):
     (512, 32, 4000, 3488, 1, 128), (2048, 12, 2048, 0, 1, 128), (4096, 256, 4096, 0, 1, 256), (300, 64, 300, 0, 0, 256), (2777, 8, 2777, 0, 0, 256), (1430, 16, 8206, 6776, 1, 256), (2482, 8, 2482, 0, 1, 128), (938, 32, 938, 0, 1, 256), (0x7fffffff, 1, 0x7fffffff, 0, 1, 256)])
 def test_attention_block_rows(lib, rows, heads, keys, offset, causal, want):
     assert lib.block_rows(C.c_longlong(rows), C.c_longlong(heads), C.c_longlong(keys), C.c_longlong(offset), causal, SMS) == want
+
+
+@pytest.mark.parametrize("k,tiles,want", [(8, 100000, True), (2047, 1024, True), (2048, 148, True), (2048, 149, False), (4096, 64, True), (4097, 64, False), (8192, 1024, False)])
+def test_results_of_pairs_in_boxes(lib, k, tiles, want):
+    assert lib.boxes(C.c_longlong(k), C.c_longlong(tiles), SMS) == want

@@ -1033,8 +1033,8 @@ Kernel lower(const Func& f) {
              << ">(const float*, const float*, float*, const tsm100::gemm_tf32x3::Params);\n";
       else if (tma)
         inst << "template __global__ void tsm100::gemm_tc::gemm_tc_kernel<" << cxx_type(out_dt) << ", " << (bt ? "true" : "false")
-             << ", " << (a.dtype == Dt::BF16 ? "true" : "false") << ">(const __grid_constant__ CUtensorMap, const __grid_constant__ CUtensorMap, " << cxx_type(out_dt)
-             << "*, const tsm100::gemm_tc::Params);\n";
+             << ", " << (a.dtype == Dt::BF16 ? "true" : "false") << ">(const __grid_constant__ CUtensorMap, const __grid_constant__ CUtensorMap, "
+             << "const __grid_constant__ CUtensorMap, const tsm100::gemm_tc::Params);\n";
       else
         inst << "template __global__ void tsm100::gemm_simt::gemm_simt_kernel<" << cxx_type(a.dtype) << ", " << cxx_type(out_dt)
              << ", 64, 64, 16, 4, 4>(const " << cxx_type(a.dtype) << "*, const " << cxx_type(a.dtype) << "*, " << cxx_type(out_dt)

@@ -19,7 +19,7 @@
 //               tensor memory; two accumulators (512 columns) alternate so the
 //               next tile's main loop overlaps this tile's epilogue.
 //   warps 2..5  epilogue: tcgen05.ld the accumulator (each warp its 32 TMEM
-//               lanes), narrow, 16-byte global stores.
+//               lanes), narrow, store_rows below.
 // B in its row-major [K,N] form is consumed as an MN-major operand, so no
 // transpose pass over B is ever made.
 //
@@ -51,13 +51,16 @@ struct alignas(8) Barriers {
   uint32_t tmem_base;
   uint32_t abort_flag;
 };
-constexpr int kSmemBytes = kStages * kStageBytes + sizeof(Barriers) + 1024;  // + alignment slack
+// C leaves through shared memory: two boxes of 32 rows x 128 bytes for each epilogue warp.
+constexpr int kBoxBytes = 32 * 128;
+constexpr int kStagingBytes = 4 * 2 * kBoxBytes;
+constexpr int kBarsOff = kStages * kStageBytes + kStagingBytes;
+constexpr int kSmemBytes = kBarsOff + sizeof(Barriers) + 1024;  // + alignment slack
+static_assert(kSmemBytes <= 227 * 1024, "shared memory budget of one CTA");
 
 struct Params {
   int32_t m, n, k, batch;
   int32_t m_blocks, n_blocks;
-  int64_t c_batch_stride;  // elements
-  int64_t ldc;             // row pitch of C in elements
   uint32_t* status;
 };
 
@@ -75,58 +78,52 @@ __device__ __forceinline__ void tile_coords(const Params& p, int tile, int& b, i
 }
 
 template <typename OutT>
-__device__ __forceinline__ void store_row_chunk(OutT* dst, const uint32_t (&acc)[32], int valid);
-
+__device__ __forceinline__ uint32_t narrow2(uint32_t lo, uint32_t hi);
 template <>
-__device__ __forceinline__ void store_row_chunk<float>(float* dst, const uint32_t (&acc)[32], int valid) {
-  if (valid >= 32) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-      reinterpret_cast<uint4*>(dst)[i] = make_uint4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
-  } else {
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-      if (i < valid) dst[i] = __uint_as_float(acc[i]);
-  }
+__device__ __forceinline__ uint32_t narrow2<__nv_bfloat16>(uint32_t lo, uint32_t hi) { return ptx::pack_bf16x2(__uint_as_float(lo), __uint_as_float(hi)); }
+template <>
+__device__ __forceinline__ uint32_t narrow2<__half>(uint32_t lo, uint32_t hi) {
+  const __half2 h = __floats2half2_rn(__uint_as_float(lo), __uint_as_float(hi));
+  return *reinterpret_cast<const uint32_t*>(&h);
 }
+template <typename OutT>
+constexpr int kBoxCols = 128 / static_cast<int>(sizeof(OutT));
 
-template <>
-__device__ __forceinline__ void store_row_chunk<__nv_bfloat16>(__nv_bfloat16* dst, const uint32_t (&acc)[32],
-                                                              int valid) {
-  if (valid >= 32) {
+// One warp's 32 rows x kBN columns of an accumulator (`tmem`: its lanes, first column) to C[b], first element (row0, col0): box by box through two
+// swizzled buffers of shared memory and TMA stores, which leave out what lies past C.  Stores from the lanes that hold the rows touch 32
+// of them with 16 bytes each, and such an epilogue of 128 x 256 took 6 us, longer than the products of K = 1000: 2897 x 4024 x 320 22.4 us, 5848 x
+// 1592 x 552 22.5, 2868 x 2848 x 944 of a batch of 4 76 us.  The caller's lane 0 has to wait for the stores before the CTA ends.
+template <typename OutT>
+__device__ __forceinline__ void store_rows(const CUtensorMap* tmap_c, uint32_t tmem, uint8_t* staging, int row0, int col0, int m, int n, int b, int lane) {
+  constexpr int kCols = kBoxCols<OutT>;
+#pragma unroll 1
+  for (int c = 0; c < kBN / kCols; ++c) {
+    if (col0 + c * kCols >= n) break;
+    uint32_t v[kCols / 32][32];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      uint4 v;
-      v.x = ptx::pack_bf16x2(__uint_as_float(acc[8 * i + 0]), __uint_as_float(acc[8 * i + 1]));
-      v.y = ptx::pack_bf16x2(__uint_as_float(acc[8 * i + 2]), __uint_as_float(acc[8 * i + 3]));
-      v.z = ptx::pack_bf16x2(__uint_as_float(acc[8 * i + 4]), __uint_as_float(acc[8 * i + 5]));
-      v.w = ptx::pack_bf16x2(__uint_as_float(acc[8 * i + 6]), __uint_as_float(acc[8 * i + 7]));
-      reinterpret_cast<uint4*>(dst)[i] = v;
-    }
-  } else {
+    for (int h = 0; h < kCols / 32; ++h) ptx::tmem_ld_32x32b_x32(tmem + c * kCols + h * 32, v[h]);
+    ptx::tmem_ld_wait();
+    uint8_t* box = staging + (c & 1) * kBoxBytes;
+    if (lane == 0) ptx::tma_store_wait_read<1>();  // the store before last has read its buffer
+    __syncwarp();
+    const uint32_t row = ptx::smem_u32(box) + lane * 128;
 #pragma unroll
-    for (int i = 0; i < 32; ++i)
-      if (i < valid) dst[i] = __float2bfloat16_rn(__uint_as_float(acc[i]));
-  }
-}
-
-template <>
-__device__ __forceinline__ void store_row_chunk<__half>(__half* dst, const uint32_t (&acc)[32], int valid) {
-  if (valid >= 32) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      uint32_t w[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        __half2 h = __floats2half2_rn(__uint_as_float(acc[8 * i + 2 * j]), __uint_as_float(acc[8 * i + 2 * j + 1]));
-        w[j] = *reinterpret_cast<uint32_t*>(&h);
+    for (int u = 0; u < 8; ++u) {
+      const uint32_t at = row + ((u ^ (lane & 7)) << 4);
+      if constexpr (sizeof(OutT) == 4) {
+        ptx::st_shared_v4(at, v[0][4 * u], v[0][4 * u + 1], v[0][4 * u + 2], v[0][4 * u + 3]);
+      } else {
+        const uint32_t(&w)[32] = v[u >> 2];
+        const int i = (u & 3) * 8;
+        ptx::st_shared_v4(at, narrow2<OutT>(w[i], w[i + 1]), narrow2<OutT>(w[i + 2], w[i + 3]), narrow2<OutT>(w[i + 4], w[i + 5]), narrow2<OutT>(w[i + 6], w[i + 7]));
       }
-      reinterpret_cast<uint4*>(dst)[i] = make_uint4(w[0], w[1], w[2], w[3]);
     }
-  } else {
-#pragma unroll
-    for (int i = 0; i < 32; ++i)
-      if (i < valid) dst[i] = __float2half_rn(__uint_as_float(acc[i]));
+    ptx::fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0 && row0 < m) {
+      ptx::tma_store_3d(tmap_c, box, col0 + c * kCols, row0, b);
+      ptx::tma_store_commit();
+    }
   }
 }
 
@@ -135,13 +132,13 @@ __device__ __forceinline__ void store_row_chunk<__half>(__half* dst, const uint3
 template <typename OutT, bool kBTransposed, bool kIsBf16>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-               OutT* __restrict__ c, const Params p) {
+               const __grid_constant__ CUtensorMap tmap_c, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   // 128-byte-swizzled tiles need 1024-byte alignment.
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + kStages * kABytes;
-  Barriers* bars = reinterpret_cast<Barriers*>(smem + kStages * kStageBytes);
+  Barriers* bars = reinterpret_cast<Barriers*>(smem + kBarsOff);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -251,6 +248,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
   } else {
     // ------------------------------ epilogue ----------------------------------
     const int quad = warp & 3;  // TMEM lanes [32*quad, 32*quad+32) belong to this warp
+    uint8_t* staging = smem + kStages * kStageBytes + (warp - 2) * 2 * kBoxBytes;
     int local = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++local) {
       const int acc = local & 1;
@@ -261,20 +259,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       const bool ready = ptx::mbar_wait(&bars->acc_full[acc], acc_phase, abort_flag, p.status, 4);
       if (!__all_sync(0xffffffffu, ready)) break;
       ptx::tcgen05_fence_after_thread_sync();
-      const int row = mb * kBM + quad * 32 + lane;
-      OutT* crow = c + static_cast<int64_t>(b) * p.c_batch_stride + static_cast<int64_t>(row) * p.ldc;
-#pragma unroll 1
-      for (int cc = 0; cc < kBN / 32; ++cc) {
-        uint32_t v[32];
-        ptx::tmem_ld_32x32b_x32(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * kBN + cc * 32, v);
-        ptx::tmem_ld_wait();
-        const int col = nb * kBN + cc * 32;
-        if (row < p.m && col < p.n) store_row_chunk<OutT>(crow + col, v, p.n - col);
-      }
+      store_rows<OutT>(&tmap_c, tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * kBN, staging, mb * kBM + quad * 32, nb * kBN, p.m, p.n, b, lane);
       ptx::tcgen05_fence_before_thread_sync();
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&bars->acc_empty[acc]);
     }
+    if (lane == 0) ptx::tma_store_wait_all<0>();
   }
 
   // ------------------------------ teardown ------------------------------------

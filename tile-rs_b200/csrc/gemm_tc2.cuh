@@ -44,11 +44,17 @@ struct alignas(8) Barriers {
   uint32_t tmem_base;
   uint32_t abort_flag;
 };
-constexpr int kSmemBytes = kStages * kStageBytes + sizeof(Barriers) + 1024;
+constexpr int kBarsOff = kStages * kStageBytes + gemm_tc::kStagingBytes;
+constexpr int kSmemBytes = kBarsOff + sizeof(Barriers) + 1024;
+static_assert(kSmemBytes <= 227 * 1024 && kBN == gemm_tc::kBN, "shared memory budget of one CTA; store_rows stores the width of a tile");
 
-using gemm_tc::Params;  // m_blocks / n_blocks count 256 x 256 pair tiles here
+struct Params {
+  gemm_tc::Params g;       // m_blocks / n_blocks count 256 x 256 pair tiles
+  int64_t c_batch_stride;  // elements
+  int64_t ldc;             // row pitch of C in elements
+};
 
-__device__ __forceinline__ void tile_coords(const Params& p, int tile, int& b, int& mb, int& nb) {
+__device__ __forceinline__ void tile_coords(const gemm_tc::Params& p, int tile, int& b, int& mb, int& nb) {
   const int per_batch = p.m_blocks * p.n_blocks;
   b = tile / per_batch;
   int t = tile - b * per_batch;
@@ -61,15 +67,73 @@ __device__ __forceinline__ void tile_coords(const Params& p, int tile, int& b, i
   nb = t / rows_in_band;
 }
 
-template <typename OutT, bool kBTransposed, bool kIsBf16>
+template <typename OutT>
+__device__ __forceinline__ void store_row_chunk(OutT* dst, const uint32_t (&acc)[32], int valid);
+
+template <>
+__device__ __forceinline__ void store_row_chunk<float>(float* dst, const uint32_t (&acc)[32], int valid) {
+  if (valid >= 32) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      reinterpret_cast<uint4*>(dst)[i] = make_uint4(acc[4 * i], acc[4 * i + 1], acc[4 * i + 2], acc[4 * i + 3]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (i < valid) dst[i] = __uint_as_float(acc[i]);
+  }
+}
+
+template <>
+__device__ __forceinline__ void store_row_chunk<__nv_bfloat16>(__nv_bfloat16* dst, const uint32_t (&acc)[32],
+                                                              int valid) {
+  if (valid >= 32) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      uint4 v;
+      v.x = ptx::pack_bf16x2(__uint_as_float(acc[8 * i + 0]), __uint_as_float(acc[8 * i + 1]));
+      v.y = ptx::pack_bf16x2(__uint_as_float(acc[8 * i + 2]), __uint_as_float(acc[8 * i + 3]));
+      v.z = ptx::pack_bf16x2(__uint_as_float(acc[8 * i + 4]), __uint_as_float(acc[8 * i + 5]));
+      v.w = ptx::pack_bf16x2(__uint_as_float(acc[8 * i + 6]), __uint_as_float(acc[8 * i + 7]));
+      reinterpret_cast<uint4*>(dst)[i] = v;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (i < valid) dst[i] = __float2bfloat16_rn(__uint_as_float(acc[i]));
+  }
+}
+
+template <>
+__device__ __forceinline__ void store_row_chunk<__half>(__half* dst, const uint32_t (&acc)[32], int valid) {
+  if (valid >= 32) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      uint32_t w[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        __half2 h = __floats2half2_rn(__uint_as_float(acc[8 * i + 2 * j]), __uint_as_float(acc[8 * i + 2 * j + 1]));
+        w[j] = *reinterpret_cast<uint32_t*>(&h);
+      }
+      reinterpret_cast<uint4*>(dst)[i] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i)
+      if (i < valid) dst[i] = __float2half_rn(__uint_as_float(acc[i]));
+  }
+}
+
+// kBoxes: C leaves through shared memory (gemm_tc.cuh: store_rows), not from the lanes that hold its rows (route.hpp: gemm16_pairs_store_boxes).
+template <typename OutT, bool kBTransposed, bool kIsBf16, bool kBoxes>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                OutT* __restrict__ c, const Params p) {
+                const __grid_constant__ CUtensorMap tmap_c, OutT* __restrict__ c, const Params params) {
+  const gemm_tc::Params& p = params.g;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_a = smem;
   uint8_t* smem_b = smem + kStages * kABytes;
-  Barriers* bars = reinterpret_cast<Barriers*>(smem + kStages * kStageBytes);
+  Barriers* bars = reinterpret_cast<Barriers*>(smem + kBarsOff);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -200,20 +264,27 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       const bool ready = ptx::mbar_wait(&bars->acc_full[acc], acc_phase, abort_flag, p.status, 34);
       if (!__all_sync(0xffffffffu, ready)) break;
       ptx::tcgen05_fence_after_thread_sync();
-      const int row = mb * kPairM + static_cast<int>(rank) * kCtaM + quad * 32 + lane;
-      OutT* crow = c + static_cast<int64_t>(b) * p.c_batch_stride + static_cast<int64_t>(row) * p.ldc;
+      const uint32_t from = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * kBN;
+      const int row0 = mb * kPairM + static_cast<int>(rank) * kCtaM + quad * 32;
+      if constexpr (kBoxes) {
+        uint8_t* staging = smem + kStages * kStageBytes + (warp - 2) * 2 * gemm_tc::kBoxBytes;
+        gemm_tc::store_rows<OutT>(&tmap_c, from, staging, row0, nb * kBN, p.m, p.n, b, lane);
+      } else {
+        OutT* crow = c + static_cast<int64_t>(b) * params.c_batch_stride + static_cast<int64_t>(row0 + lane) * params.ldc;
 #pragma unroll 1
-      for (int cc = 0; cc < kBN / 32; ++cc) {
-        uint32_t v[32];
-        ptx::tmem_ld_32x32b_x32(tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * kBN + cc * 32, v);
-        ptx::tmem_ld_wait();
-        const int col = nb * kBN + cc * 32;
-        if (row < p.m && col < p.n) gemm_tc::store_row_chunk<OutT>(crow + col, v, p.n - col);
+        for (int cc = 0; cc < kBN / 32; ++cc) {
+          uint32_t v[32];
+          ptx::tmem_ld_32x32b_x32(from + cc * 32, v);
+          ptx::tmem_ld_wait();
+          const int col = nb * kBN + cc * 32;
+          if (row0 + lane < p.m && col < p.n) store_row_chunk<OutT>(crow + col, v, p.n - col);
+        }
       }
       ptx::tcgen05_fence_before_thread_sync();
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa_shared(ptx::smem_u32(&bars->acc_empty[acc]), 0));
     }
+    if (kBoxes && lane == 0) ptx::tma_store_wait_all<0>();
   }
 
   // ------------------------------ teardown ------------------------------------

@@ -862,11 +862,19 @@ inline int32_t gemm_f32_fused_launch(std::string* err, const tsm100_gemm_desc* d
   return cuda_ok(err, bn == 64 ? pick(std::integral_constant<int, 64>{}) : pick(std::integral_constant<int, 128>{}), "gemm_f32_fused_kernel launch");
 }
 
+// C for TMA stores of 32 rows x 128 bytes (gemm_tc.cuh: store_rows).
+template <typename OutT>
+inline int32_t make_tmap_c(std::string* err, CUtensorMap* out, void* c, uint64_t m, uint64_t n, uint64_t batch, uint64_t ldc) {
+  const CUtensorMapDataType type = sizeof(OutT) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                   : std::is_same<OutT, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  return make_tmap_3d(err, out, c, n, m, batch, ldc, m * ldc, gemm_tc::kBoxCols<OutT>, 32, type, sizeof(OutT));
+}
+
 template <typename OutT, bool kBT, bool kBf16>
 inline int32_t gemm_tc_launch(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
                               uint32_t* status, cudaStream_t s) {
   namespace g = gemm_tc;
-  CUtensorMap ta, tb;
+  CUtensorMap ta, tb, tc;
   const uint64_t M = d->m, N = d->n, K = d->k, B = d->batch;
   const GemmPitch ld = gemm_pitch(d);
   const uint64_t lda = ld.lda, ldb = ld.ldb;
@@ -876,6 +884,7 @@ inline int32_t gemm_tc_launch(std::string* err, const tsm100_gemm_desc* d, const
     st = make_tmap_16bit_3d(err, &tb, b, K, N, B, ldb, N * ldb, g::kBK, g::kBN, kBf16);
   else
     st = make_tmap_16bit_3d(err, &tb, b, N, K, B, ldb, K * ldb, 64, g::kBK, kBf16);
+  if (st == TSM100_OK) st = make_tmap_c<OutT>(err, &tc, c, M, N, B, ld.ldc);
   if (st != TSM100_OK) return st;
   g::Params p;
   p.m = static_cast<int32_t>(M);
@@ -884,8 +893,6 @@ inline int32_t gemm_tc_launch(std::string* err, const tsm100_gemm_desc* d, const
   p.batch = d->batch;
   p.m_blocks = static_cast<int32_t>((M + g::kBM - 1) / g::kBM);
   p.n_blocks = static_cast<int32_t>((N + g::kBN - 1) / g::kBN);
-  p.c_batch_stride = static_cast<int64_t>(M) * ld.ldc;
-  p.ldc = ld.ldc;
   p.status = status;
   int sms = 0;
   st = sm_count(err, &sms);
@@ -895,7 +902,7 @@ inline int32_t gemm_tc_launch(std::string* err, const tsm100_gemm_desc* d, const
   cudaError_t e = set_dyn_smem_once(kern, g::kSmemBytes);
   if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(gemm_tc_kernel)");
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>(tiles, sms));
-  return cuda_ok(err, launch_chained(kern, grid, g::kThreads, g::kSmemBytes, s, 0, ta, tb, static_cast<OutT*>(c), p), "gemm_tc_kernel launch");
+  return cuda_ok(err, launch_chained(kern, grid, g::kThreads, g::kSmemBytes, s, 0, ta, tb, tc, p), "gemm_tc_kernel launch");
 }
 
 // Few output tiles: 128 columns x NT rows of C per CTA, K split over clusters (gemm_skinny.cuh).
@@ -955,7 +962,7 @@ template <typename OutT, bool kBT, bool kBf16>
 inline int32_t gemm_tc2_launch(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
                                uint32_t* status, cudaStream_t s) {
   namespace g = gemm_tc2;
-  CUtensorMap ta, tb;
+  CUtensorMap ta, tb, tc;
   const uint64_t M = d->m, N = d->n, K = d->k, B = d->batch;
   const GemmPitch ld = gemm_pitch(d);
   const uint64_t lda = ld.lda, ldb = ld.ldb;
@@ -965,27 +972,29 @@ inline int32_t gemm_tc2_launch(std::string* err, const tsm100_gemm_desc* d, cons
     st = make_tmap_16bit_3d(err, &tb, b, K, N, B, ldb, N * ldb, g::kBK, g::kCtaN, kBf16);
   else
     st = make_tmap_16bit_3d(err, &tb, b, N, K, B, ldb, K * ldb, 64, g::kBK, kBf16);
+  if (st == TSM100_OK) st = make_tmap_c<OutT>(err, &tc, c, M, N, B, ld.ldc);
   if (st != TSM100_OK) return st;
-  gemm_tc::Params p;
+  g::Params params;
+  gemm_tc::Params& p = params.g;
   p.m = static_cast<int32_t>(M);
   p.n = static_cast<int32_t>(N);
   p.k = static_cast<int32_t>(K);
   p.batch = d->batch;
   p.m_blocks = static_cast<int32_t>((M + g::kPairM - 1) / g::kPairM);
   p.n_blocks = static_cast<int32_t>((N + g::kBN - 1) / g::kBN);
-  p.c_batch_stride = static_cast<int64_t>(M) * ld.ldc;
-  p.ldc = ld.ldc;
   p.status = status;
-  auto kern = g::gemm_tc2_kernel<OutT, kBT, kBf16>;
-  cudaError_t e = set_dyn_smem_once(kern, g::kSmemBytes);
-  if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(gemm_tc2_kernel)");
+  params.c_batch_stride = static_cast<int64_t>(M) * ld.ldc;
+  params.ldc = ld.ldc;
   int sms = 0;
   st = sm_count(err, &sms);
   if (st != TSM100_OK) return st;
-  const int max_clusters = resident_clusters(kern, g::kThreads, g::kSmemBytes, 2, static_cast<unsigned>(sms & ~1), sms / 2);
   const int64_t tiles = static_cast<int64_t>(p.m_blocks) * p.n_blocks * p.batch;
+  auto kern = route::gemm16_pairs_store_boxes(d->k, tiles, sms) ? g::gemm_tc2_kernel<OutT, kBT, kBf16, true> : g::gemm_tc2_kernel<OutT, kBT, kBf16, false>;
+  cudaError_t e = set_dyn_smem_once(kern, g::kSmemBytes);
+  if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(gemm_tc2_kernel)");
+  const int max_clusters = resident_clusters(kern, g::kThreads, g::kSmemBytes, 2, static_cast<unsigned>(sms & ~1), sms / 2);
   const int64_t pairs = std::min<int64_t>(tiles, std::min<int64_t>(max_clusters, sms / 2));
-  e = launch_chained(kern, static_cast<unsigned>(2 * pairs), g::kThreads, g::kSmemBytes, s, 2, ta, tb, static_cast<OutT*>(c), p);
+  e = launch_chained(kern, static_cast<unsigned>(2 * pairs), g::kThreads, g::kSmemBytes, s, 2, ta, tb, tc, static_cast<OutT*>(c), params);
   return cuda_ok(err, e, "gemm_tc2_kernel launch");
 }
 

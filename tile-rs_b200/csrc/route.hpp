@@ -108,6 +108,12 @@ inline Gemm16 gemm16(int64_t m, int64_t n, int64_t k, int64_t batch, int sms) {
   return r;
 }
 
+// CTA pairs: does C leave through shared memory, in whole boxes, or from the lanes that hold its rows?  The boxes are out in a sixth of the time, which
+// counts where a tile's products take no longer than its end (K below 2048) or where the last wave's end is a part of the whole; in a
+// long row of long tiles the board's power decides, and the slower way is 1 to 5 % cheaper.  Rows / boxes: 4096 x 4096 x 512 of a batch of 2 39.6 / 30.0 us, x
+// 1024 53.7 / 51.2, x 2048 105.3 / 107.2, x 4096 198 / 203; 8192^3 803 / 833; 2048 x 2048 x 4096 (64 tiles) 26.1 / 25.6, 2048 x 4608 x 2048 (144) 28.4 / 26.2.
+inline bool gemm16_pairs_store_boxes(int64_t k, int64_t tiles, int sms) { return k < 2048 || (k <= 4096 && tiles <= sms); }
+
 // 16-bit products whose rows start anywhere: copies into padded scratch and the tensor cores (gemm_pad.cuh), or the FP32 pipe.  The
 // copies cost launches and traffic per row, column and output, whatever K is: FP32 pipe / padded 2000 x 3001 x
 // 17 20.6 / 31.7, x 33 29 / 32, x 65 46 / 33; 8001 x 10001 x 7 130 / 280, x 17 226 / 282, x 33 328 / 282 (hence the 2^26 products).  A CTA of the
