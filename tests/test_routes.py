@@ -228,3 +228,8 @@ def test_attention_block_rows(lib, rows, heads, keys, offset, causal, want):
 @pytest.mark.parametrize("k,tiles,want", [(8, 100000, True), (2047, 1024, True), (2048, 148, True), (2048, 149, False), (4096, 64, True), (4097, 64, False), (8192, 1024, False)])
 def test_results_of_pairs_in_boxes(lib, k, tiles, want):
     assert lib.boxes(C.c_longlong(k), C.c_longlong(tiles), SMS) == want
+
+
+@pytest.mark.parametrize("m,n,k,batch,pays", [(760, 144, 124, 1, True), (64, 1000, 81, 1, True), (64, 1000, 71, 1, False), (74, 304, 106, 1, False), (500, 117, 72, 1, True), (100, 5, 9001, 1, False)])
+def test_16_bit_products_of_odd_sizes_and_a_shorter_k(lib, m, n, k, batch, pays):
+    assert lib.padding_pays(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch)) == pays

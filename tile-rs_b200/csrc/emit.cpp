@@ -1034,7 +1034,7 @@ Kernel lower(const Func& f) {
       else if (tma)
         inst << "template __global__ void tsm100::gemm_tc::gemm_tc_kernel<" << cxx_type(out_dt) << ", " << (bt ? "true" : "false")
              << ", " << (a.dtype == Dt::BF16 ? "true" : "false") << ">(const __grid_constant__ CUtensorMap, const __grid_constant__ CUtensorMap, "
-             << "const __grid_constant__ CUtensorMap, const tsm100::gemm_tc::Params);\n";
+             << "const __grid_constant__ CUtensorMap, " << cxx_type(out_dt) << "*, const tsm100::gemm_tc::Params);\n";
       else
         inst << "template __global__ void tsm100::gemm_simt::gemm_simt_kernel<" << cxx_type(a.dtype) << ", " << cxx_type(out_dt)
              << ", 64, 64, 16, 4, 4>(const " << cxx_type(a.dtype) << "*, const " << cxx_type(a.dtype) << "*, " << cxx_type(out_dt)

@@ -1,8 +1,7 @@
 // Copies that bring 16-bit matrices whose rows do not start on 16-byte boundaries into a layout the tensor maps can
-// describe, and results back: a GEMM of odd sizes then runs on the tensor cores as the next larger one of multiples of 8.
-// Both directions are streams of a few bytes per product row and column (HBM / L2 bound); they pay as soon as the FP32-pipe
-// kernel, at a hundredth of the tensor cores' rate, would take longer than their launches: 2000 x 3001 x 2501 bf16 1365 us there
-// and 62 with the copies, 500 x 1001 x 999 166 / 15, 28 x 3134 x 4883 823 / 26.
+// describe: a GEMM of odd sizes then runs on the tensor cores as any other, and writes its result where it belongs.
+// A stream of a few bytes per row and column of the operands (HBM / L2 bound); it pays as soon as the FP32-pipe
+// kernel, at a hundredth of the tensor cores' rate, would take longer than a launch.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -14,57 +13,66 @@ namespace tsm100 {
 namespace gemm_pad {
 
 constexpr int kThreads = 256;
-constexpr int kUnpadRows = 8;
-// Up to how many CTAs the next kernel of the call is placed from the start: 300 x 1301 x 1203 bf16, whole call, 15.5 us with the 256 of other kernels,
-// 14.7 this way; 3 of 22 x 1923 x 1267 18.7 with 1024 for the copies in, 17.0 this way.
-constexpr uint32_t kFewCtasIn = 8192, kFewCtasOut = 1024;
+// Up to how many CTAs the next kernel of the call is placed from the start.
+constexpr uint32_t kFewCtas = 8192;
 
-// src [rows][cols] with row pitch ld (problems src_batch apart) -> dst [drows][dcols] packed, zeros beyond rows and cols.
-// dcols is a multiple of 8 and dst 16-byte aligned: one thread per eight values.  blockIdx.y = problem.
-__global__ void __launch_bounds__(kThreads)
-pad_kernel(const uint16_t* __restrict__ src, int64_t ld, int64_t src_batch, int32_t rows, int32_t cols,
-           uint4* __restrict__ dst, int32_t drows, int32_t dcols) {
-  ptx::launch_dependents_if_few(kFewCtasIn);
-  src = ptx::wait_prior_grid(src);
-  const uint16_t* s = src + blockIdx.y * src_batch;
-  const int64_t per_row = dcols / 8, total = drows * per_row;
-  uint4* d = dst + blockIdx.y * total;
-  for (int64_t i = blockIdx.x * static_cast<int64_t>(kThreads) + threadIdx.x; i < total; i += static_cast<int64_t>(gridDim.x) * kThreads) {
-    const int64_t r = i / per_row;
-    const int32_t c = static_cast<int32_t>(i - r * per_row) * 8;
-    uint32_t w[4] = {0u, 0u, 0u, 0u};
-    if (r < rows) {
-      const uint16_t* q = s + r * ld + c;
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (c + j < cols) w[j >> 1] |= static_cast<uint32_t>(q[j]) << ((j & 1) * 16);
+// src [rows][cols] with row pitch ld (problems `batch` elements apart) -> dst [rows][pitch] packed, zeros beyond cols.
+// pitch is a multiple of 8 and dst 16-byte aligned.
+struct Operand {
+  const uint16_t* src;
+  uint4* dst;
+  int64_t ld, batch;
+  int32_t rows, cols, pitch;
+  int32_t blocks;   // of the launch that work on it, 0: it is not copied
+};
+
+// Eight values from element `at` of a matrix that ends at `size`, as the two 16-byte vectors that hold them; a value at a time
+// where those reach past the matrix.
+__device__ __forceinline__ uint4 load8(const uint16_t* src, int64_t at, int64_t size, int valid) {
+  const uintptr_t address = reinterpret_cast<uintptr_t>(src + at), from = address & ~uintptr_t(15);
+  const uint32_t shift = static_cast<uint32_t>(address & 15);
+  uint32_t w[8] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+  if (valid >= 8 && from >= reinterpret_cast<uintptr_t>(src) && from + 32 <= reinterpret_cast<uintptr_t>(src + size)) {
+    const uint4 x = *reinterpret_cast<const uint4*>(from);
+    w[0] = x.x, w[1] = x.y, w[2] = x.z, w[3] = x.w;
+    if (shift != 0) {
+      const uint4 y = *reinterpret_cast<const uint4*>(from + 16);
+      w[4] = y.x, w[5] = y.y, w[6] = y.z, w[7] = y.w;
     }
-    d[i] = make_uint4(w[0], w[1], w[2], w[3]);
+    if (shift & 8) {
+#pragma unroll
+      for (int i = 0; i < 6; ++i) w[i] = w[i + 2];
+    }
+    if (shift & 4) {
+#pragma unroll
+      for (int i = 0; i < 5; ++i) w[i] = w[i + 1];
+    }
+    const uint32_t bits = (shift & 2) * 8;
+    return make_uint4(__funnelshift_r(w[0], w[1], bits), __funnelshift_r(w[1], w[2], bits), __funnelshift_r(w[2], w[3], bits), __funnelshift_r(w[3], w[4], bits));
   }
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (j < valid) w[j >> 1] |= static_cast<uint32_t>(src[at + j]) << ((j & 1) * 16);
+  return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// src [rows][scols] packed -> dst [rows][cols] with row pitch ld (problems dst_batch apart), cols <= scols.
-// One thread per column of ROWS rows, a warp's stores are contiguous and the loads of a thread in flight together: eight rows where there are
-// CTAs for all SMs (2000 x 3001 x 65 bf16, whole call, 31.5 us row by row, 24 this way), one where there are few.  grid (x, groups of rows in
-// strides, problem).
-template <int ROWS>
+// One thread per eight values of a row; the operands' blocks side by side in one launch.  blockIdx.y = problem.
 __global__ void __launch_bounds__(kThreads)
-unpad_kernel(const uint16_t* __restrict__ src, int32_t scols, uint16_t* __restrict__ dst, int64_t ld, int64_t dst_batch,
-             int32_t rows, int32_t cols) {
-  ptx::launch_dependents_if_few(kFewCtasOut);
-  src = ptx::wait_prior_grid(src);
-  const int32_t c = blockIdx.x * kThreads + threadIdx.x;
-  if (c >= cols) return;
-  const uint16_t* s = src + blockIdx.z * static_cast<int64_t>(rows) * scols + c;
-  uint16_t* d = dst + blockIdx.z * dst_batch + c;
-  for (int64_t r = static_cast<int64_t>(blockIdx.y) * ROWS; r < rows; r += static_cast<int64_t>(gridDim.y) * ROWS) {
-    uint16_t v[ROWS];
-#pragma unroll
-    for (int k = 0; k < ROWS; ++k)
-      if (r + k < rows) v[k] = s[(r + k) * scols];
-#pragma unroll
-    for (int k = 0; k < ROWS; ++k)
-      if (r + k < rows) d[(r + k) * ld] = v[k];
+pad_kernel(const Operand a, const Operand b) {
+  ptx::launch_dependents_if_few(kFewCtas);
+  const bool first = static_cast<int32_t>(blockIdx.x) < a.blocks;
+  const Operand& p = first ? a : b;
+  const int32_t block = first ? blockIdx.x : blockIdx.x - a.blocks;
+  const uint16_t* src = ptx::wait_prior_grid(p.src) + blockIdx.y * p.batch;
+  const uint32_t per_row = static_cast<uint32_t>(p.pitch) / 8;
+  const int64_t total = static_cast<int64_t>(p.rows) * per_row, step = static_cast<int64_t>(p.blocks) * kThreads;
+  const int64_t size = static_cast<int64_t>(p.rows - 1) * p.ld + p.cols;
+  uint4* dst = p.dst + blockIdx.y * total;
+#pragma unroll 2
+  for (int64_t i = static_cast<int64_t>(block) * kThreads + threadIdx.x; i < total; i += step) {
+    const int64_t r = total <= 0xffffffffll ? static_cast<int64_t>(static_cast<uint32_t>(i) / per_row) : i / per_row;
+    const int32_t c = static_cast<int32_t>(i - r * per_row) * 8;
+    dst[i] = load8(src, r * p.ld + c, size, p.cols - c);
   }
 }
 

@@ -76,7 +76,8 @@ template <>
 __device__ __forceinline__ __half narrow<__half>(float f) { return __float2half_rn(f); }
 
 // grid: ((batch * n_blocks + nb) * m_blocks + mb) * cluster size + rank; CTAs that share a tile of B are neighbours.
-template <typename OutT, bool kBTransposed, bool kIsBf16, int NT>
+// kLoose: rows of C start anywhere.
+template <typename OutT, bool kBTransposed, bool kIsBf16, int NT, bool kLoose>
 __global__ void __launch_bounds__(kThreads)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                    OutT* __restrict__ c, const Params p) {
@@ -238,9 +239,14 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_cons
       for (int q = 1; q < kMaxSplit; ++q)
         if (q < static_cast<int>(splits)) s.x += v[q].x, s.y += v[q].y, s.z += v[q].z, s.w += v[q].w;
       const int col = nb * kBN + (i % (kBN / 4)) * 4;
-      if (col < p.n) {  // N is a multiple of 4, rows of C start on 16-byte boundaries
+      if (col < p.n) {  // N is a multiple of 4 and rows of C start on 16-byte boundaries, unless loose
         OutT* dst = cb + static_cast<int64_t>(mb * NT + i / (kBN / 4)) * p.ldc + col;
-        if constexpr (sizeof(OutT) == 4) {
+        if constexpr (kLoose) {
+          const float x[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            if (col + j < p.n) dst[j] = narrow<OutT>(x[j]);
+        } else if constexpr (sizeof(OutT) == 4) {
           *reinterpret_cast<float4*>(dst) = s;
         } else {
           OutT o4[4] = {narrow<OutT>(s.x), narrow<OutT>(s.y), narrow<OutT>(s.z), narrow<OutT>(s.w)};

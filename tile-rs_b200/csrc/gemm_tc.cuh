@@ -61,6 +61,8 @@ static_assert(kSmemBytes <= 227 * 1024, "shared memory budget of one CTA");
 struct Params {
   int32_t m, n, k, batch;
   int32_t m_blocks, n_blocks;
+  int64_t c_batch_stride;  // elements
+  int64_t ldc;             // row pitch of C in elements
   uint32_t* status;
 };
 
@@ -93,18 +95,20 @@ constexpr int kBoxCols = 128 / static_cast<int>(sizeof(OutT));
 // swizzled buffers of shared memory and TMA stores, which leave out what lies past C.  Stores from the lanes that hold the rows touch 32
 // of them with 16 bytes each, and such an epilogue of 128 x 256 took 6 us, longer than the products of K = 1000: 2897 x 4024 x 320 22.4 us, 5848 x
 // 1592 x 552 22.5, 2868 x 2848 x 944 of a batch of 4 76 us.  The caller's lane 0 has to wait for the stores before the CTA ends.
-template <typename OutT>
-__device__ __forceinline__ void store_rows(const CUtensorMap* tmap_c, uint32_t tmem, uint8_t* staging, int row0, int col0, int m, int n, int b, int lane) {
+// kLoose: rows of C start anywhere; the boxes are copied to them from shared memory, a warp 32 columns of a row at a time (`c`: C[b]).
+template <typename OutT, bool kLoose>
+__device__ __forceinline__ void store_rows(const CUtensorMap* tmap_c, OutT* c, int64_t ldc, uint32_t tmem, uint8_t* staging, int row0, int col0, int m, int n, int b, int lane) {
   constexpr int kCols = kBoxCols<OutT>;
 #pragma unroll 1
-  for (int c = 0; c < kBN / kCols; ++c) {
-    if (col0 + c * kCols >= n) break;
+  for (int i0 = 0; i0 < kBN / kCols; ++i0) {
+    const int c0 = i0 * kCols;
+    if (col0 + c0 >= n) break;
     uint32_t v[kCols / 32][32];
 #pragma unroll
-    for (int h = 0; h < kCols / 32; ++h) ptx::tmem_ld_32x32b_x32(tmem + c * kCols + h * 32, v[h]);
+    for (int h = 0; h < kCols / 32; ++h) ptx::tmem_ld_32x32b_x32(tmem + c0 + h * 32, v[h]);
     ptx::tmem_ld_wait();
-    uint8_t* box = staging + (c & 1) * kBoxBytes;
-    if (lane == 0) ptx::tma_store_wait_read<1>();  // the store before last has read its buffer
+    uint8_t* box = staging + (i0 & 1) * kBoxBytes;
+    if (!kLoose && lane == 0) ptx::tma_store_wait_read<1>();  // the store before last has read its buffer
     __syncwarp();
     const uint32_t row = ptx::smem_u32(box) + lane * 128;
 #pragma unroll
@@ -118,10 +122,24 @@ __device__ __forceinline__ void store_rows(const CUtensorMap* tmap_c, uint32_t t
         ptx::st_shared_v4(at, narrow2<OutT>(w[i], w[i + 1]), narrow2<OutT>(w[i + 2], w[i + 3]), narrow2<OutT>(w[i + 4], w[i + 5]), narrow2<OutT>(w[i + 6], w[i + 7]));
       }
     }
+    if constexpr (kLoose) {
+      __syncwarp();
+      const int rows = min(32, m - row0);
+      OutT* dst = c + row0 * ldc + col0 + c0;
+#pragma unroll 4
+      for (int r = 0; r < rows; ++r, dst += ldc)
+#pragma unroll
+        for (int i = 0; i < kCols / 32; ++i) {
+          const int x = i * 32 + lane;
+          const OutT value = *reinterpret_cast<const OutT*>(box + r * 128 + (((x * static_cast<int>(sizeof(OutT)) >> 4) ^ (r & 7)) << 4) + (x * static_cast<int>(sizeof(OutT)) & 15));
+          if (col0 + c0 + x < n) dst[x] = value;
+        }
+      continue;
+    }
     ptx::fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0 && row0 < m) {
-      ptx::tma_store_3d(tmap_c, box, col0 + c * kCols, row0, b);
+      ptx::tma_store_3d(tmap_c, box, col0 + c0, row0, b);
       ptx::tma_store_commit();
     }
   }
@@ -129,10 +147,10 @@ __device__ __forceinline__ void store_rows(const CUtensorMap* tmap_c, uint32_t t
 
 // kBTransposed: B is stored [N,K] (K-major operand); otherwise [K,N] (MN-major).
 // kIsBf16: inputs are bf16 (else IEEE f16).
-template <typename OutT, bool kBTransposed, bool kIsBf16>
+template <typename OutT, bool kBTransposed, bool kIsBf16, bool kLoose = false>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-               const __grid_constant__ CUtensorMap tmap_c, const Params p) {
+               const __grid_constant__ CUtensorMap tmap_c, OutT* __restrict__ c, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   // 128-byte-swizzled tiles need 1024-byte alignment.
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -259,12 +277,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       const bool ready = ptx::mbar_wait(&bars->acc_full[acc], acc_phase, abort_flag, p.status, 4);
       if (!__all_sync(0xffffffffu, ready)) break;
       ptx::tcgen05_fence_after_thread_sync();
-      store_rows<OutT>(&tmap_c, tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * kBN, staging, mb * kBM + quad * 32, nb * kBN, p.m, p.n, b, lane);
+      store_rows<OutT, kLoose>(&tmap_c, c + b * p.c_batch_stride, p.ldc, tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * kBN, staging, mb * kBM + quad * 32, nb * kBN, p.m, p.n, b, lane);
       ptx::tcgen05_fence_before_thread_sync();
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&bars->acc_empty[acc]);
     }
-    if (lane == 0) ptx::tma_store_wait_all<0>();
+    if (!kLoose && lane == 0) ptx::tma_store_wait_all<0>();
   }
 
   // ------------------------------ teardown ------------------------------------

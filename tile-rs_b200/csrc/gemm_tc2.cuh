@@ -48,13 +48,9 @@ constexpr int kBarsOff = kStages * kStageBytes + gemm_tc::kStagingBytes;
 constexpr int kSmemBytes = kBarsOff + sizeof(Barriers) + 1024;
 static_assert(kSmemBytes <= 227 * 1024 && kBN == gemm_tc::kBN, "shared memory budget of one CTA; store_rows stores the width of a tile");
 
-struct Params {
-  gemm_tc::Params g;       // m_blocks / n_blocks count 256 x 256 pair tiles
-  int64_t c_batch_stride;  // elements
-  int64_t ldc;             // row pitch of C in elements
-};
+using gemm_tc::Params;  // m_blocks / n_blocks count 256 x 256 pair tiles here
 
-__device__ __forceinline__ void tile_coords(const gemm_tc::Params& p, int tile, int& b, int& mb, int& nb) {
+__device__ __forceinline__ void tile_coords(const Params& p, int tile, int& b, int& mb, int& nb) {
   const int per_batch = p.m_blocks * p.n_blocks;
   b = tile / per_batch;
   int t = tile - b * per_batch;
@@ -123,12 +119,13 @@ __device__ __forceinline__ void store_row_chunk<__half>(__half* dst, const uint3
   }
 }
 
-// kBoxes: C leaves through shared memory (gemm_tc.cuh: store_rows), not from the lanes that hold its rows (route.hpp: gemm16_pairs_store_boxes).
-template <typename OutT, bool kBTransposed, bool kIsBf16, bool kBoxes>
+// How C leaves: from the lanes that hold its rows, or through shared memory (route.hpp: gemm16_pairs_store_boxes; gemm_tc.cuh: store_rows), also to
+// rows that start anywhere.
+enum Store { kLanes, kBoxes, kLoose };
+template <typename OutT, bool kBTransposed, bool kIsBf16, Store kStore>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
-                const __grid_constant__ CUtensorMap tmap_c, OutT* __restrict__ c, const Params params) {
-  const gemm_tc::Params& p = params.g;
+                const __grid_constant__ CUtensorMap tmap_c, OutT* __restrict__ c, const Params p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_a = smem;
@@ -266,11 +263,11 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       ptx::tcgen05_fence_after_thread_sync();
       const uint32_t from = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * kBN;
       const int row0 = mb * kPairM + static_cast<int>(rank) * kCtaM + quad * 32;
-      if constexpr (kBoxes) {
+      if constexpr (kStore != kLanes) {
         uint8_t* staging = smem + kStages * kStageBytes + (warp - 2) * 2 * gemm_tc::kBoxBytes;
-        gemm_tc::store_rows<OutT>(&tmap_c, from, staging, row0, nb * kBN, p.m, p.n, b, lane);
+        gemm_tc::store_rows<OutT, kStore == kLoose>(&tmap_c, c + b * p.c_batch_stride, p.ldc, from, staging, row0, nb * kBN, p.m, p.n, b, lane);
       } else {
-        OutT* crow = c + static_cast<int64_t>(b) * params.c_batch_stride + static_cast<int64_t>(row0 + lane) * params.ldc;
+        OutT* crow = c + static_cast<int64_t>(b) * p.c_batch_stride + static_cast<int64_t>(row0 + lane) * p.ldc;
 #pragma unroll 1
         for (int cc = 0; cc < kBN / 32; ++cc) {
           uint32_t v[32];
@@ -284,7 +281,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa_shared(ptx::smem_u32(&bars->acc_empty[acc]), 0));
     }
-    if (kBoxes && lane == 0) ptx::tma_store_wait_all<0>();
+    if (kStore == kBoxes && lane == 0) ptx::tma_store_wait_all<0>();
   }
 
   // ------------------------------ teardown ------------------------------------

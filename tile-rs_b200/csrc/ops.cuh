@@ -870,11 +870,12 @@ inline int32_t make_tmap_c(std::string* err, CUtensorMap* out, void* c, uint64_t
   return make_tmap_3d(err, out, c, n, m, batch, ldc, m * ldc, gemm_tc::kBoxCols<OutT>, 32, type, sizeof(OutT));
 }
 
+// c_cols: 0, or N where rows of C may start anywhere.
 template <typename OutT, bool kBT, bool kBf16>
 inline int32_t gemm_tc_launch(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
-                              uint32_t* status, cudaStream_t s) {
+                              uint32_t* status, cudaStream_t s, int64_t c_cols = 0) {
   namespace g = gemm_tc;
-  CUtensorMap ta, tb, tc;
+  CUtensorMap ta, tb, tc = {};
   const uint64_t M = d->m, N = d->n, K = d->k, B = d->batch;
   const GemmPitch ld = gemm_pitch(d);
   const uint64_t lda = ld.lda, ldb = ld.ldb;
@@ -884,7 +885,7 @@ inline int32_t gemm_tc_launch(std::string* err, const tsm100_gemm_desc* d, const
     st = make_tmap_16bit_3d(err, &tb, b, K, N, B, ldb, N * ldb, g::kBK, g::kBN, kBf16);
   else
     st = make_tmap_16bit_3d(err, &tb, b, N, K, B, ldb, K * ldb, 64, g::kBK, kBf16);
-  if (st == TSM100_OK) st = make_tmap_c<OutT>(err, &tc, c, M, N, B, ld.ldc);
+  if (st == TSM100_OK && c_cols == 0) st = make_tmap_c<OutT>(err, &tc, c, M, N, B, ld.ldc);
   if (st != TSM100_OK) return st;
   g::Params p;
   p.m = static_cast<int32_t>(M);
@@ -893,23 +894,25 @@ inline int32_t gemm_tc_launch(std::string* err, const tsm100_gemm_desc* d, const
   p.batch = d->batch;
   p.m_blocks = static_cast<int32_t>((M + g::kBM - 1) / g::kBM);
   p.n_blocks = static_cast<int32_t>((N + g::kBN - 1) / g::kBN);
+  p.c_batch_stride = static_cast<int64_t>(M) * ld.ldc;
+  p.ldc = ld.ldc;
   p.status = status;
   int sms = 0;
   st = sm_count(err, &sms);
   if (st != TSM100_OK) return st;
   const int64_t tiles = static_cast<int64_t>(p.m_blocks) * p.n_blocks * p.batch;
-  auto kern = g::gemm_tc_kernel<OutT, kBT, kBf16>;
+  auto kern = c_cols ? g::gemm_tc_kernel<OutT, kBT, kBf16, true> : g::gemm_tc_kernel<OutT, kBT, kBf16>;
   cudaError_t e = set_dyn_smem_once(kern, g::kSmemBytes);
   if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(gemm_tc_kernel)");
   const unsigned grid = static_cast<unsigned>(std::min<int64_t>(tiles, sms));
-  return cuda_ok(err, launch_chained(kern, grid, g::kThreads, g::kSmemBytes, s, 0, ta, tb, tc, p), "gemm_tc_kernel launch");
+  return cuda_ok(err, launch_chained(kern, grid, g::kThreads, g::kSmemBytes, s, 0, ta, tb, tc, static_cast<OutT*>(c), p), "gemm_tc_kernel launch");
 }
 
 // Few output tiles: 128 columns x NT rows of C per CTA, K split over clusters (gemm_skinny.cuh).
 static_assert(gemm_skinny::kMaxSplit == route::kMaxGemmSplit && gemm_skinny::kBK == 64 && gemm_skinny::kBN == 128, "route.hpp plans in these units");
 template <typename OutT, bool kBT, bool kBf16, int NT>
 inline int32_t gemm_skinny_launch_nt(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
-                                     const route::Gemm16& plan, uint32_t* status, cudaStream_t s) {
+                                     const route::Gemm16& plan, uint32_t* status, cudaStream_t s, int64_t c_cols = 0) {
   namespace g = gemm_skinny;
   CUtensorMap ta, tb;
   const uint64_t M = d->m, N = d->n, K = d->k, B = d->batch;
@@ -925,6 +928,7 @@ inline int32_t gemm_skinny_launch_nt(std::string* err, const tsm100_gemm_desc* d
   g::Params p;
   p.m = static_cast<int32_t>(M);
   p.n = static_cast<int32_t>(N);
+
   p.k = static_cast<int32_t>(K);
   p.batch = d->batch;
   p.m_blocks = static_cast<int32_t>((M + NT - 1) / NT);
@@ -938,7 +942,9 @@ inline int32_t gemm_skinny_launch_nt(std::string* err, const tsm100_gemm_desc* d
   int sms = 0;
   if (const int32_t got = sm_count(err, &sms); got != TSM100_OK) return got;
   p.early = route::skinny_places_early(B * N * K * 2, tiles * splits, sms) ? 1 : 0;
-  auto kern = g::gemm_skinny_kernel<OutT, kBT, kBf16, NT>;
+  auto kern = g::gemm_skinny_kernel<OutT, kBT, kBf16, NT, false>;
+  if constexpr (sizeof(OutT) == 2)
+    if (c_cols) kern = g::gemm_skinny_kernel<OutT, kBT, kBf16, NT, true>;
   constexpr int smem = g::smem_bytes<NT>();
   cudaError_t e = set_dyn_smem_once(kern, smem);
   if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(gemm_skinny_kernel)");
@@ -948,21 +954,21 @@ inline int32_t gemm_skinny_launch_nt(std::string* err, const tsm100_gemm_desc* d
 }
 template <typename OutT, bool kBT, bool kBf16>
 inline int32_t gemm_skinny_launch(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
-                                  const route::Gemm16& plan, uint32_t* status, cudaStream_t s) {
+                                  const route::Gemm16& plan, uint32_t* status, cudaStream_t s, int64_t c_cols = 0) {
   switch (plan.rows) {
-    case 16: return gemm_skinny_launch_nt<OutT, kBT, kBf16, 16>(err, d, a, b, c, plan, status, s);
-    case 32: return gemm_skinny_launch_nt<OutT, kBT, kBf16, 32>(err, d, a, b, c, plan, status, s);
-    case 64: return gemm_skinny_launch_nt<OutT, kBT, kBf16, 64>(err, d, a, b, c, plan, status, s);
-    default: return gemm_skinny_launch_nt<OutT, kBT, kBf16, 128>(err, d, a, b, c, plan, status, s);
+    case 16: return gemm_skinny_launch_nt<OutT, kBT, kBf16, 16>(err, d, a, b, c, plan, status, s, c_cols);
+    case 32: return gemm_skinny_launch_nt<OutT, kBT, kBf16, 32>(err, d, a, b, c, plan, status, s, c_cols);
+    case 64: return gemm_skinny_launch_nt<OutT, kBT, kBf16, 64>(err, d, a, b, c, plan, status, s, c_cols);
+    default: return gemm_skinny_launch_nt<OutT, kBT, kBf16, 128>(err, d, a, b, c, plan, status, s, c_cols);
   }
 }
 
 // CTA-pair kernel (256 x 256 tile per two SMs), launched as clusters of two.
 template <typename OutT, bool kBT, bool kBf16>
 inline int32_t gemm_tc2_launch(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
-                               uint32_t* status, cudaStream_t s) {
+                               uint32_t* status, cudaStream_t s, int64_t c_cols = 0) {
   namespace g = gemm_tc2;
-  CUtensorMap ta, tb, tc;
+  CUtensorMap ta, tb, tc = {};
   const uint64_t M = d->m, N = d->n, K = d->k, B = d->batch;
   const GemmPitch ld = gemm_pitch(d);
   const uint64_t lda = ld.lda, ldb = ld.ldb;
@@ -972,10 +978,9 @@ inline int32_t gemm_tc2_launch(std::string* err, const tsm100_gemm_desc* d, cons
     st = make_tmap_16bit_3d(err, &tb, b, K, N, B, ldb, N * ldb, g::kBK, g::kCtaN, kBf16);
   else
     st = make_tmap_16bit_3d(err, &tb, b, N, K, B, ldb, K * ldb, 64, g::kBK, kBf16);
-  if (st == TSM100_OK) st = make_tmap_c<OutT>(err, &tc, c, M, N, B, ld.ldc);
+  if (st == TSM100_OK && c_cols == 0) st = make_tmap_c<OutT>(err, &tc, c, M, N, B, ld.ldc);
   if (st != TSM100_OK) return st;
-  g::Params params;
-  gemm_tc::Params& p = params.g;
+  gemm_tc::Params p;
   p.m = static_cast<int32_t>(M);
   p.n = static_cast<int32_t>(N);
   p.k = static_cast<int32_t>(K);
@@ -983,27 +988,35 @@ inline int32_t gemm_tc2_launch(std::string* err, const tsm100_gemm_desc* d, cons
   p.m_blocks = static_cast<int32_t>((M + g::kPairM - 1) / g::kPairM);
   p.n_blocks = static_cast<int32_t>((N + g::kBN - 1) / g::kBN);
   p.status = status;
-  params.c_batch_stride = static_cast<int64_t>(M) * ld.ldc;
-  params.ldc = ld.ldc;
+  p.c_batch_stride = static_cast<int64_t>(M) * ld.ldc;
+  p.ldc = ld.ldc;
   int sms = 0;
   st = sm_count(err, &sms);
   if (st != TSM100_OK) return st;
   const int64_t tiles = static_cast<int64_t>(p.m_blocks) * p.n_blocks * p.batch;
-  auto kern = route::gemm16_pairs_store_boxes(d->k, tiles, sms) ? g::gemm_tc2_kernel<OutT, kBT, kBf16, true> : g::gemm_tc2_kernel<OutT, kBT, kBf16, false>;
+  auto kern = c_cols ? g::gemm_tc2_kernel<OutT, kBT, kBf16, g::kLoose>
+              : route::gemm16_pairs_store_boxes(d->k, tiles, sms) ? g::gemm_tc2_kernel<OutT, kBT, kBf16, g::kBoxes> : g::gemm_tc2_kernel<OutT, kBT, kBf16, g::kLanes>;
   cudaError_t e = set_dyn_smem_once(kern, g::kSmemBytes);
   if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(gemm_tc2_kernel)");
   const int max_clusters = resident_clusters(kern, g::kThreads, g::kSmemBytes, 2, static_cast<unsigned>(sms & ~1), sms / 2);
   const int64_t pairs = std::min<int64_t>(tiles, std::min<int64_t>(max_clusters, sms / 2));
-  e = launch_chained(kern, static_cast<unsigned>(2 * pairs), g::kThreads, g::kSmemBytes, s, 2, ta, tb, tc, static_cast<OutT*>(c), params);
+  e = launch_chained(kern, static_cast<unsigned>(2 * pairs), g::kThreads, g::kSmemBytes, s, 2, ta, tb, tc, static_cast<OutT*>(c), p);
   return cuda_ok(err, e, "gemm_tc2_kernel launch");
 }
 
-inline int32_t gemm(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
-                    uint32_t* status, void* stream);
+template <typename OutT, bool kBT, bool kBf16>
+inline int32_t gemm_16bit_launch(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c, int sms, uint32_t* status,
+                                 cudaStream_t s, int64_t c_cols = 0) {
+  const route::Gemm16 plan = route::gemm16(d->m, d->n, d->k, d->batch, sms);
+  switch (plan.kind) {
+    case route::Gemm16::kPairs: return gemm_tc2_launch<OutT, kBT, kBf16>(err, d, a, b, c, status, s, c_cols);
+    case route::Gemm16::kSingles: return gemm_tc_launch<OutT, kBT, kBf16>(err, d, a, b, c, status, s, c_cols);
+    default: return gemm_skinny_launch<OutT, kBT, kBf16>(err, d, a, b, c, plan, status, s, c_cols);
+  }
+}
 
-// A 16-bit problem whose rows start anywhere, on the tensor cores: operands that need it are copied into zero-padded
-// scratch (N and K rounded up to 8), the padded problem is computed and the result copied out.  The padding adds products
-// of zeros only, and columns that are not copied out.
+// A 16-bit problem whose rows start anywhere, on the tensor cores: operands whose rows do not start on 16-byte boundaries are copied to scratch where
+// they do; the tensor maps end at N and K, and columns of C are written one by one.
 inline int32_t gemm_padded(std::string* err, const tsm100_gemm_desc* d, const void* a, const void* b, void* c,
                            uint32_t* status, cudaStream_t s) {
   namespace g = gemm_pad;
@@ -1012,45 +1025,39 @@ inline int32_t gemm_padded(std::string* err, const tsm100_gemm_desc* d, const vo
   if (st != TSM100_OK) return st;
   cudaError_t e = cudaSuccess;
   const GemmPitch ld = gemm_pitch(d);
-  const int64_t np = (d->n + 7) / 8 * 8, kp = (d->k + 7) / 8 * 8, batch = d->batch;
-  const int64_t b_rows = d->b_transposed ? d->n : d->k, b_cols = d->b_transposed ? d->k : d->n;
-  const int64_t bp_rows = d->b_transposed ? np : kp, bp_cols = d->b_transposed ? kp : np;
-  const bool pad_a = kp != d->k || ld.lda % 8 != 0 || !aligned16(a);
-  const bool pad_b = bp_rows != b_rows || bp_cols != b_cols || ld.ldb % 8 != 0 || !aligned16(b);
-  const bool pad_c = np != d->n || ld.ldc % 8 != 0 || !aligned16(c);
-  const int64_t a_elems = pad_a ? batch * d->m * kp : 0, b_elems = pad_b ? batch * bp_rows * bp_cols : 0;  // multiples of 8
-  const int64_t c_elems = pad_c ? batch * d->m * np : 0;
-  uint16_t* ws = nullptr;
-  {
-    const int32_t got = take_scratch(err, reinterpret_cast<void**>(&ws), static_cast<size_t>(a_elems + b_elems + c_elems) * 2, s);
-    if (got != TSM100_OK) return got;
-  }
-  auto pad = [&](const void* src, int64_t pitch, int64_t rows, int64_t cols, uint16_t* dst, int64_t drows, int64_t dcols) {
-    const int64_t items = drows * (dcols / 8);
-    const dim3 grid(static_cast<unsigned>(std::min<int64_t>((items + g::kThreads - 1) / g::kThreads, 16ll * sms)), static_cast<unsigned>(batch));
-    if (e == cudaSuccess)
-      e = launch_chained(g::pad_kernel, grid, g::kThreads, 0, s, 0, static_cast<const uint16_t*>(src), pitch, rows * pitch, static_cast<int32_t>(rows),
-                         static_cast<int32_t>(cols), reinterpret_cast<uint4*>(dst), static_cast<int32_t>(drows), static_cast<int32_t>(dcols));
-  };
+  const int64_t batch = d->batch, b_rows = d->b_transposed ? d->n : d->k, b_cols = d->b_transposed ? d->k : d->n;
+  const int64_t a_pitch = (d->k + 7) / 8 * 8, b_pitch = (b_cols + 7) / 8 * 8;
+  const bool pad_a = ld.lda % 8 != 0 || !aligned16(a), pad_b = ld.ldb % 8 != 0 || !aligned16(b);
+  const int64_t a_elems = pad_a ? batch * d->m * a_pitch : 0, b_elems = pad_b ? batch * b_rows * b_pitch : 0;  // multiples of 8
+  const int64_t c_cols = d->n % 8 != 0 || ld.ldc % 8 != 0 || !aligned16(c) ? d->n : 0;
   tsm100_gemm_desc t = *d;
-  t.n = np, t.k = kp;
+  t.ldc = ld.ldc;
   const void *ta = a, *tb = b;
-  void* tc = c;
-  if (pad_a) pad(a, ld.lda, d->m, d->k, ws, d->m, kp), ta = ws, t.lda = kp;
-  if (pad_b) pad(b, ld.ldb, b_rows, b_cols, ws + a_elems, bp_rows, bp_cols), tb = ws + a_elems, t.ldb = bp_cols;
-  if (pad_c) tc = ws + a_elems + b_elems, t.ldc = np;
-  st = cuda_ok(err, e, "gemm operand padding launch");
-  if (st == TSM100_OK) st = gemm(err, &t, ta, tb, tc, status, s);
-  if (st == TSM100_OK && pad_c) {
-    const int64_t across = (d->n + g::kThreads - 1) / g::kThreads;
-    const int rows_each = across * d->m * batch >= 16ll * sms ? g::kUnpadRows : 1;
-    const dim3 grid(static_cast<unsigned>(across), static_cast<unsigned>(std::min<int64_t>((d->m + rows_each - 1) / rows_each, 4096)), static_cast<unsigned>(batch));
-    e = launch_chained(rows_each == 1 ? g::unpad_kernel<1> : g::unpad_kernel<g::kUnpadRows>, grid, g::kThreads, 0, s, 0, static_cast<const uint16_t*>(tc),
-                       static_cast<int32_t>(np), static_cast<uint16_t*>(c), ld.ldc, d->m * ld.ldc, static_cast<int32_t>(d->m), static_cast<int32_t>(d->n));
-    st = cuda_ok(err, e, "gemm result copy launch");
+  uint16_t* ws = nullptr;
+  if (pad_a || pad_b) {
+    const int32_t got = take_scratch(err, reinterpret_cast<void**>(&ws), static_cast<size_t>(a_elems + b_elems) * 2, s);
+    if (got != TSM100_OK) return got;
+    auto operand = [&](bool copied, const void* src, int64_t pitch, int64_t rows, int64_t cols, uint16_t* dst, int64_t dst_pitch) {
+      const int64_t items = copied ? rows * (dst_pitch / 8) : 0;
+      return g::Operand{static_cast<const uint16_t*>(src), reinterpret_cast<uint4*>(dst), pitch, rows * pitch, static_cast<int32_t>(rows), static_cast<int32_t>(cols),
+                        static_cast<int32_t>(dst_pitch), static_cast<int32_t>(std::min<int64_t>((items + g::kThreads - 1) / g::kThreads, 16ll * sms))};
+    };
+    const g::Operand oa = operand(pad_a, a, ld.lda, d->m, d->k, ws, a_pitch), ob = operand(pad_b, b, ld.ldb, b_rows, b_cols, ws + a_elems, b_pitch);
+    if (pad_a) ta = ws, t.lda = a_pitch;
+    if (pad_b) tb = ws + a_elems, t.ldb = b_pitch;
+    e = launch_chained(g::pad_kernel, dim3(static_cast<unsigned>(oa.blocks + ob.blocks), static_cast<unsigned>(batch)), g::kThreads, 0, s, 0, oa, ob);
+    st = cuda_ok(err, e, "gemm operand padding launch");
   }
-  e = cudaFreeAsync(ws, s);
-  if (st == TSM100_OK && e != cudaSuccess) st = cuda_ok(err, e, "cudaFreeAsync");
+  if (st == TSM100_OK) {
+    if (d->dtype == TSM100_BF16)
+      st = d->b_transposed ? gemm_16bit_launch<__nv_bfloat16, true, true>(err, &t, ta, tb, c, sms, status, s, c_cols) : gemm_16bit_launch<__nv_bfloat16, false, true>(err, &t, ta, tb, c, sms, status, s, c_cols);
+    else
+      st = d->b_transposed ? gemm_16bit_launch<__half, true, false>(err, &t, ta, tb, c, sms, status, s, c_cols) : gemm_16bit_launch<__half, false, false>(err, &t, ta, tb, c, sms, status, s, c_cols);
+  }
+  if (ws) {
+    e = cudaFreeAsync(ws, s);
+    if (st == TSM100_OK && e != cudaSuccess) st = cuda_ok(err, e, "cudaFreeAsync");
+  }
   return st;
 }
 
@@ -1107,19 +1114,12 @@ inline int32_t gemm(std::string* err, const tsm100_gemm_desc* d, const void* a, 
     int sms = 0;
     int32_t st = sm_count(err, &sms);
     if (st != TSM100_OK) return st;
-    const route::Gemm16 plan = route::gemm16(d->m, d->n, d->k, d->batch, sms);
-#define TSM_GEMM_TC(OUT, BT, BF)                                                                                \
-  return plan.kind == route::Gemm16::kPairs     ? gemm_tc2_launch<OUT, BT, BF>(err, d, a, b, c, status, s) \
-         : plan.kind == route::Gemm16::kSingles ? gemm_tc_launch<OUT, BT, BF>(err, d, a, b, c, status, s)  \
-                                                : gemm_skinny_launch<OUT, BT, BF>(err, d, a, b, c, plan, status, s)
     if (bf16) {
-      if (out_f32) { if (d->b_transposed) TSM_GEMM_TC(float, true, true); else TSM_GEMM_TC(float, false, true); }
-      else { if (d->b_transposed) TSM_GEMM_TC(__nv_bfloat16, true, true); else TSM_GEMM_TC(__nv_bfloat16, false, true); }
-    } else {
-      if (out_f32) { if (d->b_transposed) TSM_GEMM_TC(float, true, false); else TSM_GEMM_TC(float, false, false); }
-      else { if (d->b_transposed) TSM_GEMM_TC(__half, true, false); else TSM_GEMM_TC(__half, false, false); }
+      if (out_f32) return d->b_transposed ? gemm_16bit_launch<float, true, true>(err, d, a, b, c, sms, status, s) : gemm_16bit_launch<float, false, true>(err, d, a, b, c, sms, status, s);
+      return d->b_transposed ? gemm_16bit_launch<__nv_bfloat16, true, true>(err, d, a, b, c, sms, status, s) : gemm_16bit_launch<__nv_bfloat16, false, true>(err, d, a, b, c, sms, status, s);
     }
-#undef TSM_GEMM_TC
+    if (out_f32) return d->b_transposed ? gemm_16bit_launch<float, true, false>(err, d, a, b, c, sms, status, s) : gemm_16bit_launch<float, false, false>(err, d, a, b, c, sms, status, s);
+    return d->b_transposed ? gemm_16bit_launch<__half, true, false>(err, d, a, b, c, sms, status, s) : gemm_16bit_launch<__half, false, false>(err, d, a, b, c, sms, status, s);
   }
   // Rows that start anywhere: copied into padded scratch where that pays.  Only for 16-bit results, whose last place hides the
   // order of the f32 sums; an f32 result keeps the FP32 pipe's rounding to nearest.

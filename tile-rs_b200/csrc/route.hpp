@@ -115,15 +115,16 @@ inline Gemm16 gemm16(int64_t m, int64_t n, int64_t k, int64_t batch, int sms) {
 inline bool gemm16_pairs_store_boxes(int64_t k, int64_t tiles, int sms) { return k < 2048 || (k <= 4096 && tiles <= sms); }
 
 // 16-bit products whose rows start anywhere: copies into padded scratch and the tensor cores (gemm_pad.cuh), or the FP32 pipe.  The
-// copies cost launches and traffic per row, column and output, whatever K is: FP32 pipe / padded 2000 x 3001 x
-// 17 20.6 / 31.7, x 33 29 / 32, x 65 46 / 33; 8001 x 10001 x 7 130 / 280, x 17 226 / 282, x 33 328 / 282 (hence the 2^26 products).  A CTA of the
-// FP32 pipe walks through K alone, 0.12 us for each step of it, so that from 128 of K on few products are enough; calls in a row, four
-// chained launches 16 us: 20 x 320 x 693 of a batch of 4 86 / 14, 3 x 1001 x 5003 418 / 16, 64 x 301 x 129 22.5 / 16, 2 x 4097 x 129 14.4 / 15.9.
+// copies cost a launch and traffic per row and column, whatever K is.  A CTA of the FP32 pipe walks through K alone, 0.12 us for each step of it, so that
+// from 72 of K on few products are enough.  FP32 pipe / padded, calls in a row: 760 x 144 x 124 20.9 / 9.7, 64 x 1000 x 81 15.4 / 9.7, 149 x 4008 x 98 20.5 / 9.6, 1000 x
+// 1001 x 81 14.3 / 9.6; from 128 of K on 20 x 320 x 693 of a batch of 4 86 / 10, 3 x 1001 x 5003 418 / 11.  A short K takes many products: 8001 x 10001 x 7 130 / 280 in
+// the form that copied the result too, x 17 226 / 282, x 33 328 / 282.
 // The tensor core's f32 sums round toward zero: all-positive f16 data 0.1 % further from the 64-bit result than its correctly rounded f16 values
 // at K = 16001, 2 % at 60001, 12 % at 120001 (normally distributed data and bf16 none), as in the kernels for aligned sizes.
 inline bool gemm16_padding_pays(int64_t m, int64_t n, int64_t k, int64_t batch) {
   const double outputs = static_cast<double>(m) * n * batch;
   if (outputs >= 512.0 && ((k >= 192 && outputs * k >= 1048576.0) || (k >= 128 && outputs * k >= 2097152.0))) return true;
+  if (k >= 72 && outputs >= 512.0 && outputs * k >= 4194304.0) return true;
   return outputs * k >= 67108864.0 && (k >= 64 || (k >= 32 && outputs >= 7340032.0));
 }
 
