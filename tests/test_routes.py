@@ -30,6 +30,10 @@ extern "C" int early(long long b_bytes, long long ctas, int sms) { return skinny
 extern "C" int row_per_warp(long long span, long long rows, int sms) { return softmax_row_per_warp(span, rows, sms); }
 extern "C" int cluster(long long span, long long rows, int sms) { return softmax_cluster(span, rows, sms); }
 extern "C" int splits(long long blocks, long long keys, int sms) { return attention_splits(blocks, keys, sms); }
+extern "C" void stream_plan(long long units, long long seq, int d, int sms, long long* out) {
+  const DecodeStream r = decode_stream(units, seq, d, sms);
+  out[0] = r.ctas, out[1] = r.tiles, out[2] = r.grain, out[3] = r.grains;
+}
 extern "C" int boxes(long long k, long long tiles, int sms) { return gemm16_pairs_store_boxes(k, tiles, sms); }
 extern "C" int block_rows(long long rows, long long heads, long long keys, long long offset, int causal, int sms) { return attention_block_rows(rows, heads, keys, offset, causal != 0, sms); }
 extern "C" int attention_f32(int d, long long keys) { return attention_f32_on_tcgen05(d, keys); }
@@ -233,3 +237,16 @@ def test_results_of_pairs_in_boxes(lib, k, tiles, want):
 @pytest.mark.parametrize("m,n,k,batch,pays", [(760, 144, 124, 1, True), (64, 1000, 81, 1, True), (64, 1000, 71, 1, False), (74, 304, 106, 1, False), (500, 117, 72, 1, True), (100, 5, 9001, 1, False)])
 def test_16_bit_products_of_odd_sizes_and_a_shorter_k(lib, m, n, k, batch, pays):
     assert lib.padding_pays(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch)) == pays
+
+
+# caches, positions, head_dim -> CTAs, and whether a cache may be parted
+@pytest.mark.parametrize("units,seq,d,ctas,parted", [
+    (136, 1729, 128, 148, True), (144, 200, 128, 144, False), (296, 300, 128, 148, False), (8, 32768, 128, 0, False), (8, 32768, 64, 148, True), (64, 1, 64, 0, False), (148, 1, 64, 148, False),
+    (80, 1120, 128, 0, False), (512, 600, 64, 148, True), (500, 0, 128, 0, False), (512, 100, 128, 0, False), (1 << 20, 77, 64, 148, False)])
+def test_decode_as_one_stream(lib, units, seq, d, ctas, parted):
+    out = (C.c_longlong * 4)()
+    lib.stream_plan(C.c_longlong(units), C.c_longlong(seq), d, SMS, out)
+    assert out[0] == ctas
+    if ctas:
+        tiles = -(-seq // (4096 // d))
+        assert out[1] == tiles and out[2] == (1 if parted else tiles) and out[2] * out[3] == units * tiles and out[3] >= ctas

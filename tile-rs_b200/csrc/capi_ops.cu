@@ -118,7 +118,7 @@ int32_t tsm100_attention_decode(tsm100_device_t dev, const tsm100_attention_deco
   int32_t st = use_device(dev);
   if (st != TSM100_OK) return st;
   std::string err;
-  return finish(ops::attention_decode(&err, desc, q, k_cache, v_cache, o, stream), err);
+  return finish(ops::attention_decode(&err, desc, q, k_cache, v_cache, o, stream, dev->status), err);
 }
 
 int32_t tsm100_gemm(tsm100_device_t dev, const tsm100_gemm_desc* desc, const void* a, const void* b, void* c,

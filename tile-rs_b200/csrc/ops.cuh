@@ -25,6 +25,7 @@
 
 #include "../../include/tile_sm100.h"
 #include "attention_decode.cuh"
+#include "attention_decode_stream.cuh"
 #include "attention_f32_tc.cuh"
 #include "attention_narrow.cuh"
 #include "attention_simt.cuh"
@@ -235,9 +236,9 @@ inline int32_t encode_fn(std::string* err, EncodeTiledFn* out) {
 // ones again: each thread keeps the last few it encoded.
 struct TmapKey {
   const void* base;
-  uint64_t dim[3], stride[2];
-  uint32_t box[2];
-  int32_t dtype;
+  uint64_t dim[4], stride[3];  // stride: bytes; dimension 0 is contiguous
+  uint32_t box[4];
+  int32_t dtype, rank;
 };
 struct TmapSlot {
   TmapKey key;
@@ -245,21 +246,11 @@ struct TmapSlot {
   bool used = false;
 };
 
-// dims (x contiguous, y, z), strides in elements of `elem_bytes`, box (box_x, box_y, 1), 128-byte swizzle (64-byte where a row of the
-// box has 64 bytes), out-of-range elements read as zero.
-inline int32_t make_tmap_3d(std::string* err, CUtensorMap* out, const void* base, uint64_t dim_x, uint64_t dim_y,
-                            uint64_t dim_z, uint64_t stride_y, uint64_t stride_z, uint32_t box_x, uint32_t box_y,
-                            CUtensorMapDataType dtype, uint32_t elem_bytes) {
+// `key` all zeros beyond its rank.  128-byte swizzle (64-byte where a row of the box has 64 bytes), out-of-range elements read as zero.
+inline int32_t make_tmap(std::string* err, CUtensorMap* out, const TmapKey& key, uint32_t elem_bytes) {
   constexpr int kSlots = 16;
   static thread_local TmapSlot cache[kSlots];
   static thread_local int next = 0;
-  TmapKey key;
-  std::memset(&key, 0, sizeof key);
-  key.base = base;
-  key.dim[0] = dim_x, key.dim[1] = dim_y, key.dim[2] = dim_z;
-  key.stride[0] = stride_y, key.stride[1] = stride_z;
-  key.box[0] = box_x, key.box[1] = box_y;
-  key.dtype = static_cast<int32_t>(dtype);
   for (int i = 0; i < kSlots; ++i)
     if (cache[i].used && std::memcmp(&cache[i].key, &key, sizeof key) == 0) {
       *out = cache[i].map;
@@ -268,15 +259,17 @@ inline int32_t make_tmap_3d(std::string* err, CUtensorMap* out, const void* base
   EncodeTiledFn fn;
   int32_t st = encode_fn(err, &fn);
   if (st != TSM100_OK) return st;
-  cuuint64_t dims[3] = {dim_x, dim_y, dim_z};
-  cuuint64_t strides[2] = {stride_y * elem_bytes, stride_z * elem_bytes};  // bytes; dimension 0 is contiguous
-  cuuint32_t box[3] = {box_x, box_y, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  if ((strides[0] & 15u) || (strides[1] & 15u) || !aligned16(base))
-    return op_fail(err, TSM100_ERR_INVALID, "tensor map needs a 16-byte aligned base and 16-byte-multiple strides");
-  CUresult r = fn(out, dtype, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  box_x * elem_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  cuuint64_t dims[4], strides[3];
+  cuuint32_t box[4], estr[4] = {1, 1, 1, 1};
+  for (int i = 0; i < key.rank; ++i) dims[i] = key.dim[i], box[i] = key.box[i];
+  for (int i = 0; i + 1 < key.rank; ++i) {
+    strides[i] = key.stride[i];
+    if (strides[i] & 15u) return op_fail(err, TSM100_ERR_INVALID, "tensor map needs a 16-byte aligned base and 16-byte-multiple strides");
+  }
+  if (!aligned16(key.base)) return op_fail(err, TSM100_ERR_INVALID, "tensor map needs a 16-byte aligned base and 16-byte-multiple strides");
+  CUresult r = fn(out, static_cast<CUtensorMapDataType>(key.dtype), static_cast<cuuint32_t>(key.rank), const_cast<void*>(key.base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, box[0] * elem_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     char buf[96];
     snprintf(buf, sizeof buf, "cuTensorMapEncodeTiled failed: CUresult %d", static_cast<int>(r));
@@ -288,6 +281,19 @@ inline int32_t make_tmap_3d(std::string* err, CUtensorMap* out, const void* base
   slot.map = *out;
   slot.used = true;
   return TSM100_OK;
+}
+// dims (x contiguous, y, z), strides in elements of `elem_bytes`, box (box_x, box_y, 1).
+inline int32_t make_tmap_3d(std::string* err, CUtensorMap* out, const void* base, uint64_t dim_x, uint64_t dim_y,
+                            uint64_t dim_z, uint64_t stride_y, uint64_t stride_z, uint32_t box_x, uint32_t box_y,
+                            CUtensorMapDataType dtype, uint32_t elem_bytes) {
+  TmapKey key;
+  std::memset(&key, 0, sizeof key);
+  key.base = base;
+  key.dim[0] = dim_x, key.dim[1] = dim_y, key.dim[2] = dim_z;
+  key.stride[0] = stride_y * elem_bytes, key.stride[1] = stride_z * elem_bytes;
+  key.box[0] = box_x, key.box[1] = box_y, key.box[2] = 1;
+  key.dtype = static_cast<int32_t>(dtype), key.rank = 3;
+  return make_tmap(err, out, key, elem_bytes);
 }
 
 // 16-bit elements (bf16 or f16).
@@ -1534,6 +1540,59 @@ inline int32_t attention_decode_global_launch(std::string* err, const tsm100_att
   return st;
 }
 
+// 16-bit caches, up to eight query heads each: the tiles of all caches dealt out evenly (attention_decode_stream.cuh).
+static_assert(attn_decode::stream::kTileBytes == route::kDecodeTileBytes, "route.hpp plans in these units");
+template <typename T, int D>
+inline int32_t attention_decode_stream_launch(std::string* err, const tsm100_attention_decode_desc* d, const T* q, const T* k, const T* v, T* o,
+                                              const route::DecodeStream& plan, uint32_t* status, cudaStream_t s) {
+  namespace ad = attn_decode::stream;
+  const uint64_t units = static_cast<uint64_t>(d->batch) * d->heads_kv;
+  CUtensorMap tk, tv;
+  TmapKey key;
+  std::memset(&key, 0, sizeof key);
+  key.base = k;
+  key.dim[0] = 64, key.dim[1] = d->max_seq, key.dim[2] = D / 64, key.dim[3] = units;
+  key.stride[0] = D * 2, key.stride[1] = 128, key.stride[2] = static_cast<uint64_t>(d->max_seq) * D * 2;
+  key.box[0] = 64, key.box[1] = ad::tile_rows<D>(), key.box[2] = D / 64, key.box[3] = 1;
+  key.dtype = static_cast<int32_t>(std::is_same<T, __half>::value ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16), key.rank = 4;
+  int32_t st = make_tmap(err, &tk, key, 2);
+  key.base = v;
+  if (st == TSM100_OK) st = make_tmap(err, &tv, key, 2);
+  if (st != TSM100_OK) return st;
+  ad::Params p;
+  p.heads_q = d->heads_q;
+  p.heads_kv = d->heads_kv;
+  p.group = d->heads_q / d->heads_kv;
+  p.head_base = 0;
+  p.heads_here = p.group;
+  p.seq_len = d->seq_len;
+  p.max_seq = d->max_seq;
+  p.tiles = plan.tiles;
+  p.grain = plan.grain;
+  p.grains = plan.grains;
+  p.scale_log2 = static_cast<float>((1.0 / std::sqrt(static_cast<double>(D))) * 1.4426950408889634);
+  p.part = nullptr;
+  p.status = status;
+  const bool merged = plan.grain != plan.tiles;
+  if (merged) {
+    st = take_scratch(err, reinterpret_cast<void**>(&p.part), static_cast<size_t>(plan.ctas) * 2 * ad::record_floats<D>() * sizeof(float), s);
+    if (st != TSM100_OK) return st;
+  }
+  auto kern = ad::attention_decode_stream_kernel<T, D>;
+  constexpr int smem = ad::smem_bytes<D>();
+  cudaError_t e = set_dyn_smem_once(kern, smem);
+  if (e == cudaSuccess)
+    e = launch_chained(kern, static_cast<unsigned>(plan.ctas), ad::kThreads, smem, s, 0, tk, tv, q, reinterpret_cast<const uint8_t*>(k), reinterpret_cast<const uint8_t*>(v), o, p);
+  if (e == cudaSuccess && merged)
+    e = launch_chained(ad::attention_decode_stream_merge_kernel<T, D>, static_cast<unsigned>(units * p.heads_here), D, 0, s, 0, o, p, static_cast<int32_t>(plan.ctas));
+  st = cuda_ok(err, e, "attention_decode_stream_kernel launch");
+  if (merged) {
+    e = cudaFreeAsync(p.part, s);
+    if (st == TSM100_OK && e != cudaSuccess) st = cuda_ok(err, e, "cudaFreeAsync");
+  }
+  return st;
+}
+
 // How many clusters of `size` CTAs of the eight-warp decode kernel the GPU holds at once (asked once per
 // kernel, size and device; 0 if such clusters cannot be placed at all).
 template <typename T, int D>
@@ -1574,7 +1633,7 @@ constexpr int kDecodeF32TensorCoreGroup = 5;
 
 template <typename T, int D>
 inline int32_t attention_decode_typed(std::string* err, const tsm100_attention_decode_desc* d, const void* q, const void* k,
-                                      const void* v, void* o, cudaStream_t s) {
+                                      const void* v, void* o, uint32_t* status, cudaStream_t s) {
   int sms = 0;
   int32_t st = sm_count(err, &sms);
   if (st != TSM100_OK) return st;
@@ -1588,6 +1647,15 @@ inline int32_t attention_decode_typed(std::string* err, const tsm100_attention_d
   const T* kp = static_cast<const T*>(k);
   const T* vp = static_cast<const T*>(v);
   T* op = static_cast<T*>(o);
+  if constexpr (sizeof(T) == 2)
+    if (status != nullptr && group <= attn_decode::stream::kRows) {
+      const route::DecodeStream plan = route::decode_stream(units, d->seq_len, D, std::min(sms, attn_decode::stream::kMaxCtas));
+      if (plan.ctas > 0) {
+        st = attention_decode_stream_launch<T, D>(err, d, qp, kp, vp, op, plan, status, s);
+        if (st != kNoScratch) return st;
+        st = TSM100_OK;
+      }
+    }
   if (sizeof(T) == 2 || group >= kDecodeF32TensorCoreGroup) {
     // 16-bit storage, or f32 with several query heads per cache: tensor cores, up to 16 query heads of a group per
     // pass; 4 warps per CTA, so the GPU is covered about four times before the ranges get shorter than 256 positions
@@ -1628,7 +1696,7 @@ inline int32_t attention_decode_typed(std::string* err, const tsm100_attention_d
 }
 
 inline int32_t attention_decode(std::string* err, const tsm100_attention_decode_desc* d, const void* q, const void* k,
-                                const void* v, void* o, void* stream) {
+                                const void* v, void* o, void* stream, uint32_t* status = nullptr) {
   if (!d || !q || !k || !v || !o) return op_fail(err, TSM100_ERR_INVALID, "attention_decode: null argument");
   if (!dtype_valid(d->dtype)) return op_fail(err, TSM100_ERR_INVALID, "attention_decode: unknown dtype");
   if (d->batch < 0 || d->heads_q <= 0 || d->heads_kv <= 0 || d->seq_len < 0 || d->max_seq < d->seq_len)
@@ -1646,12 +1714,12 @@ inline int32_t attention_decode(std::string* err, const tsm100_attention_decode_
   const bool d128 = d->head_dim == 128;
   switch (d->dtype) {
     case TSM100_F32:
-      return d128 ? attention_decode_typed<float, 128>(err, d, q, k, v, o, s) : attention_decode_typed<float, 64>(err, d, q, k, v, o, s);
+      return d128 ? attention_decode_typed<float, 128>(err, d, q, k, v, o, status, s) : attention_decode_typed<float, 64>(err, d, q, k, v, o, status, s);
     case TSM100_BF16:
-      return d128 ? attention_decode_typed<__nv_bfloat16, 128>(err, d, q, k, v, o, s)
-                  : attention_decode_typed<__nv_bfloat16, 64>(err, d, q, k, v, o, s);
+      return d128 ? attention_decode_typed<__nv_bfloat16, 128>(err, d, q, k, v, o, status, s)
+                  : attention_decode_typed<__nv_bfloat16, 64>(err, d, q, k, v, o, status, s);
     default:
-      return d128 ? attention_decode_typed<__half, 128>(err, d, q, k, v, o, s) : attention_decode_typed<__half, 64>(err, d, q, k, v, o, s);
+      return d128 ? attention_decode_typed<__half, 128>(err, d, q, k, v, o, status, s) : attention_decode_typed<__half, 64>(err, d, q, k, v, o, status, s);
   }
 }
 

@@ -220,6 +220,26 @@ inline PairTiles gemm_f32_pair_tiles(int64_t m, int64_t n, int64_t k, int64_t ba
   return best;
 }
 
+// Decode attention on 16-bit caches as one stream (attention_decode_stream.cuh): CTAs (0: another kernel), tiles per cache, and shares in multiples of
+// `grain` tiles, one or those of a whole cache.  Clusters / one stream, calls in a row with two appends, eight KV heads, four query heads each: 17 caches of 1729
+// x 128 41.9 / 30.2 us, 29 of 1312 54.2 / 35.7, 64 of 600 53.4 / 37.6, 64 of 6000 262 / 242, 2 of 8060 25.9 / 20.3, 1 of 32768 x 64 26.0 / 17.9, 17 of 1729 x 64 21.9 /
+// 18.6.  Whole caches need no merge (18 of 200 13.0 / 13.4, as graph replays 10.3 / 6.9; 37 of 300 19.9 / 17.4); shares that part caches need a second
+// launch, which 50 MB pay for (46 MB, 10 of 1120 x 128, 20.9 / 18.4 and 19.7 / 19.2 as replays; 36 MB, 29 of 600 x 64, 17.2 / 17.3 and 15.6 / 18.2; 26 MB 14.4 / 18.2).
+// A few caches of heads of 128 have their own CTAs already (1 of 32768 30.7 / 32.6).
+struct DecodeStream {
+  int64_t ctas;
+  int32_t tiles, grain;
+  int64_t grains;
+};
+constexpr int kDecodeTileBytes = 8192;  // of K or of V
+inline DecodeStream decode_stream(int64_t units, int64_t seq_len, int head_dim, int sms) {
+  const int64_t tiles = div_up(seq_len, kDecodeTileBytes / (2 * head_dim)), total = units * tiles;
+  if (total == 0 || tiles > 0x7fffffff) return {0, 0, 0, 0};
+  if (div_up(units, sms) * sms * 100 <= 108 * units) return {std::min<int64_t>(units, sms), static_cast<int32_t>(tiles), static_cast<int32_t>(tiles), units};
+  if (units * seq_len * head_dim * 4 < 50ll << 20 || (head_dim == 128 && units <= 12)) return {0, 0, 0, 0};
+  return {sms, static_cast<int32_t>(tiles), 1, total};
+}
+
 // Decode attention in clusters, as a programmatic dependent of the kernel before it?  That is worth 1.5 to 2.5 us of a call (not replayed from a
 // graph), but with one CTA on some SMs and two on others an uneven placement beside the last CTAs of that kernel may cost the time of a CTA:
 // in a row of calls, plain / chained, 10 caches of 18800 x 128 with 2 KV heads (160 CTAs) 42.7 / 48.3 us, 4 of 8000 with 8 (256) 28.9 / 33.0, 60 of
