@@ -34,6 +34,7 @@ extern "C" void stream_plan(long long units, long long seq, int d, int sms, long
   const DecodeStream r = decode_stream(units, seq, d, sms);
   out[0] = r.ctas, out[1] = r.tiles, out[2] = r.grain, out[3] = r.grains;
 }
+extern "C" int twice_stays(long long bytes, long long rows, int threads, int sms) { return softmax_twice_stays(bytes, rows, threads, sms); }
 extern "C" int boxes(long long k, long long tiles, int sms) { return gemm16_pairs_store_boxes(k, tiles, sms); }
 extern "C" int block_rows(long long rows, long long heads, long long keys, long long offset, int causal, int sms) { return attention_block_rows(rows, heads, keys, offset, causal != 0, sms); }
 extern "C" int attention_f32(int d, long long keys) { return attention_f32_on_tcgen05(d, keys); }
@@ -250,3 +251,8 @@ def test_decode_as_one_stream(lib, units, seq, d, ctas, parted):
     if ctas:
         tiles = -(-seq // (4096 // d))
         assert out[1] == tiles and out[2] == (1 if parted else tiles) and out[2] * out[3] == units * tiles and out[3] >= ctas
+
+
+@pytest.mark.parametrize("kib,rows,threads,stays", [(47, 100000, 256, True), (48, 1000, 256, False), (98, 1000, 256, False), (137, 700, 512, True), (195, 5000, 512, False), (195, 1776, 512, False), (195, 1775, 1024, True)])
+def test_softmax_ctas_that_stay(lib, kib, rows, threads, stays):
+    assert lib.twice_stays(C.c_longlong(kib * 1024), C.c_longlong(rows), threads, SMS) == stays

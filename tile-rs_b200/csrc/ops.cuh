@@ -358,10 +358,14 @@ inline int32_t softmax_typed(std::string* err, const T* x, T* y, int64_t rows, i
     int32_t st_cta = sm_count(err, &sms_cta);
     if (st_cta != TSM100_OK) return st_cta;
     const int32_t c = static_cast<int32_t>(cols);
-    // persistent CTAs: exactly as many as are resident at once, each striding over the rows
+    // f32: a row to a CTA; 16-bit: two, as soon as there are more rows than CTAs at once (softmax.cuh)
     auto launch = [&](auto kern, int threads) {
-      const int per_sm = blocks_per_sm(kern, threads);
-      const unsigned grid = static_cast<unsigned>(std::min<int64_t>(rows, static_cast<int64_t>(sms_cta) * per_sm));
+      int64_t ctas = rows;
+      if (sizeof(T) == 2) {
+        const int64_t resident = static_cast<int64_t>(sms_cta) * blocks_per_sm(kern, threads);
+        if (rows > resident) ctas = std::max(resident, (rows + 1) / 2);
+      }
+      const unsigned grid = static_cast<unsigned>(std::min<int64_t>(ctas, 0x7fffffff));
       e = launch_chained(kern, grid, threads, 0, s, 0, x, y, rows, c);
     };
     if (nvec <= 128 * 4) launch(softmax::softmax_rows_cta<T, 4, 128>, 128);
@@ -403,8 +407,9 @@ inline int32_t softmax_typed(std::string* err, const T* x, T* y, int64_t rows, i
     }
     // one CTA per row.  1000 rows of 50001 bf16: 97 us scalar, 49 here; 1212 of 97648 f32 286 / 214; 2000 of 16392 bf16 (in shared
     // memory) 45 / 31
-    const int threads = route::softmax_twice_threads(cols * static_cast<int64_t>(sizeof(T)), rows, sms);
-    const unsigned grid = static_cast<unsigned>(std::min<int64_t>(rows, sms * (1024ll / threads)));
+    const int64_t row_bytes = cols * static_cast<int64_t>(sizeof(T));
+    const int threads = route::softmax_twice_threads(row_bytes, rows, sms);
+    const unsigned grid = static_cast<unsigned>(std::min<int64_t>(rows, route::softmax_twice_stays(row_bytes, rows, threads, sms) ? sms * (1024ll / threads) : 0x7fffffff));
     auto launch = [&](auto kern) { e = launch_chained(kern, grid, threads, 0, s, 0, x, y, rows, c); };
     if (route::softmax_twice_skip((cols + PV - 1) / PV, threads, softmax::kTwiceUnroll)) {
       if (threads == 256) launch(softmax::softmax_rows_twice<T, 256, true>);

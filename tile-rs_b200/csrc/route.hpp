@@ -286,6 +286,10 @@ inline int softmax_twice_threads(int64_t row_bytes, int64_t rows, int sms) {
   if (fit >= 4 && rows > 2 * sms) return 256;
   return fit >= 2 && rows > sms ? 512 : 1024;
 }
+// Whether such CTAs stay for several rows, or a CTA goes after one.  A long row outweighs a CTA's start, and the places left by rows that end first are taken
+// at once: stay / go 1000 rows of 50001 bf16 48.5 / 44.2 us, 1016 of 35816 35.6 / 33.4, 5000 of 100000 425 / 397, 4000 of 14001 f32 89.3 / 87.1; but 3112 of 10848 f32
+// 56.3 / 57.3, 700 of 70000 bf16 (two CTAs to an SM) 43.5 / 44.5, 1000 of 60000 f32 102.8 / 104.5.
+inline bool softmax_twice_stays(int64_t row_bytes, int64_t rows, int threads, int sms) { return row_bytes < 48 * 1024 || (threads > 256 && rows < 12 * sms); }
 // Whether more than an eighth of the row's work would fall behind its end if every thread took whole steps of `unroll` vectors.  f32 1000
 // rows of 9000 18.7 with whole steps, 16.0 without; bf16 1000 of 65536 57 / 61.
 inline bool softmax_twice_skip(int64_t vectors, int threads, int unroll) {
