@@ -18,6 +18,8 @@ torch = pytest.importorskip("torch")
     (7, 999, 3001, 1, True, (0, 0, 1), 0),           # few rows, K over a cluster
     (90, 333, 1000, 3, False, (0, 3, 0), 0),
     (760, 144, 124, 1, True, (4, 4, 0), 0),          # K ends inside a vector, no copy
+    (1, 77, 73, 1, False, (0, 0, 0), 0), (3, 123, 3313, 1, True, (0, 0, 0), 0), (1, 1, 16383, 1, False, (0, 0, 0), 0), (5, 3, 999, 64, True, (0, 0, 0), 0),  # few outputs
+    (700, 901, 41, 1, True, (0, 0, 0), 0), (2500, 2501, 19, 1, False, (0, 0, 0), 0),
     (129, 257, 257, 1, False, (0, 0, 0), 1), (300, 513, 400, 1, True, (0, 0, 0), 3), (64, 1000, 81, 1, True, (0, 0, 0), 7)])
 def test_against_64_bits(dev, pkg, dtype, m, n, k, batch, bt, pads, shift):
     g = torch.Generator(device="cuda:0")

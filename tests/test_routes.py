@@ -35,6 +35,7 @@ extern "C" void stream_plan(long long units, long long seq, int d, int sms, long
   out[0] = r.ctas, out[1] = r.tiles, out[2] = r.grain, out[3] = r.grains;
 }
 extern "C" int twice_stays(long long bytes, long long rows, int threads, int sms) { return softmax_twice_stays(bytes, rows, threads, sms); }
+extern "C" int copies_pay(long long m, long long n, long long k, long long batch) { return gemm16_copies_pay(m, n, k, batch); }
 extern "C" int boxes(long long k, long long tiles, int sms) { return gemm16_pairs_store_boxes(k, tiles, sms); }
 extern "C" int block_rows(long long rows, long long heads, long long keys, long long offset, int causal, int sms) { return attention_block_rows(rows, heads, keys, offset, causal != 0, sms); }
 extern "C" int attention_f32(int d, long long keys) { return attention_f32_on_tcgen05(d, keys); }
@@ -256,3 +257,10 @@ def test_decode_as_one_stream(lib, units, seq, d, ctas, parted):
 @pytest.mark.parametrize("kib,rows,threads,stays", [(47, 100000, 256, True), (48, 1000, 256, False), (98, 1000, 256, False), (137, 700, 512, True), (195, 5000, 512, False), (195, 1776, 512, False), (195, 1775, 1024, True)])
 def test_softmax_ctas_that_stay(lib, kib, rows, threads, stays):
     assert lib.twice_stays(C.c_longlong(kib * 1024), C.c_longlong(rows), threads, SMS) == stays
+
+
+@pytest.mark.parametrize("m,n,k,batch,pays", [
+    (3, 123, 3313, 1, True), (1, 77, 72, 1, True), (1, 77, 71, 1, False), (1, 1, 16384, 1, True), (1, 1, 16385, 1, False), (64, 256, 48, 1, True), (64, 255, 48, 1, False), (500, 525, 33, 1, True),
+    (500, 524, 33, 1, False), (2000, 3000, 16, 1, True), (2000, 3000, 15, 1, False), (1, 511, 100001, 1, False), (3, 171, 100001, 1, True)])
+def test_16_bit_products_of_odd_sizes_with_one_copy(lib, m, n, k, batch, pays):
+    assert lib.copies_pay(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch)) == pays
