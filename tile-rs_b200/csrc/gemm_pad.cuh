@@ -13,9 +13,6 @@ namespace tsm100 {
 namespace gemm_pad {
 
 constexpr int kThreads = 256;
-// Up to how many CTAs the next kernel of the call is placed from the start.
-constexpr uint32_t kFewCtas = 8192;
-
 // src [rows][cols] with row pitch ld (problems `batch` elements apart) -> dst [rows][pitch] packed, zeros beyond cols.
 // pitch is a multiple of 8 and dst 16-byte aligned.
 struct Operand {
@@ -59,7 +56,7 @@ __device__ __forceinline__ uint4 load8(const uint16_t* src, int64_t at, int64_t 
 // One thread per eight values of a row; the operands' blocks side by side in one launch.  blockIdx.y = problem.
 __global__ void __launch_bounds__(kThreads)
 pad_kernel(const Operand a, const Operand b) {
-  ptx::launch_dependents_if_few(kFewCtas);
+  ptx::launch_dependents_if_few();  // 289 x 5995 x 2550 in a row of calls 36.4 us, 50.2 with the GEMM placed beside 2368 CTAs of this
   const bool first = static_cast<int32_t>(blockIdx.x) < a.blocks;
   const Operand& p = first ? a : b;
   const int32_t block = first ? blockIdx.x : blockIdx.x - a.blocks;
