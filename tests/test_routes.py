@@ -36,6 +36,7 @@ extern "C" void stream_plan(long long units, long long seq, int d, int sms, long
 }
 extern "C" int twice_stays(long long bytes, long long rows, int threads, int sms) { return softmax_twice_stays(bytes, rows, threads, sms); }
 extern "C" int copies_pay(long long m, long long n, long long k, long long batch) { return gemm16_copies_pay(m, n, k, batch); }
+extern "C" int split_ctas(long long blocks, long long keys, int sms) { return attention_split_ctas(blocks, keys, sms); }
 extern "C" int boxes(long long k, long long tiles, int sms) { return gemm16_pairs_store_boxes(k, tiles, sms); }
 extern "C" int block_rows(long long rows, long long heads, long long keys, long long offset, int causal, int sms) { return attention_block_rows(rows, heads, keys, offset, causal != 0, sms); }
 extern "C" int attention_f32(int d, long long keys) { return attention_f32_on_tcgen05(d, keys); }
@@ -264,3 +265,8 @@ def test_softmax_ctas_that_stay(lib, kib, rows, threads, stays):
     (500, 524, 33, 1, False), (2000, 3000, 16, 1, True), (2000, 3000, 15, 1, False), (1, 511, 100001, 1, False), (3, 171, 100001, 1, True)])
 def test_16_bit_products_of_odd_sizes_with_one_copy(lib, m, n, k, batch, pays):
     assert lib.copies_pay(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch)) == pays
+
+
+@pytest.mark.parametrize("blocks,keys,ctas", [(1, 4095, 1), (1, 4096, 8), (8, 5361, 10), (64, 7512, 2), (74, 8191, 2), (75, 8191, 1), (30, 4100, 4), (1, 8191, 15), (1, 8192, 8), (64, 16384, 2)])
+def test_attention_steps_of_middling_caches(lib, blocks, keys, ctas):
+    assert lib.split_ctas(C.c_longlong(blocks), C.c_longlong(keys), SMS) == ctas

@@ -1329,7 +1329,7 @@ inline int32_t attention_fwd_launch(std::string* err, const CUtensorMap& tq, con
   if (st != TSM100_OK) return st;
   uint16_t* out = static_cast<uint16_t*>(o);
   p.block_rows = 2 * at::kBQ;
-  p.splits = route::attention_splits(route::div_up(p.seq, 2 * at::kBQ) * heads, keys, sms);
+  p.splits = route::attention_split_ctas(route::div_up(p.seq, 2 * at::kBQ) * heads, keys, sms);
   if (p.splits == 1) p.block_rows = route::attention_block_rows(p.seq, heads, keys, p.q_offset, p.causal != 0, sms);
   p.q_blocks = static_cast<int32_t>(route::div_up(p.seq, p.block_rows));
   const int64_t blocks = p.q_blocks * heads;

@@ -64,6 +64,12 @@ constexpr int64_t kAttentionSplitKeys = 2048, kAttentionSplitKeysLong = 1024;
 inline int attention_splits(int64_t blocks, int64_t keys, int sms) {
   return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(sms / blocks, keys / (keys < 8192 ? kAttentionSplitKeys : kAttentionSplitKeysLong))));
 }
+// Between 4096 and 8191 keys more CTAs than that, 512 keys or more to each, where a call has them free: with rotation and appends, 2048 to a CTA / 512, 19
+// tokens on 5342, 8 heads, 51 / 27 us, 131 on 4677, 16 heads, 50 / 32, 100 on 6000, 32 heads, 60 / 36, 1700 on 4000, 4 heads, 62 / 47; 4 heads of 5585 x 64 74 / 53.
+inline int attention_split_ctas(int64_t blocks, int64_t keys, int sms) {
+  const int least = attention_splits(blocks, keys, sms);
+  return keys < 4096 || keys >= 8192 ? least : static_cast<int>(std::max<int64_t>(least, std::min<int64_t>(sms / blocks, keys / 512)));
+}
 
 // 16-bit GEMM on the tensor cores: CTA pairs (256 x 256 tiles, gemm_tc2.cuh), single CTAs (128 x 256 tiles, gemm_tc.cuh; both
 // persistent) or the few-tiles kernel (128 columns x `rows` rows of C per CTA, K over `splits` CTAs of a cluster, gemm_skinny.cuh).
