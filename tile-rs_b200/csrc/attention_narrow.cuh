@@ -59,7 +59,7 @@ static_assert(kSmemBytes <= 227 * 1024, "shared memory budget of one CTA");
 template <bool kIsBf16>
 constexpr float kPShift = kIsBf16 ? 0.0f : 7.0f;
 
-template <bool kIsBf16, bool kCache, bool kSplit>
+template <bool kIsBf16, bool kCache, bool kSplit, bool kLone = kSplit>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_narrow_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                         const __grid_constant__ CUtensorMap tmap_v, uint16_t* __restrict__ o, const Params p) {
@@ -75,13 +75,13 @@ attention_narrow_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
   const int block = kSplit ? static_cast<int>(blockIdx.x) / splits : static_cast<int>(blockIdx.x);
   int bh, kvh, qb;
   attn::block_coords(p, block, bh, kvh, qb);
-  const int q0 = qb * p.block_rows;
+  const int q0 = kLone ? qb * p.block_rows : qb * (2 * kBQ);
   const int seq_kv = kCache ? p.seq_kv : p.seq;
   const int q_off = kCache ? p.q_offset : 0;
   const int n_kv_all = (seq_kv + kBKV - 1) / kBKV;
   // number of KV steps each tile needs (causal: up to and including the step of its last row's own position)
   const int n_a_all = p.causal ? min(n_kv_all, (q0 + kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
-  const bool lone = p.block_rows == kBQ || q0 + kBQ >= p.seq;  // no tile B, as in attention_tc.cuh
+  const bool lone = kLone && (p.block_rows == kBQ || q0 + kBQ >= p.seq);  // no tile B, as in attention_tc.cuh
   const int n_b_all = lone ? n_a_all : p.causal ? min(n_kv_all, (q0 + 2 * kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
   // kSplit: this CTA's range [j0, j0 + n_b) of them, possibly empty
   const int per_rank = kSplit ? (n_b_all + splits - 1) / splits : n_b_all;

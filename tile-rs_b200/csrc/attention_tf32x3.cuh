@@ -15,7 +15,7 @@
 // B-fragment loads hit 32 banks); the score tile lives in the accumulator fragments, online
 // max / sum per row, and the accumulator layout of S is used directly as the A operand of
 // P V (the k index of that product is a permutation of the keys, applied to the V loads).
-// Larger f32 problems run on attention_f32_tc.cuh; this is the kernel for small ones.
+// Heads of 128 and more keys than route.hpp: attention_f32_on_tcgen05 draws the line at run on attention_f32_tc.cuh.
 // 16-bit tensors with a head size the tcgen05 kernel does not cover (96) use the same kernel:
 // a bf16 or f16 value is a TF32 number already (8 / 11 significant bits), its lo part is zero, so
 // Q K^T is ONE product and P V two (P is f32), still with f32-grade accuracy before the final rounding.

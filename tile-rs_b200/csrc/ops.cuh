@@ -1310,11 +1310,11 @@ inline int32_t attention_kv_band(uint64_t kv_len, int64_t kv_heads, uint64_t hea
 }
 
 // The tcgen05 attention kernels: heads of 128, and of 64 and less.
-template <bool kBf16, bool kCache, int D, bool kSplit>
+template <bool kBf16, bool kCache, int D, bool kSplit, bool kLone = kSplit>
 struct AttentionFwd {
   static auto kernel() {
-    if constexpr (D == 64) return attn_narrow::attention_narrow_kernel<kBf16, kCache, kSplit>;
-    else return attn::attention_fwd_kernel<kBf16, kCache, kSplit>;
+    if constexpr (D == 64) return attn_narrow::attention_narrow_kernel<kBf16, kCache, kSplit, kLone>;
+    else return attn::attention_fwd_kernel<kBf16, kCache, kSplit, kLone>;
   }
   static constexpr int smem() {
     if constexpr (D == 64) return attn_narrow::kSmemBytes;
@@ -1352,7 +1352,8 @@ inline int32_t attention_fwd_launch(std::string* err, const CUtensorMap& tq, con
   }
   cudaError_t e = cudaSuccess;
   if (p.splits == 1) {
-    auto kern = AttentionFwd<kBf16, kCache, D, false>::kernel();
+    const bool lone = p.block_rows == at::kBQ || p.seq - (p.q_blocks - 1) * (2 * at::kBQ) <= at::kBQ;  // some block has one tile
+    auto kern = lone ? AttentionFwd<kBf16, kCache, D, false, true>::kernel() : AttentionFwd<kBf16, kCache, D, false>::kernel();
     e = set_dyn_smem_once(kern, smem);
     if (e != cudaSuccess) return cuda_ok(err, e, "cudaFuncSetAttribute(attention_fwd_kernel)");
     return cuda_ok(err, launch_chained(kern, static_cast<unsigned>(blocks), at::kThreads, smem, s, 0, tq, tk, tv, out, p), "attention_fwd_kernel launch");

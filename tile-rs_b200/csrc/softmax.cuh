@@ -13,9 +13,9 @@
 //     128-bit coalesced streaming loads, shuffle reductions, one global read and
 //     one global write per element.  Rows of up to 256 16-byte vectors.
 //   * softmax_rows_cta   : 128 or 256 threads per row, 32 values per thread in
-//     registers, warp shuffles plus one shared-memory exchange per reduction;
-//     persistent CTAs stride over the rows.  Rows of up to 2048 vectors (the
-//     4096-wide configuration runs here with eight resident CTAs per SM).
+//     registers, warp shuffles plus one shared-memory exchange per reduction; a
+//     CTA takes one f32 row or two 16-bit rows and goes.  Rows of up to 2048
+//     vectors.
 //   * softmax_rows_warp_any, softmax_rows_cta_any: a warp or a CTA per row that
 //     starts anywhere.
 //   * softmax_rows_twice: wider rows of any alignment, one CTA each, read twice, the
