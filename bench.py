@@ -508,14 +508,18 @@ class GemmWL(Workload):
     def e2e_check(self):
         # The host-buffer call streams a large A in row blocks, each a launch of its own; the 16-bit pair kernel
         # orders its f32 sums by the waves of a launch, so a block may round a few results the other way: equal to
-        # one 16-bit rounding step, and nearly all bits equal.  f32 results and single-block problems are bit-equal.
+        # one 16-bit rounding step, and nearly all bits equal.  Tiles of an uneven last f32 wave are summed in pieces of
+        # K (4096^3 in one launch, but not in blocks of 1024 rows); either order is within 1e-6 of the 64-bit result in
+        # the norm and 1e-5 of the largest in each, so they are within twice that of one another.  Single-block problems are bit-equal.
         rows = sorted({0, self.m // 2 + 1, self.m - 1})
         p = self.units - 1
         x, y = self.c_host.array[p][rows], dev_rows_to_host(self.c[p], rows)
         if np.array_equal(x, y):
             return True
         if self.dtype == "f32":
-            return False
+            gap = x.astype(np.float64) - y
+            near = np.linalg.norm(gap) <= 2e-6 * np.linalg.norm(y) and np.abs(gap).max() <= 2e-5 * np.abs(y).max()
+            return bool(near and self.m * self.k * 4 > 16 << 20)
         xf, yf = self.ctx.oracle.bf16_to_f32(x), self.ctx.oracle.bf16_to_f32(y)
         step = np.maximum(np.abs(xf), np.abs(yf)) * np.float32(2.0 ** -7) + np.float32(1e-5)  # near zero: the f32 sums' own error (results are O(1))
         return bool((np.abs(xf - yf) <= step).all() and np.count_nonzero(x != y) <= 0.02 * x.size)
