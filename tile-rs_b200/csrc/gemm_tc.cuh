@@ -95,10 +95,13 @@ constexpr int kBoxCols = 128 / static_cast<int>(sizeof(OutT));
 // swizzled buffers of shared memory and TMA stores, which leave out what lies past C.  Stores from the lanes that hold the rows touch 32
 // of them with 16 bytes each, and such an epilogue of 128 x 256 took 6 us, longer than the products of K = 1000: 2897 x 4024 x 320 22.4 us, 5848 x
 // 1592 x 552 22.5, 2868 x 2848 x 944 of a batch of 4 76 us.  The caller's lane 0 has to wait for the stores before the CTA ends.
+// `boxes`: how many this warp has stored, over all of its tiles.  The buffers alternate by it and every box is a store group of its own, so that the wait for all
+// but the latest group covers the buffer at hand; a tile may end after an odd number of boxes, and a warp whose rows lie past C has none.
 // kLoose: rows of C start anywhere; the boxes are copied to them from shared memory, a warp 32 columns of a row at a time (`c`: C[b]).
 template <typename OutT, bool kLoose>
-__device__ __forceinline__ void store_rows(const CUtensorMap* tmap_c, OutT* c, int64_t ldc, uint32_t tmem, uint8_t* staging, int row0, int col0, int m, int n, int b, int lane) {
+__device__ __forceinline__ void store_rows(const CUtensorMap* tmap_c, OutT* c, int64_t ldc, uint32_t tmem, uint8_t* staging, uint32_t& boxes, int row0, int col0, int m, int n, int b, int lane) {
   constexpr int kCols = kBoxCols<OutT>;
+  if (row0 >= m) return;
 #pragma unroll 1
   for (int i0 = 0; i0 < kBN / kCols; ++i0) {
     const int c0 = i0 * kCols;
@@ -107,7 +110,7 @@ __device__ __forceinline__ void store_rows(const CUtensorMap* tmap_c, OutT* c, i
 #pragma unroll
     for (int h = 0; h < kCols / 32; ++h) ptx::tmem_ld_32x32b_x32(tmem + c0 + h * 32, v[h]);
     ptx::tmem_ld_wait();
-    uint8_t* box = staging + (i0 & 1) * kBoxBytes;
+    uint8_t* box = staging + (boxes++ & 1) * kBoxBytes;
     if (!kLoose && lane == 0) ptx::tma_store_wait_read<1>();  // the store before last has read its buffer
     __syncwarp();
     const uint32_t row = ptx::smem_u32(box) + lane * 128;
@@ -138,7 +141,7 @@ __device__ __forceinline__ void store_rows(const CUtensorMap* tmap_c, OutT* c, i
     }
     ptx::fence_proxy_async_smem();
     __syncwarp();
-    if (lane == 0 && row0 < m) {
+    if (lane == 0) {
       ptx::tma_store_3d(tmap_c, box, col0 + c0, row0, b);
       ptx::tma_store_commit();
     }
@@ -267,6 +270,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
     // ------------------------------ epilogue ----------------------------------
     const int quad = warp & 3;  // TMEM lanes [32*quad, 32*quad+32) belong to this warp
     uint8_t* staging = smem + kStages * kStageBytes + (warp - 2) * 2 * kBoxBytes;
+    uint32_t boxes = 0;
     int local = 0;
     for (int tile = blockIdx.x; tile < num_tiles; tile += gridDim.x, ++local) {
       const int acc = local & 1;
@@ -277,7 +281,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant
       const bool ready = ptx::mbar_wait(&bars->acc_full[acc], acc_phase, abort_flag, p.status, 4);
       if (!__all_sync(0xffffffffu, ready)) break;
       ptx::tcgen05_fence_after_thread_sync();
-      store_rows<OutT, kLoose>(&tmap_c, c + b * p.c_batch_stride, p.ldc, tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * kBN, staging, mb * kBM + quad * 32, nb * kBN, p.m, p.n, b, lane);
+      store_rows<OutT, kLoose>(&tmap_c, c + b * p.c_batch_stride, p.ldc, tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + acc * kBN, staging, boxes, mb * kBM + quad * 32, nb * kBN, p.m, p.n, b, lane);
       ptx::tcgen05_fence_before_thread_sync();
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&bars->acc_empty[acc]);

@@ -252,6 +252,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
   } else {
     // ------------------------------ epilogue (both CTAs) ----------------------
     const int quad = warp & 3;
+    uint32_t boxes = 0;
     int local = 0;
     for (int tile = pair; tile < num_tiles; tile += num_pairs, ++local) {
       const int acc = local & 1;
@@ -265,7 +266,7 @@ gemm_tc2_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constan
       const int row0 = mb * kPairM + static_cast<int>(rank) * kCtaM + quad * 32;
       if constexpr (kStore != kLanes) {
         uint8_t* staging = smem + kStages * kStageBytes + (warp - 2) * 2 * gemm_tc::kBoxBytes;
-        gemm_tc::store_rows<OutT, kStore == kLoose>(&tmap_c, c + b * p.c_batch_stride, p.ldc, from, staging, row0, nb * kBN, p.m, p.n, b, lane);
+        gemm_tc::store_rows<OutT, kStore == kLoose>(&tmap_c, c + b * p.c_batch_stride, p.ldc, from, staging, boxes, row0, nb * kBN, p.m, p.n, b, lane);
       } else {
         OutT* crow = c + static_cast<int64_t>(b) * p.c_batch_stride + static_cast<int64_t>(row0 + lane) * p.ldc;
 #pragma unroll 1
