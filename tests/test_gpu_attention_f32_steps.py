@@ -71,3 +71,36 @@ def test_scores_that_grow_with_every_step(dev, pkg, d):
         w = want(q, k, v, torch.tril(torch.ones(seq, seq, dtype=torch.bool, device="cuda:0")))
         # scores reach 8 * 84 / sqrt(d) = 84: an error of half a unit in their last place, 4e-6, goes into the exponentials
         assert float((o.double() - w).norm() / w.norm()) <= 1e-5
+
+
+def attend(dev, pkg, q, k, v):
+    o = torch.empty_like(q)
+    dev.attention(pkg.capi.F32, 1, q.shape[0], k.shape[0], q.shape[1], q.shape[2], q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), causal=False, stream=util.cur_stream(torch))
+    torch.cuda.synchronize()
+    assert dev.status() == 0
+    w = want(q, k, v, torch.ones(q.shape[1], k.shape[1], dtype=torch.bool, device="cuda:0"))
+    return float((o.double() - w).norm() / w.norm())
+
+
+@pytest.mark.parametrize("seq,d", [(96, 64), (300, 128), (200, 96), (400, 32)])
+@pytest.mark.parametrize("v_scale,k_scale", [(1e-35, 1), (1e-37, 1), (1e36, 1), (1, 1e-36), (1, 1e-30), (1, 1e36)])
+def test_tiny_and_huge_operands(dev, pkg, seq, d, v_scale, k_scale):
+    """Q is as much larger as K is smaller.  Two TF32 numbers lost bits below 2^-136 (V of 1e-37 3e-5 off), three bf16 numbers as they are below 2^-133 (3e-4); the
+    parts keep those from 2^-142 on."""
+    g = torch.Generator(device="cuda:0")
+    g.manual_seed(seq + d)
+    q, k, v = ((rnd(g, 2, seq, d).double() * s).float() for s in (1 / k_scale, k_scale, v_scale))
+    assert attend(dev, pkg, q, k, v) <= 8e-7 + 2.0 ** -142 / min(v_scale, k_scale, 1 / k_scale)
+
+
+@pytest.mark.parametrize("seq,d", [(96, 64), (300, 128), (200, 96), (400, 32)])
+def test_tiny_probabilities(dev, pkg, seq, d):
+    """One key has a weight of nearly one and a V of zero; what the others, of weights about e^-85 = 1e-37, add up to is the result."""
+    g = torch.Generator(device="cuda:0")
+    g.manual_seed(seq + d)
+    q, k, v = torch.zeros(2, seq, d, device="cuda:0"), torch.zeros(2, seq, d, device="cuda:0"), rnd(g, 2, seq, d)
+    q[..., 0] = d ** 0.5
+    k[..., 0] = torch.randint(-4, 5, (2, seq), generator=g, device="cuda:0") / 4
+    k[:, 0, 0], v[:, 0] = 85.0, 0.0
+    # scores are 123 in the exponents' units, half a unit in whose last place is 4e-6, twice
+    assert attend(dev, pkg, q, k, v) <= 1e-5

@@ -3,7 +3,7 @@
 // Semantics as attention_tf32x3.cuh (__tile_attention_f32, crates/tile_std/src/tile.rs:218-224;
 // crates/rustc_codegen_tile/src/mlir_to_linalg.rs:1781-1902, :1191-1244; grouped heads
 // crates/rustc_codegen_tile/src/mlir_to_gpu.rs:1657-1673).  Every operand, Q, K, V and the probabilities, is split into three bf16 numbers, 24 bits
-// together, and six of the nine products are taken, as in gemm_f32_fused.cuh.
+// together, and six of the nine products are taken.
 //
 // One streaming launch writes the parts of K and of V, each as planes [3][heads][keys][D]; V is read MN-major as it lies.  Then one CTA owns 128
 // query rows of one head and walks the keys in steps of 64:
@@ -19,12 +19,12 @@
 // 297 us at 1.6 GHz, 475 K cycles of which 350 K are products, and 26 us for the parts of K and V; 363 us a call in a row (189 TFLOP/s), 2.2e-7 off the
 // 64-bit result.  The form before this one took three products of two TF32 numbers in steps of 32 keys, whose scores spend most of a product on
 // reading Q, and wrote a third more for the parts, V transposed: 450 us, 9e-7; 2 heads of 1283 70 us, 48 here, 256 heads of 530 242 / 182.
-// What no bf16 number holds is bits below 2^-133, so that operands below 1e-34 have fewer: V of 1e-35 3.6e-6, of 1e-36 2.6e-5 (two TF32 numbers, whose
-// low part ends at 2^-126, 1.7e-6 and 7e-6).
+// Tiny operands and probabilities keep their bits (split2): V of 1e-36 2.9e-7 off, of 1e-37 1.5e-6, of 1e-38 1.5e-5 (two TF32 numbers 3.4e-6, 3.3e-5 and
+// 3.4e-4, three bf16 numbers as they are 2.7e-5, 2.7e-4 and 2.7e-3); that takes 0.1 % of the cycles.
 #pragma once
 
 #include "attention_simt.cuh"    // Params
-#include "gemm_f32_fused.cuh"    // split2
+#include "attention_tc.cuh"      // pack16x2
 #include "ptx.cuh"
 
 namespace tsm100 {
@@ -75,6 +75,23 @@ struct Params {
   uint32_t* status;
 };
 
+// Two values as three pairs of bf16 numbers: hi truncated (the largest f32 numbers would round up to infinity), mid what is left of them rounded to nearest,
+// lo 2^kLoShift times the rest, which has 8 bits or less.  Unscaled, it would end below the last bit that a bf16 number has, 2^-133, for values below
+// 1e-34; this way bits from 2^-142 on are kept.  lo stays smaller than hi, and sums of products with it than those of hi.
+constexpr int kLoShift = 10;
+__device__ __forceinline__ void split2(float x0, float x1, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  constexpr float kUp = 1 << kLoShift;
+  const uint32_t b0 = __float_as_uint(x0), b1 = __float_as_uint(x1);
+  hi = __byte_perm(b0, b1, 0x7632);
+  const float r0 = x0 - __uint_as_float(b0 & 0xffff0000u), r1 = x1 - __uint_as_float(b1 & 0xffff0000u);
+  mid = attn::pack16x2<true>(r0, r1);
+  float l0, l1;  // in pairs: one by one they took 0.8 % of the kernel's cycles
+  const ptx::f32x2_t m = ptx::pack_f32x2(attn::unpack16_lo<true>(mid), attn::unpack16_hi<true>(mid));
+  const ptx::f32x2_t l = ptx::fma_f32x2(m, ptx::pack_f32x2(-1.0f, -1.0f), ptx::pack_f32x2(r0, r1));
+  ptx::unpack_f32x2(ptx::mul_f32x2(l, ptx::pack_f32x2(kUp, kUp)), l0, l1);
+  lo = __byte_perm(__float_as_uint(l0), __float_as_uint(l1), 0x7632);
+}
+
 // The parts of K and of V, bf16 [3][heads][rows * D]: grid (blocks, heads, 2), a thread per eight values.
 struct SplitParams {
   const float* src[2];
@@ -92,15 +109,32 @@ split_kv_kernel(const SplitParams p) {
   const int64_t step = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < p.head_vecs; i += step) {
     const float4 x = __ldcs(src + 2 * i), y = __ldcs(src + 2 * i + 1);
-    uint32_t hi[4], mid[4], lo[4], unused = 0;
-    gemm_f32_fused::split2(x.x, x.y, hi[0], mid[0], lo[0], unused);
-    gemm_f32_fused::split2(x.z, x.w, hi[1], mid[1], lo[1], unused);
-    gemm_f32_fused::split2(y.x, y.y, hi[2], mid[2], lo[2], unused);
-    gemm_f32_fused::split2(y.z, y.w, hi[3], mid[3], lo[3], unused);
+    uint32_t hi[4], mid[4], lo[4];
+    split2(x.x, x.y, hi[0], mid[0], lo[0]);
+    split2(x.z, x.w, hi[1], mid[1], lo[1]);
+    split2(y.x, y.y, hi[2], mid[2], lo[2]);
+    split2(y.z, y.w, hi[3], mid[3], lo[3]);
     dst[i] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     dst[i + part] = make_uint4(mid[0], mid[1], mid[2], mid[3]);
     dst[i + 2 * part] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
   }
+}
+
+// What a product does with the accumulator: overwrites it, adds to it, or adds to it after bringing it down from the scale of lo.
+enum Start { kFresh, kAdd, kDown };
+__device__ __forceinline__ void product(uint32_t d, uint32_t a, uint64_t b_desc, uint32_t idesc, Start start) {
+  if (start == kDown) ptx::tcgen05_mma_f16_ts_scaled<kLoShift>(d, a, b_desc, idesc);
+  else ptx::tcgen05_mma_f16_ts(d, a, b_desc, idesc, start == kFresh ? 0u : 1u);
+}
+// The six products of the parts, the small ones first: the accumulator cuts every term off at its own last place.
+template <typename F>
+__device__ __forceinline__ void all_products(F products) {
+  products(2, 0, kFresh);
+  products(0, 2, kAdd);
+  products(1, 1, kDown);
+  products(1, 0, kAdd);
+  products(0, 1, kAdd);
+  products(0, 0, kAdd);
 }
 
 template <int D>
@@ -168,12 +202,12 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
     const uint32_t tq = tmem + (static_cast<uint32_t>(warp * 32) << 16) + kTmemQ;
 #pragma unroll
     for (int c = 0; c < D / 32; ++c) {
-      uint32_t hi[16], mid[16], lo[16], unused = 0;
+      uint32_t hi[16], mid[16], lo[16];
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const float4 x = valid ? qr[c * 8 + u] : make_float4(0.f, 0.f, 0.f, 0.f);
-        gemm_f32_fused::split2(x.x, x.y, hi[2 * u], mid[2 * u], lo[2 * u], unused);
-        gemm_f32_fused::split2(x.z, x.w, hi[2 * u + 1], mid[2 * u + 1], lo[2 * u + 1], unused);
+        split2(x.x, x.y, hi[2 * u], mid[2 * u], lo[2 * u]);
+        split2(x.z, x.w, hi[2 * u + 1], mid[2 * u + 1], lo[2 * u + 1]);
       }
       __syncwarp();
       ptx::tmem_st_32x32b_x16(tq + c * 16, hi);
@@ -231,21 +265,15 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
         const uint32_t d = tmem + kTmemS + b * kBuffer, a = tmem + kTmemQ;
         const uint32_t k_lo = static_cast<uint32_t>(k_base) | (ring16 + (k_pos(j) % kRing) * (Sh::kUnitBytes >> 4));
         if (ptx::elect_one_sync()) {
-          auto products = [&](int x, int y, bool first) {
+          auto products = [&](int x, int y, Start start) {
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
               constexpr int kPerGroup = Sh::kGroup / 16;
               const uint32_t off = y * kPart16 + (kk / kPerGroup) * (Sh::kGroupBytes >> 4) + (kk % kPerGroup) * 2;
-              ptx::tcgen05_mma_f16_ts(d, a + x * kQPart + kk * 8, desc(k_base, k_lo + off), idesc, first && kk == 0 ? 0u : 1u);
+              product(d, a + x * kQPart + kk * 8, desc(k_base, k_lo + off), idesc, kk == 0 ? start : kAdd);
             }
           };
-          // the small products first: the accumulator cuts every term off at its own last place
-          products(2, 0, true);
-          products(0, 2, false);
-          products(1, 1, false);
-          products(1, 0, false);
-          products(0, 1, false);
-          products(0, 0, false);
+          all_products(products);
           ptx::tcgen05_commit(&bars->s_full[b]);
           ptx::tcgen05_commit(&bars->kv_empty[k_pos(j) % kRing]);
         }
@@ -262,17 +290,12 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
         const uint32_t d = tmem + kTmemO, a = tmem + kTmemS + b * kBuffer;
         const uint32_t v_lo = static_cast<uint32_t>(v_base) | (ring16 + (v_pos(j) % kRing) * (Sh::kUnitBytes >> 4));
         if (ptx::elect_one_sync()) {
-          auto products = [&](int x, int y, bool first) {
+          auto products = [&](int x, int y, Start start) {
 #pragma unroll
             for (int kk = 0; kk < kBKV / 16; ++kk)
-              ptx::tcgen05_mma_f16_ts(d, a + x * kPPart + kk * 8, desc(v_base, v_lo + y * kPart16 + kk * (16 * Sh::kRow >> 4)), idesc, first && kk == 0 ? 0u : 1u);
+              product(d, a + x * kPPart + kk * 8, desc(v_base, v_lo + y * kPart16 + kk * (16 * Sh::kRow >> 4)), idesc, kk == 0 ? start : kAdd);
           };
-          products(2, 0, true);
-          products(0, 2, false);
-          products(1, 1, false);
-          products(1, 0, false);
-          products(0, 1, false);
-          products(0, 0, false);
+          all_products(products);
           ptx::tcgen05_commit(&bars->buf_free[b]);
           ptx::tcgen05_commit(&bars->o_full);
           ptx::tcgen05_commit(&bars->kv_empty[v_pos(j) % kRing]);
@@ -329,14 +352,14 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
       // The parts of the probabilities take the place of the scores.
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        uint32_t hi[16], mid[16], lo[16], unused = 0;
+        uint32_t hi[16], mid[16], lo[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           float t0, t1;
           ptx::unpack_f32x2(ptx::fma_f32x2(ptx::pack_f32x2(__uint_as_float(v[h][2 * i]), __uint_as_float(v[h][2 * i + 1])), sl2x2, nmsx2), t0, t1);
           const float e0 = ptx::ex2_approx(t0), e1 = ptx::ex2_approx(t1);
           ls[i & 1] = ptx::add_f32x2(ls[i & 1], ptx::pack_f32x2(e0, e1));
-          gemm_f32_fused::split2(e0, e1, hi[i], mid[i], lo[i], unused);
+          split2(e0, e1, hi[i], mid[i], lo[i]);
         }
         ptx::tmem_st_32x32b_x16(ts + h * 16, hi);
         ptx::tmem_st_32x32b_x16(ts + kPPart + h * 16, mid);

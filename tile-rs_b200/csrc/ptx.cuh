@@ -465,6 +465,20 @@ __device__ __forceinline__ void tcgen05_mma_f16_ts(uint32_t d_tmem, uint32_t a_t
       : "memory");
 }
 
+// The same, the accumulator times 2^-kShift before the product is added.
+template <int kShift>
+__device__ __forceinline__ void tcgen05_mma_f16_ts_scaled(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc) {
+  static_assert(kShift >= 0 && kShift <= 15, "what the instruction takes");
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "setp.ne.b32 p, 1, 0;\n"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p, %4;\n"
+      "}\n" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "n"(kShift)
+      : "memory");
+}
+
 // ---------------------------------------------------------------------------
 // tcgen05.ld: tensor memory -> registers.  Shape 32x32b: lane i of the warp
 // reads TMEM lane (32 * (warp_id % 4) + i); register j holds column base + j.
@@ -546,6 +560,11 @@ __device__ __forceinline__ void unpack_f32x2(f32x2_t v, float& lo, float& hi) {
 __device__ __forceinline__ f32x2_t fma_f32x2(f32x2_t a, f32x2_t b, f32x2_t c) {
   f32x2_t d;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ f32x2_t mul_f32x2(f32x2_t a, f32x2_t b) {
+  f32x2_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
 __device__ __forceinline__ f32x2_t add_f32x2(f32x2_t a, f32x2_t b) {
