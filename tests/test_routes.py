@@ -35,7 +35,7 @@ extern "C" void stream_plan(long long units, long long seq, int d, int sms, long
   out[0] = r.ctas, out[1] = r.tiles, out[2] = r.grain, out[3] = r.grains;
 }
 extern "C" int twice_stays(long long bytes, long long rows, int threads, int sms) { return softmax_twice_stays(bytes, rows, threads, sms); }
-extern "C" int copies_pay(long long m, long long n, long long k, long long batch) { return gemm16_copies_pay(m, n, k, batch); }
+extern "C" int copies_pay(long long m, long long n, long long k, long long batch, int bf16) { return gemm16_copies_pay(m, n, k, batch, bf16 != 0); }
 extern "C" int split_ctas(long long blocks, long long keys, int sms) { return attention_split_ctas(blocks, keys, sms); }
 extern "C" int boxes(long long k, long long tiles, int sms) { return gemm16_pairs_store_boxes(k, tiles, sms); }
 extern "C" int block_rows(long long rows, long long heads, long long keys, long long offset, int causal, int sms) { return attention_block_rows(rows, heads, keys, offset, causal != 0, sms); }
@@ -264,7 +264,13 @@ def test_softmax_ctas_that_stay(lib, kib, rows, threads, stays):
     (3, 123, 3313, 1, True), (1, 77, 72, 1, True), (1, 77, 71, 1, False), (1, 1, 16384, 1, True), (1, 1, 16385, 1, False), (64, 256, 48, 1, True), (64, 255, 48, 1, False), (500, 525, 33, 1, True),
     (500, 524, 33, 1, False), (2000, 3000, 16, 1, True), (2000, 3000, 15, 1, False), (1, 511, 100001, 1, False), (3, 171, 100001, 1, True)])
 def test_16_bit_products_of_odd_sizes_with_one_copy(lib, m, n, k, batch, pays):
-    assert lib.copies_pay(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch)) == pays
+    assert lib.copies_pay(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch), 1) == pays
+
+
+# f16 with few outputs: K only as long as sums that round toward zero do not show beside the result's own rounding
+@pytest.mark.parametrize("m,n,k,batch,pays", [(3, 123, 6144, 1, True), (3, 123, 6145, 1, False), (1, 511, 16384, 1, False), (1, 512, 16384, 1, True), (3, 171, 100001, 1, True), (1, 77, 72, 1, True), (1, 511, 100001, 1, False)])
+def test_f16_products_of_few_outputs(lib, m, n, k, batch, pays):
+    assert lib.copies_pay(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch), 0) == pays
 
 
 @pytest.mark.parametrize("blocks,keys,ctas", [(1, 4095, 1), (1, 4096, 8), (8, 5361, 10), (64, 7512, 2), (74, 8191, 2), (75, 8191, 1), (30, 4100, 4), (1, 8191, 15), (1, 8192, 8), (64, 16384, 2)])

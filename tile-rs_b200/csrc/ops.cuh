@@ -1142,7 +1142,7 @@ inline int32_t gemm(std::string* err, const tsm100_gemm_desc* d, const void* a, 
   // order of the f32 sums; an f32 result keeps the FP32 pipe's rounding to nearest.
   const int64_t n8 = (d->n + 7) / 8 * 8, k8 = (d->k + 7) / 8 * 8;
   if (status != nullptr && !out_f32 && d->batch <= 65535 && n8 <= 0x7fffffff && k8 <= 0x7fffffff &&
-      route::gemm16_copies_pay(d->m, d->n, d->k, d->batch) && (d->m + 127) / 128 * ((n8 + 255) / 256) * d->batch < 0x7fffffff) {
+      route::gemm16_copies_pay(d->m, d->n, d->k, d->batch, bf16) && (d->m + 127) / 128 * ((n8 + 255) / 256) * d->batch < 0x7fffffff) {
     const int32_t st = gemm_padded(err, d, a, b, c, status, s);
     if (st != kNoScratch) return st;
   }

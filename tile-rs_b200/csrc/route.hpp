@@ -136,12 +136,14 @@ inline bool gemm16_padding_pays(int64_t m, int64_t n, int64_t k, int64_t batch) 
 
 // The same for a call that gets both copies in one launch and no copy of the result (ops.cuh: gemm_padded): less K is enough, and few outputs are no
 // reason against it, as K is shared by a cluster.  FP32 pipe / copies, calls in a row: 3 x 123 x 3313 275 / 10.3, 1 x 77 x 97 12.3 / 10.4, x 65 9.2 / 10.4, 64 x 301 x 57 11.6 /
-// 10.4, x 41 8.9 / 10.3, 500 x 501 x 41 10.2 / 10.3, x 33 8.2 / 10.4, 2000 x 3001 x 33 30.8 / 19.8, x 17 22.6 / 19.8, 8001 x 5001 x 17 118 / 73.  A K beyond 16384 of
-// few outputs keeps the FP32 pipe's rounding to nearest.
-inline bool gemm16_copies_pay(int64_t m, int64_t n, int64_t k, int64_t batch) {
+// 10.4, x 41 8.9 / 10.3, 500 x 501 x 41 10.2 / 10.3, x 33 8.2 / 10.4, 2000 x 3001 x 33 30.8 / 19.8, x 17 22.6 / 19.8, 8001 x 5001 x 17 118 / 73.
+// Fewer than 512 outputs with a long K keep the FP32 pipe's rounding to nearest.  Where the line lies: the tensor core's sums move all-positive f16 results by less
+// than 2^-24 (norm) from the 64-bit result up to K = 6144 (rounding error 2.2e-4, times 5e-5 more at 3313, 1.7e-4 at 5999, 3.3e-4 at 8191, 1.4e-3 at 16383; FP32 pipe
+// 3e-5 at most), bf16 ones by 4e-6 of theirs at 16383; normally distributed data is nearer than on the FP32 pipe.
+inline bool gemm16_copies_pay(int64_t m, int64_t n, int64_t k, int64_t batch, bool bf16) {
   if (gemm16_padding_pays(m, n, k, batch)) return true;
   const double outputs = static_cast<double>(m) * n * batch;
-  return k <= 16384 && k >= (outputs >= 6000000.0 ? 16 : outputs >= 262144.0 ? 33 : outputs >= 16384.0 ? 48 : 72);
+  return k <= (outputs < 512.0 && !bf16 ? 6144 : 16384) && k >= (outputs >= 6000000.0 ? 16 : outputs >= 262144.0 ? 33 : outputs >= 16384.0 ? 48 : 72);
 }
 
 // f32 GEMM: operand planes and CTA pairs (gemm_tf32_tc.cuh), operands split on the way in (gemm_f32_fused.cuh), the warp-level kernel
