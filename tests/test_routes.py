@@ -23,13 +23,11 @@ extern "C" void pair_tiles(long long m, long long n, long long k, long long batc
   const PairTiles r = gemm_f32_pair_tiles(m, n, k, batch, sms);
   out[0] = r.bn, out[1] = r.whole_tiles, out[2] = r.splits;
 }
-extern "C" int padding_pays(long long m, long long n, long long k, long long batch) { return gemm16_padding_pays(m, n, k, batch); }
 extern "C" int rope_is_few(long long blocks, int heads_per, int sms) { return rope_few(blocks, heads_per, sms); }
 extern "C" int decode_chained(long long ctas, long long bytes, int sms) { return decode_is_chained(ctas, bytes, sms); }
 extern "C" int early(long long b_bytes, long long ctas, int sms) { return skinny_places_early(b_bytes, ctas, sms); }
 extern "C" int row_per_warp(long long span, long long rows, int sms) { return softmax_row_per_warp(span, rows, sms); }
 extern "C" int cluster(long long span, long long rows, int sms) { return softmax_cluster(span, rows, sms); }
-extern "C" int splits(long long blocks, long long keys, int sms) { return attention_splits(blocks, keys, sms); }
 extern "C" void stream_plan(long long units, long long seq, int d, int sms, long long* out) {
   const DecodeStream r = decode_stream(units, seq, d, sms);
   out[0] = r.ctas, out[1] = r.tiles, out[2] = r.grain, out[3] = r.grains;
@@ -101,12 +99,11 @@ def test_16_bit_plans_fit_a_launch(lib):
 
 @pytest.mark.parametrize("m,n,k,batch,pays", [
     (2000, 3001, 2501, 1, True), (500, 1001, 999, 1, True), (28, 3134, 4883, 1, True),
-    (2000, 3001, 17, 1, False), (8001, 10001, 7, 1, False), (2000, 3001, 33, 1, False), (8001, 1001, 33, 1, True), (2000, 3001, 65, 1, True),
-    (100, 101, 103, 1, False), (64, 64, 65, 500, True), (64, 64, 65, 64, False),
-    # few outputs, long K: counted in products, not in 4096ths of outputs
-    (1, 3001, 50001, 1, True), (30, 101, 1003, 64, True), (1, 501, 4001, 1, False), ((1 << 31) - 1, (1 << 31) - 1, (1 << 31) - 1, 1, True)])
+    (2000, 3001, 17, 1, True), (8001, 10001, 7, 1, False), (2000, 3001, 33, 1, True), (8001, 1001, 33, 1, True), (2000, 3001, 65, 1, True),
+    (100, 101, 103, 1, True), (64, 64, 65, 500, True), (64, 64, 65, 64, True), (64, 64, 65, 3, False),
+    (1, 3001, 50001, 1, True), (30, 101, 1003, 64, True), (1, 501, 4001, 1, True), ((1 << 31) - 1, (1 << 31) - 1, (1 << 31) - 1, 1, True)])
 def test_16_bit_products_of_odd_sizes(lib, m, n, k, batch, pays):
-    assert lib.padding_pays(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch)) == pays
+    assert lib.copies_pay(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch), 1) == pays
 
 
 @pytest.mark.parametrize("span,rows,warp", [(10, 1, True), (128, 1, True), (129, 1, False), (256, 296, False), (256, 297, True), (257, 5000, False)])
@@ -140,21 +137,21 @@ def test_rotary_head_groups(lib, blocks, heads, per):
 
 
 @pytest.mark.parametrize("blocks,keys,ctas", [
-    (1, 1, 1), (1, 3969, 1), (1, 4095, 1), (1, 4096, 2), (64, 16384, 2), (74, 1 << 20, 2), (75, 1 << 20, 1), (9, 34000, 16), (1, 1 << 20, 148), (1 << 20, 8192, 1)])
+    (1, 1, 1), (1, 3969, 1), (1, 4095, 1), (1, 4096, 8), (64, 16384, 2), (74, 1 << 20, 2), (75, 1 << 20, 1), (9, 34000, 16), (1, 1 << 20, 148), (1 << 20, 8192, 1)])
 def test_attention_steps_over_several_ctas(lib, blocks, keys, ctas):
-    assert lib.splits(C.c_longlong(blocks), C.c_longlong(keys), SMS) == ctas
+    assert lib.split_ctas(C.c_longlong(blocks), C.c_longlong(keys), SMS) == ctas
 
 
-@pytest.mark.parametrize("blocks,keys,ctas", [(1, 8191, 3), (1, 8192, 8), (4, 9030, 8), (16, 10200, 9), (64, 16384, 2), (75, 16384, 1)])
+@pytest.mark.parametrize("blocks,keys,ctas", [(1, 8191, 15), (1, 8192, 8), (4, 9030, 8), (16, 10200, 9), (64, 16384, 2), (75, 16384, 1)])
 def test_attention_steps_of_long_caches(lib, blocks, keys, ctas):
-    assert lib.splits(C.c_longlong(blocks), C.c_longlong(keys), SMS) == ctas
+    assert lib.split_ctas(C.c_longlong(blocks), C.c_longlong(keys), SMS) == ctas
 
 
 @pytest.mark.parametrize("m,n,k,batch,pays", [
-    (20, 320, 693, 4, True), (3, 1001, 5003, 1, True), (64, 301, 129, 1, True), (2, 4097, 129, 1, False), (64, 301, 127, 1, False), (25, 99, 501, 1, True),
-    (3, 171, 8001, 1, True), (1, 511, 100001, 1, False), (10, 60, 1001, 1, False)])
+    (20, 320, 693, 4, True), (3, 1001, 5003, 1, True), (64, 301, 129, 1, True), (2, 4097, 129, 1, True), (64, 301, 127, 1, True), (25, 99, 501, 1, True),
+    (3, 171, 8001, 1, True), (1, 511, 100001, 1, False), (10, 60, 1001, 1, True)])
 def test_16_bit_products_of_odd_sizes_and_a_longer_k(lib, m, n, k, batch, pays):
-    assert lib.padding_pays(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch)) == pays
+    assert lib.copies_pay(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch), 1) == pays
 
 
 @pytest.mark.parametrize("blocks,heads_per,few", [(1, 4, True), (296, 8, True), (297, 4, False), (250, 9, False), (1, 32, False)])
@@ -237,9 +234,9 @@ def test_results_of_pairs_in_boxes(lib, k, tiles, want):
     assert lib.boxes(C.c_longlong(k), C.c_longlong(tiles), SMS) == want
 
 
-@pytest.mark.parametrize("m,n,k,batch,pays", [(760, 144, 124, 1, True), (64, 1000, 81, 1, True), (64, 1000, 71, 1, False), (74, 304, 106, 1, False), (500, 117, 72, 1, True), (100, 5, 9001, 1, False)])
+@pytest.mark.parametrize("m,n,k,batch,pays", [(760, 144, 124, 1, True), (64, 1000, 81, 1, True), (64, 1000, 71, 1, True), (64, 1000, 47, 1, False), (74, 304, 106, 1, True), (500, 117, 72, 1, True), (100, 5, 9001, 1, True), (100, 5, 71, 1, False)])
 def test_16_bit_products_of_odd_sizes_and_a_shorter_k(lib, m, n, k, batch, pays):
-    assert lib.padding_pays(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch)) == pays
+    assert lib.copies_pay(C.c_longlong(m), C.c_longlong(n), C.c_longlong(k), C.c_longlong(batch), 1) == pays
 
 
 # caches, positions, head_dim -> CTAs, and whether a cache may be parted

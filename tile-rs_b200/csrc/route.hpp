@@ -55,20 +55,13 @@ inline int attention_block_rows(int64_t rows, int64_t heads, int64_t keys, int64
 }
 
 // 16-bit attention on tcgen05: how many CTAs share the KV steps of a query block.  One CTA fills an SM, so the steps are dealt out when
-// there are blocks for at most half of the SMs, 2048 keys or more to each, 1024 from 8192 keys on, where the merge of more records is
-// short beside the steps saved.  512 tokens on 15872, 32 heads (64 blocks): 212 unsplit, 122 split; the whole step of 30 tokens on 9000, 4 heads,
-// 45 us with 2048 keys to a CTA, 32 with 1024, 30 with 512; on 16000 48 / 37 / 39; 200 on 16000, 8 heads, 51 / 43 / 46.  Between 4096 and 8191
-// keys 1024 or 512 to a CTA would do as well (30 tokens on 5000 47 / 32 / 26, 512 on 7000, 8 heads, 50 / 38 / 39).  Below 4096 keys a
-// call is never split, so that a prompt in chunks gives the bits of the whole one.
-constexpr int64_t kAttentionSplitKeys = 2048, kAttentionSplitKeysLong = 1024;
-inline int attention_splits(int64_t blocks, int64_t keys, int sms) {
-  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(sms / blocks, keys / (keys < 8192 ? kAttentionSplitKeys : kAttentionSplitKeysLong))));
-}
-// Between 4096 and 8191 keys more CTAs than that, 512 keys or more to each, where a call has them free: with rotation and appends, 2048 to a CTA / 512, 19
-// tokens on 5342, 8 heads, 51 / 27 us, 131 on 4677, 16 heads, 50 / 32, 100 on 6000, 32 heads, 60 / 36, 1700 on 4000, 4 heads, 62 / 47; 4 heads of 5585 x 64 74 / 53.
+// there are blocks for at most half of the SMs: 512 keys or more to each CTA from 4096 keys on, 1024 or more from 8192 on, where the merge of more records
+// takes what the shorter chains save.  With rotation and appends, 2048 keys to a CTA / 1024 / 512: 30 tokens on 5000, 4 heads, 47 / 32 / 26 us, 19 on 5342, 8 heads,
+// 51 / - / 27, 512 on 7000, 8 heads, 50 / 38 / 39, 30 on 9000, 4 heads, 45 / 32 / 30, on 16000 48 / 37 / 39, 200 on 16000, 8 heads, 51 / 43 / 46; 512 on 15872, 32 heads (64
+// blocks), 212 unsplit, 122 split.  Below 4096 keys a call is never split, so that a prompt in chunks gives the bits of the whole one.
 inline int attention_split_ctas(int64_t blocks, int64_t keys, int sms) {
-  const int least = attention_splits(blocks, keys, sms);
-  return keys < 4096 || keys >= 8192 ? least : static_cast<int>(std::max<int64_t>(least, std::min<int64_t>(sms / blocks, keys / 512)));
+  if (keys < 4096) return 1;
+  return static_cast<int>(std::max<int64_t>(1, std::min<int64_t>(sms / blocks, keys / (keys < 8192 ? 512 : 1024))));
 }
 
 // 16-bit GEMM on the tensor cores: CTA pairs (256 x 256 tiles, gemm_tc2.cuh), single CTAs (128 x 256 tiles, gemm_tc.cuh; both
@@ -120,30 +113,18 @@ inline Gemm16 gemm16(int64_t m, int64_t n, int64_t k, int64_t batch, int sms) {
 // 1024 53.7 / 51.2, x 2048 105.3 / 107.2, x 4096 198 / 203; 8192^3 803 / 833; 2048 x 2048 x 4096 (64 tiles) 26.1 / 25.6, 2048 x 4608 x 2048 (144) 28.4 / 26.2.
 inline bool gemm16_pairs_store_boxes(int64_t k, int64_t tiles, int sms) { return k < 2048 || (k <= 4096 && tiles <= sms); }
 
-// 16-bit products whose rows start anywhere: copies into padded scratch and the tensor cores (gemm_pad.cuh), or the FP32 pipe.  The
-// copies cost a launch and traffic per row and column, whatever K is.  A CTA of the FP32 pipe walks through K alone, 0.12 us for each step of it, so that
-// from 72 of K on few products are enough.  FP32 pipe / padded, calls in a row: 760 x 144 x 124 20.9 / 9.7, 64 x 1000 x 81 15.4 / 9.7, 149 x 4008 x 98 20.5 / 9.6, 1000 x
-// 1001 x 81 14.3 / 9.6; from 128 of K on 20 x 320 x 693 of a batch of 4 86 / 10, 3 x 1001 x 5003 418 / 11.  A short K takes many products: 8001 x 10001 x 7 130 / 280 in
-// the form that copied the result too, x 17 226 / 282, x 33 328 / 282.
-// The tensor core's f32 sums round toward zero: all-positive f16 data 0.1 % further from the 64-bit result than its correctly rounded f16 values
-// at K = 16001, 2 % at 60001, 12 % at 120001 (normally distributed data and bf16 none), as in the kernels for aligned sizes.
-inline bool gemm16_padding_pays(int64_t m, int64_t n, int64_t k, int64_t batch) {
-  const double outputs = static_cast<double>(m) * n * batch;
-  if (outputs >= 512.0 && ((k >= 192 && outputs * k >= 1048576.0) || (k >= 128 && outputs * k >= 2097152.0))) return true;
-  if (k >= 72 && outputs >= 512.0 && outputs * k >= 4194304.0) return true;
-  return outputs * k >= 67108864.0 && (k >= 64 || (k >= 32 && outputs >= 7340032.0));
-}
-
-// The same for a call that gets both copies in one launch and no copy of the result (ops.cuh: gemm_padded): less K is enough, and few outputs are no
-// reason against it, as K is shared by a cluster.  FP32 pipe / copies, calls in a row: 3 x 123 x 3313 275 / 10.3, 1 x 77 x 97 12.3 / 10.4, x 65 9.2 / 10.4, 64 x 301 x 57 11.6 /
-// 10.4, x 41 8.9 / 10.3, 500 x 501 x 41 10.2 / 10.3, x 33 8.2 / 10.4, 2000 x 3001 x 33 30.8 / 19.8, x 17 22.6 / 19.8, 8001 x 5001 x 17 118 / 73.
-// Fewer than 512 outputs with a long K keep the FP32 pipe's rounding to nearest.  Where the line lies: the tensor core's sums move all-positive f16 results by less
-// than 2^-24 (norm) from the 64-bit result up to K = 6144 (rounding error 2.2e-4, times 5e-5 more at 3313, 1.7e-4 at 5999, 3.3e-4 at 8191, 1.4e-3 at 16383; FP32 pipe
-// 3e-5 at most), bf16 ones by 4e-6 of theirs at 16383; normally distributed data is nearer than on the FP32 pipe.
+// 16-bit products whose rows start anywhere: operands copied to rows that tensor maps can describe and the tensor cores (gemm_pad.cuh), or the FP32 pipe.  The
+// copies cost one launch and traffic per row and column, whatever K is; a CTA of the FP32 pipe walks through K alone, 0.12 us for each step of it.  FP32 pipe /
+// copies, calls in a row: 3 x 123 x 3313 275 / 10.3, 1 x 77 x 97 12.3 / 10.4, x 65 9.2 / 10.4, 64 x 301 x 57 11.6 / 10.4, x 41 8.9 / 10.3, 500 x 501 x 41 10.2 / 10.3, x 33 8.2 /
+// 10.4, 2000 x 3001 x 33 30.8 / 19.8, x 17 22.6 / 19.8, 8001 x 5001 x 17 118 / 73.
+// Fewer than 512 outputs with a long K keep the FP32 pipe's rounding to nearest, up to 2^26 products.  Where the line lies: the tensor core's sums, which round toward
+// zero, move all-positive f16 results by less than 2^-24 (norm) from the 64-bit result up to K = 6144 (rounding error 2.2e-4, times 2e-6 more at 127, 5e-5 at 3313,
+// 1.7e-4 at 5999, 3.3e-4 at 8191, 1.4e-3 at 16383, 2 % at 60001; FP32 pipe 3e-5 at most), bf16 ones by 4e-6 of theirs at 16383; normally distributed data is nearer
+// than on the FP32 pipe.
 inline bool gemm16_copies_pay(int64_t m, int64_t n, int64_t k, int64_t batch, bool bf16) {
-  if (gemm16_padding_pays(m, n, k, batch)) return true;
   const double outputs = static_cast<double>(m) * n * batch;
-  return k <= (outputs < 512.0 && !bf16 ? 6144 : 16384) && k >= (outputs >= 6000000.0 ? 16 : outputs >= 262144.0 ? 33 : outputs >= 16384.0 ? 48 : 72);
+  if (outputs < 512.0 && k > (bf16 ? 16384 : 6144) && outputs * k < 67108864.0) return false;
+  return k >= (outputs >= 6000000.0 ? 16 : outputs >= 262144.0 ? 33 : outputs >= 16384.0 ? 48 : 72);
 }
 
 // f32 GEMM: operand planes and CTA pairs (gemm_tf32_tc.cuh), operands split on the way in (gemm_f32_fused.cuh), the warp-level kernel
