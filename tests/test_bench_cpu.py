@@ -51,3 +51,45 @@ def test_gpu_arm_needs_a_gpu():
         pytest.skip("this check is for machines without a GPU")
     r = _run("--steps", "1", "--no-extras")
     assert r.returncode != 0 and "no CPU fallback" in (r.stderr + r.stdout)
+
+
+class _Gemm:
+    """Stands in for the device: products by numpy on host memory, f32 sums in one order for every size but `whole` rows."""
+    def __init__(self, np, whole):
+        self.np, self.whole = np, whole
+
+    def gemm(self, code, m, n, k, a, b, c, stream=None):
+        import ctypes
+        view = lambda at, *shape: self.np.ctypeslib.as_array(ctypes.cast(at, ctypes.POINTER(ctypes.c_float)), shape)
+        x, y = view(a, m, k), view(b, k, n)
+        view(c, m, n)[:] = x @ y if m != self.whole else x[:, :k // 2] @ y[:k // 2] + x[:, k // 2:] @ y[k // 2:]
+
+
+@pytest.mark.parametrize("m,spoil,ok", [(700, None, True), (700, (399, 2, 1e-6), False), (700, (1, 0, 1e-6), False), (700, (699, 7, 0.5), False), (128, None, False)])
+def test_end_to_end_check_of_f32_products(m, spoil, ok):
+    """Row blocks of 128, each compared bit for bit with a call of its size; a sum in another order over the whole only where there are several blocks."""
+    sys.path.insert(0, str(ROOT))
+    import types
+
+    import bench
+    import numpy as np
+    import torch
+    n, k = 8, 40960  # 100 rows of A are 16 MiB
+    rng = np.random.default_rng(m)
+    wl = object.__new__(bench.GemmWL)
+    wl.units, wl.m, wl.n, wl.k, wl.es, wl.dtype, wl.code = 1, m, n, k, 4, "f32", 0
+    a, b = (rng.uniform(-1, 1, shape).astype(np.float32) for shape in ((1, m, k), (1, k, n)))
+    wl.a, wl.b, wl.c = torch.from_numpy(a), torch.from_numpy(b), torch.zeros(1, m, n)
+    dev = _Gemm(np, whole=m)
+    wl.ctx = types.SimpleNamespace(dev=dev, tdev="cpu", stream=0)
+    dev.gemm(0, m, n, k, wl.a.data_ptr(), wl.b.data_ptr(), wl.c.data_ptr())
+    host = np.empty((1, m, n), np.float32)
+    assert [r for r, _ in wl._host_blocks()] == list(range(0, m, 128))
+    for row in range(0, m, 128):
+        rows = np.ascontiguousarray(a[0, row:row + 128])
+        host[0, row:row + 128] = rows @ b[0]
+    assert not np.array_equal(host, wl.c.numpy())
+    if spoil:
+        host[0, spoil[0], spoil[1]] += np.float32(spoil[2]) * max(1.0, abs(host[0, spoil[0], spoil[1]]))
+    wl.c_host = types.SimpleNamespace(array=host)
+    assert wl.e2e_check() == ok
