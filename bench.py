@@ -8,8 +8,8 @@ resident in HBM.  The headline workload is the row softmax configuration (65536 
 f32, 3*N(0,1) with 1 % of the entries at +20); every other configuration (bf16 softmax,
 f32 and bf16 GEMMs, attention forward) is measured after it, each with its own sampled
 check against the CPU oracle, CPU baseline, end-to-end (host buffers) figure and, on
-several GPUs, strong-scaling figure.  Details go under "workloads", the figures of the
-tensor-bound configurations once more, compactly, under "summary" at the end of the line.
+several GPUs, strong-scaling figure.  Their figures go under "workloads", those of the
+tensor-bound configurations under "summary" at the end of the line, the whole records to stderr.
 
 Inputs are generated once on the host (counter-based generator of the library, the seeds and
 laws of each configuration), uploaded, and read by the oracle from the same host buffers.
@@ -1017,6 +1017,48 @@ def measure(ctx, name, args, peaks, steps, warmup, headline=False, shared=None, 
     return rec, None
 
 
+def brief(r):
+    """A workload's record in a few figures."""
+    if r is None:
+        return None
+    if "error" in r:
+        return {"error": r["error"][:120]}
+    b = {"value": r["value"], "unit": r["unit"], "ms": r["ms_per_step"], "frac": r["roofline"]["frac"]}
+    if "sustained" in r:
+        b["sust"], b["sust_frac"], b["per_ghz"] = r["sustained"]["value"], r["sustained"]["roofline_frac"], r["sustained"]["tflops_per_ghz"]
+    if "verify" in r:
+        b["verify"] = "ok" if r["verify"]["ok"] else "FAILED"
+    if "cpu_baseline" in r:
+        b["cpu"], b["cores"] = r["cpu_baseline"]["value"], r["cpu_baseline"]["cores"]
+    if "e2e" in r:
+        b["e2e"] = r["e2e"]["value"]
+    if "strong" in r and "speedup_vs_one_gpu" in r["strong"]:
+        b["strong_x"] = r["strong"]["speedup_vs_one_gpu"]
+    if "context" in r and r["context"].get("torch_sdpa_tflops"):
+        b["sdpa"] = r["context"]["torch_sdpa_tflops"]
+    if "latency" in r:
+        b["host_us"], b["dev_us"] = r["latency"]["host_us_per_call"], r["latency"]["device_us_per_call_back_to_back"]
+    return b
+
+
+def result_line(args, world, threads, head, extras, failed):
+    """The one line for stdout, short enough for whoever keeps only part of a long one (all records in full were 20 KB), and the other workloads' whole
+    records for stderr."""
+    allrec = {args.workload: head, **extras}
+    line = {
+        "metric": METRIC if args.workload.startswith("softmax") else f"{args.workload} {head['unit']}",
+        "value": head["value"], "unit": head["unit"], "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
+        "ms_per_step": head["ms_per_step"], "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
+        "dtype": head["dtype"], "data": "synthetic", "config": head["config"],
+        "roofline": head["roofline"], "cpu_baseline": head.get("cpu_baseline"), "e2e": head.get("e2e"),
+        "gpu_launches": head["launches"], "clocks": head["clocks"], "verify": head.get("verify"), "strong": head.get("strong"),
+        "host_threads_per_rank": threads, "failed": failed,
+        "workloads": {n: brief(r) for n, r in extras.items() if n not in SUMMARY},
+        "summary": {n: brief(allrec.get(n)) for n in SUMMARY if n in allrec},
+    }
+    return line, {"workloads": extras}
+
+
 def run_ours(args):
     torch = _torch()
     import torch.distributed as dist
@@ -1079,40 +1121,8 @@ def run_ours(args):
             extras[name], _ = guarded(name)
 
     if rank == 0:
-        def brief(r):
-            if r is None:
-                return None
-            if "error" in r:
-                return {"error": r["error"][:120]}
-            b = {"value": r["value"], "unit": r["unit"], "ms": r["ms_per_step"], "frac": r["roofline"]["frac"]}
-            if "sustained" in r:
-                b["sust"], b["sust_frac"], b["per_ghz"] = r["sustained"]["value"], r["sustained"]["roofline_frac"], r["sustained"]["tflops_per_ghz"]
-            if "verify" in r:
-                b["verify"] = "ok" if r["verify"]["ok"] else "FAILED"
-            if "cpu_baseline" in r:
-                b["cpu"], b["cores"] = r["cpu_baseline"]["value"], r["cpu_baseline"]["cores"]
-            if "e2e" in r:
-                b["e2e"] = r["e2e"]["value"]
-            if "strong" in r and "speedup_vs_one_gpu" in r["strong"]:
-                b["strong_x"] = r["strong"]["speedup_vs_one_gpu"]
-            if "context" in r and r["context"].get("torch_sdpa_tflops"):
-                b["sdpa"] = r["context"]["torch_sdpa_tflops"]
-            if "latency" in r:
-                b["host_us"], b["dev_us"] = r["latency"]["host_us_per_call"], r["latency"]["device_us_per_call_back_to_back"]
-            return b
-
-        allrec = {args.workload: head, **extras}
-        line = {
-            "metric": METRIC if args.workload.startswith("softmax") else f"{args.workload} {head['unit']}",
-            "value": head["value"], "unit": head["unit"], "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
-            "ms_per_step": head["ms_per_step"], "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-            "dtype": head["dtype"], "data": "synthetic", "config": head["config"],
-            "roofline": head["roofline"], "cpu_baseline": head.get("cpu_baseline"), "e2e": head.get("e2e"),
-            "gpu_launches": head["launches"], "clocks": head["clocks"], "verify": head.get("verify"), "strong": head.get("strong"),
-            "host_threads_per_rank": threads, "failed": failed,
-            "workloads": extras,
-            "summary": {n: brief(allrec.get(n)) for n in SUMMARY if n in allrec},
-        }
+        line, detail = result_line(args, world, threads, head, extras, failed)
+        print(json.dumps(detail), file=sys.stderr, flush=True)
         print(json.dumps(line), flush=True)
     if world > 1:
         dist.barrier()

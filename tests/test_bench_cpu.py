@@ -93,3 +93,26 @@ def test_end_to_end_check_of_f32_products(m, spoil, ok):
         host[0, spoil[0], spoil[1]] += np.float32(spoil[2]) * max(1.0, abs(host[0, spoil[0], spoil[1]]))
     wl.c_host = types.SimpleNamespace(array=host)
     assert wl.e2e_check() == ok
+
+
+def test_the_result_line_stays_short():
+    """A line of 20 KB, with every workload's record in full, was not read whole; the records go to stderr."""
+    sys.path.insert(0, str(ROOT))
+    import types
+
+    import bench
+    roofline = {"bound": "tensor", "achieved": 1234.56, "peak": 1655.1, "unit": "TFLOP/s", "frac": 0.7459, "peak_source": "measured", "traffic": 1071900000.0}
+    clocks = {"sm_mhz": 1965.0, "sm_max_mhz": 1965.0, "reasons": ["sw_power_cap"], "samples": 16, "source": "nvml"}
+    rec = {"value": 1234.56, "unit": "TFLOP/s", "ms_per_step": 12.3456, "dtype": "bf16", "config": bench.config_for("attention_gqa_causal"), "roofline": roofline, "launches": 20,
+           "clocks": clocks, "sustained": {"value": 1234.56, "roofline_frac": 0.9999, "tflops_per_ghz": 1044.4}, "verify": {"ok": True, "tolerance": "x" * 120},
+           "cpu_baseline": {"value": 0.1234, "unit": "TFLOP/s", "cores": 16, "kind": "port", "sample": "x" * 120}, "context": {"torch_sdpa_tflops": 1231.2},
+           "e2e": {"value": 185.08, "unit": "TFLOP/s", "h2d_bytes_per_step": 4294967296, "d2h_bytes_per_step": 2147483648, "api": "x" * 120},
+           "strong": {"speedup_vs_one_gpu": 7.45}, "latency": {"host_us_per_call": 3.81, "device_us_per_call_back_to_back": 9.33}}
+    args = types.SimpleNamespace(workload="softmax_f32", steps=20, warmup=5)
+    extras = {n: rec for n in bench.ORDER if n != "softmax_f32"}
+    extras["reduce_sum_f32"] = {"error": "x" * 600}
+    line, detail = bench.result_line(args, 8, 16, rec, extras, ["reduce_sum_f32"])
+    assert len(json.dumps(line)) <= 8192 and set(line["workloads"]) | set(line["summary"]) == set(extras)
+    for key in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling", "vs_baseline", "dtype", "data", "config", "e2e", "gpu_launches", "clocks"):
+        assert key in line, key
+    assert detail["workloads"] == extras
