@@ -20,7 +20,7 @@
 // 64-bit result.  The form before this one took three products of two TF32 numbers in steps of 32 keys, whose scores spend most of a product on
 // reading Q, and wrote a third more for the parts, V transposed: 450 us, 9e-7; 2 heads of 1283 70 us, 48 here, 256 heads of 530 242 / 182.
 // Tiny operands and probabilities keep their bits (split2): V of 1e-36 2.9e-7 off, of 1e-37 1.5e-6, of 1e-38 1.5e-5 (two TF32 numbers 3.4e-6, 3.3e-5 and
-// 3.4e-4, three bf16 numbers as they are 2.7e-5, 2.7e-4 and 2.7e-3); that takes 0.1 % of the cycles.
+// 3.4e-4, three bf16 numbers as they are 2.7e-5, 2.7e-4 and 2.7e-3).  That takes 0.1 % of the cycles, 2 % with heads of 32, where the softmax is the longer part.
 #pragma once
 
 #include "attention_simt.cuh"    // Params
@@ -78,17 +78,23 @@ struct Params {
 // Two values as three pairs of bf16 numbers: hi truncated (the largest f32 numbers would round up to infinity), mid what is left of them rounded to nearest,
 // lo 2^kLoShift times the rest, which has 8 bits or less.  Unscaled, it would end below the last bit that a bf16 number has, 2^-133, for values below
 // 1e-34; this way bits from 2^-142 on are kept.  lo stays smaller than hi, and sums of products with it than those of hi.
+// kPairs: lo by packed instructions.  The attention kernel spends 0.8 % more cycles without them (16 heads of 4096 x 128, the probabilities), the split pass 3 % more with.
 constexpr int kLoShift = 10;
+template <bool kPairs>
 __device__ __forceinline__ void split2(float x0, float x1, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
   constexpr float kUp = 1 << kLoShift;
   const uint32_t b0 = __float_as_uint(x0), b1 = __float_as_uint(x1);
   hi = __byte_perm(b0, b1, 0x7632);
   const float r0 = x0 - __uint_as_float(b0 & 0xffff0000u), r1 = x1 - __uint_as_float(b1 & 0xffff0000u);
   mid = attn::pack16x2<true>(r0, r1);
-  float l0, l1;  // in pairs: one by one they took 0.8 % of the kernel's cycles
-  const ptx::f32x2_t m = ptx::pack_f32x2(attn::unpack16_lo<true>(mid), attn::unpack16_hi<true>(mid));
-  const ptx::f32x2_t l = ptx::fma_f32x2(m, ptx::pack_f32x2(-1.0f, -1.0f), ptx::pack_f32x2(r0, r1));
-  ptx::unpack_f32x2(ptx::mul_f32x2(l, ptx::pack_f32x2(kUp, kUp)), l0, l1);
+  float l0, l1;
+  if constexpr (kPairs) {
+    const ptx::f32x2_t m = ptx::pack_f32x2(attn::unpack16_lo<true>(mid), attn::unpack16_hi<true>(mid));
+    const ptx::f32x2_t l = ptx::fma_f32x2(m, ptx::pack_f32x2(-1.0f, -1.0f), ptx::pack_f32x2(r0, r1));
+    ptx::unpack_f32x2(ptx::mul_f32x2(l, ptx::pack_f32x2(kUp, kUp)), l0, l1);
+  } else {
+    l0 = (r0 - attn::unpack16_lo<true>(mid)) * kUp, l1 = (r1 - attn::unpack16_hi<true>(mid)) * kUp;
+  }
   lo = __byte_perm(__float_as_uint(l0), __float_as_uint(l1), 0x7632);
 }
 
@@ -110,10 +116,10 @@ split_kv_kernel(const SplitParams p) {
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < p.head_vecs; i += step) {
     const float4 x = __ldcs(src + 2 * i), y = __ldcs(src + 2 * i + 1);
     uint32_t hi[4], mid[4], lo[4];
-    split2(x.x, x.y, hi[0], mid[0], lo[0]);
-    split2(x.z, x.w, hi[1], mid[1], lo[1]);
-    split2(y.x, y.y, hi[2], mid[2], lo[2]);
-    split2(y.z, y.w, hi[3], mid[3], lo[3]);
+    split2<false>(x.x, x.y, hi[0], mid[0], lo[0]);
+    split2<false>(x.z, x.w, hi[1], mid[1], lo[1]);
+    split2<false>(y.x, y.y, hi[2], mid[2], lo[2]);
+    split2<false>(y.z, y.w, hi[3], mid[3], lo[3]);
     dst[i] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
     dst[i + part] = make_uint4(mid[0], mid[1], mid[2], mid[3]);
     dst[i + 2 * part] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
@@ -206,8 +212,8 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const float4 x = valid ? qr[c * 8 + u] : make_float4(0.f, 0.f, 0.f, 0.f);
-        split2(x.x, x.y, hi[2 * u], mid[2 * u], lo[2 * u]);
-        split2(x.z, x.w, hi[2 * u + 1], mid[2 * u + 1], lo[2 * u + 1]);
+        split2<true>(x.x, x.y, hi[2 * u], mid[2 * u], lo[2 * u]);
+        split2<true>(x.z, x.w, hi[2 * u + 1], mid[2 * u + 1], lo[2 * u + 1]);
       }
       __syncwarp();
       ptx::tmem_st_32x32b_x16(tq + c * 16, hi);
@@ -359,7 +365,7 @@ attention_f32_tc_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid
           ptx::unpack_f32x2(ptx::fma_f32x2(ptx::pack_f32x2(__uint_as_float(v[h][2 * i]), __uint_as_float(v[h][2 * i + 1])), sl2x2, nmsx2), t0, t1);
           const float e0 = ptx::ex2_approx(t0), e1 = ptx::ex2_approx(t1);
           ls[i & 1] = ptx::add_f32x2(ls[i & 1], ptx::pack_f32x2(e0, e1));
-          split2(e0, e1, hi[i], mid[i], lo[i]);
+          split2<true>(e0, e1, hi[i], mid[i], lo[i]);
         }
         ptx::tmem_st_32x32b_x16(ts + h * 16, hi);
         ptx::tmem_st_32x32b_x16(ts + kPPart + h * 16, mid);
