@@ -75,13 +75,13 @@ attention_narrow_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid
   const int block = kSplit ? static_cast<int>(blockIdx.x) / splits : static_cast<int>(blockIdx.x);
   int bh, kvh, qb;
   attn::block_coords(p, block, bh, kvh, qb);
-  const int q0 = kLone ? qb * p.block_rows : qb * (2 * kBQ);
+  const int q0 = kLone && !kSplit ? qb * p.block_rows : qb * (2 * kBQ);
   const int seq_kv = kCache ? p.seq_kv : p.seq;
   const int q_off = kCache ? p.q_offset : 0;
   const int n_kv_all = (seq_kv + kBKV - 1) / kBKV;
   // number of KV steps each tile needs (causal: up to and including the step of its last row's own position)
   const int n_a_all = p.causal ? min(n_kv_all, (q0 + kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
-  const bool lone = kLone && (p.block_rows == kBQ || q0 + kBQ >= p.seq);  // no tile B, as in attention_tc.cuh
+  const bool lone = kLone && ((!kSplit && p.block_rows == kBQ) || q0 + kBQ >= p.seq);  // no tile B, as in attention_tc.cuh
   const int n_b_all = lone ? n_a_all : p.causal ? min(n_kv_all, (q0 + 2 * kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
   // kSplit: this CTA's range [j0, j0 + n_b) of them, possibly empty
   const int per_rank = kSplit ? (n_b_all + splits - 1) / splits : n_b_all;

@@ -84,7 +84,7 @@ struct Params {
   int32_t heads_q, heads_kv, batch;
   int32_t causal;
   int32_t q_blocks;        // ceil(seq / block_rows)
-  int32_t block_rows;      // 256, or 128: no tile B
+  int32_t block_rows;      // 256, or 128: no tile B (not where the keys of a block are shared out)
   int32_t kv_band;         // causal launch order: KV heads per band (>= 1), see the block index mapping in the kernel
   float scale_log2;        // (1/sqrt(d)) * log2(e)
   uint32_t* status;
@@ -167,7 +167,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   const int block = kSplit ? static_cast<int>(blockIdx.x) / splits : static_cast<int>(blockIdx.x);
   int bh, kvh, qb;
   block_coords(p, block, bh, kvh, qb);
-  const int q0 = kLone ? qb * p.block_rows : qb * (2 * kBQ);
+  const int q0 = kLone && !kSplit ? qb * p.block_rows : qb * (2 * kBQ);
   const int seq_kv = kCache ? p.seq_kv : p.seq;
   const int q_off = kCache ? p.q_offset : 0;
   const int n_kv_all = (seq_kv + kBKV - 1) / kBKV;
@@ -175,7 +175,7 @@ attention_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   const int n_a_all = p.causal ? min(n_kv_all, (q0 + kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
   // A block of 128 rows or fewer (a short prompt, the end of a sequence) has no tile B, whose products and exponentials would slow tile A down:
   // 2060 cycles a step instead of 3240.  Rotation, appends and attention of 30 tokens on 3000, 4 heads, 49.9 -> 39.0 us, of 100 on 12000, 32 heads, 65.4 -> 51.7.
-  const bool lone = kLone && (p.block_rows == kBQ || q0 + kBQ >= p.seq);
+  const bool lone = kLone && ((!kSplit && p.block_rows == kBQ) || q0 + kBQ >= p.seq);
   const int n_b_all = lone ? n_a_all : p.causal ? min(n_kv_all, (q0 + 2 * kBQ - 1 + q_off) / kBKV + 1) : n_kv_all;
   // kSplit: this CTA's range [j0, j0 + n_b) of them, possibly empty
   const int per_rank = kSplit ? (n_b_all + splits - 1) / splits : n_b_all;
@@ -581,11 +581,11 @@ attention_merge_kernel(uint16_t* __restrict__ o, const Params p) {
   const int block = static_cast<int>(blockIdx.x) / kGroups, c0 = static_cast<int>(blockIdx.x) % kGroups * 16;
   int bh, kvh, qb;
   block_coords(p, block, bh, kvh, qb);
-  const int row = threadIdx.x, qrow = qb * p.block_rows + row;
+  const int row = threadIdx.x, qrow = qb * (2 * kBQ) + row;
   const int cols = D == 64 ? p.head_dim : D;
   ptx::launch_dependents();
   ptx::wait_prior_grid();
-  if (qrow >= p.seq || row >= p.block_rows || c0 >= cols) return;
+  if (qrow >= p.seq || c0 >= cols) return;
   const int64_t rec0 = static_cast<int64_t>(block) * p.splits;
   float gm = -INFINITY;
 #pragma unroll 8
