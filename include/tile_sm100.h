@@ -136,10 +136,13 @@ int32_t tsm100_launch(tsm100_module_t mod, const char* name, uint32_t blocks, vo
 /* ---- operators on device memory ---------------------------------------- */
 /* Scratch.  Some operators take device memory for the length of a call:
  *   tsm100_gemm, f32, 64 tiles of 128 x 256 and K >= 256 or more: 8 bytes per element of A and B (and 4 per 128 x 128 of C);
- *   tsm100_gemm, 16 bit, sizes or rows that are no multiple of 16 bytes, 2^26 products or more: padded copies of A, B, C;
- *   tsm100_attention and _prefill, f32, 64 query rows and 256 keys or more: twice the bytes of K and V;
+ *   tsm100_gemm, 16 bit in and out, rows of A or B that do not start on 16-byte boundaries, from K = 16 on for many results and
+ *   K = 72 for few: a copy of A, of B, or of both;
+ *   tsm100_attention and _prefill, f32, heads of 128, of 64 and 96 with more than 64 keys, of 32 with more than 160: 1.5 times the
+ *   bytes of K and V;
  *   the same in 16 bit, 4096 keys or more and query blocks for at most half of the SMs: up to 20 MB;
- *   tsm100_attention_decode, 16 bit, few caches of 1024 positions or more: up to 1.3 MB.
+ *   tsm100_attention_decode, 16 bit, few caches of 1024 positions or more, or 50 MB of caches with up to eight query heads to
+ *   each: up to 1.3 MB.
  * It is taken and returned on the caller's stream, from a pool of the library's own on each device (the device's default
  * memory pool is neither used nor changed).  The pool keeps up to 1/16 of the device's memory for later calls and gives it
  * back when the device's last handle is closed.  When the device has no memory left, such a call takes a form without

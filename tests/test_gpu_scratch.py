@@ -40,10 +40,17 @@ def calls(capi):
                           [rnd(100, 4, 128), rnd(2, 5100, 128, seed=2), rnd(2, 5100, 128, seed=3)], torch.zeros(100, 4, 128, dtype=half, device="cuda:0")),
         "decode of few caches": ("attention_decode", capi.AttentionDecodeDesc(capi.BF16, 1, 16, 8, 9000, 9000, 128),
                                  [rnd(16, 128), rnd(8, 9000, 128, seed=2), rnd(8, 9000, 128, seed=3)], torch.zeros(16, 128, dtype=half, device="cuda:0")),
+        "decode as one stream": ("attention_decode", capi.AttentionDecodeDesc(capi.BF16, 17, 32, 8, 801, 805, 128),
+                                 [rnd(17, 32, 128), rnd(17, 8, 805, 128, seed=2), rnd(17, 8, 805, 128, seed=3)], torch.zeros(17, 32, 128, dtype=half, device="cuda:0")),
+        "f32 attention of few keys": ("attention", capi.AttentionDesc(capi.F32, 1, 1, 4, 2, 40, 128), [rnd(4, 40, 128, dtype=f32), rnd(2, 40, 128, dtype=f32, seed=2),
+                                                                                                       rnd(2, 40, 128, dtype=f32, seed=3)], torch.zeros(4, 40, 128, device="cuda:0")),
+        "16-bit GEMM of a short odd K": ("gemm", gemm(capi.F16, capi.F16, 0, 1, 760, 145, 127), [rnd(760, 127, dtype=torch.float16), rnd(127, 145, dtype=torch.float16, seed=2)],
+                                         torch.zeros(760, 145, dtype=torch.float16, device="cuda:0")),
     }
 
 
-NAMES = ["f32 GEMM", "f32 GEMM of odd sizes", "16-bit GEMM of odd sizes", "f32 attention", "split prefill", "decode of few caches"]
+NAMES = ["f32 GEMM", "f32 GEMM of odd sizes", "16-bit GEMM of odd sizes", "f32 attention", "split prefill", "decode of few caches", "decode as one stream", "f32 attention of few keys",
+         "16-bit GEMM of a short odd K"]
 
 
 def run(capi, dev, call):
@@ -120,7 +127,7 @@ using namespace tsm100;
 CALL(gemm, tsm100_gemm_desc, o, status, s)
 CALL(attention, tsm100_attention_desc, v, o, status, s)
 CALL(attention_prefill, tsm100_attention_prefill_desc, v, o, status, s)
-CALL(attention_decode, tsm100_attention_decode_desc, v, o, s)
+CALL(attention_decode, tsm100_attention_decode_desc, v, o, s, status)
 """
 
 
