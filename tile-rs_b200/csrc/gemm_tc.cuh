@@ -93,8 +93,8 @@ constexpr int kBoxCols = 128 / static_cast<int>(sizeof(OutT));
 
 // One warp's 32 rows x kBN columns of an accumulator (`tmem`: its lanes, first column) to C[b], first element (row0, col0): box by box through two
 // swizzled buffers of shared memory and TMA stores, which leave out what lies past C.  Stores from the lanes that hold the rows touch 32
-// of them with 16 bytes each, and such an epilogue of 128 x 256 took 6 us, longer than the products of K = 1000: 2897 x 4024 x 320 22.4 us, 5848 x
-// 1592 x 552 22.5, 2868 x 2848 x 944 of a batch of 4 76 us.  The caller's lane 0 has to wait for the stores before the CTA ends.
+// of them with 16 bytes each, and such an epilogue of 128 x 256 took 6 us, longer than the products of K = 1000: lanes / boxes 2897 x 4024 x 320 20.1 / 14.1 us, 5848 x
+// 1592 x 552 22.9 / 19.2, 2868 x 2848 x 944 of a batch of 4 63.7 / 56.0.  The caller's lane 0 has to wait for the stores before the CTA ends.
 // `boxes`: how many this warp has stored, over all of its tiles.  The buffers alternate by it and every box is a store group of its own, so that the wait for all
 // but the latest group covers the buffer at hand; a tile may end after an odd number of boxes, and a warp whose rows lie past C has none.
 // kLoose: rows of C start anywhere; the boxes are copied to them from shared memory, a warp 32 columns of a row at a time (`c`: C[b]).

@@ -945,7 +945,6 @@ inline int32_t gemm_skinny_launch_nt(std::string* err, const tsm100_gemm_desc* d
   g::Params p;
   p.m = static_cast<int32_t>(M);
   p.n = static_cast<int32_t>(N);
-
   p.k = static_cast<int32_t>(K);
   p.batch = d->batch;
   p.m_blocks = static_cast<int32_t>((M + NT - 1) / NT);

@@ -170,8 +170,8 @@ inline GemmF32 gemm_f32(int64_t m, int64_t n, int64_t k, int64_t batch, bool ali
   // 4.4 us on 64 columns, 5.5 on 128, a further wave 1.4 and 2.3, a k-block what stands below: rows that start anywhere are loaded value by
   // value, B stored [K][N] in columns, and both cost more where a CTA loads 128 columns.  All clusters have to fit the GPU at
   // once, one CTA per SM (1419 x 372 x 680 as 36 clusters of four 23 us, in two waves, of two 16); of clusters of 2, 3, ... 8 a B200
-  // holds 74, 45, 33, 26, 22, 15 and 15.  Any size of cluster, not powers of two alone: 2410 x 108 x 2256 26.8 -> 20.1, 549 x 1064 x 900 23.2 -> 19.8,
-  // 1900 x 261 x 2591 58 -> 48, 267 x 724 x 792 13.2 -> 11.6.
+  // holds 74, 45, 33, 26, 22, 15 and 15.  Any size of cluster, not powers of two alone: 2410 x 108 x 2256 27.5 -> 21.2, 549 x 1064 x 900 24.0 -> 20.9,
+  // 1900 x 261 x 2591 62 -> 54, 267 x 724 x 792 14.8 -> 12.6.
   const int64_t kb64 = aligned ? 810 : 880, kb128 = aligned ? (b_transposed ? 1020 : 1170) : (b_transposed ? 1200 : 1270);
   int64_t best = INT64_MAX;
   for (int bn = 64; bn <= 128; bn += 64)
